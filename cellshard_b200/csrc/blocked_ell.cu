@@ -17,8 +17,9 @@
 //           blockColIdx (set bits in ascending order, CS_INVALID_COL padding).
 //
 // Values of duplicate columns inside one row resolve to the last occurrence
-// (the reference's overwrite order): such rows are detected with a block-wide
-// vote and scattered by one thread in CSR order.
+// (the reference's overwrite order).  A row whose columns ascend has none (a
+// block-wide vote); a row in another order is checked with one bit per cell,
+// and only a row that repeats a column is scattered by one thread in CSR order.
 #include "common.cuh"
 
 #include <cstdlib>
@@ -262,8 +263,9 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
 // scattered into a zeroed buffer by the threads, then one thread hands the
 // whole padded row to the copy engine and the CTA moves on while it streams
 // out.  A buffer is re-zeroed only after the bulk store that read it has
-// finished reading.  Rows whose columns are not strictly increasing are
-// redone in CSR order by one thread (the reference's overwrite order).
+// finished reading.  A row whose columns are not strictly increasing marks
+// one bit per cell in `seen`; one that repeats a column is redone in CSR order
+// by one thread (the reference's overwrite order).
 template <int NBUF>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
@@ -275,7 +277,9 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t row_bytes = ell_cols * 2u;
     const uint32_t stride = (row_bytes + 127u) & ~127u;
     uint2 *ix = reinterpret_cast<uint2 *>(tma_smem + (std::size_t) NBUF * stride);
-    uint32_t *rp = reinterpret_cast<uint32_t *>(ix + words); // [B + 1] row pointers of the block
+    const uint32_t seen_words = (ell_cols + 31u) / 32u;
+    uint32_t *seen = reinterpret_cast<uint32_t *>(ix + words); // [seen_words] occupied cells of an unordered row
+    uint32_t *rp = seen + seen_words;                          // [B + 1] row pointers of the block
     __shared__ uint32_t count_smem;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t row_blocks = (rows + B - 1u) / B;
@@ -354,13 +358,18 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             }
             int unordered = 0;
             uint32_t row_nnz = 0u;
-            auto place = [&](uint32_t i, uint32_t c, uint16_t v) {
-                if (c >= cols) return;
+            // cell of column c, or 0xffffffff where it has none
+            auto cell = [&](uint32_t c) -> uint32_t {
+                if (c >= cols) return 0xffffffffu;
                 const uint32_t bc = div_b(c, B, shift);
                 const uint2 x = ix[bc >> 5];
                 const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
-                if (slot >= width) return;
-                buf[slot * B + (c - bc * B)] = v;
+                return slot < width ? slot * B + (c - bc * B) : 0xffffffffu;
+            };
+            auto place = [&](uint32_t c, uint16_t v) {
+                const uint32_t p = cell(c);
+                if (p == 0xffffffffu) return;
+                buf[p] = v;
                 row_nnz += half_nonzero(v);
             };
             if (!ptr_bad) {
@@ -372,27 +381,39 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                     if (lane == 31u && i + 1u < e) nxt = __ldg(idx + i + 1u);
                     if (i < e) {
                         if (i + 1u < e && cc[k] >= nxt) unordered = 1;
-                        place(i, cc[k], cv[k]);
+                        place(cc[k], cv[k]);
                     }
                 }
                 for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) {
                     const uint32_t c = __ldg(idx + i);
                     if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
-                    place(i, c, val[i]);
+                    place(c, val[i]);
                 }
             }
+            int repeated = 0;
             if (__syncthreads_or(unordered)) {
+                for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
+                __syncthreads();
+                auto mark = [&](uint32_t c) {
+                    const uint32_t p = cell(c);
+                    if (p == 0xffffffffu) return;
+                    const uint32_t bit = 1u << (p & 31u);
+                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
+                };
+#pragma unroll
+                for (int k = 0; k < PF; ++k)
+                    if (a + threadIdx.x + (uint32_t) k * kEmitThreads < e) mark(cc[k]);
+                for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) mark(__ldg(idx + i));
+                repeated = __syncthreads_or(repeated);
+            }
+            if (repeated) {
                 for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
                     *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
                 __syncthreads();
                 if (threadIdx.x == 0) {
                     for (uint32_t i = a; i < e; ++i) {
-                        const uint32_t c = idx[i];
-                        if (c >= cols) continue;
-                        const uint32_t bc = div_b(c, B, shift);
-                        const uint2 x = ix[bc >> 5];
-                        const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
-                        if (slot < width) buf[slot * B + (c - bc * B)] = val[i];
+                        const uint32_t p = cell(idx[i]);
+                        if (p != 0xffffffffu) buf[p] = val[i];
                     }
                 }
                 __syncthreads();
@@ -490,8 +511,9 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
     if (tma_ok) {
         const int nbuf = stride <= 8192u ? 8 : (stride <= 16384u ? 4 : (stride <= 32768u ? 2 : 1));
         const std::size_t tsmem =
-            (std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) + ((std::size_t) B + 1u) * 4u;
-        if (tsmem <= 72u * 1024u) {
+            (std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) +
+            ((dst->ell_cols + 31u) / 32u + (std::size_t) B + 1u) * 4u;
+        if (tsmem <= 75u * 1024u) { // three CTAs per SM
             const uint32_t row_blocks = (src->rows + B - 1u) / B;
             uint32_t tgrid = (uint32_t) sm_count() * 3u;
             if (tgrid > row_blocks) tgrid = row_blocks;

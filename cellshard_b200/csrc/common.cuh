@@ -204,6 +204,13 @@ std::size_t sort_pairs_u32_scratch_bytes(uint32_t n);
 int sort_pairs_u32(const uint32_t *keys, const uint32_t *vals, uint32_t n, uint32_t *out_keys, uint32_t *out_vals,
                    void *tmp, std::size_t tmp_bytes, cudaStream_t stream);
 
+// COO entries put in row order, stable (transpose.cu).  scratch_bytes is 0
+// where it does not apply (no entries, too many rows, columns too wide).
+std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t cols);
+int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row, const uint32_t *col,
+                   const uint32_t *map, const uint16_t *val, uint32_t *out_ptr, uint32_t *out_col, uint16_t *out_val,
+                   void *scratch, std::size_t scratch_bytes, cudaStream_t stream);
+
 // Owned device memory and stream for the synchronous host entry points.
 struct dmem {
     void *p = nullptr;

@@ -178,10 +178,16 @@ __global__ void __launch_bounds__(kThreads) tr_scatter_kernel(const uint32_t *__
 // Both passes rank entries in input order (warp match on the digit plus
 // per-warp running counts), so the result is the stable transpose.
 // Needs cDim < 2^24 and uDim <= 262,144.
+//
+// The same two passes also put COO entries in row order (partition_rows_*
+// below): the key is then the entry's row, the payload its column, and the low
+// digit has LB = 8 to 11 bits so that up to 2,097,152 rows stay within the
+// 1,024 pass-1 buckets.
 // ---------------------------------------------------------------------------
 constexpr unsigned kTpThreads = 256;
 constexpr unsigned kTpWarps = kTpThreads / 32;
-constexpr uint32_t kTpBucketBits = 8;
+constexpr uint32_t kTpBucketBits = 8; // low digit of the transpose
+constexpr uint32_t kTpMaxLowBits = 11;
 constexpr uint32_t kTpMaxBuckets = 1024;
 constexpr uint32_t kTpTile1 = 8192;  // entries per pass-1 tile (staged whole in shared memory)
 constexpr uint32_t kTpChunk = 8192;  // entries per pass-2 chunk (staged whole in shared memory)
@@ -200,15 +206,18 @@ struct tp2_layout {
     uint32_t *hist2;        // [256 * max_chunks + 1], digit-major
     void *scan_tmp;
     std::size_t scan_bytes, bytes;
-    uint32_t K, tiles1, max_chunks;
+    uint32_t K, tiles1, max_chunks, low_bits;
 };
 
 bool tp2_applicable(uint32_t cDim, uint32_t uDim) {
     return cDim < (1u << 24) && uDim <= kTpMaxBuckets * 256u;
 }
 
-void tp2_make_layout(uint32_t cDim, uint32_t uDim, uint32_t nnz, void *base, std::size_t cap, tp2_layout *l) {
-    l->K = (uDim + 255u) >> kTpBucketBits;
+void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granules, void *base, std::size_t cap,
+                     tp2_layout *l) {
+    const uint32_t D = 1u << low_bits;
+    l->low_bits = low_bits;
+    l->K = (uint32_t) (((uint64_t) uDim + D - 1u) >> low_bits);
     if (l->K == 0u) l->K = 1u;
     l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + kTpTile1 - 1u) / kTpTile1);
     l->max_chunks = nnz / kTpChunk + l->K + 1u;
@@ -217,14 +226,14 @@ void tp2_make_layout(uint32_t cDim, uint32_t uDim, uint32_t nnz, void *base, std
     l->hist1 = c.take<uint32_t>((std::size_t) l->K * l->tiles1 + 1u);
     l->tmp_key = c.take<uint32_t>((std::size_t) nnz + 1u);
     l->tmp_val = c.take<uint16_t>((std::size_t) nnz + 8u);
-    l->gran_row = c.take<uint32_t>((std::size_t) nnz / kTpGran + 1u);
+    l->gran_row = granules ? c.take<uint32_t>((std::size_t) nnz / kTpGran + 1u) : nullptr;
     l->chunk_bucket = c.take<uint32_t>(l->max_chunks);
     l->chunk_begin = c.take<uint32_t>(l->max_chunks);
     l->chunk_end = c.take<uint32_t>(l->max_chunks);
     l->chunk_first = c.take<uint32_t>((std::size_t) l->K + 1u);
-    l->hist2 = c.take<uint32_t>((std::size_t) 256u * l->max_chunks + 1u);
+    l->hist2 = c.take<uint32_t>((std::size_t) D * l->max_chunks + 1u);
     std::size_t sb = scan_u32_scratch_bytes((std::size_t) l->K * l->tiles1);
-    const std::size_t sb2 = scan_u32_scratch_bytes((std::size_t) 256u * l->max_chunks);
+    const std::size_t sb2 = scan_u32_scratch_bytes((std::size_t) D * l->max_chunks);
     const std::size_t sb3 = scan_u32_scratch_bytes(uDim);
     if (sb2 > sb) sb = sb2;
     if (sb3 > sb) sb = sb3;
@@ -245,7 +254,8 @@ __global__ void __launch_bounds__(256) tp_gran_rows_kernel(const uint32_t *__res
 
 // Pass-1 histogram: tile t is entries [t * kTpTile1, (t + 1) * kTpTile1).
 __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__restrict__ idx, uint32_t nnz,
-                                                             uint32_t uDim, uint32_t K, uint32_t tiles1,
+                                                             uint32_t uDim, uint32_t low_bits, uint32_t K,
+                                                             uint32_t tiles1,
                                                              uint32_t *__restrict__ hist1, uint32_t *status) {
     extern __shared__ uint32_t tp_h[];
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) tp_h[k] = 0u;
@@ -263,7 +273,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__
 #pragma unroll
         for (unsigned u = 0; u < U; ++u) {
             if (c[u] < uDim)
-                atomicAdd(tp_h + (c[u] >> kTpBucketBits), 1u);
+                atomicAdd(tp_h + (c[u] >> low_bits), 1u);
             else if (i0 + u * blockDim.x + threadIdx.x < e)
                 bad = CS_STATUS_INDEX_RANGE;
         }
@@ -273,22 +283,23 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__
     if (bad) status_or(status, bad);
 }
 
-// Block-wide exclusive scan of n <= 4 * blockDim.x values in place (each
-// thread scans up to 4 consecutive entries); out[n] receives the total.
+// Block-wide exclusive scan of n <= Q * blockDim.x values in place (each
+// thread scans up to Q consecutive entries); out[n] receives the total.
+template <int Q>
 __device__ __forceinline__ void block_scan_small(uint32_t *v, uint32_t n, uint32_t *smem33) {
     const uint32_t t = threadIdx.x;
-    uint32_t loc[4], sum = 0u;
+    uint32_t loc[Q], sum = 0u;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t k = t * 4u + q;
+    for (int q = 0; q < Q; ++q) {
+        const uint32_t k = t * (unsigned) Q + q;
         loc[q] = k < n ? v[k] : 0u;
         sum += loc[q];
     }
     uint32_t tot;
     uint32_t run = block_exclusive_scan(sum, smem33, tot);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t k = t * 4u + q;
+    for (int q = 0; q < Q; ++q) {
+        const uint32_t k = t * (unsigned) Q + q;
         if (k < n) v[k] = run;
         run += loc[q];
     }
@@ -351,15 +362,23 @@ __device__ __forceinline__ void tp_stage_prefix(const tp_stage &sg, uint32_t D) 
     }
 }
 
-// Pass 1: tile t = entries [t * kTpTile1, ...) of the CSR, reordered by
-// bucket (column >> 8) in shared memory, stable, then written out as one run
-// per bucket.  Keys are (row << 8 | column & 255).
+// Pass 1: tile t = entries [t * kTpTile1, ...) of the input, reordered by
+// bucket (key >> low_bits) in shared memory, stable, then written out as one
+// run per bucket.  Packed keys are (payload << low_bits | low digit).
+// kCoo false: the key is the CSR entry's column, the payload its row, found
+// from `ptr`.  kCoo true: the key `idx` is the COO entry's row, the payload
+// its (mapped) column; random rows make a warp's 32 keys nearly all distinct,
+// so peers come from ballots (one per bucket bit) instead of match.any.
+template <bool kCoo>
 __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t *__restrict__ ptr,
                                                                 const uint32_t *__restrict__ idx,
                                                                 const uint16_t *__restrict__ val, uint32_t cDim,
-                                                                uint32_t uDim, uint32_t nnz, uint32_t K,
-                                                                uint32_t tiles1, const uint32_t *__restrict__ hist1,
+                                                                uint32_t uDim, uint32_t nnz, uint32_t coo_low_bits,
+                                                                uint32_t K, uint32_t tiles1,
+                                                                const uint32_t *__restrict__ hist1,
                                                                 const uint32_t *__restrict__ gran_row,
+                                                                const uint32_t *__restrict__ pay,
+                                                                const uint32_t *__restrict__ pay_map,
                                                                 uint32_t *__restrict__ tmp_key,
                                                                 uint16_t *__restrict__ tmp_val) {
     extern __shared__ __align__(16) uint32_t tp_s[];
@@ -383,12 +402,14 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
     }
     for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
     __syncthreads();
-    block_scan_small(sg.lb, K, scan33);
+    block_scan_small<4>(sg.lb, K, scan33);
     const unsigned lt = (1u << lane) - 1u;
     uint16_t *my_cnt = sg.cnt + warp * K;
     uint16_t *my_bas = sg.bas + warp * K;
     static_assert(kTpSub / kTpWarps == kTpGran, "a warp's step range is one row granule");
-    uint32_t ncc[kTpBatches], nrc;
+    const uint32_t low_bits = kCoo ? coo_low_bits : kTpBucketBits;
+    uint32_t ncc[kTpBatches], npp[kTpBatches], nrc = 0u;
+    const uint32_t low_mask = (1u << low_bits) - 1u;
     uint16_t nvv[kTpBatches];
     auto fetch = [&](uint32_t sc) {
         const uint32_t n = min(kTpSub, e - sc);
@@ -399,8 +420,9 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
             const bool in = i < we;
             ncc[q] = in ? __ldg(idx + i) : uDim;
             nvv[q] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
+            if constexpr (kCoo) npp[q] = in ? __ldg(pay + i) : 0u;
         }
-        nrc = wa < we ? min(__ldg(gran_row + wa / kTpGran), cDim - 1u) : 0u;
+        if constexpr (!kCoo) nrc = wa < we ? min(__ldg(gran_row + wa / kTpGran), cDim - 1u) : 0u;
     };
     fetch(a);
     for (uint32_t sc0 = a; sc0 < e; sc0 += kTpSub) {
@@ -413,33 +435,36 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
         for (unsigned q = 0; q < kTpBatches; ++q) {
             cc[q] = ncc[q];
             vv[q] = nvv[q];
+            if constexpr (kCoo) rl[q] = pay_map != nullptr && cc[q] < uDim ? __ldg(pay_map + npp[q]) : npp[q];
         }
         uint32_t r_cur = nrc;
         if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
-            const uint32_t i = wa + q * 32u + lane;
-            const bool in = i < we;
-            // row of entry i: walk forward from the warp's current row; a
-            // batch that spans many short rows finishes by binary search
-            uint32_t r = r_cur;
-            for (unsigned step = 0;; ++step) {
-                const bool adv = in && r + 1u < cDim && __ldg(ptr + r + 1u) <= i;
-                if (!__any_sync(0xffffffffu, adv)) break;
-                if (step == 3u) {
-                    if (adv) {
-                        const uint32_t lo = r + 1u;
-                        r = lo + major_of(ptr + lo, cDim - lo, i);
+            if constexpr (!kCoo) {
+                const uint32_t i = wa + q * 32u + lane;
+                const bool in = i < we;
+                // row of entry i: walk forward from the warp's current row; a
+                // batch that spans many short rows finishes by binary search
+                uint32_t r = r_cur;
+                for (unsigned step = 0;; ++step) {
+                    const bool adv = in && r + 1u < cDim && __ldg(ptr + r + 1u) <= i;
+                    if (!__any_sync(0xffffffffu, adv)) break;
+                    if (step == 3u) {
+                        if (adv) {
+                            const uint32_t lo = r + 1u;
+                            r = lo + major_of(ptr + lo, cDim - lo, i);
+                        }
+                        break;
                     }
-                    break;
+                    r += adv ? 1u : 0u;
                 }
-                r += adv ? 1u : 0u;
+                rl[q] = r;
+                r_cur = __shfl_sync(0xffffffffu, r, 31);
             }
-            rl[q] = r;
-            r_cur = __shfl_sync(0xffffffffu, r, 31);
             const bool ok = cc[q] < uDim;
-            const uint32_t k = cc[q] >> kTpBucketBits;
-            pk[q] = tp_peers(k, ok);
+            const uint32_t k = cc[q] >> low_bits;
+            pk[q] = kCoo ? warp_match_digit<10>(k, ok) : tp_peers(k, ok);
             if (ok && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[k] += (uint16_t) __popc(pk[q]);
             __syncwarp();
         }
@@ -449,13 +474,13 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
             const bool ok = cc[q] < uDim;
-            const uint32_t k = cc[q] >> kTpBucketBits;
+            const uint32_t k = cc[q] >> low_bits;
             uint32_t lp = 0u;
             if (ok) lp = my_bas[k] + __popc(pk[q] & lt);
             __syncwarp();
             if (ok) {
                 if (lp < kTpTile1)
-                    st[lp] = (unsigned long long) ((rl[q] << kTpBucketBits) | (cc[q] & 255u)) |
+                    st[lp] = (unsigned long long) ((rl[q] << low_bits) | (cc[q] & low_mask)) |
                              ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
                 if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
             }
@@ -522,13 +547,17 @@ __global__ void __launch_bounds__(1024) tp_chunks_kernel(const uint32_t *__restr
     }
 }
 
+// one histogram per warp while eight of them fit (LB = 8), one per CTA above
+template <int LB>
 __global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ tmp_key,
                                                              const uint32_t *__restrict__ chunk_begin,
                                                              const uint32_t *__restrict__ chunk_end,
                                                              uint32_t max_chunks, uint32_t *__restrict__ hist2) {
-    __shared__ uint32_t h[kTpWarps][256];
-    const unsigned warp = threadIdx.x >> 5;
-    for (uint32_t d = threadIdx.x; d < kTpWarps * 256u; d += blockDim.x) (&h[0][0])[d] = 0u;
+    constexpr uint32_t D = 1u << LB;
+    constexpr unsigned kCopies = LB == 8 ? kTpWarps : 1u;
+    __shared__ uint32_t h[kCopies][D];
+    const unsigned copy = (threadIdx.x >> 5) % kCopies;
+    for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
     __syncthreads();
     const uint32_t b = chunk_begin[blockIdx.x], e = chunk_end[blockIdx.x];
     constexpr unsigned U = 4;
@@ -537,31 +566,36 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__
 #pragma unroll
         for (unsigned u = 0; u < U; ++u) {
             const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-            kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu;
+            kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu; // no packed key: see partition_low_bits
         }
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-            if (kk[u] != 0xffffffffu) atomicAdd(&h[warp][kk[u] & 255u], 1u);
+            if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][kk[u] & (D - 1u)], 1u);
     }
     __syncthreads();
-    uint32_t t = 0u;
-    for (unsigned w = 0; w < kTpWarps; ++w) t += h[w][threadIdx.x];
-    hist2[(std::size_t) threadIdx.x * max_chunks + blockIdx.x] = t;
+    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+        uint32_t t = 0u;
+#pragma unroll
+        for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
+        hist2[(std::size_t) d * max_chunks + blockIdx.x] = t;
+    }
 }
 
-// column totals from the digit-major scan: count(k*256+d) = P[d][last] - P[d][first]
+// key totals from the digit-major scan: count(k * D + d) = P[d][last] - P[d][first]
 __global__ void __launch_bounds__(256) tp_colcount_kernel(const uint32_t *__restrict__ hist2, uint32_t max_chunks,
                                                           const uint32_t *__restrict__ chunk_first, uint32_t uDim,
-                                                          uint32_t *__restrict__ counts) {
-    const uint32_t k = blockIdx.x, d = threadIdx.x;
-    const uint32_t c = k * 256u + d;
-    if (c >= uDim) return;
+                                                          uint32_t low_bits, uint32_t *__restrict__ counts) {
+    const uint32_t k = blockIdx.x;
     const uint32_t f = chunk_first[k], l = chunk_first[k + 1u];
-    counts[c] = hist2[(std::size_t) d * max_chunks + l] - hist2[(std::size_t) d * max_chunks + f];
+    for (uint32_t d = threadIdx.x; d < 1u << low_bits; d += blockDim.x) {
+        const uint32_t c = (k << low_bits) + d;
+        if (c < uDim) counts[c] = hist2[(std::size_t) d * max_chunks + l] - hist2[(std::size_t) d * max_chunks + f];
+    }
 }
 
-// Pass 2: a chunk of one bucket reordered by the low column byte in shared
-// memory (stable), then written out as one run per column.
+// Pass 2: a chunk of one bucket reordered by the low digit in shared memory
+// (stable), then written out as one run per key.
+template <int LB>
 __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
                                                                 const uint16_t *__restrict__ tmp_val,
                                                                 const uint32_t *__restrict__ chunk_bucket,
@@ -573,15 +607,16 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
                                                                 uint32_t *__restrict__ out_idx,
                                                                 uint16_t *__restrict__ out_val) {
     extern __shared__ __align__(16) uint32_t tp_s2[];
-    __shared__ uint32_t gbase[256];
-    __shared__ uint32_t lb[257];
-    __shared__ uint32_t fill[256];
+    constexpr uint32_t D = 1u << LB;
+    __shared__ uint32_t gbase[D];
+    __shared__ uint32_t lb[D + 1u];
+    __shared__ uint32_t fill[D];
     __shared__ uint32_t scan33[33];
     uint32_t *st_key = tp_s2;                                              // [kTpChunk]
     uint16_t *st_val = reinterpret_cast<uint16_t *>(st_key + kTpChunk);   // [kTpChunk]
     tp_stage sg;
-    sg.cnt = st_val + kTpChunk;                                            // [kTpWarps][256]
-    sg.bas = sg.cnt + kTpWarps * 256u;                                     // [kTpWarps][256]
+    sg.cnt = st_val + kTpChunk;                                            // [kTpWarps][D]
+    sg.bas = sg.cnt + kTpWarps * D;                                     // [kTpWarps][D]
     sg.lb = lb;
     sg.fill = fill;
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -589,22 +624,21 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
     if (b >= e) return;
     const uint32_t k = chunk_bucket[blockIdx.x];
     const uint32_t f = chunk_first[k];
-    {
-        const uint32_t d = threadIdx.x; // kTpThreads == 256
-        const uint32_t c = k * 256u + d;
+    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
+        const uint32_t c = k * D + d;
         const std::size_t row = (std::size_t) d * max_chunks;
         const uint32_t h = hist2[row + blockIdx.x];
         lb[d] = hist2[row + blockIdx.x + 1u] - h;
         gbase[d] = c < uDim ? out_ptr[c] + h - hist2[row + f] : 0u;
         fill[d] = 0u;
 #pragma unroll
-        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * 256u + d] = 0u;
+        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
     }
     __syncthreads();
-    block_scan_small(lb, 256u, scan33);
+    block_scan_small<(D / kTpThreads)>(lb, D, scan33);
     const unsigned lt = (1u << lane) - 1u;
-    uint16_t *my_cnt = sg.cnt + warp * 256u;
-    uint16_t *my_bas = sg.bas + warp * 256u;
+    uint16_t *my_cnt = sg.cnt + warp * D;
+    uint16_t *my_bas = sg.bas + warp * D;
     uint32_t nkk[kTpBatches];
     uint16_t nvv[kTpBatches];
     auto fetch = [&](uint32_t sc) {
@@ -634,18 +668,18 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
             const bool in = wa + q * 32u + lane < we;
-            const uint32_t d = kk[q] & 255u;
-            pk[q] = warp_match_digit<8>(d, in);
+            const uint32_t d = kk[q] & (D - 1u);
+            pk[q] = warp_match_digit<LB>(d, in);
             if (in && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[d] += (uint16_t) __popc(pk[q]);
             __syncwarp();
         }
         __syncthreads();
-        tp_stage_prefix(sg, 256u);
+        tp_stage_prefix(sg, D);
         __syncthreads();
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
             const bool in = wa + q * 32u + lane < we;
-            const uint32_t d = kk[q] & 255u;
+            const uint32_t d = kk[q] & (D - 1u);
             uint32_t lp = 0u;
             if (in) lp = my_bas[d] + __popc(pk[q] & lt);
             __syncwarp();
@@ -659,56 +693,91 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
             __syncwarp();
         }
     }
-    gbase[threadIdx.x] -= lb[threadIdx.x]; // global slot of staging slot 0 for digit d
+    // global slot of staging slot 0 for digit d
+    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
     __syncthreads();
     const uint32_t n = min(e - b, kTpChunk);
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
         const uint32_t key = st_key[j];
-        const uint32_t g = gbase[key & 255u] + j;
-        out_idx[g] = key >> kTpBucketBits;
+        const uint32_t g = gbase[key & (D - 1u)] + j;
+        out_idx[g] = key >> LB;
         out_val[g] = st_val[j];
     }
 }
 
-constexpr std::size_t kTpScatter2Smem = (std::size_t) kTpChunk * 6u + (std::size_t) 2u * kTpWarps * 256u * 2u;
+constexpr std::size_t tp_scatter2_smem(uint32_t low_bits) {
+    return (std::size_t) kTpChunk * 6u + ((std::size_t) 2u * kTpWarps * 2u << low_bits);
+}
+
+// Chunks, counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).
+template <int LB>
+int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
+                   cudaStream_t stream) {
+    constexpr std::size_t smem = tp_scatter2_smem(LB);
+    auto s2 = tp_scatter2_kernel<LB>;
+    if (!cuda_ok(cudaFuncSetAttribute(s2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
+                 "scatter2 smem attribute"))
+        return 0;
+    tp_chunks_kernel<<<1, 1024, 0, stream>>>(l.hist1, l.tiles1, l.K, l.max_chunks, l.chunk_bucket, l.chunk_begin,
+                                             l.chunk_end, l.chunk_first);
+    if (!launch_ok("tp_chunks_kernel")) return 0;
+    tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_begin, l.chunk_end, l.max_chunks,
+                                                                 l.hist2);
+    if (!launch_ok("tp_hist2_kernel")) return 0;
+    if (!scan_exclusive_u32(l.hist2, l.hist2, (std::size_t) l.max_chunks << LB, true, l.scan_tmp, l.scan_bytes,
+                            stream))
+        return 0;
+    tp_colcount_kernel<<<l.K, 256, 0, stream>>>(l.hist2, l.max_chunks, l.chunk_first, uDim, LB, out_ptr);
+    if (!launch_ok("tp_colcount_kernel")) return 0;
+    if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
+    s2<<<l.max_chunks, kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_bucket, l.chunk_begin, l.chunk_end,
+                                                   l.chunk_first, l.max_chunks, l.hist2, out_ptr, uDim, out_idx,
+                                                   out_val);
+    return launch_ok("tp_scatter2_kernel");
+}
+
+template <bool kCoo>
+int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *ptr, const uint32_t *key,
+                  const uint16_t *val, const uint32_t *pay, const uint32_t *pay_map, const tp2_layout &l,
+                  cudaStream_t stream) {
+    const std::size_t s1_smem = tp_scatter1_smem(l.K);
+    auto s1 = tp_scatter1_kernel<kCoo>;
+    if (!cuda_ok(cudaFuncSetAttribute(s1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s1_smem),
+                 "scatter1 smem attribute"))
+        return 0;
+    tp_hist1_kernel<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K,
+                                                                              l.tiles1, l.hist1, l.status);
+    if (!launch_ok("tp_hist1_kernel")) return 0;
+    if (!scan_exclusive_u32(l.hist1, l.hist1, (std::size_t) l.K * l.tiles1, true, l.scan_tmp, l.scan_bytes, stream))
+        return 0;
+    s1<<<l.tiles1, kTpThreads, s1_smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.low_bits, l.K, l.tiles1, l.hist1,
+                                                  l.gran_row, pay, pay_map, l.tmp_key, l.tmp_val);
+    return launch_ok("tp_scatter1_kernel");
+}
 
 int transpose2_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *ptr, const uint32_t *idx,
                       const uint16_t *val, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
                       const tp2_layout &l, cudaStream_t stream) {
-    const std::size_t h1_smem = (std::size_t) l.K * 4u;
-    const std::size_t s1_smem = tp_scatter1_smem(l.K);
-    auto s1 = tp_scatter1_kernel;
-    if (!cuda_ok(cudaFuncSetAttribute(s1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s1_smem),
-                 "scatter1 smem attribute") ||
-        !cuda_ok(cudaFuncSetAttribute(tp_scatter2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int) kTpScatter2Smem),
-                 "scatter2 smem attribute"))
-        return 0;
     tp_gran_rows_kernel<<<(cDim + 255u) / 256u, 256, 0, stream>>>(ptr, cDim, l.gran_row);
     if (!launch_ok("tp_gran_rows_kernel")) return 0;
-    tp_hist1_kernel<<<l.tiles1, kTpThreads, h1_smem, stream>>>(idx, nnz, uDim, l.K, l.tiles1, l.hist1, l.status);
-    if (!launch_ok("tp_hist1_kernel")) return 0;
-    if (!scan_exclusive_u32(l.hist1, l.hist1, (std::size_t) l.K * l.tiles1, true, l.scan_tmp, l.scan_bytes, stream))
-        return 0;
-    s1<<<l.tiles1, kTpThreads, s1_smem, stream>>>(ptr, idx, val, cDim, uDim, nnz, l.K, l.tiles1, l.hist1,
-                                                  l.gran_row, l.tmp_key, l.tmp_val);
-    if (!launch_ok("tp_scatter1_kernel")) return 0;
-    tp_chunks_kernel<<<1, 1024, 0, stream>>>(l.hist1, l.tiles1, l.K, l.max_chunks, l.chunk_bucket, l.chunk_begin,
-                                             l.chunk_end, l.chunk_first);
-    if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_hist2_kernel<<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_begin, l.chunk_end, l.max_chunks,
-                                                             l.hist2);
-    if (!launch_ok("tp_hist2_kernel")) return 0;
-    if (!scan_exclusive_u32(l.hist2, l.hist2, (std::size_t) 256u * l.max_chunks, true, l.scan_tmp, l.scan_bytes,
-                            stream))
-        return 0;
-    tp_colcount_kernel<<<l.K, 256, 0, stream>>>(l.hist2, l.max_chunks, l.chunk_first, uDim, out_ptr);
-    if (!launch_ok("tp_colcount_kernel")) return 0;
-    if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
-    tp_scatter2_kernel<<<l.max_chunks, kTpThreads, kTpScatter2Smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_bucket, l.chunk_begin,
-                                                                l.chunk_end, l.chunk_first, l.max_chunks, l.hist2,
-                                                                out_ptr, uDim, out_idx, out_val);
-    return launch_ok("tp_scatter2_kernel");
+    return tp_first_pass<false>(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, l, stream) &&
+           tp_second_pass<(int) kTpBucketBits>(uDim, l, out_ptr, out_idx, out_val, stream);
+}
+
+uint32_t bits_below(uint64_t v) { // bits that hold 0 .. v - 1
+    uint32_t b = 0u;
+    while (((uint64_t) 1u << b) < v) ++b;
+    return b;
+}
+
+// Low digit of the row partition: the fewest bits that keep the buckets within
+// kTpMaxBuckets; 0 where the partition does not apply (more rows than that
+// allows, or a column and the digit do not fit one packed word together, with
+// the word of all ones left over as "no entry").
+uint32_t partition_low_bits(uint32_t rows, uint32_t cols) {
+    uint32_t lb = kTpBucketBits;
+    while (lb <= kTpMaxLowBits && (uint64_t) rows > ((uint64_t) kTpMaxBuckets << lb)) ++lb;
+    return lb <= kTpMaxLowBits && bits_below((uint64_t) cols + 1u) + lb <= 32u ? lb : 0u;
 }
 
 } // namespace
@@ -718,7 +787,7 @@ int transpose_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t 
                      std::size_t scratch_bytes, cudaStream_t stream) {
     if (tp2_applicable(cDim, uDim)) {
         tp2_layout l2;
-        tp2_make_layout(cDim, uDim, nnz, scratch, scratch_bytes, &l2);
+        tp2_make_layout(uDim, nnz, kTpBucketBits, true, scratch, scratch_bytes, &l2);
         if (scratch == nullptr || l2.bytes > scratch_bytes) {
             set_error("compressed_transpose: scratch %zu < %zu bytes", scratch_bytes, l2.bytes);
             return 0;
@@ -756,10 +825,48 @@ int transpose_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t 
     return launch_ok("tr_scatter_kernel");
 }
 
+// COO entries in row order (stable: a row's entries keep their order): row
+// pointers, columns (through `map` when given) and values.  Every row is below
+// `rows` and every mapped column below `cols`.  Two passes move 22 bytes an
+// entry in runs; the two stable 32-bit sorts and the random gathers that this
+// replaces moved over 100, most of them one sector per entry.
+std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t cols) {
+    const uint32_t lb = partition_low_bits(rows, cols);
+    if (n == 0u || rows == 0u || lb == 0u) return 0u;
+    tp2_layout l;
+    tp2_make_layout(rows, n, lb, false, nullptr, 0, &l);
+    return l.bytes;
+}
+
+int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row, const uint32_t *col,
+                   const uint32_t *map, const uint16_t *val, uint32_t *out_ptr, uint32_t *out_col, uint16_t *out_val,
+                   void *scratch, std::size_t scratch_bytes, cudaStream_t stream) {
+    const uint32_t lb = partition_low_bits(rows, cols);
+    if (n == 0u || rows == 0u || lb == 0u) {
+        set_error("partition_rows: %u rows by %u columns outside its range", rows, cols);
+        return 0;
+    }
+    tp2_layout l;
+    tp2_make_layout(rows, n, lb, false, scratch, scratch_bytes, &l);
+    if (scratch == nullptr || l.bytes > scratch_bytes) {
+        set_error("partition_rows: scratch %zu < %zu bytes", scratch_bytes, l.bytes);
+        return 0;
+    }
+    if (!cuda_ok(cudaMemsetAsync(l.status, 0, 16, stream), "partition status memset") ||
+        !tp_first_pass<true>(0u, rows, n, nullptr, row, val, col, map, l, stream))
+        return 0;
+    switch (lb) {
+        case 8u: return tp_second_pass<8>(rows, l, out_ptr, out_col, out_val, stream);
+        case 9u: return tp_second_pass<9>(rows, l, out_ptr, out_col, out_val, stream);
+        case 10u: return tp_second_pass<10>(rows, l, out_ptr, out_col, out_val, stream);
+        default: return tp_second_pass<11>(rows, l, out_ptr, out_col, out_val, stream);
+    }
+}
+
 std::size_t transpose_scratch(uint32_t cDim, uint32_t uDim, uint32_t nnz) {
     if (tp2_applicable(cDim, uDim)) {
         tp2_layout l2;
-        tp2_make_layout(cDim, uDim, nnz, nullptr, 0, &l2);
+        tp2_make_layout(uDim, nnz, kTpBucketBits, true, nullptr, 0, &l2);
         return l2.bytes;
     }
     tr_layout l;

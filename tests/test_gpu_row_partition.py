@@ -1,0 +1,86 @@
+"""COO entries out of row order (put in row order by two counting-sort passes)
+and CSR rows out of column order, to Blocked-ELL, against the restatement: the
+edges of the 8,192-entry tiles, the low-digit widths, rows longer than a tile,
+repeated cells near and far apart, and more rows than the passes take."""
+
+import numpy as np
+import pytest
+
+from cases import np_u16, np_u32, to_device_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _entries(rows, cols, n, seed, hot=0, repeat=0):
+    rng = np.random.default_rng(seed)
+    row = rng.integers(0, rows, n).astype(np.uint32)
+    col = rng.integers(0, cols, n).astype(np.uint32)
+    if hot:  # one row holds most entries
+        row[rng.random(n) < 0.8] = hot
+    # distinct cells, then `repeat` copies of earlier cells at random later places
+    _, first = np.unique(row.astype(np.int64) * cols + col, return_index=True)
+    keep = rng.permutation(first)
+    row, col = row[keep], col[keep]
+    if repeat:
+        k = rng.integers(0, len(row), repeat)
+        at = np.sort(rng.integers(0, len(row) + 1, repeat))
+        row, col = np.insert(row, at, row[k]), np.insert(col, at, col[k])
+    val = rng.integers(1, 2000, len(row)).astype(np.float16)
+    val[rng.random(len(row)) < 0.02] = 0
+    return row, col, val.view(np.uint16)
+
+
+@pytest.mark.parametrize("rows,cols,n,block,hot,repeat,remap", [
+    (2, 9, 12, 8, 0, 0, False),
+    (700, 900, 8_192, 16, 0, 0, False),          # one whole tile (before repeats fall out)
+    (700, 900, 20_001, 16, 0, 300, True),        # repeats within a tile and across tiles
+    (513, 40_000, 60_000, 16, 300, 20, False),   # a row of several tiles
+    (262_144, 24, 30_000, 8, 0, 0, False),       # the most rows of an 8-bit low digit
+    (262_145, 24, 30_000, 8, 0, 50, False),      # 9 bits
+    (600_000, 24, 30_000, 8, 0, 0, True),        # 10 bits
+    (1_300_000, 16, 30_000, 8, 0, 10, False),    # 11 bits
+    (2_097_153, 8, 20_000, 8, 0, 10, False),     # past the partition: the sorts
+])
+def test_shuffled_coo(cuda, orc, rows, cols, n, block, hot, repeat, remap):
+    import torch
+
+    from cellshard_b200.device import blocked_ell_from_coo
+
+    row, col, val = _entries(rows, cols, n, rows + n, hot, repeat)
+    fmap = np.random.default_rng(1).permutation(cols).astype(np.uint32) if remap else None
+
+    def dev(a, t):
+        return torch.from_numpy(np.ascontiguousarray(a).view(t).copy()).cuda()
+
+    out, counts, status, total = blocked_ell_from_coo(
+        rows, cols, dev(row, np.int32), dev(col, np.int32), dev(val, np.float16), block, cols,
+        dev(fmap, np.int32) if remap else None)
+    ref = orc.blocked_ell_from_coo(rows, cols, row, col, val, block, fmap)
+    assert status == 0 and out.ell_cols == ref["ell_cols"] and total == ref["total_blocks"]
+    assert np.array_equal(np_u32(out.bci), ref["bci"])
+    assert np.array_equal(np_u16(out.val), ref["val"])
+    assert counts == [ref["nnz_host"], ref["nnz_gpu"]]
+
+
+@pytest.mark.parametrize("cols,block,repeat", [(500, 8, False), (9_000, 16, False), (9_000, 16, True),
+                                               (32_768, 16, True), (32_768, 2, False)])
+def test_csr_rows_in_any_column_order(cuda, orc, cols, block, repeat):
+    from cellshard_b200.device import blocked_ell_from_csr
+
+    rng = np.random.default_rng(cols + block)
+    rows = 37
+    parts = []
+    for r in range(rows):
+        c = rng.permutation(cols)[:int(rng.integers(0, min(cols, 5_000)))]
+        if r % 3 == 0:
+            c = np.sort(c)
+        if repeat and r % 4 == 1 and len(c) > 1:
+            c = np.append(c, c[rng.integers(0, len(c), 3)])
+        parts.append(c)
+    ptr = np.concatenate([[0], np.cumsum([len(c) for c in parts])]).astype(np.uint32)
+    idx = np.concatenate(parts).astype(np.uint32)
+    val = rng.integers(0, 2000, len(idx)).astype(np.float16).view(np.uint16)
+    out = blocked_ell_from_csr(to_device_csr(rows, cols, ptr, idx, val), block)
+    ref = orc.blocked_ell_from_csr(rows, cols, ptr, idx, val, block)
+    assert out.ell_cols == ref["ell_cols"] and out.nnz == ref["nnz"]
+    assert np.array_equal(np_u32(out.bci), ref["bci"]) and np.array_equal(np_u16(out.val), ref["val"])
