@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(kThreads) tr_scatter_kernel(const uint32_t *__
 // sectors open, far beyond L2.  Here the column key is sorted in two stable
 // counting-sort passes whose open write frontier is small:
 //   pass 1  by bucket = column >> 8 (<= 1,024 buckets), tiles of 8,192
-//           consecutive entries; entries become packed keys
-//           (row << 8 | column & 255) + values.
+//           consecutive entries; entries become packed words (row >> 5,
+//           column & 255, row & 31) + values: the upper bits are the place of
+//           the entry's bit in pass 2's bitmap.
 //   pass 2  inside each bucket by column & 255, in chunks of <= 8,192 that
 //           never cross a bucket, writing straight into the CSC.
 // Each tile or chunk is reordered whole in shared memory and leaves as one
@@ -193,20 +194,33 @@ constexpr uint32_t kTpTile1 = 8192;  // entries per pass-1 tile (staged whole in
 constexpr uint32_t kTpChunk = 8192;  // entries per pass-2 chunk (staged whole in shared memory)
 constexpr uint32_t kTpGran = 256;    // entries per warp per step; rows are looked up per granule
 
+constexpr uint32_t kTpSlice = 64;    // tiles or chunks per slice of the offset scan
+
+// Counts of a pass, one row per tile or chunk and one column per digit, and
+// what the scan over the rows of a segment makes of them: pass 1 has one
+// segment (all tiles), pass 2 one per bucket (its chunks).
+struct tp_counts {
+    uint16_t *cnt;      // [rows][D]
+    uint32_t *base;     // [rows][D] global slot of the row's first entry of the digit
+    uint32_t *slices;   // [slices][D] sums, then exclusive prefixes inside the segment
+};
+
 struct tp2_layout {
     uint32_t *status;
-    uint32_t *hist1;       // [K * tiles1 + 1], bucket-major
+    tp_counts one, two;
+    uint32_t *total1;      // [K] entries of each bucket
+    uint32_t *start1;      // [K + 1] first pass-1 slot of each bucket
     uint32_t *tmp_key;     // [nnz]
     uint16_t *tmp_val;     // [nnz]
     uint32_t *chunk_bucket; // [max_chunks]
-    uint32_t *chunk_begin;  // [max_chunks]
-    uint32_t *chunk_end;    // [max_chunks]
-    uint32_t *chunk_first;  // [K + 1]
+    uint2 *chunk_range;     // [max_chunks] entries
+    uint32_t *slice_bucket; // [max_slices]
+    uint2 *slice_range;     // [max_slices] chunks
+    uint32_t *slice_first;  // [K + 1]
     uint32_t *gran_row;     // [nnz / kTpGran + 1] row holding entry j * kTpGran
-    uint32_t *hist2;        // [256 * max_chunks + 1], digit-major
     void *scan_tmp;
     std::size_t scan_bytes, bytes;
-    uint32_t K, tiles1, max_chunks, low_bits;
+    uint32_t K, tiles1, max_chunks, slices1, max_slices, low_bits;
 };
 
 bool tp2_applicable(uint32_t cDim, uint32_t uDim) {
@@ -221,24 +235,29 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     if (l->K == 0u) l->K = 1u;
     l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + kTpTile1 - 1u) / kTpTile1);
     l->max_chunks = nnz / kTpChunk + l->K + 1u;
+    l->slices1 = (l->tiles1 + kTpSlice - 1u) / kTpSlice;
+    l->max_slices = l->max_chunks / kTpSlice + l->K + 1u;
     scratch_carver c(base, cap);
     l->status = c.take<uint32_t>(4);
-    l->hist1 = c.take<uint32_t>((std::size_t) l->K * l->tiles1 + 1u);
+    auto counts = [&](tp_counts *t, std::size_t rows, std::size_t slices, std::size_t digits) {
+        t->cnt = c.take<uint16_t>(rows * digits);
+        t->base = c.take<uint32_t>(rows * digits);
+        t->slices = c.take<uint32_t>(slices * digits);
+    };
+    counts(&l->one, l->tiles1, l->slices1, l->K);
+    counts(&l->two, l->max_chunks, l->max_slices, D);
+    l->total1 = c.take<uint32_t>(l->K);
+    l->start1 = c.take<uint32_t>((std::size_t) l->K + 1u);
     l->tmp_key = c.take<uint32_t>((std::size_t) nnz + 1u);
     l->tmp_val = c.take<uint16_t>((std::size_t) nnz + 8u);
     l->gran_row = granules ? c.take<uint32_t>((std::size_t) nnz / kTpGran + 1u) : nullptr;
     l->chunk_bucket = c.take<uint32_t>(l->max_chunks);
-    l->chunk_begin = c.take<uint32_t>(l->max_chunks);
-    l->chunk_end = c.take<uint32_t>(l->max_chunks);
-    l->chunk_first = c.take<uint32_t>((std::size_t) l->K + 1u);
-    l->hist2 = c.take<uint32_t>((std::size_t) D * l->max_chunks + 1u);
-    std::size_t sb = scan_u32_scratch_bytes((std::size_t) l->K * l->tiles1);
-    const std::size_t sb2 = scan_u32_scratch_bytes((std::size_t) D * l->max_chunks);
-    const std::size_t sb3 = scan_u32_scratch_bytes(uDim);
-    if (sb2 > sb) sb = sb2;
-    if (sb3 > sb) sb = sb3;
-    l->scan_bytes = sb;
-    l->scan_tmp = c.take<char>(sb);
+    l->chunk_range = c.take<uint2>(l->max_chunks);
+    l->slice_bucket = c.take<uint32_t>(l->max_slices);
+    l->slice_range = c.take<uint2>(l->max_slices);
+    l->slice_first = c.take<uint32_t>((std::size_t) l->K + 1u);
+    l->scan_bytes = scan_u32_scratch_bytes(uDim);
+    l->scan_tmp = c.take<char>(l->scan_bytes);
     l->bytes = c.used;
 }
 
@@ -255,8 +274,7 @@ __global__ void __launch_bounds__(256) tp_gran_rows_kernel(const uint32_t *__res
 // Pass-1 histogram: tile t is entries [t * kTpTile1, (t + 1) * kTpTile1).
 __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__restrict__ idx, uint32_t nnz,
                                                              uint32_t uDim, uint32_t low_bits, uint32_t K,
-                                                             uint32_t tiles1,
-                                                             uint32_t *__restrict__ hist1, uint32_t *status) {
+                                                             uint16_t *__restrict__ cnt, uint32_t *status) {
     extern __shared__ uint32_t tp_h[];
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) tp_h[k] = 0u;
     __syncthreads();
@@ -279,8 +297,85 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__
         }
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) hist1[(std::size_t) k * tiles1 + blockIdx.x] = tp_h[k];
+    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) cnt[(std::size_t) blockIdx.x * K + k] = (uint16_t) tp_h[k];
     if (bad) status_or(status, bad);
+}
+
+// The offset scan, over slices of kTpSlice rows so that a segment of many rows
+// is not one serial chain: slice sums, a scan of each segment's slices, then
+// the rows of every slice.  Rows are D counters wide and a warp reads 32 of
+// them together (the counts used to lie digit by digit, one sector apart for a
+// CTA that wants its row of them; scanned as one array of 12 M words they took
+// 100 us and 256 scattered reads per chunk at 300,000 x 32,768).
+__device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, uint32_t rows) {
+    if (range != nullptr) return range[blockIdx.x];
+    return make_uint2(blockIdx.x * kTpSlice, min(rows, (blockIdx.x + 1u) * kTpSlice));
+}
+
+__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
+                                                            uint32_t rows, const uint2 *__restrict__ range,
+                                                            uint32_t *__restrict__ slices) {
+    const uint2 r = tp_slice_rows(range, rows);
+    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+        uint32_t sum = 0u;
+#pragma unroll 16
+        for (uint32_t i = r.x; i < r.y; ++i) sum += __ldg(cnt + (std::size_t) i * D + d);
+        slices[(std::size_t) blockIdx.x * D + d] = sum;
+    }
+}
+
+// One segment (blockIdx.x) and 32 digits (blockIdx.y) per CTA: 32 threads per
+// digit, each over a run of the segment's slices.  totals[segment * D + d] for
+// digits below `limit` in all.
+__global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restrict__ slices, uint32_t D,
+                                                             const uint32_t *__restrict__ seg_first, uint32_t n_slices,
+                                                             uint32_t limit, uint32_t *__restrict__ totals) {
+    __shared__ uint32_t part[32][33];
+    const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, d = blockIdx.y * 32u + x;
+    const uint32_t s0 = seg_first != nullptr ? seg_first[blockIdx.x] : 0u;
+    const uint32_t s1 = seg_first != nullptr ? seg_first[blockIdx.x + 1u] : n_slices;
+    const uint32_t per = (s1 - s0 + 31u) / 32u;
+    const uint32_t a = min(s1, s0 + y * per), e = min(s1, a + per);
+    uint32_t sum = 0u;
+    if (d < D)
+        for (uint32_t i = a; i < e; ++i) sum += slices[(std::size_t) i * D + d];
+    part[y][x] = sum;
+    __syncthreads();
+    // warp y scans digit y of the 32
+    {
+        const uint32_t v = part[x][y], incl = warp_inclusive_scan(v);
+        part[x][y] = incl - v;
+        const std::size_t c = (std::size_t) blockIdx.x * D + blockIdx.y * 32u + y;
+        if (x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
+    }
+    __syncthreads();
+    if (d < D) {
+        uint32_t run = part[y][x];
+        for (uint32_t i = a; i < e; ++i) {
+            const uint32_t v = slices[(std::size_t) i * D + d];
+            slices[(std::size_t) i * D + d] = run;
+            run += v;
+        }
+    }
+}
+
+// start[segment * D + d]: global slot of the digit's first entry
+__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
+                                                             uint32_t rows, const uint2 *__restrict__ range,
+                                                             const uint32_t *__restrict__ segment,
+                                                             const uint32_t *__restrict__ slices,
+                                                             const uint32_t *__restrict__ start, uint32_t limit,
+                                                             uint32_t *__restrict__ base) {
+    const uint2 r = tp_slice_rows(range, rows);
+    const std::size_t c0 = (segment != nullptr ? (std::size_t) segment[blockIdx.x] : 0u) * D;
+    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+        uint32_t run = slices[(std::size_t) blockIdx.x * D + d] + (c0 + d < limit ? start[c0 + d] : 0u);
+#pragma unroll 16
+        for (uint32_t i = r.x; i < r.y; ++i) {
+            base[(std::size_t) i * D + d] = run;
+            run += __ldg(cnt + (std::size_t) i * D + d);
+        }
+    }
 }
 
 // Block-wide exclusive scan of n <= Q * blockDim.x values in place (each
@@ -305,6 +400,19 @@ __device__ __forceinline__ void block_scan_small(uint32_t *v, uint32_t n, uint32
     }
     if (t == 0) v[n] = tot;
     __syncthreads();
+}
+
+// An entry between the passes: its payload (row; COO: column) around the low digit.
+__device__ __forceinline__ uint32_t tp_pack(uint32_t pay, uint32_t digit, uint32_t low_bits) {
+    return (pay >> 5) << (low_bits + 5u) | digit << 5 | (pay & 31u);
+}
+template <int LB>
+__device__ __forceinline__ uint32_t tp_digit(uint32_t key) {
+    return key >> 5 & ((1u << LB) - 1u);
+}
+template <int LB>
+__device__ __forceinline__ uint32_t tp_payload(uint32_t key) {
+    return key >> (LB + 5) << 5 | (key & 31u);
 }
 
 constexpr uint32_t kTpSub = 2048;                        // entries counted and placed per step
@@ -347,12 +455,13 @@ struct tp_stage {
     uint32_t *fill; // [D]
 };
 
+template <unsigned WARPS>
 __device__ __forceinline__ void tp_stage_prefix(const tp_stage &sg, uint32_t D) {
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t t = sg.lb[d] + sg.fill[d];
         const uint32_t t0 = t;
 #pragma unroll
-        for (unsigned w = 0; w < kTpWarps; ++w) {
+        for (unsigned w = 0; w < WARPS; ++w) {
             const uint32_t c = sg.cnt[w * D + d];
             sg.cnt[w * D + d] = 0u;
             sg.bas[w * D + d] = (uint16_t) t;
@@ -364,18 +473,18 @@ __device__ __forceinline__ void tp_stage_prefix(const tp_stage &sg, uint32_t D) 
 
 // Pass 1: tile t = entries [t * kTpTile1, ...) of the input, reordered by
 // bucket (key >> low_bits) in shared memory, stable, then written out as one
-// run per bucket.  Packed keys are (payload << low_bits | low digit).
+// run per bucket.
 // kCoo false: the key is the CSR entry's column, the payload its row, found
 // from `ptr`.  kCoo true: the key `idx` is the COO entry's row, the payload
 // its (mapped) column; random rows make a warp's 32 keys nearly all distinct,
 // so peers come from ballots (one per bucket bit) instead of match.any.
+// Packed words are (payload >> 5, low digit, payload & 31).
 template <bool kCoo>
 __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t *__restrict__ ptr,
                                                                 const uint32_t *__restrict__ idx,
                                                                 const uint16_t *__restrict__ val, uint32_t cDim,
                                                                 uint32_t uDim, uint32_t nnz, uint32_t coo_low_bits,
-                                                                uint32_t K, uint32_t tiles1,
-                                                                const uint32_t *__restrict__ hist1,
+                                                                uint32_t K, const tp_counts one,
                                                                 const uint32_t *__restrict__ gran_row,
                                                                 const uint32_t *__restrict__ pay,
                                                                 const uint32_t *__restrict__ pay_map,
@@ -395,9 +504,8 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
     const uint32_t a = blockIdx.x * kTpTile1, e = min(nnz, a + kTpTile1);
     if (a >= e) return;
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
-        const uint32_t h = hist1[(std::size_t) k * tiles1 + blockIdx.x];
-        run[k] = h;
-        sg.lb[k] = hist1[(std::size_t) k * tiles1 + blockIdx.x + 1u] - h;
+        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        sg.lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
         sg.fill[k] = 0u;
     }
     for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
@@ -469,7 +577,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
             __syncwarp();
         }
         __syncthreads();
-        tp_stage_prefix(sg, K);
+        tp_stage_prefix<kTpWarps>(sg, K);
         __syncthreads();
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
@@ -480,7 +588,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
             __syncwarp();
             if (ok) {
                 if (lp < kTpTile1)
-                    st[lp] = (unsigned long long) ((rl[q] << low_bits) | (cc[q] & low_mask)) |
+                    st[lp] = (unsigned long long) tp_pack(rl[q], cc[q] & low_mask, low_bits) |
                              ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
                 if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
             }
@@ -504,62 +612,81 @@ std::size_t tp_scatter1_smem(uint32_t K) {
     return (std::size_t) kTpTile1 * 8u + ((std::size_t) 3u * K + 1u) * 4u + (std::size_t) 2u * kTpWarps * K * 2u;
 }
 
-// one CTA: cut every bucket's entry range into chunks of <= kTpChunk entries
-__global__ void __launch_bounds__(1024) tp_chunks_kernel(const uint32_t *__restrict__ hist1, uint32_t tiles1,
-                                                         uint32_t K, uint32_t max_chunks,
-                                                         uint32_t *__restrict__ chunk_bucket,
-                                                         uint32_t *__restrict__ chunk_begin,
-                                                         uint32_t *__restrict__ chunk_end,
-                                                         uint32_t *__restrict__ chunk_first) {
-    __shared__ uint32_t smem[33];
-    const uint32_t total = hist1[(std::size_t) K * tiles1];
-    uint32_t carry = 0u;
-    for (uint32_t k0 = 0; k0 < K; k0 += blockDim.x) {
-        const uint32_t k = k0 + threadIdx.x;
-        uint32_t b = 0u, n = 0u, nc = 0u;
-        if (k < K) {
-            b = hist1[(std::size_t) k * tiles1];
-            const uint32_t e = k + 1u < K ? hist1[(std::size_t) (k + 1u) * tiles1] : total;
-            n = e - b;
-            nc = (n + kTpChunk - 1u) / kTpChunk;
-        }
-        uint32_t tot;
-        const uint32_t ex = block_exclusive_scan(nc, smem, tot);
-        if (k < K) {
-            chunk_first[k] = carry + ex;
-            for (uint32_t j = 0; j < nc; ++j) {
-                const uint32_t id = carry + ex + j;
-                if (id < max_chunks) {
-                    chunk_bucket[id] = k;
-                    chunk_begin[id] = b + j * kTpChunk;
-                    chunk_end[id] = min(b + n, b + (j + 1u) * kTpChunk);
-                }
-            }
-        }
-        carry += tot;
+// One CTA: bucket starts from their totals, then every bucket's entry range is
+// cut at the multiples of kTpChunk and its chunks into slices; a scan of the
+// buckets' chunk counts, and a thread per chunk finds its bucket in it (a
+// thread per bucket writing its chunks one by one took 84 us for 48,000).
+__device__ __forceinline__ uint32_t tp_find(const uint32_t *first, uint32_t K, uint32_t id) {
+    uint32_t lo = 0u, hi = K - 1u; // last k with first[k] <= id
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1u) >> 1;
+        if (first[mid] <= id)
+            lo = mid;
+        else
+            hi = mid - 1u;
     }
-    if (threadIdx.x == 0) chunk_first[K] = carry;
-    // unused chunk slots carry empty ranges so their histograms are zero
-    for (uint32_t id = carry + threadIdx.x; id < max_chunks; id += blockDim.x) {
-        chunk_bucket[id] = 0u;
-        chunk_begin[id] = 0u;
-        chunk_end[id] = 0u;
+    return lo;
+}
+
+__global__ void __launch_bounds__(1024) tp_chunks_kernel(const tp2_layout l) {
+    __shared__ uint32_t smem[33];
+    __shared__ uint32_t first[kTpMaxBuckets + 1u], begin[kTpMaxBuckets + 1u], slice[kTpMaxBuckets + 1u];
+    const uint32_t k = threadIdx.x, K = l.K; // K <= kTpMaxBuckets == blockDim.x
+    uint32_t total;
+    const uint32_t n = k < K ? l.total1[k] : 0u;
+    const uint32_t b = block_exclusive_scan(n, smem, total);
+    if (k < K) begin[k] = l.start1[k] = b;
+    if (k == 0u) begin[K] = l.start1[K] = total;
+    const uint32_t nc = n != 0u ? (b + n - 1u) / kTpChunk + 1u - b / kTpChunk : 0u;
+    uint32_t chunks, slices;
+    const uint32_t fc = block_exclusive_scan(nc, smem, chunks);
+    const uint32_t fs = block_exclusive_scan((nc + kTpSlice - 1u) / kTpSlice, smem, slices);
+    if (k < K) {
+        first[k] = fc;
+        slice[k] = l.slice_first[k] = fs;
+    }
+    if (k == 0u) {
+        first[K] = chunks;
+        slice[K] = l.slice_first[K] = slices;
+    }
+    __syncthreads();
+    for (uint32_t id = threadIdx.x; id < l.max_chunks; id += blockDim.x) {
+        uint32_t bk = 0u;
+        uint2 r = make_uint2(0u, 0u); // unused chunks are empty
+        if (id < chunks) {
+            bk = tp_find(first, K, id);
+            const uint32_t cell = begin[bk] / kTpChunk + (id - first[bk]);
+            r.x = max(begin[bk], cell * kTpChunk);
+            r.y = cell == 0xffffffffu / kTpChunk ? begin[bk + 1u] : min(begin[bk + 1u], (cell + 1u) * kTpChunk);
+        }
+        l.chunk_bucket[id] = bk;
+        l.chunk_range[id] = r;
+    }
+    for (uint32_t id = threadIdx.x; id < l.max_slices; id += blockDim.x) {
+        uint32_t bk = 0u;
+        uint2 r = make_uint2(0u, 0u);
+        if (id < slices) {
+            bk = tp_find(slice, K, id);
+            r.x = first[bk] + (id - slice[bk]) * kTpSlice;
+            r.y = min(first[bk + 1u], r.x + kTpSlice);
+        }
+        l.slice_bucket[id] = bk;
+        l.slice_range[id] = r;
     }
 }
 
 // one histogram per warp while eight of them fit (LB = 8), one per CTA above
 template <int LB>
 __global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ tmp_key,
-                                                             const uint32_t *__restrict__ chunk_begin,
-                                                             const uint32_t *__restrict__ chunk_end,
-                                                             uint32_t max_chunks, uint32_t *__restrict__ hist2) {
+                                                             const uint2 *__restrict__ chunk_range,
+                                                             uint16_t *__restrict__ cnt) {
     constexpr uint32_t D = 1u << LB;
     constexpr unsigned kCopies = LB == 8 ? kTpWarps : 1u;
     __shared__ uint32_t h[kCopies][D];
     const unsigned copy = (threadIdx.x >> 5) % kCopies;
     for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
     __syncthreads();
-    const uint32_t b = chunk_begin[blockIdx.x], e = chunk_end[blockIdx.x];
+    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
     constexpr unsigned U = 4;
     for (uint32_t i0 = b; i0 < e; i0 += U * blockDim.x) {
         uint32_t kk[U];
@@ -570,79 +697,34 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__
         }
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-            if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][kk[u] & (D - 1u)], 1u);
+            if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][tp_digit<LB>(kk[u])], 1u);
     }
     __syncthreads();
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t t = 0u;
 #pragma unroll
         for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
-        hist2[(std::size_t) d * max_chunks + blockIdx.x] = t;
+        cnt[(std::size_t) blockIdx.x * D + d] = (uint16_t) t;
     }
 }
 
-// key totals from the digit-major scan: count(k * D + d) = P[d][last] - P[d][first]
-__global__ void __launch_bounds__(256) tp_colcount_kernel(const uint32_t *__restrict__ hist2, uint32_t max_chunks,
-                                                          const uint32_t *__restrict__ chunk_first, uint32_t uDim,
-                                                          uint32_t low_bits, uint32_t *__restrict__ counts) {
-    const uint32_t k = blockIdx.x;
-    const uint32_t f = chunk_first[k], l = chunk_first[k + 1u];
-    for (uint32_t d = threadIdx.x; d < 1u << low_bits; d += blockDim.x) {
-        const uint32_t c = (k << low_bits) + d;
-        if (c < uDim) counts[c] = hist2[(std::size_t) d * max_chunks + l] - hist2[(std::size_t) d * max_chunks + f];
-    }
-}
-
-// Pass 2: a chunk of one bucket reordered by the low digit in shared memory
-// (stable), then written out as one run per key.
-template <int LB>
-__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
-                                                                const uint16_t *__restrict__ tmp_val,
-                                                                const uint32_t *__restrict__ chunk_bucket,
-                                                                const uint32_t *__restrict__ chunk_begin,
-                                                                const uint32_t *__restrict__ chunk_end,
-                                                                const uint32_t *__restrict__ chunk_first,
-                                                                uint32_t max_chunks, const uint32_t *__restrict__ hist2,
-                                                                const uint32_t *__restrict__ out_ptr, uint32_t uDim,
-                                                                uint32_t *__restrict__ out_idx,
-                                                                uint16_t *__restrict__ out_val) {
-    extern __shared__ __align__(16) uint32_t tp_s2[];
+// Stable ranking of one pass-2 chunk [b, e) into the stage by ballots: each
+// step gives every warp 256 consecutive entries in eight 32-entry batches; a
+// batch's peers (lanes with the same digit) come from one ballot per digit bit.
+// lb holds each digit's first staging slot; fill and cnt are zero on entry.
+template <int LB, unsigned WARPS>
+__device__ void tp_rank_ballots(const uint32_t *__restrict__ tmp_key, const uint16_t *__restrict__ tmp_val, uint32_t b,
+                                uint32_t e, const tp_stage &sg, uint32_t *st_key, uint16_t *st_val) {
     constexpr uint32_t D = 1u << LB;
-    __shared__ uint32_t gbase[D];
-    __shared__ uint32_t lb[D + 1u];
-    __shared__ uint32_t fill[D];
-    __shared__ uint32_t scan33[33];
-    uint32_t *st_key = tp_s2;                                              // [kTpChunk]
-    uint16_t *st_val = reinterpret_cast<uint16_t *>(st_key + kTpChunk);   // [kTpChunk]
-    tp_stage sg;
-    sg.cnt = st_val + kTpChunk;                                            // [kTpWarps][D]
-    sg.bas = sg.cnt + kTpWarps * D;                                     // [kTpWarps][D]
-    sg.lb = lb;
-    sg.fill = fill;
+    constexpr uint32_t kStep = WARPS * kTpGran;
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t b = chunk_begin[blockIdx.x], e = chunk_end[blockIdx.x];
-    if (b >= e) return;
-    const uint32_t k = chunk_bucket[blockIdx.x];
-    const uint32_t f = chunk_first[k];
-    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
-        const uint32_t c = k * D + d;
-        const std::size_t row = (std::size_t) d * max_chunks;
-        const uint32_t h = hist2[row + blockIdx.x];
-        lb[d] = hist2[row + blockIdx.x + 1u] - h;
-        gbase[d] = c < uDim ? out_ptr[c] + h - hist2[row + f] : 0u;
-        fill[d] = 0u;
-#pragma unroll
-        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
-    }
-    __syncthreads();
-    block_scan_small<(D / kTpThreads)>(lb, D, scan33);
     const unsigned lt = (1u << lane) - 1u;
     uint16_t *my_cnt = sg.cnt + warp * D;
     uint16_t *my_bas = sg.bas + warp * D;
     uint32_t nkk[kTpBatches];
     uint16_t nvv[kTpBatches];
     auto fetch = [&](uint32_t sc) {
-        const uint32_t n = min(kTpSub, e - sc);
+        const uint32_t n = min(kStep, e - sc);
         const uint32_t wa = sc + min(n, warp * kTpGran), we = sc + min(n, (warp + 1u) * kTpGran);
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
@@ -653,8 +735,8 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
         }
     };
     fetch(b);
-    for (uint32_t sc0 = b; sc0 < e; sc0 += kTpSub) {
-        const uint32_t n = min(kTpSub, e - sc0);
+    for (uint32_t sc0 = b; sc0 < e; sc0 += kStep) {
+        const uint32_t n = min(kStep, e - sc0);
         const uint32_t wa = sc0 + min(n, warp * kTpGran);
         const uint32_t we = sc0 + min(n, (warp + 1u) * kTpGran);
         uint32_t kk[kTpBatches], pk[kTpBatches];
@@ -664,22 +746,22 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
             kk[q] = nkk[q];
             vv[q] = nvv[q];
         }
-        if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
+        if (sc0 + kStep < e) fetch(sc0 + kStep);
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
             const bool in = wa + q * 32u + lane < we;
-            const uint32_t d = kk[q] & (D - 1u);
+            const uint32_t d = tp_digit<LB>(kk[q]);
             pk[q] = warp_match_digit<LB>(d, in);
             if (in && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[d] += (uint16_t) __popc(pk[q]);
             __syncwarp();
         }
         __syncthreads();
-        tp_stage_prefix(sg, D);
+        tp_stage_prefix<WARPS>(sg, D);
         __syncthreads();
 #pragma unroll
         for (unsigned q = 0; q < kTpBatches; ++q) {
             const bool in = wa + q * 32u + lane < we;
-            const uint32_t d = kk[q] & (D - 1u);
+            const uint32_t d = tp_digit<LB>(kk[q]);
             uint32_t lp = 0u;
             if (in) lp = my_bas[d] + __popc(pk[q] & lt);
             __syncwarp();
@@ -693,15 +775,199 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
             __syncwarp();
         }
     }
+}
+
+// Pass 2 of entries in any payload order (the COO rows): a chunk of one bucket
+// reordered by the low digit in shared memory (stable), then written out as
+// one run per key.
+template <int LB>
+__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
+                                                                const uint16_t *__restrict__ tmp_val,
+                                                                const uint2 *__restrict__ chunk_range,
+                                                                const tp_counts two, uint32_t *__restrict__ out_idx,
+                                                                uint16_t *__restrict__ out_val) {
+    extern __shared__ __align__(16) uint32_t tp_s2[];
+    constexpr uint32_t D = 1u << LB;
+    __shared__ uint32_t gbase[D];
+    __shared__ uint32_t lb[D + 1u];
+    __shared__ uint32_t fill[D];
+    __shared__ uint32_t scan33[33];
+    uint32_t *st_key = tp_s2;                                              // [kTpChunk]
+    uint16_t *st_val = reinterpret_cast<uint16_t *>(st_key + kTpChunk);   // [kTpChunk]
+    tp_stage sg;
+    sg.cnt = st_val + kTpChunk;                                            // [kTpWarps][D]
+    sg.bas = sg.cnt + kTpWarps * D;                                        // [kTpWarps][D]
+    sg.lb = lb;
+    sg.fill = fill;
+    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
+    if (b >= e) return;
+    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
+        lb[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
+        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
+        fill[d] = 0u;
+#pragma unroll
+        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
+    }
+    __syncthreads();
+    block_scan_small<(D / kTpThreads)>(lb, D, scan33);
+    tp_rank_ballots<LB, kTpWarps>(tmp_key, tmp_val, b, e, sg, st_key, st_val);
     // global slot of staging slot 0 for digit d
     for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
     __syncthreads();
     const uint32_t n = min(e - b, kTpChunk);
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
         const uint32_t key = st_key[j];
-        const uint32_t g = gbase[key & (D - 1u)] + j;
-        out_idx[g] = key >> LB;
+        const uint32_t g = gbase[tp_digit<LB>(key)] + j;
+        out_idx[g] = tp_payload<LB>(key);
         out_val[g] = st_val[j];
+    }
+}
+
+// Pass 2 of the transpose.  Pass 1 is stable, so the rows of a chunk never
+// decrease, and the rank of an entry among its column's is the number of
+// earlier ROWS of the chunk that hold the column: a bitmap over (32-row word,
+// column) filled by atomicOr in any order, popcounts prefixed per column (the
+// prefix starts at the column's staging slot, so one lookup gives the slot).
+// The bitmap covers 32 * kTpSpanWords rows; a chunk that spans more goes round
+// by round (rows ascending), one that would take over kTpRounds by ballots.
+// A row that holds a column twice leaves fewer bits than entries: its chunk is
+// ranked by ballots.  A matrix with under kTpRowsKernelMin entries per row and
+// 256 columns takes the ballot kernel for all chunks: at 300,000 x 32,768 and
+// density 0.02 (5 entries) the whole transpose takes 2.76 ms this way and 2.96
+// by ballots, at 0.01 (2.6) 1.64 and 1.61, at 0.006 1.12 and 1.06.
+// 300,000 x 32,768, 393 M entries: 1.80 ms (4.7 GB) where ballots in every
+// chunk took 2.45; bound by shared-memory wavefronts (34 per 32 entries).
+constexpr double kTpRowsKernelMin = 3.0;
+constexpr unsigned kTpThreads2 = 512;
+constexpr unsigned kTpWarps2 = kTpThreads2 / 32;
+constexpr uint32_t kTpSpanWords = 36; // two CTAs per SM with the stage
+constexpr uint32_t kTpSpanKeys = kTpSpanWords << (kTpBucketBits + 5u); // packed words of a span
+constexpr uint32_t kTpRounds = 4;
+constexpr unsigned kTpPerThread = kTpChunk / kTpThreads2;
+
+struct tp_rows_smem {
+    uint32_t key[kTpChunk];                // staged words
+    uint32_t bits[kTpSpanWords * 256];     // ballots: cnt, bas
+    uint16_t pre[kTpSpanWords * 256];
+    uint16_t val[kTpChunk];                // staged values
+    uint32_t gbase[256], lb[257], fill[256], scan33[33], dup;
+};
+static_assert(sizeof(uint32_t) * kTpSpanWords * 256u >= 2u * kTpWarps2 * 256u * sizeof(uint16_t),
+              "the ballot counters fit the bitmap's place");
+
+__global__ void __launch_bounds__(kTpThreads2, 2)
+    tp_scatter2_rows_kernel(const uint32_t *__restrict__ tmp_key, const uint16_t *__restrict__ tmp_val,
+                            const uint2 *__restrict__ chunk_range, const tp_counts two,
+                            uint32_t *__restrict__ out_idx, uint16_t *__restrict__ out_val) {
+    extern __shared__ __align__(16) unsigned char tp_rs[];
+    tp_rows_smem &sm = *reinterpret_cast<tp_rows_smem *>(tp_rs);
+    constexpr int LB = (int) kTpBucketBits;
+    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
+    if (b >= e) return;
+    const unsigned t = threadIdx.x;
+    const uint32_t n = min(e - b, kTpChunk);
+    // consecutive lanes take consecutive entries: ~3 rows of ascending columns,
+    // few of which meet in one bitmap word
+    uint32_t kk[kTpPerThread];
+    uint32_t vv[kTpPerThread / 2u];
+    const uint32_t *kp = tmp_key + b + t;
+    const unsigned short *vp = reinterpret_cast<const unsigned short *>(tmp_val) + b + t;
+    if (n == kTpChunk) {
+#pragma unroll
+        for (unsigned q = 0; q < kTpPerThread; ++q) kk[q] = __ldcs(kp + q * kTpThreads2);
+#pragma unroll
+        for (unsigned q = 0; q < kTpPerThread; q += 2u)
+            vv[q / 2u] = (uint32_t) __ldcs(vp + q * kTpThreads2) | (uint32_t) __ldcs(vp + (q + 1u) * kTpThreads2) << 16;
+    } else {
+#pragma unroll
+        for (unsigned q = 0; q < kTpPerThread; ++q) {
+            const bool in = q * kTpThreads2 + t < n;
+            kk[q] = in ? __ldcs(kp + q * kTpThreads2) : 0xffffffffu;
+            const uint32_t v = in ? (uint32_t) __ldcs(vp + q * kTpThreads2) : 0u;
+            vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
+        }
+    }
+    if (t < 256u) {
+        sm.lb[t] = two.cnt[(std::size_t) blockIdx.x * 256u + t];
+        sm.gbase[t] = two.base[(std::size_t) blockIdx.x * 256u + t];
+    }
+    if (t == 0u) sm.dup = 0u;
+    const uint32_t w_first = __ldg(tmp_key + b) >> (LB + 5), w_last = __ldg(tmp_key + e - 1u) >> (LB + 5);
+    __syncthreads();
+    block_scan_small<1>(sm.lb, 256u, sm.scan33);
+    if (t < 256u) {
+        sm.fill[t] = sm.lb[t];
+        sm.gbase[t] -= sm.lb[t]; // global slot of staging slot 0
+    }
+    bool ballots = (w_last - w_first) / kTpSpanWords >= kTpRounds;
+    if (!ballots) {
+        for (uint32_t w0 = w_first; w0 <= w_last; w0 += kTpSpanWords) {
+            const uint32_t words = min(kTpSpanWords, w_last - w0 + 1u), k0 = w0 << (LB + 5);
+            for (uint32_t w = t; w < words * 64u; w += kTpThreads2)
+                reinterpret_cast<uint4 *>(sm.bits)[w] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+#pragma unroll
+            for (unsigned q = 0; q < kTpPerThread; ++q) {
+                const uint32_t x = kk[q] - k0; // no entry: past every span
+                if (x < kTpSpanKeys) atomicOr(sm.bits + (x >> 5), 1u << (x & 31u));
+            }
+            __syncthreads();
+            // two threads per column, each with half of the words: the prefix
+            // starts at the column's next staging slot
+            {
+                constexpr uint32_t kHalf = kTpSpanWords / 2u;
+                const uint32_t d = t >> 1, h = t & 1u;
+                uint32_t c[kHalf], sum = 0u;
+#pragma unroll
+                for (uint32_t w = 0; w < kHalf; ++w) {
+                    c[w] = h * kHalf + w < words ? __popc(sm.bits[(h * kHalf + w) * 256u + d]) : 0u;
+                    sum += c[w];
+                }
+                const uint32_t other = __shfl_xor_sync(0xffffffffu, sum, 1);
+                uint32_t run = sm.fill[d] + (h ? other : 0u);
+#pragma unroll
+                for (uint32_t w = 0; w < kHalf; ++w) {
+                    sm.pre[(h * kHalf + w) * 256u + d] = (uint16_t) run;
+                    run += c[w];
+                }
+                __syncwarp();
+                if (h) sm.fill[d] = run;
+            }
+            __syncthreads();
+#pragma unroll
+            for (unsigned q = 0; q < kTpPerThread; ++q) {
+                const uint32_t x = kk[q] - k0;
+                if (x < kTpSpanKeys) {
+                    const uint32_t lp = sm.pre[x >> 5] + __popc(sm.bits[x >> 5] & ((1u << (x & 31u)) - 1u));
+                    sm.key[lp] = kk[q]; // lp < n: the column's slots start at lb and hold its entries
+                    sm.val[lp] = (uint16_t) ((q & 1u) ? vv[q / 2u] >> 16 : vv[q / 2u]);
+                }
+            }
+            __syncthreads();
+        }
+        if (t < 256u && sm.fill[t] != sm.lb[t + 1u]) sm.dup = 1u;
+        __syncthreads();
+        ballots = sm.dup != 0u;
+    }
+    if (ballots) {
+        __syncthreads();
+        tp_stage sg;
+        sg.cnt = reinterpret_cast<uint16_t *>(sm.bits);
+        sg.bas = sg.cnt + kTpWarps2 * 256u;
+        sg.lb = sm.lb;
+        sg.fill = sm.fill;
+        if (t < 256u) sm.fill[t] = 0u;
+        for (uint32_t w = t; w < kTpWarps2 * 256u; w += kTpThreads2) sg.cnt[w] = 0u;
+        __syncthreads();
+        tp_rank_ballots<LB, kTpWarps2>(tmp_key, tmp_val, b, e, sg, sm.key, sm.val);
+        __syncthreads();
+    }
+#pragma unroll 4
+    for (uint32_t j = t; j < n; j += kTpThreads2) {
+        const uint32_t key = sm.key[j];
+        const uint32_t g = sm.gbase[tp_digit<LB>(key)] + j;
+        out_idx[g] = tp_payload<LB>(key);
+        out_val[g] = sm.val[j];
     }
 }
 
@@ -709,30 +975,30 @@ constexpr std::size_t tp_scatter2_smem(uint32_t low_bits) {
     return (std::size_t) kTpChunk * 6u + ((std::size_t) 2u * kTpWarps * 2u << low_bits);
 }
 
-// Chunks, counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).
-template <int LB>
+// Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).
+// kRows: the payloads of a bucket never decrease (the transpose's rows).
+template <int LB, bool kRows>
 int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
                    cudaStream_t stream) {
-    constexpr std::size_t smem = tp_scatter2_smem(LB);
-    auto s2 = tp_scatter2_kernel<LB>;
+    static_assert(!kRows || LB == (int) kTpBucketBits, "the row ranking has 256 digits");
+    constexpr std::size_t smem = kRows ? sizeof(tp_rows_smem) : tp_scatter2_smem(LB);
+    auto s2 = kRows ? tp_scatter2_rows_kernel : tp_scatter2_kernel<LB>;
     if (!cuda_ok(cudaFuncSetAttribute(s2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
                  "scatter2 smem attribute"))
         return 0;
-    tp_chunks_kernel<<<1, 1024, 0, stream>>>(l.hist1, l.tiles1, l.K, l.max_chunks, l.chunk_bucket, l.chunk_begin,
-                                             l.chunk_end, l.chunk_first);
-    if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_begin, l.chunk_end, l.max_chunks,
-                                                                 l.hist2);
+    tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_range, l.two.cnt);
     if (!launch_ok("tp_hist2_kernel")) return 0;
-    if (!scan_exclusive_u32(l.hist2, l.hist2, (std::size_t) l.max_chunks << LB, true, l.scan_tmp, l.scan_bytes,
-                            stream))
-        return 0;
-    tp_colcount_kernel<<<l.K, 256, 0, stream>>>(l.hist2, l.max_chunks, l.chunk_first, uDim, LB, out_ptr);
-    if (!launch_ok("tp_colcount_kernel")) return 0;
+    constexpr uint32_t D = 1u << LB;
+    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, l.slice_range, l.two.slices);
+    if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(l.two.slices, D, l.slice_first, 0u, uDim, out_ptr);
+    if (!launch_ok("tp_slice_scan_kernel")) return 0;
     if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
-    s2<<<l.max_chunks, kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_bucket, l.chunk_begin, l.chunk_end,
-                                                   l.chunk_first, l.max_chunks, l.hist2, out_ptr, uDim, out_idx,
-                                                   out_val);
+    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, l.slice_range, l.slice_bucket,
+                                                            l.two.slices, out_ptr, uDim, l.two.base);
+    if (!launch_ok("tp_slice_apply_kernel")) return 0;
+    s2<<<l.max_chunks, kRows ? kTpThreads2 : kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range, l.two,
+                                                                         out_idx, out_val);
     return launch_ok("tp_scatter2_kernel");
 }
 
@@ -746,12 +1012,20 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
                  "scatter1 smem attribute"))
         return 0;
     tp_hist1_kernel<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K,
-                                                                              l.tiles1, l.hist1, l.status);
+                                                                              l.one.cnt, l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
-    if (!scan_exclusive_u32(l.hist1, l.hist1, (std::size_t) l.K * l.tiles1, true, l.scan_tmp, l.scan_bytes, stream))
-        return 0;
-    s1<<<l.tiles1, kTpThreads, s1_smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.low_bits, l.K, l.tiles1, l.hist1,
-                                                  l.gran_row, pay, pay_map, l.tmp_key, l.tmp_val);
+    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, nullptr, l.one.slices);
+    if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(l.one.slices, l.K, nullptr, l.slices1, l.K,
+                                                                          l.total1);
+    if (!launch_ok("tp_slice_scan_kernel")) return 0;
+    tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
+    if (!launch_ok("tp_chunks_kernel")) return 0;
+    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, nullptr, nullptr, l.one.slices,
+                                                         l.start1, l.K, l.one.base);
+    if (!launch_ok("tp_slice_apply_kernel")) return 0;
+    s1<<<l.tiles1, kTpThreads, s1_smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.low_bits, l.K, l.one, l.gran_row,
+                                                  pay, pay_map, l.tmp_key, l.tmp_val);
     return launch_ok("tp_scatter1_kernel");
 }
 
@@ -761,7 +1035,9 @@ int transpose2_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t
     tp_gran_rows_kernel<<<(cDim + 255u) / 256u, 256, 0, stream>>>(ptr, cDim, l.gran_row);
     if (!launch_ok("tp_gran_rows_kernel")) return 0;
     return tp_first_pass<false>(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, l, stream) &&
-           tp_second_pass<(int) kTpBucketBits>(uDim, l, out_ptr, out_idx, out_val, stream);
+           ((double) nnz >= kTpRowsKernelMin * (double) cDim * (double) l.K
+                ? tp_second_pass<(int) kTpBucketBits, true>(uDim, l, out_ptr, out_idx, out_val, stream)
+                : tp_second_pass<(int) kTpBucketBits, false>(uDim, l, out_ptr, out_idx, out_val, stream));
 }
 
 uint32_t bits_below(uint64_t v) { // bits that hold 0 .. v - 1
@@ -856,10 +1132,10 @@ int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row
         !tp_first_pass<true>(0u, rows, n, nullptr, row, val, col, map, l, stream))
         return 0;
     switch (lb) {
-        case 8u: return tp_second_pass<8>(rows, l, out_ptr, out_col, out_val, stream);
-        case 9u: return tp_second_pass<9>(rows, l, out_ptr, out_col, out_val, stream);
-        case 10u: return tp_second_pass<10>(rows, l, out_ptr, out_col, out_val, stream);
-        default: return tp_second_pass<11>(rows, l, out_ptr, out_col, out_val, stream);
+        case 8u: return tp_second_pass<8, false>(rows, l, out_ptr, out_col, out_val, stream);
+        case 9u: return tp_second_pass<9, false>(rows, l, out_ptr, out_col, out_val, stream);
+        case 10u: return tp_second_pass<10, false>(rows, l, out_ptr, out_col, out_val, stream);
+        default: return tp_second_pass<11, false>(rows, l, out_ptr, out_col, out_val, stream);
     }
 }
 

@@ -1,0 +1,53 @@
+"""Transpose where the second pass ranks by rows: chunks that span one round of
+rows, several, and too many (ranked by ballots), chunks holding a repeated
+column, buckets that start off a vector boundary, the most buckets."""
+
+import numpy as np
+import pytest
+
+from cases import np_u16, np_u32, to_device_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(rows, cols, per_row, seed, repeat=0, unsorted=False):
+    rng = np.random.default_rng(seed)
+    n = rng.poisson(per_row, rows)
+    row = np.repeat(np.arange(rows), n)
+    col = rng.integers(0, cols, len(row))
+    key = np.unique(row.astype(np.int64) * cols + col)  # each cell once, columns ascending
+    row, col = (key // cols), (key % cols)
+    if repeat:
+        at = rng.choice(len(row), repeat, replace=False)
+        row, col = np.insert(row, at, row[at]), np.insert(col, at, col[at])
+    if unsorted:  # each row's columns in any order
+        p = np.lexsort((rng.random(len(row)), row))
+        row, col = row[p], col[p]
+    ptr = np.zeros(rows + 1, np.uint32)
+    np.cumsum(np.bincount(row, minlength=rows), out=ptr[1:])
+    return ptr, col.astype(np.uint32), rng.integers(1, 60000, len(col)).astype(np.uint16)
+
+
+@pytest.mark.parametrize("rows,cols,per_row,repeat,unsorted", [
+    (700, 300, 60, 0, False),          # one round
+    (6_000, 300, 9, 0, False),         # spans around the bitmap's 1,152 rows
+    (6_000, 300, 9, 40, False),        # with repeated columns in most chunks
+    (30_000, 300, 6.5, 0, True),       # two rounds, columns in any order; a sparse second bucket
+    (40_000, 256, 3.3, 0, False),      # three rounds
+    (40_000, 256, 3.3, 3, False),      # a repeated column in few chunks
+    (30_000, 300, 3, 3, True),         # too sparse for the row ranking
+    (60_000, 256, 0.5, 0, False),
+    (60_000, 777, 2, 5, True),         # more than one bucket, sparse, repeated
+    (1_153, 513, 30, 0, False),        # the span's edge, a bucket of one column
+    (40, 262_144, 3_000, 0, False),    # the most buckets, chunks far from full
+    (8_192, 1, 0.9, 0, False),         # one column
+])
+def test_transpose_ranks(cuda, orc, rows, cols, per_row, repeat, unsorted):
+    from cellshard_b200.device import transpose
+
+    ptr, idx, val = _csr(rows, cols, per_row, rows + cols, repeat, unsorted)
+    t = transpose(to_device_csr(rows, cols, ptr, idx, val))
+    rptr, ridx, rval = orc.csr_transpose(rows, cols, ptr, idx, val)
+    assert np.array_equal(np_u32(t.ptr), rptr)
+    assert np.array_equal(np_u32(t.idx), ridx)
+    assert np.array_equal(np_u16(t.val), rval)
