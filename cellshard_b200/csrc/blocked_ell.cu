@@ -5,7 +5,7 @@
 // blocks with epoch marks; :294-342 sorts them with qsort, maps block -> slot
 // and scatters values into a memset output).  Here:
 //
-//   shape   one warp per row block sets a shared-memory bitmap over column
+//   shape   one to eight warps per row block set a shared-memory bitmap over column
 //           blocks from the row block's contiguous CSR index range; popc gives
 //           the distinct count, atomicMax the global ell_width.  The bitmaps
 //           are kept in scratch for the emit pass.
@@ -28,7 +28,6 @@
 namespace csb {
 namespace {
 
-constexpr unsigned kShapeWarps = 4;
 constexpr unsigned kEmitThreads = 256;
 constexpr unsigned kSegHalves = 32768; // 64 KB row segment in shared memory
 
@@ -36,27 +35,39 @@ __device__ __forceinline__ uint32_t div_b(uint32_t c, uint32_t B, int shift) {
     return shift >= 0 ? (c >> shift) : (c / B);
 }
 
-__global__ void __launch_bounds__(kShapeWarps * 32) bell_shape_kernel(
+// WARPS warps per row block.  Bound by the latency of the column loads, so as
+// many vectors as possible are in flight: up to 8 per thread, and 8 warps on a
+// row block of thousands of entries (a warp per row block left 16 % of the
+// warp slots filled at 30,000 rows of 1,311 entries).
+template <unsigned WARPS>
+__global__ void __launch_bounds__(WARPS * 32) bell_shape_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, uint32_t rows, uint32_t cols, uint32_t nnz,
     uint32_t B, int shift, uint32_t row_blocks, uint32_t words, uint32_t *__restrict__ bitmaps,
     unsigned long long *__restrict__ shape, uint32_t *status) {
-    extern __shared__ uint32_t shape_smem[];
-    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint32_t *bits = shape_smem + (std::size_t) warp * words;
-    uint32_t local_max = 0u;
+    extern __shared__ uint32_t bits[]; // [words]
+    __shared__ uint32_t warp_count[WARPS];
+    constexpr uint32_t T = WARPS * 32u;
+    const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    uint32_t local_max = 0u; // thread 0
     unsigned long long local_total = 0ull;
     uint32_t bad = 0u;
-    for (uint32_t rb = blockIdx.x * kShapeWarps + warp; rb < row_blocks; rb += gridDim.x * kShapeWarps) {
-        for (uint32_t w = lane; w < words; w += 32u) bits[w] = 0u;
-        __syncwarp();
+    auto sync = [&]() {
+        if constexpr (WARPS == 1u)
+            __syncwarp();
+        else
+            __syncthreads();
+    };
+    for (uint32_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {
+        for (uint32_t w = t; w < words; w += T) bits[w] = 0u;
         const uint32_t r0 = rb * B;
         const uint32_t r1 = min(rows, r0 + B);
-        uint32_t ptr_bad = 0u;
-        for (uint32_t r = r0 + lane; r < r1; r += 32u) {
+        int ptr_bad = 0;
+        for (uint32_t r = r0 + t; r < r1; r += T) {
             const uint32_t a = ptr[r], b = ptr[r + 1u];
-            if (b < a || b > nnz) ptr_bad = 1u;
+            if (b < a || b > nnz) ptr_bad = 1;
         }
-        ptr_bad = __any_sync(0xffffffffu, ptr_bad);
+        ptr_bad = WARPS == 1u ? __any_sync(0xffffffffu, ptr_bad) : __syncthreads_or(ptr_bad);
+        if constexpr (WARPS == 1u) __syncwarp();
         if (ptr_bad) {
             bad |= CS_STATUS_BAD_POINTERS;
         } else {
@@ -72,7 +83,7 @@ __global__ void __launch_bounds__(kShapeWarps * 32) bell_shape_kernel(
             // scalar head to a 16-byte boundary, 16-byte body, scalar tail
             const bool vec = (reinterpret_cast<uintptr_t>(idx) & 15u) == 0u;
             const uint32_t head_end = vec ? min(e, (b + 3u) & ~3u) : e;
-            for (uint32_t i = b + lane; i < head_end; i += 32u) mark(idx[i]);
+            for (uint32_t i = b + t; i < head_end; i += T) mark(idx[i]);
             if (vec) {
                 const uint32_t nvec = (e - head_end) >> 2;
                 const uint4 *v4 = reinterpret_cast<const uint4 *>(idx + head_end);
@@ -97,39 +108,45 @@ __global__ void __launch_bounds__(kShapeWarps * 32) bell_shape_kernel(
                     }
                     if (m != 0u) atomicOr(bits + word, m);
                 };
-                // eight vectors per lane loaded before any is marked
+                // eight vectors per thread loaded before any is marked
                 constexpr unsigned kV = 8;
-                for (uint32_t k0 = lane; k0 < nvec; k0 += 32u * kV) {
+                for (uint32_t k0 = t; k0 < nvec; k0 += T * kV) {
                     uint4 q[kV];
 #pragma unroll
                     for (unsigned u = 0; u < kV; ++u) {
-                        const uint32_t k = k0 + 32u * u;
+                        const uint32_t k = k0 + T * u;
                         q[u] = k < nvec ? __ldg(v4 + k) : make_uint4(0u, 0u, 0u, 0u);
                     }
 #pragma unroll
                     for (unsigned u = 0; u < kV; ++u)
-                        if (k0 + 32u * u < nvec) mark4(q[u]);
+                        if (k0 + T * u < nvec) mark4(q[u]);
                 }
-                for (uint32_t i = head_end + (nvec << 2) + lane; i < e; i += 32u) mark(idx[i]);
+                for (uint32_t i = head_end + (nvec << 2) + t; i < e; i += T) mark(idx[i]);
             }
         }
-        __syncwarp();
+        sync();
         uint32_t cnt = 0u;
-        for (uint32_t w = lane; w < words; w += 32u) {
+        for (uint32_t w = t; w < words; w += T) {
             const uint32_t word = bits[w];
             cnt += __popc(word);
             if (bitmaps != nullptr) bitmaps[(std::size_t) rb * words + w] = word;
         }
         cnt = __reduce_add_sync(0xffffffffu, cnt);
-        local_max = max(local_max, cnt);
-        local_total += cnt;
-        __syncwarp();
+        if (lane == 0u) warp_count[warp] = cnt;
+        sync(); // also before the next row block clears the bitmap
+        if (t == 0u) {
+            uint32_t all = 0u;
+#pragma unroll
+            for (unsigned w = 0; w < WARPS; ++w) all += warp_count[w];
+            local_max = max(local_max, all);
+            local_total += all;
+        }
     }
     bad = __reduce_or_sync(0xffffffffu, bad);
-    if (lane == 0u) {
+    if (lane == 0u) status_or(status, bad);
+    if (t == 0u) {
         if (local_max != 0u) atomicMax(shape, (unsigned long long) local_max);
         if (local_total != 0ull) atomicAdd(shape + 1, local_total);
-        status_or(status, bad);
     }
 }
 
@@ -140,7 +157,8 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
     uint32_t *__restrict__ d_nnz, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char emit_smem[];
     uint16_t *buf = reinterpret_cast<uint16_t *>(emit_smem);                  // [kSegHalves]
-    uint2 *ix = reinterpret_cast<uint2 *>(emit_smem + kSegHalves * sizeof(uint16_t)); // [words]
+    uint32_t *seen = reinterpret_cast<uint32_t *>(buf + kSegHalves);          // [kSegHalves / 32]
+    uint2 *ix = reinterpret_cast<uint2 *>(seen + kSegHalves / 32u);           // [words]
     __shared__ uint32_t count_smem;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const bool vec_ok = ((ell_cols & 7u) == 0u) && ((reinterpret_cast<uintptr_t>(out_val) & 15u) == 0u);
@@ -184,7 +202,7 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
         }
         const uint32_t a = ptr[r], e = ptr[r + 1u];
         const bool ptr_bad = e < a || e > nnz;
-        // rows whose columns are not strictly increasing take the ordered path
+        // rows whose columns are not strictly increasing are checked for repeats
         int unordered = 0;
         if (!ptr_bad) {
             for (uint32_t i = a + threadIdx.x; i + 1u < e; i += blockDim.x)
@@ -203,25 +221,32 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
             }
             __syncthreads();
             if (!ptr_bad) {
-                if (!unordered) {
+                // cell of column c inside the segment, or seg_len where it has none
+                auto cell = [&](uint32_t c) -> uint32_t {
+                    if (c >= cols) return seg_len;
+                    const uint32_t bc = div_b(c, B, shift);
+                    const uint2 x = ix[bc >> 5];
+                    const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
+                    if (slot >= width) return seg_len;
+                    return min(slot * B + (c - bc * B) - seg0, seg_len);
+                };
+                for (uint32_t i = a + threadIdx.x; i < e; i += blockDim.x) {
+                    const uint32_t pos = cell(idx[i]);
+                    if (pos < seg_len) buf[pos] = val[i];
+                }
+                if (unordered) { // one bit per cell; a repeated cell keeps its last entry
+                    for (uint32_t k = threadIdx.x; k < kSegHalves / 32u; k += blockDim.x) seen[k] = 0u;
+                    __syncthreads();
+                    int repeated = 0;
                     for (uint32_t i = a + threadIdx.x; i < e; i += blockDim.x) {
-                        const uint32_t c = idx[i];
-                        if (c >= cols) continue;
-                        const uint32_t bc = div_b(c, B, shift);
-                        const uint2 x = ix[bc >> 5];
-                        const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
-                        const uint32_t pos = slot * B + (c - bc * B) - seg0;
-                        if (slot < width && pos < seg_len) buf[pos] = val[i];
+                        const uint32_t pos = cell(idx[i]), bit = 1u << (pos & 31u);
+                        if (pos < seg_len && (atomicOr(seen + (pos >> 5), bit) & bit)) repeated = 1;
                     }
-                } else if (threadIdx.x == 0) {
-                    for (uint32_t i = a; i < e; ++i) {
-                        const uint32_t c = idx[i];
-                        if (c >= cols) continue;
-                        const uint32_t bc = div_b(c, B, shift);
-                        const uint2 x = ix[bc >> 5];
-                        const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
-                        const uint32_t pos = slot * B + (c - bc * B) - seg0;
-                        if (slot < width && pos < seg_len) buf[pos] = val[i];
+                    if (__syncthreads_or(repeated) && threadIdx.x == 0) {
+                        for (uint32_t i = a; i < e; ++i) {
+                            const uint32_t pos = cell(idx[i]);
+                            if (pos < seg_len) buf[pos] = val[i];
+                        }
                     }
                 }
             } else {
@@ -257,15 +282,43 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
 }
 
 
-// Emit with shared-memory row staging and bulk (TMA) stores.  A CTA takes
-// whole row blocks (the block's column index is loaded once for its B rows)
-// and owns NBUF row buffers (~64 KB in total, three CTAs per SM): a row is
-// scattered into a zeroed buffer by the threads, then one thread hands the
-// whole padded row to the copy engine and the CTA moves on while it streams
-// out.  A buffer is re-zeroed only after the bulk store that read it has
-// finished reading.  A row whose columns are not strictly increasing marks
-// one bit per cell in `seen`; one that repeats a column is redone in CSR order
-// by one thread (the reference's overwrite order).
+// A row block's block columns (set bits in ascending order, invalid columns
+// after them), by the whole CTA.
+__device__ __forceinline__ void write_block_columns(const uint2 *ix, uint32_t words, uint32_t width, uint32_t count,
+                                                    uint32_t *__restrict__ row_bci) {
+    for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
+        uint32_t word = ix[w].x;
+        uint32_t pos = ix[w].y;
+        while (word != 0u) {
+            const uint32_t bit = __ffs(word) - 1u;
+            if (pos < width) row_bci[pos] = w * 32u + bit;
+            ++pos;
+            word &= word - 1u;
+        }
+    }
+    for (uint32_t s2 = count + threadIdx.x; s2 < width; s2 += blockDim.x) row_bci[s2] = CS_INVALID_COL;
+}
+
+// Emit with shared-memory row staging and bulk (TMA) stores, a CTA per row.  A
+// CTA takes whole row blocks (the block's column index is loaded once for its
+// B rows) and owns NBUF row buffers (~64 KB in total, three CTAs per SM): a
+// row is scattered into an all-zero buffer by the threads, then one thread
+// hands the whole padded row to the copy engine and the CTA moves on while it
+// streams out.  Bound by the write stream, which only runs while a CTA's
+// buffer is being read, so the time between two stores counts:
+// - a buffer is cleared by taking back the cells of the row it held (their
+//   positions stay in registers; 5 two-byte stores a thread instead of 16
+//   16-byte ones at 1,311 entries in 32,768 columns);
+// - a warp takes consecutive entries, so the check that columns ascend needs
+//   one load per warp and row from beyond its registers, and that load is
+//   issued with the row's prefetch.
+// 131,071 x 32,768 (9.6 GB moved): 1.70 ms, 1.89 before (whole buffers
+// re-zeroed, a dependent load per warp and 32 entries, five barriers a row).
+// Rows without entries take 1.41; asking the next row block into L2 ahead made
+// it slower (1.86), as did doing so by bulk prefetch.
+// A row whose columns are not strictly increasing marks one bit per cell in
+// `seen`; one that repeats a column is redone in CSR order by one thread (the
+// reference's overwrite order).
 template <int NBUF>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
@@ -273,7 +326,9 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci, uint16_t *__restrict__ out_val,
     uint32_t *__restrict__ d_nnz, uint32_t *status) {
     extern __shared__ __align__(128) unsigned char tma_smem[];
-    constexpr int PF = 8; // entries per thread prefetched for the next row
+    constexpr int PF = 8;                    // entries per thread prefetched for the next row
+    constexpr bool kTakeBack = NBUF <= 2;    // small rows: a few vector stores clear them
+    constexpr uint32_t kNone = 0xffffu;      // ell_cols <= kSegHalves < 0xffff
     const uint32_t row_bytes = ell_cols * 2u;
     const uint32_t stride = (row_bytes + 127u) & ~127u;
     uint2 *ix = reinterpret_cast<uint2 *>(tma_smem + (std::size_t) NBUF * stride);
@@ -286,15 +341,25 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     for (uint32_t k = threadIdx.x * 16u; k < NBUF * stride; k += blockDim.x * 16u)
         *reinterpret_cast<uint4 *>(tma_smem + k) = make_uint4(0u, 0u, 0u, 0u);
     uint32_t my_nnz = 0u, bad = 0u, iter = 0u;
-    uint32_t nc[PF];
+    uint32_t nc[PF], n_beyond; // the next row's entries; the one after the warp's last (lane 31)
     uint16_t nv[PF];
+    // positions of the rows that the NBUF buffers hold, newest first, and
+    // whether a row's cells are all among them
+    uint32_t held[kTakeBack ? NBUF : 1][PF / 2];
+    bool held_all[kTakeBack ? NBUF : 1];
+    // warp w's entries of a row of n: [w * 32 * nb, (w + 1) * 32 * nb), nb = batches per warp
+    auto batches = [&](uint32_t n) { return min((uint32_t) PF, (n + kEmitThreads - 1u) / kEmitThreads); };
     auto prefetch = [&](uint32_t a, uint32_t e) {
+        const uint32_t nb = batches(e - a), first = a + warp * nb * 32u + lane;
 #pragma unroll
         for (int k = 0; k < PF; ++k) {
-            const uint32_t i = a + threadIdx.x + (uint32_t) k * kEmitThreads;
-            nc[k] = i < e ? __ldg(idx + i) : 0xffffffffu;
-            nv[k] = i < e ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
+            const uint32_t i = first + (uint32_t) k * 32u;
+            const bool in = (uint32_t) k < nb && i < e;
+            nc[k] = in ? __ldg(idx + i) : 0xffffffffu;
+            nv[k] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
         }
+        const uint32_t beyond = a + (warp + 1u) * nb * 32u;
+        n_beyond = lane == 31u && beyond < e ? __ldg(idx + beyond) : 0xffffffffu;
     };
     for (uint32_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {
         const uint32_t r_beg = rb * B, r_end = min(rows, rb * B + B);
@@ -315,11 +380,215 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
         __syncthreads();
         const uint32_t count = count_smem;
         if (count > width) bad |= CS_STATUS_INDEX_RANGE;
-        if (out_bci != nullptr) {
+        {
+            const uint32_t a0 = rp[0], e0 = rp[1];
+            prefetch(a0, (e0 < a0 || e0 > nnz) ? a0 : e0);
+        }
+        if (out_bci != nullptr) write_block_columns(ix, words, width, count, out_bci + (std::size_t) rb * width);
+        for (uint32_t r = r_beg; r < r_end; ++r, ++iter) {
+            uint32_t cc[PF];
+            uint16_t cv[PF];
+#pragma unroll
+            for (int k = 0; k < PF; ++k) {
+                cc[k] = nc[k];
+                cv[k] = nv[k];
+            }
+            const uint32_t beyond = n_beyond;
+            const uint32_t a = rp[r - r_beg];
+            uint32_t e = rp[r - r_beg + 1u];
+            if (e < a || e > nnz) {
+                bad |= CS_STATUS_BAD_POINTERS;
+                e = a; // an empty row
+            }
+            const uint32_t n = e - a, nb = batches(n);
+            if (r + 1u < r_end) {
+                const uint32_t a1 = rp[r - r_beg + 1u], e1 = rp[r - r_beg + 2u];
+                prefetch(a1, (e1 < a1 || e1 > nnz) ? a1 : e1);
+            }
+            uint16_t *buf = reinterpret_cast<uint16_t *>(tma_smem + (std::size_t) (iter % NBUF) * stride);
+            if (iter >= (uint32_t) NBUF) {
+                if (threadIdx.x == 0) bulk_wait_read<NBUF - 1>();
+                __syncthreads();
+                if (kTakeBack && held_all[NBUF <= 2 ? NBUF - 1 : 0]) {
+#pragma unroll
+                    for (int k = 0; k < PF / 2; ++k) {
+                        const uint32_t pp = held[NBUF <= 2 ? NBUF - 1 : 0][k];
+                        if ((pp & 0xffffu) != kNone) buf[pp & 0xffffu] = 0u;
+                        if (pp >> 16 != kNone) buf[pp >> 16] = 0u;
+                    }
+                } else {
+                    for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
+                        *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                __syncthreads();
+            }
+            int unordered = 0;
+            uint32_t row_nnz = 0u;
+            // cell of column c, or kNone where it has none
+            auto cell = [&](uint32_t c) -> uint32_t {
+                if (c >= cols) return kNone;
+                const uint32_t bc = div_b(c, B, shift);
+                const uint2 x = ix[bc >> 5];
+                const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
+                return slot < width ? slot * B + (c - bc * B) : kNone;
+            };
+            auto place = [&](uint32_t c, uint16_t v) {
+                const uint32_t p = cell(c);
+                if (p != kNone) {
+                    buf[p] = v;
+                    row_nnz += half_nonzero(v);
+                }
+                return p;
+            };
+            uint32_t pos[PF / 2];
+#pragma unroll
+            for (int k = 0; k < PF / 2; ++k) pos[k] = kNone << 16 | kNone;
+            const uint32_t first = a + warp * nb * 32u + lane;
+#pragma unroll
+            for (int k = 0; k < PF; ++k) {
+                if ((uint32_t) k < nb) { // uniform
+                    const uint32_t i = first + (uint32_t) k * 32u;
+                    uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
+                    const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
+                    if (lane == 31u) nxt = (uint32_t) k + 1u < nb ? head : beyond;
+                    if (i < e) {
+                        if (i + 1u < e && cc[k] >= nxt) unordered = 1;
+                        const uint32_t p = place(cc[k], cv[k]);
+                        pos[k / 2] = (k & 1) ? (pos[k / 2] & 0xffffu) | p << 16 : (pos[k / 2] & 0xffff0000u) | p;
+                    }
+                }
+            }
+            for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) {
+                const uint32_t c = __ldg(idx + i);
+                if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
+                place(c, val[i]);
+            }
+            bool all_held = n <= PF * kEmitThreads;
+            fence_proxy_async_smem();
+            if (__syncthreads_or(unordered)) {
+                int repeated = 0;
+                for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
+                __syncthreads();
+                auto mark = [&](uint32_t p) {
+                    if (p == kNone) return;
+                    const uint32_t bit = 1u << (p & 31u);
+                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
+                };
+#pragma unroll
+                for (int k = 0; k < PF / 2; ++k) {
+                    mark(pos[k] & 0xffffu);
+                    mark(pos[k] >> 16);
+                }
+                for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) mark(cell(__ldg(idx + i)));
+                if (__syncthreads_or(repeated)) {
+                    if (threadIdx.x == 0) {
+                        for (uint32_t i = a; i < e; ++i) {
+                            const uint32_t p = cell(idx[i]);
+                            if (p != kNone) buf[p] = val[i];
+                        }
+                    }
+                    __syncthreads();
+                    row_nnz = 0u;
+                    for (uint32_t k = threadIdx.x; k < ell_cols; k += blockDim.x) row_nnz += half_nonzero(buf[k]);
+                    fence_proxy_async_smem();
+                    __syncthreads();
+                }
+            }
+            my_nnz += row_nnz;
+            if constexpr (kTakeBack) {
+#pragma unroll
+                for (int q = NBUF - 1; q > 0; --q) {
+                    held_all[q] = held_all[q - 1];
+#pragma unroll
+                    for (int k = 0; k < PF / 2; ++k) held[q][k] = held[q - 1][k];
+                }
+                held_all[0] = all_held;
+#pragma unroll
+                for (int k = 0; k < PF / 2; ++k) held[0][k] = pos[k];
+            }
+            if (threadIdx.x == 0) {
+                bulk_store_s2g(out_val + (std::size_t) r * ell_cols, buf, row_bytes);
+                bulk_commit();
+            }
+        }
+    }
+    if (threadIdx.x == 0) bulk_wait_all();
+    my_nnz = __reduce_add_sync(0xffffffffu, my_nnz);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (lane == 0u) {
+        if (my_nnz != 0u) atomicAdd(d_nnz, my_nnz);
+        status_or(status, bad);
+    }
+}
+
+// The same for rows of up to 8 KB, a warp per row: no CTA barrier, and
+// NBUF buffers per warp.  A warp takes `unit_rows` rows of one row block, fewer
+// than B where whole row blocks would leave warps idle.
+// 8,192 x 2,000 at 6 %: 31 us; 52 with a CTA per row (512 row blocks on 444
+// CTAs, five barriers a row).  100,000 x 2,000 at 1 %: 77 us against 353.
+constexpr unsigned kEmitWarps = kEmitThreads / 32;
+template <int NBUF>
+__global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
+    const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
+    uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
+    uint32_t unit_rows, const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci,
+    uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status) {
+    extern __shared__ __align__(128) unsigned char tma_smem[];
+    constexpr int PF = 8;
+    const uint32_t row_bytes = ell_cols * 2u;
+    const uint32_t stride = (row_bytes + 127u) & ~127u;
+    const uint32_t seen_words = (ell_cols + 31u) / 32u;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned char *bufs = tma_smem + (std::size_t) warp * NBUF * stride;
+    uint2 *ix = reinterpret_cast<uint2 *>(tma_smem + (std::size_t) kEmitWarps * NBUF * stride) + warp * words;
+    uint32_t *seen = reinterpret_cast<uint32_t *>(tma_smem + (std::size_t) kEmitWarps * NBUF * stride +
+                                                  (std::size_t) kEmitWarps * words * sizeof(uint2)) + warp * seen_words;
+    const uint32_t row_blocks = (rows + B - 1u) / B, per_block = (B + unit_rows - 1u) / unit_rows;
+    const uint64_t units = (uint64_t) row_blocks * per_block;
+    uint32_t my_nnz = 0u, bad = 0u, iter = 0u;
+    uint32_t nc[PF];
+    uint16_t nv[PF];
+    auto prefetch = [&](uint32_t a, uint32_t e) {
+#pragma unroll
+        for (int k = 0; k < PF; ++k) {
+            const uint32_t i = a + (uint32_t) k * 32u + lane;
+            nc[k] = i < e ? __ldg(idx + i) : 0xffffffffu;
+            nv[k] = i < e ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
+        }
+    };
+    for (uint64_t u = blockIdx.x * kEmitWarps + warp; u < units; u += (uint64_t) gridDim.x * kEmitWarps) {
+        const uint32_t rb = (uint32_t) (u / per_block), part = (uint32_t) (u % per_block);
+        const uint32_t b_end = min(rows, rb * B + B);
+        const uint32_t r_beg = min(b_end, rb * B + part * unit_rows), r_end = min(b_end, r_beg + unit_rows);
+        __syncwarp(); // the last unit's lookups are done
+        uint32_t count = 0u;
+        for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
+            const uint32_t w = w0 + lane;
+            const uint32_t word = w < words ? __ldg(bitmaps + (std::size_t) rb * words + w) : 0u;
+            const uint32_t c = __popc(word);
+            const uint32_t incl = warp_inclusive_scan(c);
+            if (w < words) ix[w] = make_uint2(word, count + incl - c);
+            count += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        __syncwarp();
+        if (count > width) bad |= CS_STATUS_INDEX_RANGE;
+        uint32_t a1 = 0u, e1 = 0u; // the next row's entries, bad pointers as an empty row
+        auto bounds = [&](uint32_t r) {
+            a1 = __ldg(ptr + r);
+            e1 = __ldg(ptr + r + 1u);
+            if (e1 < a1 || e1 > nnz) {
+                bad |= CS_STATUS_BAD_POINTERS;
+                e1 = a1;
+            }
+        };
+        if (r_beg < r_end) {
+            bounds(r_beg);
+            prefetch(a1, e1);
+        }
+        if (part == 0u && out_bci != nullptr) {
             uint32_t *row_bci = out_bci + (std::size_t) rb * width;
-            for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
-                uint32_t word = ix[w].x;
-                uint32_t pos = ix[w].y;
+            for (uint32_t w = lane; w < words; w += 32u) {
+                uint32_t word = ix[w].x, pos = ix[w].y;
                 while (word != 0u) {
                     const uint32_t bit = __ffs(word) - 1u;
                     if (pos < width) row_bci[pos] = w * 32u + bit;
@@ -327,11 +596,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                     word &= word - 1u;
                 }
             }
-            for (uint32_t s2 = count + threadIdx.x; s2 < width; s2 += blockDim.x) row_bci[s2] = CS_INVALID_COL;
-        }
-        {
-            const uint32_t a0 = rp[0], e0 = rp[1];
-            prefetch(a0, (e0 < a0 || e0 > nnz) ? a0 : e0);
+            for (uint32_t s2 = count + lane; s2 < width; s2 += 32u) row_bci[s2] = CS_INVALID_COL;
         }
         for (uint32_t r = r_beg; r < r_end; ++r, ++iter) {
             uint32_t cc[PF];
@@ -341,24 +606,19 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                 cc[k] = nc[k];
                 cv[k] = nv[k];
             }
-            const uint32_t a = rp[r - r_beg], e = rp[r - r_beg + 1u];
-            const bool ptr_bad = e < a || e > nnz;
-            if (ptr_bad) bad |= CS_STATUS_BAD_POINTERS;
+            const uint32_t a = a1, e = e1;
             if (r + 1u < r_end) {
-                const uint32_t a1 = rp[r - r_beg + 1u], e1 = rp[r - r_beg + 2u];
-                prefetch(a1, (e1 < a1 || e1 > nnz) ? a1 : e1);
+                bounds(r + 1u);
+                prefetch(a1, e1);
             }
-            uint16_t *buf = reinterpret_cast<uint16_t *>(tma_smem + (std::size_t) (iter % NBUF) * stride);
-            if (iter >= (uint32_t) NBUF) {
-                if (threadIdx.x == 0) bulk_wait_read<NBUF - 1>();
-                __syncthreads();
-                for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
-                    *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
-                __syncthreads();
-            }
+            uint16_t *buf = reinterpret_cast<uint16_t *>(bufs + (std::size_t) (iter % NBUF) * stride);
+            if (lane == 0u && iter >= (uint32_t) NBUF) bulk_wait_read<NBUF - 1>();
+            __syncwarp();
+            for (uint32_t k = lane * 8u; k < ell_cols; k += 256u)
+                *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
+            __syncwarp();
             int unordered = 0;
             uint32_t row_nnz = 0u;
-            // cell of column c, or 0xffffffff where it has none
             auto cell = [&](uint32_t c) -> uint32_t {
                 if (c >= cols) return 0xffffffffu;
                 const uint32_t bc = div_b(c, B, shift);
@@ -372,64 +632,54 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                 buf[p] = v;
                 row_nnz += half_nonzero(v);
             };
-            if (!ptr_bad) {
 #pragma unroll
-                for (int k = 0; k < PF; ++k) {
-                    const uint32_t i = a + threadIdx.x + (uint32_t) k * kEmitThreads;
-                    // the next entry belongs to the next lane (or, for lane 31, the next warp)
+            for (int k = 0; k < PF; ++k) {
+                if (a + (uint32_t) k * 32u < e) { // uniform
+                    const uint32_t i = a + (uint32_t) k * 32u + lane;
                     uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
-                    if (lane == 31u && i + 1u < e) nxt = __ldg(idx + i + 1u);
+                    const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
+                    if (lane == 31u) nxt = k + 1 < PF ? head : (i + 1u < e ? __ldg(idx + i + 1u) : 0u);
                     if (i < e) {
                         if (i + 1u < e && cc[k] >= nxt) unordered = 1;
                         place(cc[k], cv[k]);
                     }
                 }
-                for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) {
-                    const uint32_t c = __ldg(idx + i);
-                    if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
-                    place(c, val[i]);
+            }
+            for (uint32_t i = a + PF * 32u + lane; i < e; i += 32u) {
+                const uint32_t c = __ldg(idx + i);
+                if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
+                place(c, val[i]);
+            }
+            if (__any_sync(0xffffffffu, unordered)) {
+                int repeated = 0;
+                for (uint32_t k = lane; k < seen_words; k += 32u) seen[k] = 0u;
+                __syncwarp();
+                for (uint32_t i = a + lane; i < e; i += 32u) {
+                    const uint32_t p = cell(__ldg(idx + i)), bit = 1u << (p & 31u);
+                    if (p != 0xffffffffu && (atomicOr(seen + (p >> 5), bit) & bit)) repeated = 1;
                 }
-            }
-            int repeated = 0;
-            if (__syncthreads_or(unordered)) {
-                for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
-                __syncthreads();
-                auto mark = [&](uint32_t c) {
-                    const uint32_t p = cell(c);
-                    if (p == 0xffffffffu) return;
-                    const uint32_t bit = 1u << (p & 31u);
-                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
-                };
-#pragma unroll
-                for (int k = 0; k < PF; ++k)
-                    if (a + threadIdx.x + (uint32_t) k * kEmitThreads < e) mark(cc[k]);
-                for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) mark(__ldg(idx + i));
-                repeated = __syncthreads_or(repeated);
-            }
-            if (repeated) {
-                for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
-                    *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    for (uint32_t i = a; i < e; ++i) {
-                        const uint32_t p = cell(idx[i]);
-                        if (p != 0xffffffffu) buf[p] = val[i];
+                if (__any_sync(0xffffffffu, repeated)) {
+                    if (lane == 0u) {
+                        for (uint32_t i = a; i < e; ++i) {
+                            const uint32_t p = cell(idx[i]);
+                            if (p != 0xffffffffu) buf[p] = val[i];
+                        }
                     }
+                    __syncwarp();
+                    row_nnz = 0u;
+                    for (uint32_t k = lane; k < ell_cols; k += 32u) row_nnz += half_nonzero(buf[k]);
                 }
-                __syncthreads();
-                row_nnz = 0u;
-                for (uint32_t k = threadIdx.x; k < ell_cols; k += blockDim.x) row_nnz += half_nonzero(buf[k]);
             }
             my_nnz += row_nnz;
             fence_proxy_async_smem();
-            __syncthreads();
-            if (threadIdx.x == 0) {
+            __syncwarp();
+            if (lane == 0u) {
                 bulk_store_s2g(out_val + (std::size_t) r * ell_cols, buf, row_bytes);
                 bulk_commit();
             }
         }
     }
-    if (threadIdx.x == 0) bulk_wait_all();
+    if (lane == 0u) bulk_wait_all();
     my_nnz = __reduce_add_sync(0xffffffffu, my_nnz);
     bad = __reduce_or_sync(0xffffffffu, bad);
     if (lane == 0u) {
@@ -483,18 +733,21 @@ int blocked_ell_shape_launch(const cs_compressed_view *src, uint32_t B, uint64_t
     const uint32_t row_blocks = (src->rows + B - 1u) / B;
     const uint32_t words = col_words(src->cols, B);
     if (row_blocks == 0u || words == 0u) return 1;
-    const std::size_t smem = (std::size_t) kShapeWarps * words * sizeof(uint32_t);
-    if (smem > 48u * 1024u &&
-        !cuda_ok(cudaFuncSetAttribute(bell_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                 "bell_shape smem attribute"))
-        return 0;
-    uint32_t grid = (row_blocks + kShapeWarps - 1u) / kShapeWarps;
-    const uint32_t cap = (uint32_t) sm_count() * 32u;
-    if (grid > cap) grid = cap;
-    bell_shape_kernel<<<grid, kShapeWarps * 32, smem, stream>>>(
-        src->majorPtr, src->minorIdx, src->rows, src->cols, src->nnz, B, pow2_shift(B), row_blocks, words, bitmaps,
-        reinterpret_cast<unsigned long long *>(d_shape), d_status);
-    return launch_ok("bell_shape_kernel");
+    const std::size_t smem = (std::size_t) words * sizeof(uint32_t);
+    auto launch = [&](auto kern, unsigned warps) {
+        const unsigned grid = resident_grid((const void *) kern, warps * 32u, smem, row_blocks);
+        kern<<<grid, warps * 32u, smem, stream>>>(src->majorPtr, src->minorIdx, src->rows, src->cols, src->nnz, B,
+                                                  pow2_shift(B), row_blocks, words, bitmaps,
+                                                  reinterpret_cast<unsigned long long *>(d_shape), d_status);
+        return launch_ok("bell_shape_kernel");
+    };
+    // short row blocks keep one warp busy; longer ones take four, or eight where
+    // there are too few row blocks to fill the device otherwise (us by 1 / 4 / 8
+    // warps: 6,250 row blocks of 320 entries 15 / 19 / 34, of 1,920 entries
+    // 31 / 28 / 42; 8,192 of 21,000 222 / 194 / 204; 1,875 of them 116 / 68 / 61)
+    if (src->nnz / row_blocks <= 1024u) return launch(bell_shape_kernel<1>, 1u);
+    if (row_blocks > 4096u) return launch(bell_shape_kernel<4>, 4u);
+    return launch(bell_shape_kernel<8>, 8u);
 }
 
 int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
@@ -508,13 +761,42 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
     const std::size_t stride = (row_bytes + 127u) & ~(std::size_t) 127u;
     const bool tma_ok = (dst->ell_cols % 8u) == 0u && (reinterpret_cast<uintptr_t>(dst->val) & 15u) == 0u &&
                         dst->ell_cols <= kSegHalves;
+    const uint32_t row_blocks = (uint32_t) (((uint64_t) src->rows + B - 1u) / B);
+    const std::size_t seen_bytes = ((dst->ell_cols + 31u) / 32u) * sizeof(uint32_t);
+    const std::size_t kSmem = 75u * 1024u; // three CTAs per SM
+    if (tma_ok && stride <= 8192u) {
+        const int nbuf = stride <= 2048u ? 4 : (stride <= 4096u ? 2 : 1);
+        const std::size_t wsmem =
+            kEmitWarps * ((std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) + seen_bytes);
+        if (wsmem <= kSmem) {
+            // rows of a row block stay together while that gives every warp two units
+            const uint32_t warps = (uint32_t) sm_count() * 3u * kEmitWarps;
+            uint32_t unit_rows = B;
+            while (unit_rows > 1u && (uint64_t) row_blocks * ((B + unit_rows - 1u) / unit_rows) < 2u * (uint64_t) warps)
+                unit_rows = (unit_rows + 1u) / 2u;
+            const uint64_t units = (uint64_t) row_blocks * ((B + unit_rows - 1u) / unit_rows);
+            uint32_t grid = (uint32_t) sm_count() * 3u;
+            if (grid > (units + kEmitWarps - 1u) / kEmitWarps) grid = (uint32_t) ((units + kEmitWarps - 1u) / kEmitWarps);
+            auto launch = [&](auto kern) {
+                if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) wsmem),
+                             "bell_emit_warp smem attribute"))
+                    return 0;
+                kern<<<grid, kEmitThreads, wsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
+                                                            src->cols, src->nnz, B, pow2_shift(B), words, width,
+                                                            dst->ell_cols, unit_rows, bitmaps, dst->blockColIdx,
+                                                            dst->val, d_nnz, d_status);
+                return launch_ok("bell_emit_warp_kernel");
+            };
+            if (nbuf == 4) return launch(bell_emit_warp_kernel<4>);
+            if (nbuf == 2) return launch(bell_emit_warp_kernel<2>);
+            return launch(bell_emit_warp_kernel<1>);
+        }
+    }
     if (tma_ok) {
         const int nbuf = stride <= 8192u ? 8 : (stride <= 16384u ? 4 : (stride <= 32768u ? 2 : 1));
-        const std::size_t tsmem =
-            (std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) +
-            ((dst->ell_cols + 31u) / 32u + (std::size_t) B + 1u) * 4u;
-        if (tsmem <= 75u * 1024u) { // three CTAs per SM
-            const uint32_t row_blocks = (src->rows + B - 1u) / B;
+        const std::size_t tsmem = (std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) + seen_bytes +
+                                  ((std::size_t) B + 1u) * 4u;
+        if (tsmem <= kSmem) {
             uint32_t tgrid = (uint32_t) sm_count() * 3u;
             if (tgrid > row_blocks) tgrid = row_blocks;
             auto launch = [&](auto kern) {
@@ -533,7 +815,8 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
             return launch(bell_emit_tma_kernel<1>);
         }
     }
-    const std::size_t smem = (std::size_t) kSegHalves * sizeof(uint16_t) + (std::size_t) words * sizeof(uint2);
+    const std::size_t smem = (std::size_t) kSegHalves * sizeof(uint16_t) + kSegHalves / 8u +
+                             (std::size_t) words * sizeof(uint2);
     if (!cuda_ok(cudaFuncSetAttribute(bell_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
                  "bell_emit smem attribute"))
         return 0;

@@ -62,8 +62,12 @@ def test_shuffled_coo(cuda, orc, rows, cols, n, block, hot, repeat, remap):
     assert counts == [ref["nnz_host"], ref["nnz_gpu"]]
 
 
-@pytest.mark.parametrize("cols,block,repeat", [(500, 8, False), (9_000, 16, False), (9_000, 16, True),
-                                               (32_768, 16, True), (32_768, 2, False)])
+@pytest.mark.parametrize("cols,block,repeat", [
+    (500, 8, False), (500, 8, True), (1_100, 24, True), (2_100, 16, False), (4_096, 16, True),  # a warp per row
+    (4_104, 8, True), (9_000, 16, False), (9_000, 16, True), (16_384, 32, True),               # a CTA per row
+    (32_768, 16, True), (32_768, 2, False),                                                    # one row buffer
+    (333, 3, True), (40_000, 16, True),                                                        # no bulk stores
+])
 def test_csr_rows_in_any_column_order(cuda, orc, cols, block, repeat):
     from cellshard_b200.device import blocked_ell_from_csr
 
@@ -71,6 +75,7 @@ def test_csr_rows_in_any_column_order(cuda, orc, cols, block, repeat):
     rows = 37
     parts = []
     for r in range(rows):
+        # full row blocks of every kind: some rows past the 2,048 entries that registers hold
         c = rng.permutation(cols)[:int(rng.integers(0, min(cols, 5_000)))]
         if r % 3 == 0:
             c = np.sort(c)
