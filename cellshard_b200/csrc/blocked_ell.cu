@@ -31,6 +31,17 @@ namespace {
 constexpr unsigned kEmitThreads = 256;
 constexpr unsigned kSegHalves = 32768; // 64 KB row segment in shared memory
 
+// How an emit treats rows out of column order.  Default: checked row by row, a
+// repeated column keeps its last value.  With a flag, all rows come in any
+// order, and either (first) a repeated column only sets the flag, or (second)
+// the emit runs only where the flag is set.
+struct emit_order {
+    uint32_t *flag;
+    bool first;
+    __device__ __forceinline__ bool skips() const { return flag != nullptr && !first && *flag == 0u; }
+    __device__ __forceinline__ bool flag_repeats() const { return flag != nullptr && first; }
+};
+
 __device__ __forceinline__ uint32_t div_b(uint32_t c, uint32_t B, int shift) {
     return shift >= 0 ? (c >> shift) : (c / B);
 }
@@ -154,7 +165,8 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci, uint16_t *__restrict__ out_val,
-    uint32_t *__restrict__ d_nnz, uint32_t *status) {
+    uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
+    if (order.skips()) return;
     extern __shared__ __align__(16) unsigned char emit_smem[];
     uint16_t *buf = reinterpret_cast<uint16_t *>(emit_smem);                  // [kSegHalves]
     uint32_t *seen = reinterpret_cast<uint32_t *>(buf + kSegHalves);          // [kSegHalves / 32]
@@ -243,7 +255,8 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
                         if (pos < seg_len && (atomicOr(seen + (pos >> 5), bit) & bit)) repeated = 1;
                     }
                     if (__syncthreads_or(repeated) && threadIdx.x == 0) {
-                        for (uint32_t i = a; i < e; ++i) {
+                        if (order.flag_repeats()) atomicOr(order.flag, 1u);
+                        for (uint32_t i = a; i < e && !order.flag_repeats(); ++i) {
                             const uint32_t pos = cell(idx[i]);
                             if (pos < seg_len) buf[pos] = val[i];
                         }
@@ -319,12 +332,15 @@ __device__ __forceinline__ void write_block_columns(const uint2 *ix, uint32_t wo
 // A row whose columns are not strictly increasing marks one bit per cell in
 // `seen`; one that repeats a column is redone in CSR order by one thread (the
 // reference's overwrite order).
-template <int NBUF>
+// kAny (rows in any column order, as the COO partition leaves them): every row
+// marks its cells while it places them, with no order check.
+template <int NBUF, bool kAny>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci, uint16_t *__restrict__ out_val,
-    uint32_t *__restrict__ d_nnz, uint32_t *status) {
+    uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
+    if (kAny && order.skips()) return;
     extern __shared__ __align__(128) unsigned char tma_smem[];
     constexpr int PF = 8;                    // entries per thread prefetched for the next row
     constexpr bool kTakeBack = NBUF <= 2;    // small rows: a few vector stores clear them
@@ -341,7 +357,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     for (uint32_t k = threadIdx.x * 16u; k < NBUF * stride; k += blockDim.x * 16u)
         *reinterpret_cast<uint4 *>(tma_smem + k) = make_uint4(0u, 0u, 0u, 0u);
     uint32_t my_nnz = 0u, bad = 0u, iter = 0u;
-    uint32_t nc[PF], n_beyond; // the next row's entries; the one after the warp's last (lane 31)
+    uint32_t nc[PF], n_beyond = 0u; // the next row's entries; the one after the warp's last (lane 31)
     uint16_t nv[PF];
     // positions of the rows that the NBUF buffers hold, newest first, and
     // whether a row's cells are all among them
@@ -358,8 +374,10 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             nc[k] = in ? __ldg(idx + i) : 0xffffffffu;
             nv[k] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
         }
-        const uint32_t beyond = a + (warp + 1u) * nb * 32u;
-        n_beyond = lane == 31u && beyond < e ? __ldg(idx + beyond) : 0xffffffffu;
+        if constexpr (!kAny) {
+            const uint32_t beyond = a + (warp + 1u) * nb * 32u;
+            n_beyond = lane == 31u && beyond < e ? __ldg(idx + beyond) : 0xffffffffu;
+        }
     };
     for (uint32_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {
         const uint32_t r_beg = rb * B, r_end = min(rows, rb * B + B);
@@ -420,9 +438,13 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                     for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
                         *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
                 }
+                if constexpr (!kAny) __syncthreads();
+            }
+            if constexpr (kAny) {
+                for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
                 __syncthreads();
             }
-            int unordered = 0;
+            int unordered = 0, repeated = 0;
             uint32_t row_nnz = 0u;
             // cell of column c, or kNone where it has none
             auto cell = [&](uint32_t c) -> uint32_t {
@@ -432,9 +454,15 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                 const uint32_t slot = x.y + __popc(x.x & ((1u << (bc & 31u)) - 1u));
                 return slot < width ? slot * B + (c - bc * B) : kNone;
             };
+            auto mark = [&](uint32_t p) {
+                if (p == kNone) return;
+                const uint32_t bit = 1u << (p & 31u);
+                if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
+            };
             auto place = [&](uint32_t c, uint16_t v) {
                 const uint32_t p = cell(c);
                 if (p != kNone) {
+                    if constexpr (kAny) mark(p);
                     buf[p] = v;
                     row_nnz += half_nonzero(v);
                 }
@@ -448,11 +476,13 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             for (int k = 0; k < PF; ++k) {
                 if ((uint32_t) k < nb) { // uniform
                     const uint32_t i = first + (uint32_t) k * 32u;
-                    uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
-                    const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
-                    if (lane == 31u) nxt = (uint32_t) k + 1u < nb ? head : beyond;
-                    if (i < e) {
+                    if constexpr (!kAny) {
+                        uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
+                        const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
+                        if (lane == 31u) nxt = (uint32_t) k + 1u < nb ? head : beyond;
                         if (i + 1u < e && cc[k] >= nxt) unordered = 1;
+                    }
+                    if (i < e) {
                         const uint32_t p = place(cc[k], cv[k]);
                         pos[k / 2] = (k & 1) ? (pos[k / 2] & 0xffffu) | p << 16 : (pos[k / 2] & 0xffff0000u) | p;
                     }
@@ -460,39 +490,38 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             }
             for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) {
                 const uint32_t c = __ldg(idx + i);
-                if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
+                if (!kAny && i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
                 place(c, val[i]);
             }
             bool all_held = n <= PF * kEmitThreads;
             fence_proxy_async_smem();
-            if (__syncthreads_or(unordered)) {
-                int repeated = 0;
+            if constexpr (kAny) {
+                repeated = __syncthreads_or(repeated);
+            } else if (__syncthreads_or(unordered)) {
                 for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
                 __syncthreads();
-                auto mark = [&](uint32_t p) {
-                    if (p == kNone) return;
-                    const uint32_t bit = 1u << (p & 31u);
-                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
-                };
 #pragma unroll
                 for (int k = 0; k < PF / 2; ++k) {
                     mark(pos[k] & 0xffffu);
                     mark(pos[k] >> 16);
                 }
                 for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) mark(cell(__ldg(idx + i)));
-                if (__syncthreads_or(repeated)) {
-                    if (threadIdx.x == 0) {
-                        for (uint32_t i = a; i < e; ++i) {
-                            const uint32_t p = cell(idx[i]);
-                            if (p != kNone) buf[p] = val[i];
-                        }
+                repeated = __syncthreads_or(repeated);
+            }
+            if (kAny && order.first) {
+                if (repeated && threadIdx.x == 0) atomicOr(order.flag, 1u);
+            } else if (repeated) {
+                if (threadIdx.x == 0) {
+                    for (uint32_t i = a; i < e; ++i) {
+                        const uint32_t p = cell(idx[i]);
+                        if (p != kNone) buf[p] = val[i];
                     }
-                    __syncthreads();
-                    row_nnz = 0u;
-                    for (uint32_t k = threadIdx.x; k < ell_cols; k += blockDim.x) row_nnz += half_nonzero(buf[k]);
-                    fence_proxy_async_smem();
-                    __syncthreads();
                 }
+                __syncthreads();
+                row_nnz = 0u;
+                for (uint32_t k = threadIdx.x; k < ell_cols; k += blockDim.x) row_nnz += half_nonzero(buf[k]);
+                fence_proxy_async_smem();
+                __syncthreads();
             }
             my_nnz += row_nnz;
             if constexpr (kTakeBack) {
@@ -527,12 +556,13 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
 // 8,192 x 2,000 at 6 %: 31 us; 52 with a CTA per row (512 row blocks on 444
 // CTAs, five barriers a row).  100,000 x 2,000 at 1 %: 77 us against 353.
 constexpr unsigned kEmitWarps = kEmitThreads / 32;
-template <int NBUF>
+template <int NBUF, bool kAny>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     uint32_t unit_rows, const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci,
-    uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status) {
+    uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
+    if (kAny && order.skips()) return;
     extern __shared__ __align__(128) unsigned char tma_smem[];
     constexpr int PF = 8;
     const uint32_t row_bytes = ell_cols * 2u;
@@ -616,8 +646,10 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             __syncwarp();
             for (uint32_t k = lane * 8u; k < ell_cols; k += 256u)
                 *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
+            if constexpr (kAny)
+                for (uint32_t k = lane; k < seen_words; k += 32u) seen[k] = 0u;
             __syncwarp();
-            int unordered = 0;
+            int unordered = 0, repeated = 0;
             uint32_t row_nnz = 0u;
             auto cell = [&](uint32_t c) -> uint32_t {
                 if (c >= cols) return 0xffffffffu;
@@ -629,6 +661,10 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             auto place = [&](uint32_t c, uint16_t v) {
                 const uint32_t p = cell(c);
                 if (p == 0xffffffffu) return;
+                if constexpr (kAny) {
+                    const uint32_t bit = 1u << (p & 31u);
+                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
+                }
                 buf[p] = v;
                 row_nnz += half_nonzero(v);
             };
@@ -636,39 +672,42 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             for (int k = 0; k < PF; ++k) {
                 if (a + (uint32_t) k * 32u < e) { // uniform
                     const uint32_t i = a + (uint32_t) k * 32u + lane;
-                    uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
-                    const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
-                    if (lane == 31u) nxt = k + 1 < PF ? head : (i + 1u < e ? __ldg(idx + i + 1u) : 0u);
-                    if (i < e) {
+                    if constexpr (!kAny) {
+                        uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
+                        const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
+                        if (lane == 31u) nxt = k + 1 < PF ? head : (i + 1u < e ? __ldg(idx + i + 1u) : 0u);
                         if (i + 1u < e && cc[k] >= nxt) unordered = 1;
-                        place(cc[k], cv[k]);
                     }
+                    if (i < e) place(cc[k], cv[k]);
                 }
             }
             for (uint32_t i = a + PF * 32u + lane; i < e; i += 32u) {
                 const uint32_t c = __ldg(idx + i);
-                if (i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
+                if (!kAny && i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
                 place(c, val[i]);
             }
-            if (__any_sync(0xffffffffu, unordered)) {
-                int repeated = 0;
+            if (!kAny && __any_sync(0xffffffffu, unordered)) {
                 for (uint32_t k = lane; k < seen_words; k += 32u) seen[k] = 0u;
                 __syncwarp();
                 for (uint32_t i = a + lane; i < e; i += 32u) {
                     const uint32_t p = cell(__ldg(idx + i)), bit = 1u << (p & 31u);
                     if (p != 0xffffffffu && (atomicOr(seen + (p >> 5), bit) & bit)) repeated = 1;
                 }
-                if (__any_sync(0xffffffffu, repeated)) {
-                    if (lane == 0u) {
-                        for (uint32_t i = a; i < e; ++i) {
-                            const uint32_t p = cell(idx[i]);
-                            if (p != 0xffffffffu) buf[p] = val[i];
-                        }
+            }
+            repeated = __any_sync(0xffffffffu, repeated);
+            if (kAny && order.first) {
+                if (repeated && lane == 0u) atomicOr(order.flag, 1u);
+            } else if (repeated) {
+                __syncwarp();
+                if (lane == 0u) {
+                    for (uint32_t i = a; i < e; ++i) {
+                        const uint32_t p = cell(idx[i]);
+                        if (p != 0xffffffffu) buf[p] = val[i];
                     }
-                    __syncwarp();
-                    row_nnz = 0u;
-                    for (uint32_t k = lane; k < ell_cols; k += 32u) row_nnz += half_nonzero(buf[k]);
                 }
+                __syncwarp();
+                row_nnz = 0u;
+                for (uint32_t k = lane; k < ell_cols; k += 32u) row_nnz += half_nonzero(buf[k]);
             }
             my_nnz += row_nnz;
             fence_proxy_async_smem();
@@ -750,8 +789,10 @@ int blocked_ell_shape_launch(const cs_compressed_view *src, uint32_t B, uint64_t
     return launch(bell_shape_kernel<8>, 8u);
 }
 
-int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
-                            const uint32_t *bitmaps, uint32_t *d_status, cudaStream_t stream) {
+namespace {
+template <bool kAny>
+int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
+                const uint32_t *bitmaps, uint32_t *d_status, const emit_order order, cudaStream_t stream) {
     const uint32_t B = dst->block_size;
     const uint32_t words = col_words(src->cols, B);
     const uint32_t width = dst->ell_cols / B;
@@ -784,12 +825,12 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
                 kern<<<grid, kEmitThreads, wsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                             src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                             dst->ell_cols, unit_rows, bitmaps, dst->blockColIdx,
-                                                            dst->val, d_nnz, d_status);
+                                                            dst->val, d_nnz, d_status, order);
                 return launch_ok("bell_emit_warp_kernel");
             };
-            if (nbuf == 4) return launch(bell_emit_warp_kernel<4>);
-            if (nbuf == 2) return launch(bell_emit_warp_kernel<2>);
-            return launch(bell_emit_warp_kernel<1>);
+            if (nbuf == 4) return launch(bell_emit_warp_kernel<4, kAny>);
+            if (nbuf == 2) return launch(bell_emit_warp_kernel<2, kAny>);
+            return launch(bell_emit_warp_kernel<1, kAny>);
         }
     }
     if (tma_ok) {
@@ -806,13 +847,13 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
                 kern<<<tgrid, kEmitThreads, tsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                               src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                               dst->ell_cols, bitmaps, dst->blockColIdx, dst->val,
-                                                              d_nnz, d_status);
+                                                              d_nnz, d_status, order);
                 return launch_ok("bell_emit_tma_kernel");
             };
-            if (nbuf == 8) return launch(bell_emit_tma_kernel<8>);
-            if (nbuf == 4) return launch(bell_emit_tma_kernel<4>);
-            if (nbuf == 2) return launch(bell_emit_tma_kernel<2>);
-            return launch(bell_emit_tma_kernel<1>);
+            if (nbuf == 8) return launch(bell_emit_tma_kernel<8, kAny>);
+            if (nbuf == 4) return launch(bell_emit_tma_kernel<4, kAny>);
+            if (nbuf == 2) return launch(bell_emit_tma_kernel<2, kAny>);
+            return launch(bell_emit_tma_kernel<1, kAny>);
         }
     }
     const std::size_t smem = (std::size_t) kSegHalves * sizeof(uint16_t) + kSegHalves / 8u +
@@ -826,8 +867,19 @@ int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_
     bell_emit_kernel<<<grid, kEmitThreads, smem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                            src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                            dst->ell_cols, bitmaps, dst->blockColIdx, dst->val, d_nnz,
-                                                           d_status);
+                                                           d_status, order);
     return launch_ok("bell_emit_kernel");
+}
+} // namespace
+
+int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
+                            const uint32_t *bitmaps, uint32_t *d_status, cudaStream_t stream) {
+    return emit_launch<false>(src, dst, d_nnz, bitmaps, d_status, emit_order{nullptr, false}, stream);
+}
+
+int blocked_ell_emit_any_order(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
+                               const uint32_t *bitmaps, uint32_t *flag, bool flag_repeats, cudaStream_t stream) {
+    return emit_launch<true>(src, dst, d_nnz, bitmaps, nullptr, emit_order{flag, flag_repeats}, stream);
 }
 
 // ---------------------------------------------------------------------------

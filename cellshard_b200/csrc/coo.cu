@@ -9,15 +9,17 @@
 // Here, when every mapped column is below `cols` (and the column-block
 // bitmaps of the CSR kernels stay small), the CSR route: entries whose rows
 // never decrease -- COO written row by row -- get row pointers from their row
-// runs; other entries are put in row order by the two counting-sort passes of
-// the transpose (partition_rows: 8-byte entries in runs, a row's entries
-// keeping their COO order); then the library's CSR -> Blocked-ELL shape and
-// emit, which place a row's values whatever the order of its columns (a
-// repeated column keeps its last value) and count nnz the same way.  The
+// runs; other entries are put by rows in two counting-sort passes
+// (partition_rows: 6-byte entries in runs, a row's entries in any order); then
+// the library's CSR -> Blocked-ELL shape and emit, which place a row's values
+// whatever the order of its columns and count nnz the same way.  Only a
+// repeated (row, column), whose last value stays, needs the entries' order: the
+// emit flags it, and the partition (stable this time) and the emit, launched
+// again behind the flag, then run.  The
 // partition takes up to 2,097,152 rows whose row digit and column fit one
 // word; past that the entries are stably sorted by column and then by row and
 // gathered.  100,000 x 32,768, 131 M shuffled entries, plan + emit: 19.9 ms
-// by the two sorts (6.1 + 2.6 ms of it random gathers), 4.7 ms now.
+// by the two sorts (6.1 + 2.6 ms of it random gathers), 3.3 ms now.
 // Otherwise:
 //   scan    one pass over the entries: rows in range and columns inside
 //           the column map (others dropped and flagged), the largest mapped
@@ -43,7 +45,8 @@ namespace {
 
 constexpr uint32_t kInvalid = 0xffffffffu;
 
-// words: [0] largest mapped column, [1] dropped entries, [2] width, [3] route
+// words (16): [8] the partition route found a repeated (row, column);
+// [0] largest mapped column, [1] dropped entries, [2] width, [3] route
 // (0 two sorts, 1 one sort, 2 CSR), [4] key shift, [5] kept entries, [6] rows
 // decrease somewhere, [7] the CSR route's nnz
 constexpr uint32_t kRouteTwoSorts = 0u, kRouteOneSort = 1u, kRouteCsr = 2u, kRouteCsrSorted = 3u;
@@ -72,7 +75,7 @@ void carve(void *base, uint32_t n, uint32_t rows, uint32_t cols, uint32_t B, coo
     const uint32_t RB = (uint32_t) (((uint64_t) rows + B - 1u) / B);
     scratch_carver c(base, ~std::size_t(0));
     const std::size_t n1 = (std::size_t) n + 1u;
-    x->words = c.take<uint32_t>(8);
+    x->words = c.take<uint32_t>(16);
     x->shape = c.take<unsigned long long>(2);
     x->csr_ptr = c.take<uint32_t>((std::size_t) rows + 1u);
     x->mcol = c.take<uint32_t>(n1);
@@ -534,10 +537,18 @@ int coo_emit(const cs_coo_view *src, const uint32_t *map, uint32_t cols, const v
     }
     if (route == kRouteCsr || route == kRouteCsrSorted) {
         const cs_compressed_view v = csr_of(src, map, cols, x, route == kRouteCsrSorted);
-        if (!cuda_ok(cudaMemsetAsync(x.words + 7, 0, 4, stream), "csr nnz clear") ||
-            !cs_b200_blocked_ell_emit(&v, dst, x.words + 7, x.csr_tmp, x.csr_bytes, nullptr,
-                                      reinterpret_cast<cs_stream_t>(stream)))
+        if (!cuda_ok(cudaMemsetAsync(x.words + 7, 0, 8, stream), "csr nnz clear")) return 0;
+        if (route == kRouteCsrSorted && x.part_bytes != 0u) {
+            const uint32_t *bits = (const uint32_t *) x.csr_tmp;
+            if (!blocked_ell_emit_any_order(&v, dst, x.words + 7, bits, x.words + 8, true, stream) ||
+                !partition_rows_stable(x.words + 8, x.words + 7, n, src->rows, cols, src->rowIdx, src->colIdx, map,
+                                       src->val, x.csr_ptr, x.mcol, x.sval, x.part_tmp, x.part_bytes, stream) ||
+                !blocked_ell_emit_any_order(&v, dst, x.words + 7, bits, x.words + 8, false, stream))
+                return 0;
+        } else if (!cs_b200_blocked_ell_emit(&v, dst, x.words + 7, x.csr_tmp, x.csr_bytes, nullptr,
+                                             reinterpret_cast<cs_stream_t>(stream))) {
             return 0;
+        }
         coo_nnz_from_csr_kernel<<<1, 32, 0, stream>>>(x.words + 7, (unsigned long long *) d_nnz);
         return launch_ok("coo_nnz_from_csr_kernel");
     }

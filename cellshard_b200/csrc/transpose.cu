@@ -190,7 +190,12 @@ constexpr unsigned kTpWarps = kTpThreads / 32;
 constexpr uint32_t kTpBucketBits = 8; // low digit of the transpose
 constexpr uint32_t kTpMaxLowBits = 11;
 constexpr uint32_t kTpMaxBuckets = 1024;
-constexpr uint32_t kTpTile1 = 8192;  // entries per pass-1 tile (staged whole in shared memory)
+// entries per pass-1 tile (staged whole in shared memory): CSR rows leave runs of
+// many entries even in small tiles, and more CTAs per SM overlap their phases
+// (300,000 x 32,768: 4.69 ms against 4.98 with 8,192); COO entries are random,
+// and a tile of twice the entries writes runs twice as long
+constexpr uint32_t kTpTileCsr = 4096;
+constexpr uint32_t kTpTileCoo = 8192;
 constexpr uint32_t kTpChunk = 8192;  // entries per pass-2 chunk (staged whole in shared memory)
 constexpr uint32_t kTpGran = 256;    // entries per warp per step; rows are looked up per granule
 
@@ -233,7 +238,8 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     l->low_bits = low_bits;
     l->K = (uint32_t) (((uint64_t) uDim + D - 1u) >> low_bits);
     if (l->K == 0u) l->K = 1u;
-    l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + kTpTile1 - 1u) / kTpTile1);
+    const uint32_t tile = granules ? kTpTileCsr : kTpTileCoo;
+    l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + tile - 1u) / tile);
     l->max_chunks = nnz / kTpChunk + l->K + 1u;
     l->slices1 = (l->tiles1 + kTpSlice - 1u) / kTpSlice;
     l->max_slices = l->max_chunks / kTpSlice + l->K + 1u;
@@ -271,30 +277,58 @@ __global__ void __launch_bounds__(256) tp_gran_rows_kernel(const uint32_t *__res
     for (std::size_t j = ((std::size_t) lo + kTpGran - 1u) / kTpGran; j * kTpGran < hi; ++j) gran_row[j] = r;
 }
 
-// Pass-1 histogram: tile t is entries [t * kTpTile1, (t + 1) * kTpTile1).
+// Pass-1 histogram: tile t is entries [t * TILE, (t + 1) * TILE).  A
+// thread's whole share is in flight at once, 16 bytes a load where the keys
+// are aligned, and neighbouring entries of one bucket are added together.
+// 393 M entries in 128 buckets: 285 us (361 with an atomic per entry and four
+// 4-byte loads in flight).
+template <uint32_t TILE, bool VEC>
 __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__restrict__ idx, uint32_t nnz,
                                                              uint32_t uDim, uint32_t low_bits, uint32_t K,
                                                              uint16_t *__restrict__ cnt, uint32_t *status) {
     extern __shared__ uint32_t tp_h[];
+    const uint32_t a = blockIdx.x * TILE, n = min(nnz - a, TILE);
+    constexpr unsigned V = TILE / (4u * kTpThreads); // vectors per thread
+    uint32_t c[V][4];
+    if (VEC && n == TILE) {
+#pragma unroll
+        for (unsigned v = 0; v < V; ++v) {
+            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(idx + a) + v * kTpThreads + threadIdx.x);
+            c[v][0] = x.x;
+            c[v][1] = x.y;
+            c[v][2] = x.z;
+            c[v][3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (unsigned v = 0; v < V; ++v)
+#pragma unroll
+            for (unsigned j = 0; j < 4u; ++j) {
+                const uint32_t i = (v * kTpThreads + threadIdx.x) * 4u + j;
+                c[v][j] = i < n ? __ldg(idx + a + i) : uDim;
+            }
+    }
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) tp_h[k] = 0u;
     __syncthreads();
-    const uint32_t a = blockIdx.x * kTpTile1, e = min(nnz, a + kTpTile1);
     uint32_t bad = 0u;
-    constexpr unsigned U = 4;
-    for (uint32_t i0 = a; i0 < e; i0 += U * blockDim.x) {
-        uint32_t c[U];
 #pragma unroll
-        for (unsigned u = 0; u < U; ++u) {
-            const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-            c[u] = i < e ? __ldg(idx + i) : uDim;
-        }
+    for (unsigned v = 0; v < V; ++v) {
+        uint32_t k = 0u, run = 0u;
 #pragma unroll
-        for (unsigned u = 0; u < U; ++u) {
-            if (c[u] < uDim)
-                atomicAdd(tp_h + (c[u] >> low_bits), 1u);
-            else if (i0 + u * blockDim.x + threadIdx.x < e)
-                bad = CS_STATUS_INDEX_RANGE;
+        for (unsigned j = 0; j < 4u; ++j) {
+            const uint32_t x = c[v][j];
+            if (x >= uDim) {
+                if ((v * kTpThreads + threadIdx.x) * 4u + j < n) bad = CS_STATUS_INDEX_RANGE;
+                continue;
+            }
+            if ((x >> low_bits) != k) {
+                if (run != 0u) atomicAdd(tp_h + k, run);
+                k = x >> low_bits;
+                run = 0u;
+            }
+            ++run;
         }
+        if (run != 0u) atomicAdd(tp_h + k, run);
     }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) cnt[(std::size_t) blockIdx.x * K + k] = (uint16_t) tp_h[k];
@@ -312,9 +346,11 @@ __device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, 
     return make_uint2(blockIdx.x * kTpSlice, min(rows, (blockIdx.x + 1u) * kTpSlice));
 }
 
-__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
-                                                            uint32_t rows, const uint2 *__restrict__ range,
+// flag (here and below): nothing runs where it is given and clear.
+__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint32_t *__restrict__ flag,
+                                                            const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, const uint2 *__restrict__ range,
                                                             uint32_t *__restrict__ slices) {
+    if (flag != nullptr && *flag == 0u) return;
     const uint2 r = tp_slice_rows(range, rows);
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t sum = 0u;
@@ -326,11 +362,13 @@ __global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__re
 
 // One segment (blockIdx.x) and 32 digits (blockIdx.y) per CTA: 32 threads per
 // digit, each over a run of the segment's slices.  totals[segment * D + d] for
-// digits below `limit` in all.
-__global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restrict__ slices, uint32_t D,
+// digits below `limit` in all (null: not wanted).
+__global__ void __launch_bounds__(1024) tp_slice_scan_kernel(const uint32_t *__restrict__ flag,
+                                                             uint32_t *__restrict__ slices, uint32_t D,
                                                              const uint32_t *__restrict__ seg_first, uint32_t n_slices,
                                                              uint32_t limit, uint32_t *__restrict__ totals) {
     __shared__ uint32_t part[32][33];
+    if (flag != nullptr && *flag == 0u) return;
     const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, d = blockIdx.y * 32u + x;
     const uint32_t s0 = seg_first != nullptr ? seg_first[blockIdx.x] : 0u;
     const uint32_t s1 = seg_first != nullptr ? seg_first[blockIdx.x + 1u] : n_slices;
@@ -346,7 +384,7 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restric
         const uint32_t v = part[x][y], incl = warp_inclusive_scan(v);
         part[x][y] = incl - v;
         const std::size_t c = (std::size_t) blockIdx.x * D + blockIdx.y * 32u + y;
-        if (x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
+        if (totals != nullptr && x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
     }
     __syncthreads();
     if (d < D) {
@@ -360,12 +398,13 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restric
 }
 
 // start[segment * D + d]: global slot of the digit's first entry
-__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
-                                                             uint32_t rows, const uint2 *__restrict__ range,
+__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint32_t *__restrict__ flag,
+                                                             const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, const uint2 *__restrict__ range,
                                                              const uint32_t *__restrict__ segment,
                                                              const uint32_t *__restrict__ slices,
                                                              const uint32_t *__restrict__ start, uint32_t limit,
                                                              uint32_t *__restrict__ base) {
+    if (flag != nullptr && *flag == 0u) return;
     const uint2 r = tp_slice_rows(range, rows);
     const std::size_t c0 = (segment != nullptr ? (std::size_t) segment[blockIdx.x] : 0u) * D;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
@@ -471,136 +510,267 @@ __device__ __forceinline__ void tp_stage_prefix(const tp_stage &sg, uint32_t D) 
     }
 }
 
-// Pass 1: tile t = entries [t * kTpTile1, ...) of the input, reordered by
-// bucket (key >> low_bits) in shared memory, stable, then written out as one
-// run per bucket.
-// kCoo false: the key is the CSR entry's column, the payload its row, found
-// from `ptr`.  kCoo true: the key `idx` is the COO entry's row, the payload
-// its (mapped) column; random rows make a warp's 32 keys nearly all distinct,
-// so peers come from ballots (one per bucket bit) instead of match.any.
-// Packed words are (payload >> 5, low digit, payload & 31).
-template <bool kCoo>
-__global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t *__restrict__ ptr,
-                                                                const uint32_t *__restrict__ idx,
-                                                                const uint16_t *__restrict__ val, uint32_t cDim,
-                                                                uint32_t uDim, uint32_t nnz, uint32_t coo_low_bits,
-                                                                uint32_t K, const tp_counts one,
-                                                                const uint32_t *__restrict__ gran_row,
-                                                                const uint32_t *__restrict__ pay,
-                                                                const uint32_t *__restrict__ pay_map,
-                                                                uint32_t *__restrict__ tmp_key,
-                                                                uint16_t *__restrict__ tmp_val) {
+// Pass 1 of the transpose: the key is the CSR entry's column, the payload its
+// row.  Consecutive entries of a row ascend, so the entries of one bucket stand
+// in runs (~10 at 1,311 entries in 128 buckets), and what is sorted is the
+// tile's list of runs: heads by a shuffle and a ballot per 32 entries, the runs
+// ranked by bucket (per-warp counts, then in order), and every entry moves by
+// its run's displacement.  Rows in any column order only make the runs shorter.
+// Row starts inside the tile are bits over its entries too: the row of an entry
+// is the number of starts up to it, looked up in the tile's list of rows.
+// 60,000 x 32,768, 79 M entries: 435 us; 457 with match.any on every 32 entries,
+// two barriers per 2,048 entries and a row pointer read per batch; 481 ranking
+// entry by entry at run ends.  Bound by the phases that a CTA goes through one
+// after the other (load 80, rank 190, write 120 us when run alone).
+constexpr unsigned kTpThreads1 = 256;
+constexpr unsigned kTpWarps1 = kTpThreads1 / 32;
+constexpr unsigned kTpBatches1 = kTpTileCsr / kTpThreads1; // 32-entry batches per warp
+constexpr uint32_t kTpTileWords = kTpTileCsr / 32u;
+static_assert(kTpTileWords <= kTpThreads1, "a thread per word of the tile's bits");
+constexpr uint32_t kTpTileRows = 2048;                   // listed rows: a tile with more, or in a gap of more
+constexpr uint32_t kTpTileSpan = 32768;                  // empty rows than this, searches the row pointers
+
+struct tp_tile_smem {
+    union {
+        unsigned long long st[kTpTileCsr]; // staged entries: packed word | value << 32 | bucket << 48
+        struct {
+            uint32_t runs[kTpTileCsr];     // first entry | bucket << 16
+            uint32_t cnt[kTpWarps1 * kTpMaxBuckets / 2u]; // [warp][K2] pairs of u16: counts, then staging slots
+        };
+    };
+    uint16_t move[kTpTileCsr];             // a run's staging slot - its first entry
+    uint32_t heads[kTpTileWords], starts[kTpTileWords]; // bits: run heads, row starts
+    uint16_t heads_pre[kTpTileWords], starts_pre[kTpTileWords];
+    uint16_t row_of[kTpTileRows];        // row - the tile's first row
+    uint32_t scan33[33], scan33b[33];
+};
+
+__global__ void __launch_bounds__(kTpThreads1, 4)
+    tp_scatter1_csr_kernel(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx,
+                           const uint16_t *__restrict__ val, uint32_t cDim, uint32_t uDim, uint32_t nnz, uint32_t K,
+                           const tp_counts one, const uint32_t *__restrict__ gran_row, uint32_t *__restrict__ tmp_key,
+                           uint16_t *__restrict__ tmp_val) {
+    extern __shared__ __align__(16) unsigned char tp_ts[];
+    tp_tile_smem &sm = *reinterpret_cast<tp_tile_smem *>(tp_ts);
+    uint32_t *run = reinterpret_cast<uint32_t *>(tp_ts + sizeof(tp_tile_smem)); // [K] global base per bucket
+    uint32_t *lb = run + K;                                                     // [K + 1]
+    constexpr uint32_t kNone = 0xffffu; // bucket of an entry out of range or past the tile
+    const uint32_t K2 = (K + 1u) / 2u;
+    const unsigned t = threadIdx.x, warp = t >> 5, lane = t & 31u;
+    const unsigned le = 0xffffffffu >> (31u - lane);
+    const uint32_t a = blockIdx.x * kTpTileCsr, n = min(nnz - a, kTpTileCsr), e = a + n;
+    const uint32_t w0 = warp * (kTpBatches1 * 32u); // the warp's first entry in the tile
+    uint32_t cc[kTpBatches1], vv[kTpBatches1 / 2u];
+    if (n == kTpTileCsr) {
+#pragma unroll
+        for (unsigned q = 0; q < kTpBatches1; ++q) cc[q] = __ldcs(idx + a + w0 + q * 32u + lane);
+#pragma unroll
+        for (unsigned q = 0; q < kTpBatches1; q += 2u) {
+            const unsigned short *p = reinterpret_cast<const unsigned short *>(val) + a + w0 + q * 32u + lane;
+            vv[q / 2u] = (uint32_t) __ldcs(p) | (uint32_t) __ldcs(p + 32) << 16;
+        }
+    } else {
+#pragma unroll
+        for (unsigned q = 0; q < kTpBatches1; ++q) {
+            const uint32_t i = w0 + q * 32u + lane;
+            cc[q] = i < n ? __ldcs(idx + a + i) : 0xffffffffu;
+            const uint32_t v = i < n ? (uint32_t) __ldcs(reinterpret_cast<const unsigned short *>(val) + a + i) : 0u;
+            vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
+        }
+    }
+    for (uint32_t k = t; k < K; k += kTpThreads1) {
+        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
+    }
+    for (uint32_t k = t; k < kTpWarps1 * K2; k += kTpThreads1) sm.cnt[k] = 0u;
+    if (t < kTpTileWords) sm.starts[t] = 0u;
+    // rows that may start inside the tile; the tile's first entry lies in r_begin
+    const uint32_t r_begin = min(__ldg(gran_row + a / kTpGran), cDim - 1u);
+    const uint32_t r_end = e < nnz ? min(__ldg(gran_row + e / kTpGran), cDim - 1u) : major_of(ptr, cDim, e - 1u);
+    const bool near = r_end < r_begin || r_end - r_begin <= kTpTileSpan;
+    __syncthreads();
+    block_scan_small<4>(lb, K, sm.scan33);
+    // run heads (a warp's first entry is one) and row starts (of rows with entries)
+#pragma unroll
+    for (unsigned q = 0; q < kTpBatches1; ++q) {
+        const uint32_t k = cc[q] < uDim ? cc[q] >> kTpBucketBits : kNone;
+        uint32_t up = __shfl_up_sync(0xffffffffu, k, 1);
+        if (q != 0u) {
+            const uint32_t before = __shfl_sync(0xffffffffu, cc[q - (q != 0u)], 31);
+            if (lane == 0u) up = before < uDim ? before >> kTpBucketBits : kNone;
+        }
+        const uint32_t h = __ballot_sync(0xffffffffu, k != up || (q == 0u && lane == 0u));
+        if (lane == 0u) sm.heads[w0 / 32u + q] = h;
+    }
+    for (uint32_t r = r_begin + 1u + t; near && r <= r_end; r += kTpThreads1) {
+        const uint32_t x = __ldg(ptr + r) - a;
+        if (x < n && x != 0u && __ldg(ptr + r + 1u) != x + a) atomicOr(sm.starts + (x >> 5), 1u << (x & 31u));
+    }
+    __syncthreads();
+    uint32_t n_runs, n_starts;
+    {
+        const uint32_t both = t < kTpTileWords ? __popc(sm.heads[t]) | __popc(sm.starts[t]) << 16 : 0u;
+        uint32_t total; // both counts are at most kTpTileCsr
+        const uint32_t before = block_exclusive_scan(both, sm.scan33, total);
+        if (t < kTpTileWords) {
+            sm.heads_pre[t] = (uint16_t) before;
+            sm.starts_pre[t] = (uint16_t) (before >> 16);
+        }
+        n_runs = total & 0xffffu;
+        n_starts = total >> 16;
+    }
+    __syncthreads();
+    const bool listed = near && n_starts < kTpTileRows;
+#pragma unroll
+    for (unsigned q = 0; q < kTpBatches1; ++q) {
+        const uint32_t word = w0 / 32u + q, h = sm.heads[word];
+        const uint32_t k = cc[q] < uDim ? cc[q] >> kTpBucketBits : kNone;
+        if (h >> lane & 1u) sm.runs[sm.heads_pre[word] + __popc(h & (le >> 1))] = (w0 + q * 32u + lane) | k << 16;
+    }
+    if (listed) {
+        if (t == 0u) sm.row_of[0] = 0u;
+        for (uint32_t r = r_begin + 1u + t; r <= r_end; r += kTpThreads1) {
+            const uint32_t x = __ldg(ptr + r) - a;
+            if (x < n && x != 0u && __ldg(ptr + r + 1u) != x + a)
+                sm.row_of[sm.starts_pre[x >> 5] + __popc(sm.starts[x >> 5] & ((1u << (x & 31u)) - 1u)) + 1u] =
+                    (uint16_t) (r - r_begin);
+        }
+    }
+    __syncthreads();
+    // each warp takes consecutive runs: entries per bucket, staging slots, then
+    // its runs in order
+    uint32_t *my_cnt = sm.cnt + warp * K2;
+    uint16_t *my_bas = reinterpret_cast<uint16_t *>(my_cnt);
+    const uint32_t per = (n_runs + kTpThreads1 - 1u) / kTpThreads1 * 32u;
+    const uint32_t u0 = min(n_runs, warp * per), u1 = min(n_runs, u0 + per);
+    auto length = [&](uint32_t u, uint32_t rec) {
+        return (u + 1u < n_runs ? sm.runs[u + 1u] & 0xffffu : kTpTileCsr) - (rec & 0xffffu);
+    };
+    for (uint32_t u = u0 + lane; u < u1; u += 32u) {
+        const uint32_t rec = sm.runs[u], k = rec >> 16;
+        if (k != kNone) atomicAdd(my_cnt + (k >> 1), length(u, rec) << (16u * (k & 1u)));
+    }
+    __syncthreads();
+    for (uint32_t k2 = t; k2 < K2; k2 += kTpThreads1) {
+        uint32_t s0 = lb[2u * k2], s1 = 2u * k2 + 1u < K ? lb[2u * k2 + 1u] : 0u;
+#pragma unroll
+        for (unsigned w = 0; w < kTpWarps1; ++w) {
+            const uint32_t c = sm.cnt[w * K2 + k2];
+            sm.cnt[w * K2 + k2] = s0 | s1 << 16;
+            s0 += c & 0xffffu;
+            s1 += c >> 16;
+        }
+    }
+    __syncthreads();
+    for (uint32_t v0 = u0; v0 < u1; v0 += 32u) {
+        const uint32_t u = v0 + lane;
+        const uint32_t rec = u < u1 ? sm.runs[u] : kNone << 16, k = rec >> 16;
+        // one run per bucket and turn, the first of its bucket's first
+        uint32_t peers = tp_peers(k, k != kNone);
+        while (__any_sync(0xffffffffu, peers != 0u)) {
+            const bool mine = peers != 0u && (peers & (le >> 1)) == 0u;
+            if (mine) {
+                const uint32_t slot = my_bas[k];
+                sm.move[u] = (uint16_t) (slot - (rec & 0xffffu));
+                my_bas[k] = (uint16_t) (slot + length(u, rec));
+            }
+            const uint32_t done = __ballot_sync(0xffffffffu, mine);
+            peers = mine ? 0u : peers & ~done;
+            __syncwarp();
+        }
+    }
+    __syncthreads(); // the stage takes the place of the runs and the counts
+    auto in_place = [](uint32_t r) { return r >> 5 << (kTpBucketBits + 5u) | (r & 31u); };
+    // the row that goes on into the next batch, as its bits of the packed word
+    uint32_t row_bits = listed ? in_place(r_begin + sm.row_of[sm.starts_pre[w0 / 32u]]) : 0u;
+#pragma unroll
+    for (unsigned q = 0; q < kTpBatches1; ++q) {
+        const uint32_t word = w0 / 32u + q, c = cc[q], pos = w0 + q * 32u + lane;
+        const uint32_t sb = sm.starts[word];
+        if (!listed)
+            row_bits = in_place(major_of(ptr, cDim, min(a + pos, e - 1u)));
+        else if (sb != 0u)
+            row_bits = in_place(r_begin + sm.row_of[sm.starts_pre[word] + __popc(sb & le)]);
+        const uint32_t lp = (pos + sm.move[sm.heads_pre[word] + __popc(sm.heads[word] & le) - 1u]) & 0xffffu;
+        if (c < uDim)
+            sm.st[lp] = (unsigned long long) (row_bits | (c & 255u) << 5) |
+                        (unsigned long long) (((q & 1u) ? vv[q / 2u] >> 16 : vv[q / 2u] & 0xffffu) |
+                                              c >> kTpBucketBits << 16)
+                            << 32;
+        if (sb != 0u) row_bits = __shfl_sync(0xffffffffu, row_bits, 31);
+    }
+    __syncthreads();
+    const uint32_t placed = min(lb[K], kTpTileCsr);
+    for (uint32_t k = t; k < K; k += kTpThreads1) run[k] -= lb[k]; // the global slot of staging slot 0
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t j = t; j < placed; j += kTpThreads1) {
+        const unsigned long long v = sm.st[j];
+        const uint32_t g = run[(uint32_t) (v >> 48)] + j;
+        tmp_key[g] = (uint32_t) v;
+        tmp_val[g] = (uint16_t) (v >> 32);
+    }
+}
+
+std::size_t tp_scatter1_csr_smem(uint32_t K) { return sizeof(tp_tile_smem) + ((std::size_t) 2u * K + 1u) * 4u; }
+
+// Pass 1 of COO entries: the key is the entry's row, the payload its (mapped)
+// column.  Random rows leave nothing to rank by but the counters themselves: a
+// thread's entries take their places in a bucket by shared atomics, in any
+// order, which costs ~50 warp instructions per 32 entries against ~230 of the
+// ballots below.  Only a repeated (row, column) needs the order of the entries,
+// and the Blocked-ELL emit finds those: the ballot kernels then run again.
+constexpr unsigned kTpThreadsCoo = 512;
+constexpr unsigned kTpPerCoo = kTpTileCoo / kTpThreadsCoo;
+
+__global__ void __launch_bounds__(kTpThreadsCoo, 2)
+    tp_scatter1_coo_kernel(const uint32_t *__restrict__ key, const uint16_t *__restrict__ val,
+                           const uint32_t *__restrict__ pay, const uint32_t *__restrict__ pay_map, uint32_t uDim,
+                           uint32_t nnz, uint32_t low_bits, uint32_t K, const tp_counts one,
+                           uint32_t *__restrict__ tmp_key, uint16_t *__restrict__ tmp_val) {
     extern __shared__ __align__(16) uint32_t tp_s[];
     __shared__ uint32_t scan33[33];
-    // staged entry: key | value << 32 | bucket << 48
-    unsigned long long *st = reinterpret_cast<unsigned long long *>(tp_s); // [kTpTile1]
-    uint32_t *run = reinterpret_cast<uint32_t *>(st + kTpTile1);           // [K] global base per bucket
-    tp_stage sg;
-    sg.lb = run + K;                                                       // [K + 1]
-    sg.fill = sg.lb + K + 1u;                                              // [K]
-    sg.cnt = reinterpret_cast<uint16_t *>(sg.fill + K);                    // [kTpWarps][K]
-    sg.bas = sg.cnt + kTpWarps * K;                                        // [kTpWarps][K]
-    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t a = blockIdx.x * kTpTile1, e = min(nnz, a + kTpTile1);
-    if (a >= e) return;
-    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
+    // staged entry: packed word | value << 32 | bucket << 48
+    unsigned long long *st = reinterpret_cast<unsigned long long *>(tp_s); // [kTpTileCoo]
+    uint32_t *run = reinterpret_cast<uint32_t *>(st + kTpTileCoo);         // [K] global base per bucket
+    uint32_t *at = run + K;                                                // [K + 1] next staging slot
+    const unsigned t = threadIdx.x;
+    const uint32_t a = blockIdx.x * kTpTileCoo, n = min(nnz - a, kTpTileCoo);
+    uint32_t rr[kTpPerCoo], pp[kTpPerCoo], vv[kTpPerCoo / 2u];
+#pragma unroll
+    for (unsigned q = 0; q < kTpPerCoo; ++q) {
+        const uint32_t i = q * kTpThreadsCoo + t;
+        rr[q] = i < n ? __ldcs(key + a + i) : 0xffffffffu;
+        pp[q] = i < n ? __ldcs(pay + a + i) : 0u;
+        const uint32_t v = i < n ? (uint32_t) __ldcs(reinterpret_cast<const unsigned short *>(val) + a + i) : 0u;
+        vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
+    }
+    for (uint32_t k = t; k < K; k += kTpThreadsCoo) {
         run[k] = one.base[(std::size_t) blockIdx.x * K + k];
-        sg.lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
-        sg.fill[k] = 0u;
+        at[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
     }
-    for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
+    if (pay_map != nullptr)
+#pragma unroll
+        for (unsigned q = 0; q < kTpPerCoo; ++q)
+            if (rr[q] < uDim) pp[q] = __ldg(pay_map + pp[q]);
     __syncthreads();
-    block_scan_small<4>(sg.lb, K, scan33);
-    const unsigned lt = (1u << lane) - 1u;
-    uint16_t *my_cnt = sg.cnt + warp * K;
-    uint16_t *my_bas = sg.bas + warp * K;
-    static_assert(kTpSub / kTpWarps == kTpGran, "a warp's step range is one row granule");
-    const uint32_t low_bits = kCoo ? coo_low_bits : kTpBucketBits;
-    uint32_t ncc[kTpBatches], npp[kTpBatches], nrc = 0u;
+    block_scan_small<2>(at, K, scan33);
+    const uint32_t placed = min(at[K], kTpTileCoo);
+    for (uint32_t k = t; k < K; k += kTpThreadsCoo) run[k] -= at[k]; // the global slot of staging slot 0
+    __syncthreads();
     const uint32_t low_mask = (1u << low_bits) - 1u;
-    uint16_t nvv[kTpBatches];
-    auto fetch = [&](uint32_t sc) {
-        const uint32_t n = min(kTpSub, e - sc);
-        const uint32_t wa = sc + min(n, warp * kTpGran), we = sc + min(n, (warp + 1u) * kTpGran);
 #pragma unroll
-        for (unsigned q = 0; q < kTpBatches; ++q) {
-            const uint32_t i = wa + q * 32u + lane;
-            const bool in = i < we;
-            ncc[q] = in ? __ldg(idx + i) : uDim;
-            nvv[q] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
-            if constexpr (kCoo) npp[q] = in ? __ldg(pay + i) : 0u;
-        }
-        if constexpr (!kCoo) nrc = wa < we ? min(__ldg(gran_row + wa / kTpGran), cDim - 1u) : 0u;
-    };
-    fetch(a);
-    for (uint32_t sc0 = a; sc0 < e; sc0 += kTpSub) {
-        const uint32_t n = min(kTpSub, e - sc0);
-        const uint32_t wa = sc0 + min(n, warp * kTpGran);
-        const uint32_t we = sc0 + min(n, (warp + 1u) * kTpGran);
-        uint32_t cc[kTpBatches], pk[kTpBatches], rl[kTpBatches];
-        uint16_t vv[kTpBatches];
-#pragma unroll
-        for (unsigned q = 0; q < kTpBatches; ++q) {
-            cc[q] = ncc[q];
-            vv[q] = nvv[q];
-            if constexpr (kCoo) rl[q] = pay_map != nullptr && cc[q] < uDim ? __ldg(pay_map + npp[q]) : npp[q];
-        }
-        uint32_t r_cur = nrc;
-        if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
-#pragma unroll
-        for (unsigned q = 0; q < kTpBatches; ++q) {
-            if constexpr (!kCoo) {
-                const uint32_t i = wa + q * 32u + lane;
-                const bool in = i < we;
-                // row of entry i: walk forward from the warp's current row; a
-                // batch that spans many short rows finishes by binary search
-                uint32_t r = r_cur;
-                for (unsigned step = 0;; ++step) {
-                    const bool adv = in && r + 1u < cDim && __ldg(ptr + r + 1u) <= i;
-                    if (!__any_sync(0xffffffffu, adv)) break;
-                    if (step == 3u) {
-                        if (adv) {
-                            const uint32_t lo = r + 1u;
-                            r = lo + major_of(ptr + lo, cDim - lo, i);
-                        }
-                        break;
-                    }
-                    r += adv ? 1u : 0u;
-                }
-                rl[q] = r;
-                r_cur = __shfl_sync(0xffffffffu, r, 31);
-            }
-            const bool ok = cc[q] < uDim;
-            const uint32_t k = cc[q] >> low_bits;
-            pk[q] = kCoo ? warp_match_digit<10>(k, ok) : tp_peers(k, ok);
-            if (ok && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[k] += (uint16_t) __popc(pk[q]);
-            __syncwarp();
-        }
-        __syncthreads();
-        tp_stage_prefix<kTpWarps>(sg, K);
-        __syncthreads();
-#pragma unroll
-        for (unsigned q = 0; q < kTpBatches; ++q) {
-            const bool ok = cc[q] < uDim;
-            const uint32_t k = cc[q] >> low_bits;
-            uint32_t lp = 0u;
-            if (ok) lp = my_bas[k] + __popc(pk[q] & lt);
-            __syncwarp();
-            if (ok) {
-                if (lp < kTpTile1)
-                    st[lp] = (unsigned long long) tp_pack(rl[q], cc[q] & low_mask, low_bits) |
-                             ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
-                if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
-            }
-            __syncwarp();
-        }
+    for (unsigned q = 0; q < kTpPerCoo; ++q) {
+        if (rr[q] >= uDim) continue;
+        const uint32_t k = rr[q] >> low_bits;
+        const uint32_t lp = atomicAdd(at + k, 1u);
+        if (lp < kTpTileCoo)
+            st[lp] = (unsigned long long) tp_pack(pp[q], rr[q] & low_mask, low_bits) |
+                     (unsigned long long) (((q & 1u) ? vv[q / 2u] >> 16 : vv[q / 2u] & 0xffffu) | k << 16) << 32;
     }
     __syncthreads();
-    const uint32_t placed = min(sg.lb[K], kTpTile1);
-    // run[k] - lb[k]: the global slot of staging slot 0 for bucket k
-    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) run[k] -= sg.lb[k];
-    __syncthreads();
-    for (uint32_t j = threadIdx.x; j < placed; j += blockDim.x) {
+#pragma unroll 4
+    for (uint32_t j = t; j < placed; j += kTpThreadsCoo) {
         const unsigned long long v = st[j];
         const uint32_t g = run[(uint32_t) (v >> 48)] + j;
         tmp_key[g] = (uint32_t) v;
@@ -608,8 +778,114 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_kernel(const uint32_t 
     }
 }
 
+std::size_t tp_scatter1_coo_smem(uint32_t K) {
+    return (std::size_t) kTpTileCoo * 8u + ((std::size_t) 2u * K + 1u) * 4u;
+}
+
+// The same in the order of the entries (stable), where `flag` is set: a
+// tile's entries are ranked in 32-entry batches by ballots, one per bucket bit.
+// Clears *nnz for the emit that follows.
+__global__ void __launch_bounds__(kTpThreads) tp_scatter1_coo_stable_kernel(
+    const uint32_t *__restrict__ flag, uint32_t *__restrict__ nnz_count, const uint32_t *__restrict__ idx,
+    const uint16_t *__restrict__ val, uint32_t uDim, uint32_t nnz, uint32_t low_bits, uint32_t K, uint32_t tiles1,
+    const tp_counts one, const uint32_t *__restrict__ pay, const uint32_t *__restrict__ pay_map,
+    uint32_t *__restrict__ tmp_key, uint16_t *__restrict__ tmp_val) {
+    if (*flag == 0u) return;
+    if (blockIdx.x == 0u && threadIdx.x == 0u) *nnz_count = 0u;
+    extern __shared__ __align__(16) uint32_t tp_s[];
+    __shared__ uint32_t scan33[33];
+    // staged entry: key | value << 32 | bucket << 48
+    unsigned long long *st = reinterpret_cast<unsigned long long *>(tp_s); // [kTpTileCoo]
+    uint32_t *run = reinterpret_cast<uint32_t *>(st + kTpTileCoo);           // [K] global base per bucket
+    tp_stage sg;
+    sg.lb = run + K;                                                       // [K + 1]
+    sg.fill = sg.lb + K + 1u;                                              // [K]
+    sg.cnt = reinterpret_cast<uint16_t *>(sg.fill + K);                    // [kTpWarps][K]
+    sg.bas = sg.cnt + kTpWarps * K;                                        // [kTpWarps][K]
+    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    for (uint32_t tile = blockIdx.x; tile < tiles1; tile += gridDim.x) {
+        __syncthreads();
+        const uint32_t a = tile * kTpTileCoo, e = min(nnz - a, kTpTileCoo) + a;
+        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
+            run[k] = one.base[(std::size_t) tile * K + k];
+            sg.lb[k] = one.cnt[(std::size_t) tile * K + k];
+            sg.fill[k] = 0u;
+        }
+        for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
+        __syncthreads();
+        block_scan_small<4>(sg.lb, K, scan33);
+        const unsigned lt = (1u << lane) - 1u;
+        uint16_t *my_cnt = sg.cnt + warp * K;
+        uint16_t *my_bas = sg.bas + warp * K;
+        uint32_t ncc[kTpBatches], npp[kTpBatches];
+        const uint32_t low_mask = (1u << low_bits) - 1u;
+        uint16_t nvv[kTpBatches];
+        auto fetch = [&](uint32_t sc) {
+            const uint32_t n = min(kTpSub, e - sc);
+            const uint32_t wa = sc + min(n, warp * kTpGran), we = sc + min(n, (warp + 1u) * kTpGran);
+#pragma unroll
+            for (unsigned q = 0; q < kTpBatches; ++q) {
+                const uint32_t i = wa + q * 32u + lane;
+                const bool in = i < we;
+                ncc[q] = in ? __ldg(idx + i) : uDim;
+                nvv[q] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
+                npp[q] = in ? __ldg(pay + i) : 0u;
+            }
+        };
+        fetch(a);
+        for (uint32_t sc0 = a; sc0 < e; sc0 += kTpSub) {
+            uint32_t cc[kTpBatches], pk[kTpBatches], rl[kTpBatches];
+            uint16_t vv[kTpBatches];
+#pragma unroll
+            for (unsigned q = 0; q < kTpBatches; ++q) {
+                cc[q] = ncc[q];
+                vv[q] = nvv[q];
+                rl[q] = pay_map != nullptr && cc[q] < uDim ? __ldg(pay_map + npp[q]) : npp[q];
+            }
+            if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
+#pragma unroll
+            for (unsigned q = 0; q < kTpBatches; ++q) {
+                const bool ok = cc[q] < uDim;
+                const uint32_t k = cc[q] >> low_bits;
+                pk[q] = warp_match_digit<10>(k, ok);
+                if (ok && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[k] += (uint16_t) __popc(pk[q]);
+                __syncwarp();
+            }
+            __syncthreads();
+            tp_stage_prefix<kTpWarps>(sg, K);
+            __syncthreads();
+#pragma unroll
+            for (unsigned q = 0; q < kTpBatches; ++q) {
+                const bool ok = cc[q] < uDim;
+                const uint32_t k = cc[q] >> low_bits;
+                uint32_t lp = 0u;
+                if (ok) lp = my_bas[k] + __popc(pk[q] & lt);
+                __syncwarp();
+                if (ok) {
+                    if (lp < kTpTileCoo)
+                        st[lp] = (unsigned long long) tp_pack(rl[q], cc[q] & low_mask, low_bits) |
+                                 ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
+                    if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
+                }
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        const uint32_t placed = min(sg.lb[K], kTpTileCoo);
+        // run[k] - lb[k]: the global slot of staging slot 0 for bucket k
+        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) run[k] -= sg.lb[k];
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < placed; j += blockDim.x) {
+            const unsigned long long v = st[j];
+            const uint32_t g = run[(uint32_t) (v >> 48)] + j;
+            tmp_key[g] = (uint32_t) v;
+            tmp_val[g] = (uint16_t) (v >> 32);
+        }
+    }
+}
+
 std::size_t tp_scatter1_smem(uint32_t K) {
-    return (std::size_t) kTpTile1 * 8u + ((std::size_t) 3u * K + 1u) * 4u + (std::size_t) 2u * kTpWarps * K * 2u;
+    return (std::size_t) kTpTileCoo * 8u + ((std::size_t) 3u * K + 1u) * 4u + (std::size_t) 2u * kTpWarps * K * 2u;
 }
 
 // One CTA: bucket starts from their totals, then every bucket's entry range is
@@ -677,34 +953,39 @@ __global__ void __launch_bounds__(1024) tp_chunks_kernel(const tp2_layout l) {
 
 // one histogram per warp while eight of them fit (LB = 8), one per CTA above
 template <int LB>
-__global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ tmp_key,
-                                                             const uint2 *__restrict__ chunk_range,
+__global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ flag,
+                                                             const uint32_t *__restrict__ tmp_key,
+                                                             const uint2 *__restrict__ chunk_range, uint32_t chunks,
                                                              uint16_t *__restrict__ cnt) {
     constexpr uint32_t D = 1u << LB;
     constexpr unsigned kCopies = LB == 8 ? kTpWarps : 1u;
     __shared__ uint32_t h[kCopies][D];
+    if (flag != nullptr && *flag == 0u) return;
     const unsigned copy = (threadIdx.x >> 5) % kCopies;
-    for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
-    __syncthreads();
-    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
-    constexpr unsigned U = 4;
-    for (uint32_t i0 = b; i0 < e; i0 += U * blockDim.x) {
-        uint32_t kk[U];
+    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+        for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
+        __syncthreads();
+        const uint32_t b = chunk_range[chunk].x, e = chunk_range[chunk].y;
+        constexpr unsigned U = 4;
+        for (uint32_t i0 = b; i0 < e; i0 += U * blockDim.x) {
+            uint32_t kk[U];
 #pragma unroll
-        for (unsigned u = 0; u < U; ++u) {
-            const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-            kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu; // no packed key: see partition_low_bits
+            for (unsigned u = 0; u < U; ++u) {
+                const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+                kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu; // no packed key: see partition_low_bits
+            }
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u)
+                if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][tp_digit<LB>(kk[u])], 1u);
         }
+        __syncthreads();
+        for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+            uint32_t t = 0u;
 #pragma unroll
-        for (unsigned u = 0; u < U; ++u)
-            if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][tp_digit<LB>(kk[u])], 1u);
-    }
-    __syncthreads();
-    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
-        uint32_t t = 0u;
-#pragma unroll
-        for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
-        cnt[(std::size_t) blockIdx.x * D + d] = (uint16_t) t;
+            for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
+            cnt[(std::size_t) chunk * D + d] = (uint16_t) t;
+        }
+        if (chunk + gridDim.x < chunks) __syncthreads();
     }
 }
 
@@ -777,15 +1058,17 @@ __device__ void tp_rank_ballots(const uint32_t *__restrict__ tmp_key, const uint
     }
 }
 
-// Pass 2 of entries in any payload order (the COO rows): a chunk of one bucket
-// reordered by the low digit in shared memory (stable), then written out as
-// one run per key.
+// Pass 2 by ballots: a chunk of one bucket reordered by the low digit in shared
+// memory (stable), then written out as one run per key.  Sparse transposes, and
+// COO entries where `flag` is set (null: always).
 template <int LB>
-__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
+__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ flag,
+                                                                const uint32_t *__restrict__ tmp_key,
                                                                 const uint16_t *__restrict__ tmp_val,
-                                                                const uint2 *__restrict__ chunk_range,
+                                                                const uint2 *__restrict__ chunk_range, uint32_t chunks,
                                                                 const tp_counts two, uint32_t *__restrict__ out_idx,
                                                                 uint16_t *__restrict__ out_val) {
+    if (flag != nullptr && *flag == 0u) return;
     extern __shared__ __align__(16) uint32_t tp_s2[];
     constexpr uint32_t D = 1u << LB;
     __shared__ uint32_t gbase[D];
@@ -799,28 +1082,89 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
     sg.bas = sg.cnt + kTpWarps * D;                                        // [kTpWarps][D]
     sg.lb = lb;
     sg.fill = fill;
+    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+        const uint32_t b = chunk_range[chunk].x, e = chunk_range[chunk].y;
+        if (b >= e) continue;
+        __syncthreads();
+        for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
+            lb[d] = two.cnt[(std::size_t) chunk * D + d];
+            gbase[d] = two.base[(std::size_t) chunk * D + d];
+            fill[d] = 0u;
+#pragma unroll
+            for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
+        }
+        __syncthreads();
+        block_scan_small<(D / kTpThreads)>(lb, D, scan33);
+        tp_rank_ballots<LB, kTpWarps>(tmp_key, tmp_val, b, e, sg, st_key, st_val);
+        // global slot of staging slot 0 for digit d
+        for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
+        __syncthreads();
+        const uint32_t n = min(e - b, kTpChunk);
+        for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+            const uint32_t key = st_key[j];
+            const uint32_t g = gbase[tp_digit<LB>(key)] + j;
+            out_idx[g] = tp_payload<LB>(key);
+            out_val[g] = st_val[j];
+        }
+    }
+}
+
+// Pass 2 of COO entries, in any order inside a row: as tp_scatter1_coo_kernel,
+// by shared atomics on the row's next staging slot.
+template <int LB>
+__global__ void __launch_bounds__(kTpThreadsCoo, 2)
+    tp_scatter2_coo_kernel(const uint32_t *__restrict__ tmp_key, const uint16_t *__restrict__ tmp_val,
+                           const uint2 *__restrict__ chunk_range, const tp_counts two, uint32_t *__restrict__ out_idx,
+                           uint16_t *__restrict__ out_val) {
+    extern __shared__ __align__(16) uint32_t tp_s2[];
+    constexpr uint32_t D = 1u << LB;
+    __shared__ uint32_t scan33[33];
+    uint32_t *st_key = tp_s2;                                            // [kTpChunk]
+    uint16_t *st_val = reinterpret_cast<uint16_t *>(st_key + kTpChunk); // [kTpChunk]
+    uint32_t *gbase = reinterpret_cast<uint32_t *>(st_val + kTpChunk);  // [D]
+    uint32_t *at = gbase + D;                                           // [D + 1] next staging slot
+    const unsigned t = threadIdx.x;
     const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
     if (b >= e) return;
-    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
-        lb[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
-        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
-        fill[d] = 0u;
+    const uint32_t n = min(e - b, kTpChunk);
+    constexpr unsigned kPer = kTpChunk / kTpThreadsCoo;
+    uint32_t kk[kPer], vv[kPer / 2u];
 #pragma unroll
-        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
+    for (unsigned q = 0; q < kPer; ++q) {
+        const uint32_t i = q * kTpThreadsCoo + t;
+        kk[q] = i < n ? __ldcs(tmp_key + b + i) : 0xffffffffu; // no packed key: see partition_low_bits
+        const uint32_t v = i < n ? (uint32_t) __ldcs(reinterpret_cast<const unsigned short *>(tmp_val) + b + i) : 0u;
+        vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
+    }
+    for (uint32_t d = t; d < D; d += kTpThreadsCoo) {
+        at[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
+        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
     }
     __syncthreads();
-    block_scan_small<(D / kTpThreads)>(lb, D, scan33);
-    tp_rank_ballots<LB, kTpWarps>(tmp_key, tmp_val, b, e, sg, st_key, st_val);
-    // global slot of staging slot 0 for digit d
-    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
+    block_scan_small<(D + kTpThreadsCoo - 1u) / kTpThreadsCoo>(at, D, scan33);
+    for (uint32_t d = t; d < D; d += kTpThreadsCoo) gbase[d] -= at[d]; // global slot of staging slot 0
     __syncthreads();
-    const uint32_t n = min(e - b, kTpChunk);
-    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+#pragma unroll
+    for (unsigned q = 0; q < kPer; ++q) {
+        if (kk[q] == 0xffffffffu) continue;
+        const uint32_t lp = atomicAdd(at + tp_digit<LB>(kk[q]), 1u);
+        if (lp < kTpChunk) {
+            st_key[lp] = kk[q];
+            st_val[lp] = (uint16_t) ((q & 1u) ? vv[q / 2u] >> 16 : vv[q / 2u]);
+        }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t j = t; j < n; j += kTpThreadsCoo) {
         const uint32_t key = st_key[j];
         const uint32_t g = gbase[tp_digit<LB>(key)] + j;
         out_idx[g] = tp_payload<LB>(key);
         out_val[g] = st_val[j];
     }
+}
+
+constexpr std::size_t tp_scatter2_coo_smem(uint32_t low_bits) {
+    return (std::size_t) kTpChunk * 6u + ((std::size_t) 2u << low_bits) * 4u + 4u;
 }
 
 // Pass 2 of the transpose.  Pass 1 is stable, so the rows of a chunk never
@@ -975,57 +1319,93 @@ constexpr std::size_t tp_scatter2_smem(uint32_t low_bits) {
     return (std::size_t) kTpChunk * 6u + ((std::size_t) 2u * kTpWarps * 2u << low_bits);
 }
 
-// Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).
-// kRows: the payloads of a bucket never decrease (the transpose's rows).
-template <int LB, bool kRows>
+enum class tp_rank { rows, ballots, any }; // how a pass-2 chunk is ranked
+
+template <typename K>
+int tp_smem(K kernel, std::size_t smem, const char *what) {
+    return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem), what);
+}
+
+// Counts of `l`'s pass-1 result (low digit of LB bits), the row pointers and
+// every chunk's offsets; with a flag, the chunks' offsets again where it is
+// set, in grids of one wave.
+template <int LB>
+int tp_count_chunks(const uint32_t *flag, uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, cudaStream_t stream) {
+    constexpr uint32_t D = 1u << LB;
+    const unsigned grid = flag == nullptr
+                              ? l.max_chunks
+                              : resident_grid((const void *) tp_hist2_kernel<LB>, kTpThreads, 0, l.max_chunks);
+    tp_hist2_kernel<LB><<<grid, kTpThreads, 0, stream>>>(flag, l.tmp_key, l.chunk_range, l.max_chunks, l.two.cnt);
+    if (!launch_ok("tp_hist2_kernel")) return 0;
+    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, l.slice_range, l.two.slices);
+    if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(flag, l.two.slices, D, l.slice_first, 0u, uDim,
+                                                                  flag == nullptr ? out_ptr : nullptr);
+    if (!launch_ok("tp_slice_scan_kernel")) return 0;
+    if (flag == nullptr &&
+        !scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream))
+        return 0;
+    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, l.slice_range, l.slice_bucket,
+                                                            l.two.slices, out_ptr, uDim, l.two.base);
+    return launch_ok("tp_slice_apply_kernel");
+}
+
+// Pass 2.  rows: the payloads of a bucket never decrease (the transpose); any:
+// entries of one key in any order (COO).
+template <int LB, tp_rank kRank>
 int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
                    cudaStream_t stream) {
-    static_assert(!kRows || LB == (int) kTpBucketBits, "the row ranking has 256 digits");
-    constexpr std::size_t smem = kRows ? sizeof(tp_rows_smem) : tp_scatter2_smem(LB);
-    auto s2 = kRows ? tp_scatter2_rows_kernel : tp_scatter2_kernel<LB>;
-    if (!cuda_ok(cudaFuncSetAttribute(s2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                 "scatter2 smem attribute"))
-        return 0;
-    tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_range, l.two.cnt);
-    if (!launch_ok("tp_hist2_kernel")) return 0;
-    constexpr uint32_t D = 1u << LB;
-    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, l.slice_range, l.two.slices);
-    if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(l.two.slices, D, l.slice_first, 0u, uDim, out_ptr);
-    if (!launch_ok("tp_slice_scan_kernel")) return 0;
-    if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
-    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, l.slice_range, l.slice_bucket,
-                                                            l.two.slices, out_ptr, uDim, l.two.base);
-    if (!launch_ok("tp_slice_apply_kernel")) return 0;
-    s2<<<l.max_chunks, kRows ? kTpThreads2 : kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range, l.two,
-                                                                         out_idx, out_val);
+    static_assert(kRank != tp_rank::rows || LB == (int) kTpBucketBits, "the row ranking has 256 digits");
+    if (!tp_count_chunks<LB>(nullptr, uDim, l, out_ptr, stream)) return 0;
+    if constexpr (kRank == tp_rank::rows) {
+        if (!tp_smem(tp_scatter2_rows_kernel, sizeof(tp_rows_smem), "scatter2 smem attribute")) return 0;
+        tp_scatter2_rows_kernel<<<l.max_chunks, kTpThreads2, sizeof(tp_rows_smem), stream>>>(
+            l.tmp_key, l.tmp_val, l.chunk_range, l.two, out_idx, out_val);
+    } else if constexpr (kRank == tp_rank::any) {
+        constexpr std::size_t smem = tp_scatter2_coo_smem(LB);
+        if (!tp_smem(tp_scatter2_coo_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
+        tp_scatter2_coo_kernel<LB><<<l.max_chunks, kTpThreadsCoo, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range,
+                                                                                  l.two, out_idx, out_val);
+    } else {
+        constexpr std::size_t smem = tp_scatter2_smem(LB);
+        if (!tp_smem(tp_scatter2_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
+        tp_scatter2_kernel<LB><<<l.max_chunks, kTpThreads, smem, stream>>>(nullptr, l.tmp_key, l.tmp_val, l.chunk_range,
+                                                                           l.max_chunks, l.two, out_idx, out_val);
+    }
     return launch_ok("tp_scatter2_kernel");
 }
 
-template <bool kCoo>
+// Pass 1: `ptr` is null for COO (payloads `pay` through `pay_map`).
 int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *ptr, const uint32_t *key,
                   const uint16_t *val, const uint32_t *pay, const uint32_t *pay_map, const tp2_layout &l,
                   cudaStream_t stream) {
-    const std::size_t s1_smem = tp_scatter1_smem(l.K);
-    auto s1 = tp_scatter1_kernel<kCoo>;
-    if (!cuda_ok(cudaFuncSetAttribute(s1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s1_smem),
-                 "scatter1 smem attribute"))
-        return 0;
-    tp_hist1_kernel<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K,
-                                                                              l.one.cnt, l.status);
+    const bool csr = ptr != nullptr, vec = (reinterpret_cast<uintptr_t>(key) & 15u) == 0u;
+    auto hist1 = csr ? (vec ? tp_hist1_kernel<kTpTileCsr, true> : tp_hist1_kernel<kTpTileCsr, false>)
+                     : (vec ? tp_hist1_kernel<kTpTileCoo, true> : tp_hist1_kernel<kTpTileCoo, false>);
+    hist1<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K, l.one.cnt,
+                                                                    l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, nullptr, l.one.slices);
+    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, nullptr, l.one.slices);
     if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(l.one.slices, l.K, nullptr, l.slices1, l.K,
+    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(nullptr, l.one.slices, l.K, nullptr, l.slices1, l.K,
                                                                           l.total1);
     if (!launch_ok("tp_slice_scan_kernel")) return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
     if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, nullptr, nullptr, l.one.slices,
+    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, nullptr, nullptr, l.one.slices,
                                                          l.start1, l.K, l.one.base);
     if (!launch_ok("tp_slice_apply_kernel")) return 0;
-    s1<<<l.tiles1, kTpThreads, s1_smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.low_bits, l.K, l.one, l.gran_row,
-                                                  pay, pay_map, l.tmp_key, l.tmp_val);
+    if (csr) {
+        const std::size_t smem = tp_scatter1_csr_smem(l.K);
+        if (!tp_smem(tp_scatter1_csr_kernel, smem, "scatter1 smem attribute")) return 0;
+        tp_scatter1_csr_kernel<<<l.tiles1, kTpThreads1, smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.K, l.one,
+                                                                        l.gran_row, l.tmp_key, l.tmp_val);
+    } else {
+        const std::size_t smem = tp_scatter1_coo_smem(l.K);
+        if (!tp_smem(tp_scatter1_coo_kernel, smem, "scatter1 smem attribute")) return 0;
+        tp_scatter1_coo_kernel<<<l.tiles1, kTpThreadsCoo, smem, stream>>>(key, val, pay, pay_map, uDim, nnz, l.low_bits,
+                                                                          l.K, l.one, l.tmp_key, l.tmp_val);
+    }
     return launch_ok("tp_scatter1_kernel");
 }
 
@@ -1034,10 +1414,10 @@ int transpose2_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t
                       const tp2_layout &l, cudaStream_t stream) {
     tp_gran_rows_kernel<<<(cDim + 255u) / 256u, 256, 0, stream>>>(ptr, cDim, l.gran_row);
     if (!launch_ok("tp_gran_rows_kernel")) return 0;
-    return tp_first_pass<false>(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, l, stream) &&
+    return tp_first_pass(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, l, stream) &&
            ((double) nnz >= kTpRowsKernelMin * (double) cDim * (double) l.K
-                ? tp_second_pass<(int) kTpBucketBits, true>(uDim, l, out_ptr, out_idx, out_val, stream)
-                : tp_second_pass<(int) kTpBucketBits, false>(uDim, l, out_ptr, out_idx, out_val, stream));
+                ? tp_second_pass<(int) kTpBucketBits, tp_rank::rows>(uDim, l, out_ptr, out_idx, out_val, stream)
+                : tp_second_pass<(int) kTpBucketBits, tp_rank::ballots>(uDim, l, out_ptr, out_idx, out_val, stream));
 }
 
 uint32_t bits_below(uint64_t v) { // bits that hold 0 .. v - 1
@@ -1101,11 +1481,11 @@ int transpose_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t 
     return launch_ok("tr_scatter_kernel");
 }
 
-// COO entries in row order (stable: a row's entries keep their order): row
-// pointers, columns (through `map` when given) and values.  Every row is below
-// `rows` and every mapped column below `cols`.  Two passes move 22 bytes an
-// entry in runs; the two stable 32-bit sorts and the random gathers that this
-// replaces moved over 100, most of them one sector per entry.
+// COO entries by rows: row pointers, columns (through `map` when given) and
+// values, a row's entries in any order.  Every row is below `rows` and every
+// mapped column below `cols`.  Two passes move 22 bytes an entry in runs; the
+// two stable 32-bit sorts and the random gathers that this replaces moved over
+// 100, most of them one sector per entry.
 std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t cols) {
     const uint32_t lb = partition_low_bits(rows, cols);
     if (n == 0u || rows == 0u || lb == 0u) return 0u;
@@ -1129,13 +1509,55 @@ int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row
         return 0;
     }
     if (!cuda_ok(cudaMemsetAsync(l.status, 0, 16, stream), "partition status memset") ||
-        !tp_first_pass<true>(0u, rows, n, nullptr, row, val, col, map, l, stream))
+        !tp_first_pass(0u, rows, n, nullptr, row, val, col, map, l, stream))
         return 0;
     switch (lb) {
-        case 8u: return tp_second_pass<8, false>(rows, l, out_ptr, out_col, out_val, stream);
-        case 9u: return tp_second_pass<9, false>(rows, l, out_ptr, out_col, out_val, stream);
-        case 10u: return tp_second_pass<10, false>(rows, l, out_ptr, out_col, out_val, stream);
-        default: return tp_second_pass<11, false>(rows, l, out_ptr, out_col, out_val, stream);
+        case 8u: return tp_second_pass<8, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
+        case 9u: return tp_second_pass<9, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
+        case 10u: return tp_second_pass<10, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
+        default: return tp_second_pass<11, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
+    }
+}
+
+// The same entries again in their own order (stable), where *flag is set, from
+// the pass-1 offsets and chunks that partition_rows left in `scratch` (a chunk
+// may end inside a tile's run, so its counts are taken anew); *nnz_count is
+// cleared with it.  Where the flag is clear, the launches are all it costs.
+template <int LB>
+static int partition_rows_stable_lb(uint32_t rows, const tp2_layout &l, const uint32_t *flag, const uint32_t *row_ptr,
+                                    uint32_t *out_col, uint16_t *out_val, cudaStream_t stream) {
+    constexpr std::size_t smem = tp_scatter2_smem(LB);
+    if (!tp_count_chunks<LB>(flag, rows, l, const_cast<uint32_t *>(row_ptr), stream)) return 0; // read only
+    if (!tp_smem(tp_scatter2_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
+    tp_scatter2_kernel<LB><<<resident_grid((const void *) tp_scatter2_kernel<LB>, kTpThreads, smem, l.max_chunks),
+                             kTpThreads, smem, stream>>>(flag, l.tmp_key, l.tmp_val, l.chunk_range, l.max_chunks, l.two,
+                                                         out_col, out_val);
+    return launch_ok("tp_scatter2_kernel");
+}
+
+int partition_rows_stable(const uint32_t *flag, uint32_t *nnz_count, uint32_t n, uint32_t rows, uint32_t cols,
+                          const uint32_t *row, const uint32_t *col, const uint32_t *map, const uint16_t *val,
+                          const uint32_t *row_ptr, uint32_t *out_col, uint16_t *out_val, void *scratch,
+                          std::size_t scratch_bytes, cudaStream_t stream) {
+    const uint32_t lb = partition_low_bits(rows, cols);
+    tp2_layout l;
+    tp2_make_layout(rows, n, lb == 0u ? kTpBucketBits : lb, false, scratch, scratch_bytes, &l);
+    if (n == 0u || rows == 0u || lb == 0u || scratch == nullptr || l.bytes > scratch_bytes) {
+        set_error("partition_rows_stable: outside its range");
+        return 0;
+    }
+    const std::size_t smem = tp_scatter1_smem(l.K);
+    if (!tp_smem(tp_scatter1_coo_stable_kernel, smem, "scatter1 smem attribute")) return 0;
+    tp_scatter1_coo_stable_kernel<<<resident_grid((const void *) tp_scatter1_coo_stable_kernel, kTpThreads, smem,
+                                                  l.tiles1),
+                                    kTpThreads, smem, stream>>>(flag, nnz_count, row, val, rows, n, l.low_bits, l.K,
+                                                                l.tiles1, l.one, col, map, l.tmp_key, l.tmp_val);
+    if (!launch_ok("tp_scatter1_kernel")) return 0;
+    switch (lb) {
+        case 8u: return partition_rows_stable_lb<8>(rows, l, flag, row_ptr, out_col, out_val, stream);
+        case 9u: return partition_rows_stable_lb<9>(rows, l, flag, row_ptr, out_col, out_val, stream);
+        case 10u: return partition_rows_stable_lb<10>(rows, l, flag, row_ptr, out_col, out_val, stream);
+        default: return partition_rows_stable_lb<11>(rows, l, flag, row_ptr, out_col, out_val, stream);
     }
 }
 

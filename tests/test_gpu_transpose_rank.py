@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 def _csr(rows, cols, per_row, seed, repeat=0, unsorted=False):
     rng = np.random.default_rng(seed)
     n = rng.poisson(per_row, rows)
+    n[rng.integers(0, rows, rows // 3)] = 0
     row = np.repeat(np.arange(rows), n)
     col = rng.integers(0, cols, len(row))
     key = np.unique(row.astype(np.int64) * cols + col)  # each cell once, columns ascending
@@ -41,6 +42,8 @@ def _csr(rows, cols, per_row, seed, repeat=0, unsorted=False):
     (1_153, 513, 30, 0, False),        # the span's edge, a bucket of one column
     (40, 262_144, 3_000, 0, False),    # the most buckets, chunks far from full
     (8_192, 1, 0.9, 0, False),         # one column
+    (8_192, 3_000, 1.2, 4, True),      # tiles of thousands of rows: pointers searched
+    (3, 100_000, 20_000, 0, False),    # rows of several tiles
 ])
 def test_transpose_ranks(cuda, orc, rows, cols, per_row, repeat, unsorted):
     from cellshard_b200.device import transpose
@@ -50,4 +53,20 @@ def test_transpose_ranks(cuda, orc, rows, cols, per_row, repeat, unsorted):
     rptr, ridx, rval = orc.csr_transpose(rows, cols, ptr, idx, val)
     assert np.array_equal(np_u32(t.ptr), rptr)
     assert np.array_equal(np_u32(t.idx), ridx)
+    assert np.array_equal(np_u16(t.val), rval)
+
+
+@pytest.mark.parametrize("gap", [30_000, 100_000])
+def test_gap_of_empty_rows_inside_a_tile(cuda, orc, gap):
+    """Two rows of entries with thousands of empty rows between and after them."""
+    from cellshard_b200.device import transpose
+
+    cols = 600
+    idx = np.concatenate([np.arange(0, cols, 2), np.arange(0, cols, 3)]).astype(np.uint32)
+    ptr = np.zeros(gap + 8, np.uint32)
+    ptr[3:gap], ptr[gap:] = 300, 500
+    val = np.arange(1, 501, dtype=np.uint16)
+    t = transpose(to_device_csr(gap + 7, cols, ptr, idx, val))
+    rptr, ridx, rval = orc.csr_transpose(gap + 7, cols, ptr, idx, val)
+    assert np.array_equal(np_u32(t.ptr), rptr) and np.array_equal(np_u32(t.idx), ridx)
     assert np.array_equal(np_u16(t.val), rval)
