@@ -27,20 +27,18 @@
 //   of one slice, cost = fixed packed bytes + 6 bytes per slot, a segment as
 //   wide as its last row, exactly `requested` non-empty segments before
 //   equal-width neighbours merge) with its monotone convex-hull and its tie
-//   rules.  The programme is sequential over the sorted widths: it runs on the
-//   host over the widths copied back (4 bytes per row), as in the reference,
-//   its levels pipelined over host threads; counting, sorting and copying run
-//   on the device.  One programme of 8
-//   levels serves all eight candidates of choose_bucket_count_for_sliced_part
-//   (:1572-1596): level k's costs and cuts do not depend on how many levels
-//   follow.
+//   rules.  Every split it can choose cuts between two widths (see
+//   sliced_split), so it runs on the host over the distinct widths and their
+//   row counts -- a histogram filled by the counting kernel -- while the device
+//   sorts; only a part with fewer distinct widths than buckets goes row by row.
+//   One programme of 8 levels serves all eight candidates of
+//   choose_bucket_count_for_sliced_part (:1572-1596): level k's costs and cuts
+//   do not depend on how many levels follow.
 #include "common.cuh"
 
-#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
-#include <thread>
 #include <vector>
 
 namespace csb {
@@ -564,25 +562,41 @@ __device__ __forceinline__ uint32_t slice_of(const cs_sliced_ell_view &v, uint32
     return lo;
 }
 
+// Live slots of every row, a warp per row, eight loads a lane in flight;
+// hist (null: not wanted) counts the rows of each width.
 __global__ void __launch_bounds__(256) sell_row_width_kernel(const cs_sliced_ell_view src,
-                                                             uint32_t *__restrict__ widths) {
+                                                             uint32_t *__restrict__ widths,
+                                                             uint32_t *__restrict__ hist) {
     const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < src.rows; row += warps) {
         const uint32_t s = slice_of(src, row);
         uint32_t n = 0u;
         if (s < src.slice_count) {
             const uint32_t w = src.slice_widths[s];
-            const uint32_t *c = src.col_idx + src.slice_slot_offsets[s] + (std::size_t) (row - src.slice_row_offsets[s]) * w;
-            for (uint32_t k = lane; k < w; k += 32u) n += __ldg(c + k) != kInvalid;
+            const uint32_t *c = src.col_idx + src.slice_slot_offsets[s] +
+                                (std::size_t) (row - src.slice_row_offsets[s]) * w;
+            constexpr unsigned U = 8;
+            for (uint32_t k0 = lane; k0 < w; k0 += 32u * U) {
+                uint32_t x[U];
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u) x[u] = k0 + 32u * u < w ? __ldcs(c + k0 + 32u * u) : kInvalid;
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u) n += x[u] != kInvalid;
+            }
         }
         n = __reduce_add_sync(0xffffffffu, n);
-        if (lane == 0u) widths[row] = n;
+        if (lane == 0u) {
+            widths[row] = n;
+            if (hist != nullptr) atomicAdd(hist + n, 1u);
+        }
     }
 }
 
 // One warp per execution row: the row's live slots compacted by ballot rank,
-// padding after them.
+// padding after them.  A row is read up to its last live slot only (the plan
+// counted them): slots behind it, most of a slice's padding, are not touched.
 __global__ void __launch_bounds__(256) sell_exec_fill_kernel(const cs_sliced_ell_view src,
+                                                             const uint32_t *__restrict__ live_of,
                                                              const uint32_t *__restrict__ order,
                                                              const seg_rec *__restrict__ rec,
                                                              const plan_head *__restrict__ head,
@@ -600,6 +614,7 @@ __global__ void __launch_bounds__(256) sell_exec_fill_kernel(const cs_sliced_ell
         if (s < src.slice_count) {
             const uint32_t sw = src.slice_widths[s];
             const std::size_t base = src.slice_slot_offsets[s] + (std::size_t) (row - src.slice_row_offsets[s]) * sw;
+            const uint32_t live = live_of[row];
             // 128 slots per step: four column loads per lane; the live values of
             // a step are loaded together with the next step's columns, then four
             // ballot-ranked stores
@@ -607,28 +622,33 @@ __global__ void __launch_bounds__(256) sell_exec_fill_kernel(const cs_sliced_ell
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const uint32_t k = 32u * u + lane;
-                cn[u] = k < sw ? __ldcs(src.col_idx + base + k) : kInvalid;
+                cn[u] = k < sw && live != 0u ? __ldcs(src.col_idx + base + k) : kInvalid;
             }
-            for (uint32_t k0 = 0; k0 < sw; k0 += 128u) {
+            for (uint32_t k0 = 0; k0 < sw && off < live; k0 += 128u) {
                 uint32_t c[4];
+                unsigned m[4];
                 uint16_t x[4];
+                uint32_t after = off; // live slots up to the end of this step
 #pragma unroll
-                for (int u = 0; u < 4; ++u) c[u] = cn[u];
+                for (int u = 0; u < 4; ++u) {
+                    c[u] = cn[u];
+                    m[u] = __ballot_sync(0xffffffffu, c[u] != kInvalid);
+                    after += __popc(m[u]);
+                }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     x[u] = c[u] != kInvalid ? __ldcs(src.val + base + k0 + 32u * u + lane) : (uint16_t) 0u;
                     const uint32_t k = k0 + 128u + 32u * u + lane;
-                    cn[u] = k < sw ? __ldcs(src.col_idx + base + k) : kInvalid;
+                    cn[u] = after < live && k < sw ? __ldcs(src.col_idx + base + k) : kInvalid;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const unsigned m = __ballot_sync(0xffffffffu, c[u] != kInvalid);
                     if (c[u] != kInvalid) {
-                        const uint32_t at = off + __popc(m & ((1u << lane) - 1u));
+                        const uint32_t at = off + __popc(m[u] & ((1u << lane) - 1u));
                         dc[at] = c[u];
                         dv[at] = x[u];
                     }
-                    off += __popc(m);
+                    off += __popc(m[u]);
                 }
             }
         }
@@ -657,28 +677,36 @@ int check_sell(const cs_sliced_ell_view *part, const char *who) {
 }
 
 // The split programme (build_sliced_execution_bucket_layout :1312-1412) for
-// levels 1..K over ascending widths; cut(k, r) = first row of the last of k
-// segments covering rows [0, r).
+// levels 1..K over ascending widths.  A unit is a row, or all rows of one
+// width: unit j ends at row end[j] and has width w[j]; cut(k, j) = first unit
+// of the last of k segments covering units [0, j).
+//
+// Units of whole widths give the row programme's cuts exactly while K is at
+// most the number of widths.  All k-segment splits pay the same fixed bytes.
+// A cut inside the rows of one width v costs as much as no cut where its
+// segment ends at width v too, and strictly more than the cut behind those rows
+// where it ends wider; with at most as many segments as widths some cut between
+// widths is then unused, and adding it saves (wider - narrower) slots for each
+// row before it.  So every optimal split cuts between widths only, at every
+// level of the traceback, and the smallest optimal cut is the same in both.
+// (The hull's tie rule is just that: of concurrent lines the middle one goes,
+// and the pointer stays on a tie, so a query returns its smallest minimiser.)
 struct sliced_split {
-    uint32_t rows = 0, K = 0;
-    std::unique_ptr<uint32_t[]> cuts; // (K + 1) x (rows + 1)
-    std::vector<uint64_t> cost_at_rows; // level k's cost of all rows
+    uint32_t units = 0, K = 0;
+    std::vector<uint32_t> end; // [units + 1], end[0] = 0
+    std::vector<uint32_t> cuts; // (K + 1) x (units + 1)
+    std::vector<uint64_t> cost_at_end; // level k's cost of all units
 
     static constexpr uint64_t kInf = ~0ull / 4u;
-    static constexpr uint32_t kBlockRows = 4096u;
 
     struct line {
         int64_t slope, icpt;
         uint32_t cut;
     };
 
-    // One level over rows k..rows: prev = level k-1's costs, curr = this
-    // level's.  When `ready` is set, level k-1 runs in another thread and
-    // `ready` holds the last row it has finished: rows are taken in blocks
-    // once the previous level has passed them (bounded only by its progress,
-    // which always advances).
-    void level(uint32_t k, const std::vector<uint32_t> &w, const uint64_t *prev, uint64_t *curr,
-               const std::atomic<uint32_t> *ready, std::atomic<uint32_t> *done) {
+    // One level over units k..all: prev = level k-1's costs, curr = this level's.
+    void level(uint32_t k, const std::vector<uint32_t> &w, const std::vector<uint64_t> &prev,
+               std::vector<uint64_t> &curr, std::vector<line> &hull) {
         const uint64_t fixed = packed_sell_bytes(1u, 0u), slot = 6u;
         auto at = [](const line &l, uint32_t x) { return l.icpt + l.slope * (int64_t) x; };
         auto redundant = [](const line &a, const line &m, const line &b) {
@@ -686,104 +714,69 @@ struct sliced_split {
             const __int128 right = (__int128) (m.icpt - a.icpt) * (__int128) (a.slope - b.slope);
             return left <= right;
         };
-        std::unique_ptr<line[]> hull(new line[(std::size_t) rows + 1u]); // written before read
         std::size_t n = 0u, h = 0u;
-        uint32_t *cut = cuts.get() + (std::size_t) k * (rows + 1u);
-        uint32_t avail = ready != nullptr ? ready->load(std::memory_order_acquire) : rows;
-        while (avail < k - 1u) {
-            std::this_thread::yield();
-            avail = ready->load(std::memory_order_acquire);
-        }
-        if (prev[k - 1u] != kInf) hull[n++] = line{-(int64_t) slot * (int64_t) (k - 1u), (int64_t) prev[k - 1u], k - 1u};
-        for (uint32_t r0 = k; r0 <= rows; r0 += kBlockRows) {
-            const uint32_t r1 = r0 + kBlockRows - 1u < rows ? r0 + kBlockRows - 1u : rows;
-            while (avail < r1) {
-                std::this_thread::yield();
-                avail = ready->load(std::memory_order_acquire);
+        uint32_t *cut = cuts.data() + (std::size_t) k * (units + 1u);
+        if (prev[k - 1u] != kInf)
+            hull[n++] = line{-(int64_t) slot * (int64_t) end[k - 1u], (int64_t) prev[k - 1u], k - 1u};
+        for (uint32_t j = k; j <= units; ++j) {
+            const uint32_t x = w[j - 1u];
+            while (h + 1u < n && at(hull[h + 1u], x) < at(hull[h], x)) ++h;
+            if (h < n) {
+                curr[j] = fixed + slot * (uint64_t) x * (uint64_t) end[j] + (uint64_t) at(hull[h], x);
+                cut[j] = hull[h].cut;
+            } else {
+                curr[j] = kInf;
+                cut[j] = 0u;
             }
-            for (uint32_t r = r0; r <= r1; ++r) {
-                const uint32_t x = w[r - 1u];
-                while (h + 1u < n && at(hull[h + 1u], x) < at(hull[h], x)) ++h;
-                if (h < n) {
-                    curr[r] = fixed + slot * (uint64_t) x * (uint64_t) r + (uint64_t) at(hull[h], x);
-                    cut[r] = hull[h].cut;
-                } else {
-                    curr[r] = kInf;
-                    cut[r] = 0u;
-                }
-                if (prev[r] != kInf) {
-                    const line l{-(int64_t) slot * (int64_t) r, (int64_t) prev[r], r};
-                    while (n >= h + 2u && redundant(hull[n - 2u], hull[n - 1u], l)) --n;
-                    hull[n++] = l;
-                }
+            if (prev[j] != kInf) {
+                const line l{-(int64_t) slot * (int64_t) end[j], (int64_t) prev[j], j};
+                while (n >= h + 2u && redundant(hull[n - 2u], hull[n - 1u], l)) --n;
+                hull[n++] = l;
             }
-            if (done != nullptr) done->store(r1, std::memory_order_release);
         }
-        if (done != nullptr) done->store(rows, std::memory_order_release);
     }
 
-    // Levels 1..K.  Each level's loop is sequential (its hull depends on every
-    // earlier row), but level k only needs level k-1's costs of rows up to the
-    // one it is at, so the levels run as a pipeline, one thread each, level k
-    // a block of rows behind level k-1; every cost and cut is the one the
-    // sequential order computes.
-    bool run(const std::vector<uint32_t> &w, uint32_t levels) {
-        rows = (uint32_t) w.size();
+    // Levels 1..K; `ends` holds the row that each unit ends at.
+    void run(const std::vector<uint32_t> &w, const std::vector<uint32_t> &ends, uint32_t levels) {
+        units = (uint32_t) w.size();
         K = levels;
-        // level 0: no rows cost 0, any row unreachable; a level k >= 1 writes
-        // every entry r >= k, the only ones level k + 1 reads
-        std::vector<std::unique_ptr<uint64_t[]>> cost((std::size_t) K + 1u);
-        for (auto &c : cost) c.reset(new uint64_t[(std::size_t) rows + 1u]);
-        for (uint32_t r = 0; r <= rows; ++r) cost[0][r] = r == 0u ? 0u : kInf;
-        cuts.reset(new uint32_t[((std::size_t) K + 1u) * ((std::size_t) rows + 1u)]);
-        cost_at_rows.assign((std::size_t) K + 1u, kInf);
-        const unsigned hw = std::thread::hardware_concurrency();
-        if (K <= 1u || rows < 2u * kBlockRows || K > 16u || hw < 2u) {
-            for (uint32_t k = 1; k <= K; ++k) level(k, w, cost[k - 1u].get(), cost[k].get(), nullptr, nullptr);
-        } else {
-            std::vector<std::atomic<uint32_t>> progress((std::size_t) K + 1u);
-            progress[0].store(rows);
-            for (uint32_t k = 1; k <= K; ++k) progress[k].store(0u);
-            std::vector<std::thread> th;
-            th.reserve(K);
-            uint32_t started = 0u;
-            try {
-                for (uint32_t k = 1; k <= K; ++k, ++started)
-                    th.emplace_back([&, k] { level(k, w, cost[k - 1u].get(), cost[k].get(), &progress[k - 1u],
-                                                   &progress[k]); });
-            } catch (...) {
-                // no thread for level `started + 1`: the remaining levels run here,
-                // after the started ones (each still waits on its predecessor)
-            }
-            for (uint32_t k = started + 1u; k <= K; ++k)
-                level(k, w, cost[k - 1u].get(), cost[k].get(), &progress[k - 1u], &progress[k]);
-            for (auto &t : th) t.join();
+        end.assign(1, 0u);
+        end.insert(end.end(), ends.begin(), ends.end());
+        // level 0: no units cost 0, any unit unreachable; a level k >= 1 writes
+        // every entry j >= k, the only ones level k + 1 reads
+        std::vector<uint64_t> prev((std::size_t) units + 1u, kInf), curr((std::size_t) units + 1u, kInf);
+        std::vector<line> hull((std::size_t) units + 1u);
+        prev[0] = 0u;
+        cuts.assign(((std::size_t) K + 1u) * ((std::size_t) units + 1u), 0u);
+        cost_at_end.assign((std::size_t) K + 1u, kInf);
+        for (uint32_t k = 1; k <= K; ++k) {
+            level(k, w, prev, curr, hull);
+            cost_at_end[k] = curr[units];
+            prev.swap(curr);
         }
-        for (uint32_t k = 1; k <= K; ++k) cost_at_rows[k] = cost[k][rows];
-        return true;
     }
     // Segments of the k-level split after equal-width neighbours merge.
     bool layout(const std::vector<uint32_t> &w, uint32_t k, std::vector<uint32_t> *offs,
                 std::vector<uint32_t> *widths) const {
         offs->assign(1, 0u);
         widths->clear();
-        if (rows == 0u) return true;
-        if (cost_at_rows[k] == kInf) return false;
+        if (units == 0u) return true;
+        if (cost_at_end[k] == kInf) return false;
         std::vector<uint32_t> raw_off((std::size_t) k + 1u), raw_w(k);
-        uint32_t r = rows;
-        raw_off[k] = rows;
-        for (uint32_t j = k; j != 0u; --j) {
-            const uint32_t begin = cuts.get()[(std::size_t) j * (rows + 1u) + r];
-            raw_off[j - 1u] = begin;
-            raw_w[j - 1u] = w[r - 1u];
-            r = begin;
+        uint32_t j = units;
+        raw_off[k] = end[units];
+        for (uint32_t q = k; q != 0u; --q) {
+            const uint32_t begin = cuts[(std::size_t) q * (units + 1u) + j];
+            raw_off[q - 1u] = end[begin];
+            raw_w[q - 1u] = w[j - 1u];
+            j = begin;
         }
-        for (uint32_t j = 0; j < k; ++j) {
-            if (!widths->empty() && widths->back() == raw_w[j]) {
-                offs->back() = raw_off[j + 1u];
+        for (uint32_t q = 0; q < k; ++q) {
+            if (!widths->empty() && widths->back() == raw_w[q]) {
+                offs->back() = raw_off[q + 1u];
             } else {
-                widths->push_back(raw_w[j]);
-                offs->push_back(raw_off[j + 1u]);
+                widths->push_back(raw_w[q]);
+                offs->push_back(raw_off[q + 1u]);
             }
         }
         return true;
@@ -833,17 +826,58 @@ int sell_plan(const cs_sliced_ell_view *part, uint32_t requested, void *scratch,
         set_error("bucketed_sliced_ell_plan: %llu slots but null columns or values", (unsigned long long) total);
         return 0;
     }
-    std::vector<uint32_t> w(rows);
+    // the rows' widths as (width, rows up to its last): from a histogram in the
+    // place of the sorted widths, or, where widths outnumber rows, from those
+    std::vector<uint32_t> w, ends;
     if (rows != 0u) {
-        sell_row_width_kernel<<<resident_grid((const void *) sell_row_width_kernel, 256, 0, ((std::size_t) rows + 7u) / 8u),
-                                256, 0, stream>>>(*part, x.widths);
-        if (!launch_ok("sell_row_width_kernel")) return 0;
-        if (!sort_pairs_u32(x.widths, nullptr, rows, x.sorted, x.order, x.sort_tmp, x.sort_bytes, stream)) return 0;
-        if (!cuda_ok(cudaMemcpyAsync(w.data(), x.sorted, (std::size_t) rows * 4u, cudaMemcpyDeviceToHost, stream),
-                     "D2H sorted widths") ||
-            !cuda_ok(cudaStreamSynchronize(stream), "plan sync"))
+        uint32_t widest = 0u;
+        for (const uint32_t sw : src_w) widest = widest > sw ? widest : sw;
+        const bool counted = widest <= rows; // x.sorted has rows + 1 words
+        uint32_t *hist = counted ? x.sorted : nullptr;
+        if (counted && !cuda_ok(cudaMemsetAsync(hist, 0, ((std::size_t) widest + 1u) * 4u, stream), "width histogram"))
             return 0;
+        sell_row_width_kernel<<<resident_grid((const void *) sell_row_width_kernel, 256, 0,
+                                              ((std::size_t) rows + 7u) / 8u),
+                                256, 0, stream>>>(*part, x.widths, hist);
+        if (!launch_ok("sell_row_width_kernel")) return 0;
+        if (counted) {
+            std::vector<uint32_t> of((std::size_t) widest + 1u);
+            if (!cuda_ok(cudaMemcpyAsync(of.data(), hist, of.size() * 4u, cudaMemcpyDeviceToHost, stream),
+                         "D2H width histogram") ||
+                !cuda_ok(cudaStreamSynchronize(stream), "width sync"))
+                return 0;
+            uint32_t upto = 0u;
+            for (uint32_t v = 0; v <= widest; ++v) {
+                if (of[v] == 0u) continue;
+                upto += of[v];
+                w.push_back(v);
+                ends.push_back(upto);
+            }
+        }
+        if (!sort_pairs_u32(x.widths, nullptr, rows, x.sorted, x.order, x.sort_tmp, x.sort_bytes, stream)) return 0;
+        if (!counted) {
+            std::vector<uint32_t> sorted(rows);
+            if (!cuda_ok(cudaMemcpyAsync(sorted.data(), x.sorted, (std::size_t) rows * 4u, cudaMemcpyDeviceToHost,
+                                         stream), "D2H sorted widths") ||
+                !cuda_ok(cudaStreamSynchronize(stream), "plan sync"))
+                return 0;
+            for (uint32_t r = 0; r < rows; ++r) {
+                if (w.empty() || w.back() != sorted[r]) {
+                    w.push_back(sorted[r]);
+                    ends.push_back(r);
+                }
+                ends.back() = r + 1u;
+            }
+        }
     }
+    auto by_rows = [](const std::vector<uint32_t> &gw, const std::vector<uint32_t> &ge, std::vector<uint32_t> *rw,
+                      std::vector<uint32_t> *re) {
+        for (std::size_t g = 0; g < gw.size(); ++g)
+            for (uint32_t r = g == 0u ? 0u : ge[g - 1u]; r < ge[g]; ++r) {
+                rw->push_back(gw[g]);
+                re->push_back(r + 1u);
+            }
+    };
     plan_head h{};
     h.units = rows;
     h.block_size = 1u;
@@ -853,7 +887,13 @@ int sell_plan(const cs_sliced_ell_view *part, uint32_t requested, void *scratch,
     if (rows != 0u) {
         sliced_split dp;
         const uint32_t levels = bound;
-        dp.run(w, levels);
+        if (levels > w.size()) { // more segments than widths: rows of one width get split
+            std::vector<uint32_t> rw, re;
+            by_rows(w, ends, &rw, &re);
+            w.swap(rw);
+            ends.swap(re);
+        }
+        dp.run(w, ends, levels);
         auto kept = [&](uint32_t b, std::vector<uint32_t> *o, std::vector<uint32_t> *wd, uint64_t *bytes) {
             if (!dp.layout(w, b, o, wd)) return false;
             *bytes = sliced_layout_bytes(*o, *wd);
@@ -888,9 +928,11 @@ int sell_plan(const cs_sliced_ell_view *part, uint32_t requested, void *scratch,
     std::vector<char> host(sizeof(plan_head) + ((std::size_t) h.S + 1u) * sizeof(seg_rec));
     seg_rec *rec = (seg_rec *) (host.data() + sizeof(plan_head));
     uint64_t slots = 0u;
+    std::size_t unit = 0u;
     for (uint32_t s = 0; s < h.S; ++s) {
         uint32_t nnz = 0u; // the reference's u32 sum of the rows' live slots
-        for (uint32_t p = offs[s]; p < offs[s + 1u]; ++p) nnz += w[p];
+        for (; unit < w.size() && ends[unit] <= offs[s + 1u]; ++unit)
+            nnz += w[unit] * (ends[unit] - (unit == 0u ? 0u : ends[unit - 1u]));
         rec[s] = seg_rec{offs[s], offs[s], widths[s], 0u, slots, slots, nnz};
         slots += (uint64_t) (offs[s + 1u] - offs[s]) * widths[s];
     }
@@ -925,7 +967,7 @@ int sell_fill(const cs_sliced_ell_view *part, const void *scratch, const cs_exec
     exec_scratch x;
     carve(const_cast<void *>(scratch), part->rows, 1u, &x);
     sell_exec_fill_kernel<<<resident_grid((const void *) sell_exec_fill_kernel, 256, 0, ((std::size_t) part->rows + 7u) / 8u),
-                            256, 0, stream>>>(*part, x.order, x.rec, x.head, seg_col, seg_val, e2c, c2e);
+                            256, 0, stream>>>(*part, x.widths, x.order, x.rec, x.head, seg_col, seg_val, e2c, c2e);
     return launch_ok("sell_exec_fill_kernel");
 }
 

@@ -376,12 +376,11 @@ def bucketed_sliced_ell(sell: SlicedELL, requested: int, stream=None) -> Buckete
     _abi.check(lib.cs_b200_bucketed_sliced_ell_fill(C.byref(v), ptr(scratch), C.byref(plan), col.data_ptr(),
                                                     val.data_ptr(), ptr(e2c), ptr(c2e), s), "bucketed_sliced_ell_fill")
     segments, o = [], 0
-    for k in range(S):
-        n, w = int(unit_off[k + 1] - unit_off[k]), int(widths[k])
-        z = torch.zeros(1, dtype=torch.int32, device="cuda")
-        segments.append(SlicedELL(n, sell.cols, 0, n, torch.tensor([0, n], dtype=torch.int32, device="cuda"),
-                                  torch.tensor([w], dtype=torch.int32, device="cuda"), z,
-                                  col[o:o + n * w], val[o:o + n * w]))
+    # every segment's one-slice table in one upload: row offsets [0, n], width, slot offset 0
+    sizes = [(int(unit_off[k + 1] - unit_off[k]), int(widths[k])) for k in range(S)]
+    tables = torch.tensor([[0, n, w, 0] for n, w in sizes] or [[0] * 4], dtype=torch.int64).to(torch.int32).cuda()
+    for t, (n, w) in zip(tables.unbind(), sizes):
+        segments.append(SlicedELL(n, sell.cols, 0, n, t[0:2], t[2:3], t[3:4], col[o:o + n * w], val[o:o + n * w]))
         o += n * w
     return BucketedPartition(_plan_dict(plan), segments, [int(x) for x in row_off[:S + 1]], e2c, c2e, None, None,
                              col, val)
