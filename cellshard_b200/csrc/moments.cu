@@ -31,7 +31,7 @@ constexpr unsigned kSortThreads = 256; // 8 warps x 128 rows
 constexpr unsigned kSortWarps = kSortThreads / 32;
 constexpr unsigned kAccThreads = 256;
 constexpr unsigned kBatch = 8;         // rows per fp32 batch sum
-constexpr unsigned kDefaultChunkRows = 2048;
+constexpr unsigned kDefaultChunkRows = 2048; // the most that is taken by default
 constexpr unsigned kMaxChunkRows = 8192;
 constexpr unsigned kIndexWarps = 4;
 constexpr unsigned kMaxIndexWords = 2048; // column blocks / 32 per row block
@@ -57,6 +57,25 @@ struct moments_layout {
     uint32_t row_blocks, words, tiles, max_chunks, chunk_rows, col_blocks;
 };
 
+// Rows per chunk where the caller leaves it open.  A chunk's CTAs walk its rows
+// one batch after the other, so a small matrix in chunks of 2,048 rows runs on a
+// few SMs (8,192 x 2,000, 8 groups: 12 CTAs); every chunk costs 32 bytes of
+// partials a column, 16 / chunk_rows of the rows' own bytes.  Halved to 256
+// rows (6 %) while there are under 1,000 CTAs, and on to 64 only while there
+// are under two per SM.  us per call by 2,048 / 256 / 64 rows: 8,192 x 2,000
+// 95 / 49 / 33; 100,000 x 5,000 (16 groups) 349 / 179 / 258; 20,000 x 8,000 (64
+// groups) 80 / 80 / 103; 50,000 x 32,768 493 / 531 / 735 (1,024 taken: 494).
+uint32_t default_chunk_rows(uint32_t rows, uint32_t col_blocks, uint32_t block_size, uint32_t groups) {
+    const uint64_t segs = (uint64_t) col_blocks * ((block_size + 7u) / 8u);
+    const uint64_t tiles = (segs + kAccThreads - 1u) / kAccThreads;
+    // about half of the groups end in a chunk of their own
+    auto ctas = [&](uint32_t chunk) { return (rows / chunk + groups / 2u) * tiles; };
+    uint32_t chunk = kDefaultChunkRows;
+    while (chunk > 256u && ctas(chunk) < 1000u) chunk /= 2u;
+    while (chunk > 64u && ctas(chunk) < 296u) chunk /= 2u;
+    return chunk;
+}
+
 bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *p, void *base, std::size_t cap,
                  moments_layout *lay) {
     const uint32_t B = src->block_size;
@@ -64,7 +83,7 @@ bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *
     lay->col_blocks = (src->cols + B - 1u) / B;
     lay->words = (lay->col_blocks + 31u) / 32u;
     lay->tiles = (src->rows + kTileRows - 1u) / kTileRows;
-    lay->chunk_rows = p->chunk_rows == 0u ? kDefaultChunkRows : p->chunk_rows;
+    lay->chunk_rows = p->chunk_rows == 0u ? default_chunk_rows(src->rows, lay->col_blocks, B, p->group_count) : p->chunk_rows;
     const std::size_t G = p->group_count;
     lay->max_chunks = (uint32_t) ((src->rows + lay->chunk_rows - 1u) / lay->chunk_rows + G);
     scratch_carver c(base, cap);
@@ -463,6 +482,7 @@ __global__ void __launch_bounds__(256) moments_combine_kernel(
     if (kept) {
         if (scheme == CS_MOMENTS_TWOSUM_F64_COMBINE) {
             double s = 0.0, q = 0.0;
+#pragma unroll 8
             for (uint32_t c = c0; c < c1; ++c) {
                 const float *p = partials + (std::size_t) c * 4u * cols;
                 s += (double) p[f] + (double) p[cols + f];

@@ -72,6 +72,14 @@ extern "C" int cs_b200_group_moments_blocked_ell_noalloc(const cs_blocked_ell_vi
                                                           const uint8_t *d_feature_keep, const uint32_t *d_row_labels,
                                                           const cs_group_moments_params *params,
                                                           const cs_group_moments_out *out, cs_stream_t stream) {
+    // chunks of 2,048 rows by default: shorter ones, which the entry point with
+    // caller scratch takes for small matrices, would need more of the static array
+    cs_group_moments_params whole;
+    if (params != nullptr && params->chunk_rows == 0u) {
+        whole = *params;
+        whole.chunk_rows = 2048u;
+        params = &whole;
+    }
     const std::size_t need = group_moments_scratch_needed(src, params);
     if (need == 0) return 0;
     if (need > (std::size_t) CS_NOALLOC_SCRATCH_BYTES) {

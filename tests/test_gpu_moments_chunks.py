@@ -1,0 +1,58 @@
+"""Grouped moments where the default chunk size differs (64 rows on small
+matrices up to 2,048): whole counts, so every sum is exact in 64 bits; the
+allocation-free entry point accepts what its static scratch always held."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from cases import random_csr, to_device_csr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,cols,density,block,groups", [
+    (1, 40, 0.5, 8, 3),
+    (2_047, 333, 0.05, 16, 1),
+    (5_000, 2_100, 0.01, 32, 300),
+    (20_000, 700, 0.02, 8, 2),
+    (3_001, 9_000, 0.004, 16, 5),
+])
+def test_default_chunks(cuda, rows, cols, density, block, groups):
+    import torch
+
+    from cellshard_b200 import _abi, runtime
+    from cellshard_b200.device import blocked_ell_from_csr, ptr as dptr, stream_handle
+
+    p, idx, val = random_csr(rows, cols, density, rows, 0.1)
+    bell = blocked_ell_from_csr(to_device_csr(rows, cols, p, idx, val), block)
+    rng = np.random.default_rng(rows)
+    keep, lab = rng.random(rows) < 0.8, rng.integers(0, groups, rows)
+    rk = torch.from_numpy(keep.astype(np.uint8)).cuda()
+    labels = torch.from_numpy(lab.astype(np.int32)).cuda()
+    row = np.repeat(np.arange(rows), np.diff(p.astype(np.int64)))
+    x = val.view(np.float16).astype(np.float64)
+    ok = keep[row]
+    want = [np.zeros((groups, cols)), np.zeros((groups, cols))]
+    for w, v in zip(want, (x, x * x)):
+        np.add.at(w, (lab[row][ok], idx[ok].astype(np.int64)), v[ok])
+    got = runtime.compute_sparse_group_moments(bell, groups, rk, None, labels)
+    for w, k in zip(want, ("sum", "sumsq")):
+        assert np.array_equal(got[k].cpu().numpy().astype(np.float64), w), k  # below 2^24: exact in fp32
+    assert np.array_equal(got["group_rows"].cpu().numpy(), np.bincount(lab[keep], minlength=groups))
+    if bell.ell_cols == 0:
+        return
+    lib = _abi.load()
+    out = {k: torch.empty(groups, cols, device="cuda") for k in ("sum", "sumsq")}
+    o = _abi.GroupMomentsOut(dptr(out["sum"]), dptr(out["sumsq"]))
+    prm, v = _abi.GroupMomentsParams(groups, 2, 1, 0), bell.view()
+    n = C.c_size_t()
+    old = _abi.GroupMomentsParams(groups, 2, 1, 2048)
+    _abi.check(lib.cs_b200_group_moments_scratch_bytes(C.byref(v), C.byref(old), C.byref(n)), "scratch")
+    done = lib.cs_b200_group_moments_blocked_ell_noalloc(C.byref(v), dptr(rk), None, dptr(labels), C.byref(prm),
+                                                         C.byref(o), stream_handle())
+    assert done == (1 if n.value <= 64 << 20 else 0)
+    if done:
+        for w, k in zip(want, ("sum", "sumsq")):
+            assert np.array_equal(out[k].cpu().numpy().astype(np.float64), w), k
