@@ -3,16 +3,21 @@
 // real (column, value) pairs go into the first n slots in CSR order, the rest
 // is padding (CS_INVALID_COL, 0) -- sliced_ell_from_compressed.cuh:49-80.
 //
-// A group of GL lanes (GL in {32, 16, 8, 4}) writes one row.  The output is
-// written 4 slots per lane with 16-byte column and 8-byte value stores once
-// base + k is a multiple of 4; the unaligned head (< 4 slots) and the tail are
-// written one slot at a time.  Requires col_idx 16-byte and val 8-byte
-// aligned.
+// A group of GL lanes (GL in {32, 16, 8, 4}) writes one row.  Real slots are
+// copied lane by lane, so loads and stores are whole lines whatever the two
+// rows' alignments, kEmitFlight of them in flight per lane before the first is
+// stored: a row is one latency per GL * kEmitFlight entries, and with 24 warps
+// an SM that latency is what bounds the copy.  (Four slots a lane with 16-byte
+// stores took eight scattered loads and one latency per 4 * GL slots.)  The
+// padding needs no loads: 16-byte column and 8-byte value stores between an
+// unaligned head and tail.  Requires col_idx 16-byte and val 8-byte aligned.
 #pragma once
 
 #include "common.cuh"
 
 namespace csb {
+
+constexpr unsigned kEmitFlight = 8;
 
 template <unsigned GL>
 __device__ __forceinline__ void sell_emit_row_vec(const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val,
@@ -20,44 +25,45 @@ __device__ __forceinline__ void sell_emit_row_vec(const uint32_t *__restrict__ i
                                                   uint32_t *__restrict__ col_idx, uint16_t *__restrict__ out_val,
                                                   unsigned gl) {
     if (n > w) n = w;
-    const uint32_t head = min((uint32_t) ((4u - (uint32_t) (base & 3u)) & 3u), w);
-    if (gl < head) {
-        const bool real = gl < n;
-        col_idx[base + gl] = real ? __ldg(idx + a + gl) : CS_INVALID_COL;
-        out_val[base + gl] = real ? __ldg(reinterpret_cast<const unsigned short *>(val) + a + gl) : (uint16_t) 0u;
-    }
-    const uint32_t body_end = head + ((w - head) & ~3u);
-    for (uint32_t k = head + 4u * gl; k < body_end; k += 4u * GL) {
-        uint4 ci;
-        uint2 vv;
-        if (k + 4u <= n) {
-            const uint32_t *ip = idx + a + k;
-            const unsigned short *vp = reinterpret_cast<const unsigned short *>(val) + a + k;
-            ci = make_uint4(__ldg(ip), __ldg(ip + 1), __ldg(ip + 2), __ldg(ip + 3));
-            vv.x = (uint32_t) __ldg(vp) | ((uint32_t) __ldg(vp + 1) << 16);
-            vv.y = (uint32_t) __ldg(vp + 2) | ((uint32_t) __ldg(vp + 3) << 16);
-        } else if (k >= n) {
-            ci = make_uint4(CS_INVALID_COL, CS_INVALID_COL, CS_INVALID_COL, CS_INVALID_COL);
-            vv = make_uint2(0u, 0u);
-        } else {
-            uint32_t c[4];
-            uint32_t v[4];
+    const uint32_t *ip = idx + a;
+    const unsigned short *vp = reinterpret_cast<const unsigned short *>(val) + a;
+    uint32_t *cp = col_idx + base;
+    uint16_t *op = out_val + base;
+    for (uint32_t k0 = gl; k0 < n; k0 += GL * kEmitFlight) {
+        uint32_t c[kEmitFlight];
+        uint16_t v[kEmitFlight];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool real = k + j < n;
-                c[j] = real ? __ldg(idx + a + k + j) : CS_INVALID_COL;
-                v[j] = real ? (uint32_t) __ldg(reinterpret_cast<const unsigned short *>(val) + a + k + j) : 0u;
+        for (unsigned u = 0; u < kEmitFlight; ++u) {
+            const uint32_t k = k0 + GL * u;
+            if (k < n) {
+                c[u] = __ldcs(ip + k);
+                v[u] = __ldcs(vp + k);
             }
-            ci = make_uint4(c[0], c[1], c[2], c[3]);
-            vv = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
         }
-        *reinterpret_cast<uint4 *>(col_idx + base + k) = ci;
-        *reinterpret_cast<uint2 *>(out_val + base + k) = vv;
+#pragma unroll
+        for (unsigned u = 0; u < kEmitFlight; ++u) {
+            const uint32_t k = k0 + GL * u;
+            if (k < n) {
+                __stcs(cp + k, c[u]);
+                __stcs(reinterpret_cast<unsigned short *>(op) + k, (unsigned short) v[u]);
+            }
+        }
     }
-    for (uint32_t k = body_end + gl; k < w; k += GL) {
-        const bool real = k < n;
-        col_idx[base + k] = real ? __ldg(idx + a + k) : CS_INVALID_COL;
-        out_val[base + k] = real ? __ldg(reinterpret_cast<const unsigned short *>(val) + a + k) : (uint16_t) 0u;
+    // padding [n, w): up to three slots to a vector boundary, vectors, a tail
+    const uint32_t head = min(w, n + ((4u - (uint32_t) ((base + n) & 3u)) & 3u));
+    const uint32_t body_end = head + ((w - head) & ~3u);
+    if (n + gl < head) {
+        cp[n + gl] = CS_INVALID_COL;
+        op[n + gl] = 0u;
+    }
+    for (uint32_t k = head + 4u * gl; k < body_end; k += 4u * GL) {
+        __stcs(reinterpret_cast<uint4 *>(cp + k),
+               make_uint4(CS_INVALID_COL, CS_INVALID_COL, CS_INVALID_COL, CS_INVALID_COL));
+        __stcs(reinterpret_cast<uint2 *>(op + k), make_uint2(0u, 0u));
+    }
+    if (body_end + gl < w) {
+        cp[body_end + gl] = CS_INVALID_COL;
+        op[body_end + gl] = 0u;
     }
 }
 
