@@ -550,17 +550,18 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     }
 }
 
-// The same for rows of up to 8 KB, a warp per row: no CTA barrier, and
-// NBUF buffers per warp.  A warp takes `unit_rows` rows of one row block, fewer
-// than B where whole row blocks would leave warps idle.
-// 8,192 x 2,000 at 6 %: 31 us; 52 with a CTA per row (512 row blocks on 444
-// CTAs, five barriers a row).  100,000 x 2,000 at 1 %: 77 us against 353.
+// The same for rows of up to 12 KB, a warp per row: no CTA barrier, and NBUF
+// buffers per warp.  A warp takes `run_rows` consecutive rows at a time, over
+// row-block borders, so that all warps get the same number of them (whole row
+// blocks, or even parts of them, left a second round to a few warps).
+// 8,192 x 2,000 at 6 %: 15 us; 52 with a CTA per row (512 row blocks on 444
+// CTAs, five barriers a row).  100,000 x 2,000 at 1 %: 86 us against 353.
 constexpr unsigned kEmitWarps = kEmitThreads / 32;
 template <int NBUF, bool kAny>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
-    uint32_t unit_rows, const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci,
+    uint32_t run_rows, const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci,
     uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
     if (kAny && order.skips()) return;
     extern __shared__ __align__(128) unsigned char tma_smem[];
@@ -573,8 +574,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
     uint2 *ix = reinterpret_cast<uint2 *>(tma_smem + (std::size_t) kEmitWarps * NBUF * stride) + warp * words;
     uint32_t *seen = reinterpret_cast<uint32_t *>(tma_smem + (std::size_t) kEmitWarps * NBUF * stride +
                                                   (std::size_t) kEmitWarps * words * sizeof(uint2)) + warp * seen_words;
-    const uint32_t row_blocks = (rows + B - 1u) / B, per_block = (B + unit_rows - 1u) / unit_rows;
-    const uint64_t units = (uint64_t) row_blocks * per_block;
+    const uint64_t runs = ((uint64_t) rows + run_rows - 1u) / run_rows;
     uint32_t my_nnz = 0u, bad = 0u, iter = 0u;
     uint32_t nc[PF];
     uint16_t nv[PF];
@@ -586,49 +586,51 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             nv[k] = i < e ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
         }
     };
-    for (uint64_t u = blockIdx.x * kEmitWarps + warp; u < units; u += (uint64_t) gridDim.x * kEmitWarps) {
-        const uint32_t rb = (uint32_t) (u / per_block), part = (uint32_t) (u % per_block);
-        const uint32_t b_end = min(rows, rb * B + B);
-        const uint32_t r_beg = min(b_end, rb * B + part * unit_rows), r_end = min(b_end, r_beg + unit_rows);
-        __syncwarp(); // the last unit's lookups are done
-        uint32_t count = 0u;
-        for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
-            const uint32_t w = w0 + lane;
-            const uint32_t word = w < words ? __ldg(bitmaps + (std::size_t) rb * words + w) : 0u;
-            const uint32_t c = __popc(word);
-            const uint32_t incl = warp_inclusive_scan(c);
-            if (w < words) ix[w] = make_uint2(word, count + incl - c);
-            count += __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t a1 = 0u, e1 = 0u; // the next row's entries, bad pointers as an empty row
+    auto bounds = [&](uint32_t r) {
+        a1 = __ldg(ptr + r);
+        e1 = __ldg(ptr + r + 1u);
+        if (e1 < a1 || e1 > nnz) {
+            bad |= CS_STATUS_BAD_POINTERS;
+            e1 = a1;
         }
-        __syncwarp();
-        if (count > width) bad |= CS_STATUS_INDEX_RANGE;
-        uint32_t a1 = 0u, e1 = 0u; // the next row's entries, bad pointers as an empty row
-        auto bounds = [&](uint32_t r) {
-            a1 = __ldg(ptr + r);
-            e1 = __ldg(ptr + r + 1u);
-            if (e1 < a1 || e1 > nnz) {
-                bad |= CS_STATUS_BAD_POINTERS;
-                e1 = a1;
-            }
-        };
-        if (r_beg < r_end) {
-            bounds(r_beg);
-            prefetch(a1, e1);
-        }
-        if (part == 0u && out_bci != nullptr) {
-            uint32_t *row_bci = out_bci + (std::size_t) rb * width;
-            for (uint32_t w = lane; w < words; w += 32u) {
-                uint32_t word = ix[w].x, pos = ix[w].y;
-                while (word != 0u) {
-                    const uint32_t bit = __ffs(word) - 1u;
-                    if (pos < width) row_bci[pos] = w * 32u + bit;
-                    ++pos;
-                    word &= word - 1u;
+    };
+    uint32_t rb_now = 0xffffffffu; // the row block that ix holds
+    for (uint64_t u = blockIdx.x * kEmitWarps + warp; u < runs; u += (uint64_t) gridDim.x * kEmitWarps) {
+        const uint32_t r_beg = (uint32_t) (u * run_rows);
+        const uint32_t r_end = (uint32_t) min((uint64_t) rows, (u + 1u) * run_rows);
+        bounds(r_beg);
+        prefetch(a1, e1);
+        for (uint32_t r = r_beg; r < r_end; ++r, ++iter) {
+            const uint32_t rb = div_b(r, B, shift);
+            if (rb != rb_now) {
+                __syncwarp(); // the last row's lookups are done
+                uint32_t count = 0u;
+                for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
+                    const uint32_t w = w0 + lane;
+                    const uint32_t word = w < words ? __ldg(bitmaps + (std::size_t) rb * words + w) : 0u;
+                    const uint32_t c = __popc(word);
+                    const uint32_t incl = warp_inclusive_scan(c);
+                    if (w < words) ix[w] = make_uint2(word, count + incl - c);
+                    count += __shfl_sync(0xffffffffu, incl, 31);
+                }
+                __syncwarp();
+                rb_now = rb;
+                if (count > width) bad |= CS_STATUS_INDEX_RANGE;
+                if (r == rb * B && out_bci != nullptr) { // the block's first row writes its columns
+                    uint32_t *row_bci = out_bci + (std::size_t) rb * width;
+                    for (uint32_t w = lane; w < words; w += 32u) {
+                        uint32_t word = ix[w].x, pos = ix[w].y;
+                        while (word != 0u) {
+                            const uint32_t bit = __ffs(word) - 1u;
+                            if (pos < width) row_bci[pos] = w * 32u + bit;
+                            ++pos;
+                            word &= word - 1u;
+                        }
+                    }
+                    for (uint32_t s2 = count + lane; s2 < width; s2 += 32u) row_bci[s2] = CS_INVALID_COL;
                 }
             }
-            for (uint32_t s2 = count + lane; s2 < width; s2 += 32u) row_bci[s2] = CS_INVALID_COL;
-        }
-        for (uint32_t r = r_beg; r < r_end; ++r, ++iter) {
             uint32_t cc[PF];
             uint16_t cv[PF];
 #pragma unroll
@@ -668,23 +670,34 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
                 buf[p] = v;
                 row_nnz += half_nonzero(v);
             };
+            // PF batches of 32 a step: the first from the prefetch, a longer row's
+            // next ones loaded together (one by one they took a latency each)
+            for (uint32_t i0 = a; i0 < e; i0 += PF * 32u) {
+                if (i0 != a) {
 #pragma unroll
-            for (int k = 0; k < PF; ++k) {
-                if (a + (uint32_t) k * 32u < e) { // uniform
-                    const uint32_t i = a + (uint32_t) k * 32u + lane;
-                    if constexpr (!kAny) {
-                        uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
-                        const uint32_t head = __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
-                        if (lane == 31u) nxt = k + 1 < PF ? head : (i + 1u < e ? __ldg(idx + i + 1u) : 0u);
-                        if (i + 1u < e && cc[k] >= nxt) unordered = 1;
+                    for (int k = 0; k < PF; ++k) {
+                        const uint32_t i = i0 + (uint32_t) k * 32u + lane;
+                        cc[k] = i < e ? __ldg(idx + i) : 0xffffffffu;
+                        cv[k] = i < e ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
                     }
-                    if (i < e) place(cc[k], cv[k]);
                 }
-            }
-            for (uint32_t i = a + PF * 32u + lane; i < e; i += 32u) {
-                const uint32_t c = __ldg(idx + i);
-                if (!kAny && i + 1u < e && c >= __ldg(idx + i + 1u)) unordered = 1;
-                place(c, val[i]);
+                const uint32_t beyond = i0 + PF * 32u; // the entry after the step's last (lane 31)
+                uint32_t after = 0u;
+                if (!kAny && lane == 31u && beyond < e) after = __ldg(idx + beyond);
+#pragma unroll
+                for (int k = 0; k < PF; ++k) {
+                    if (i0 + (uint32_t) k * 32u < e) { // uniform
+                        const uint32_t i = i0 + (uint32_t) k * 32u + lane;
+                        if constexpr (!kAny) {
+                            uint32_t nxt = __shfl_down_sync(0xffffffffu, cc[k], 1);
+                            const uint32_t head =
+                                __shfl_sync(0xffffffffu, k + 1 < PF ? cc[k + 1 < PF ? k + 1 : 0] : 0u, 0);
+                            if (lane == 31u) nxt = k + 1 < PF ? head : after;
+                            if (i + 1u < e && cc[k] >= nxt) unordered = 1;
+                        }
+                        if (i < e) place(cc[k], cv[k]);
+                    }
+                }
             }
             if (!kAny && __any_sync(0xffffffffu, unordered)) {
                 for (uint32_t k = lane; k < seen_words; k += 32u) seen[k] = 0u;
@@ -804,27 +817,29 @@ int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, u
                         dst->ell_cols <= kSegHalves;
     const uint32_t row_blocks = (uint32_t) (((uint64_t) src->rows + B - 1u) / B);
     const std::size_t seen_bytes = ((dst->ell_cols + 31u) / 32u) * sizeof(uint32_t);
-    const std::size_t kSmem = 75u * 1024u; // three CTAs per SM
-    if (tma_ok && stride <= 8192u) {
+    const std::size_t kSmem = 75u * 1024u, kSmem2 = 112u * 1024u; // three CTAs per SM, two
+    // a warp per row up to 12 KB a row (100,000 x 5,003 at 2 %: 204 us against 320
+    // by a CTA per row); at 16 KB one CTA fits and it is the slower (810 against 392)
+    if (tma_ok && stride <= 12288u) {
         const int nbuf = stride <= 2048u ? 4 : (stride <= 4096u ? 2 : 1);
         const std::size_t wsmem =
             kEmitWarps * ((std::size_t) nbuf * stride + (std::size_t) words * sizeof(uint2) + seen_bytes);
-        if (wsmem <= kSmem) {
-            // rows of a row block stay together while that gives every warp two units
-            const uint32_t warps = (uint32_t) sm_count() * 3u * kEmitWarps;
-            uint32_t unit_rows = B;
-            while (unit_rows > 1u && (uint64_t) row_blocks * ((B + unit_rows - 1u) / unit_rows) < 2u * (uint64_t) warps)
-                unit_rows = (unit_rows + 1u) / 2u;
-            const uint64_t units = (uint64_t) row_blocks * ((B + unit_rows - 1u) / unit_rows);
-            uint32_t grid = (uint32_t) sm_count() * 3u;
-            if (grid > (units + kEmitWarps - 1u) / kEmitWarps) grid = (uint32_t) ((units + kEmitWarps - 1u) / kEmitWarps);
+        if (wsmem <= kSmem2) {
+            const uint32_t per_sm = wsmem <= kSmem ? 3u : 2u;
+            // equal runs for all warps, of at most 64 rows (rows may differ in size)
+            const uint32_t warps = (uint32_t) sm_count() * per_sm * kEmitWarps;
+            uint32_t run_rows = (src->rows + warps - 1u) / warps;
+            if (run_rows > 64u) run_rows = 64u;
+            const uint64_t runs = ((uint64_t) src->rows + run_rows - 1u) / run_rows;
+            uint32_t grid = (uint32_t) sm_count() * per_sm;
+            if (grid > (runs + kEmitWarps - 1u) / kEmitWarps) grid = (uint32_t) ((runs + kEmitWarps - 1u) / kEmitWarps);
             auto launch = [&](auto kern) {
                 if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) wsmem),
                              "bell_emit_warp smem attribute"))
                     return 0;
                 kern<<<grid, kEmitThreads, wsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                             src->cols, src->nnz, B, pow2_shift(B), words, width,
-                                                            dst->ell_cols, unit_rows, bitmaps, dst->blockColIdx,
+                                                            dst->ell_cols, run_rows, bitmaps, dst->blockColIdx,
                                                             dst->val, d_nnz, d_status, order);
                 return launch_ok("bell_emit_warp_kernel");
             };

@@ -457,9 +457,9 @@ int coo_plan(const cs_coo_view *src, const uint32_t *map, uint32_t cols, uint32_
             return 0;
         s->width = (uint32_t) shape[0];
         s->groups = shape[1];
+        // copied from pageable memory: taken before the call returns, so nothing waits
         const uint32_t words[4] = {s->width, route, 0u, s->n_valid};
-        return cuda_ok(cudaMemcpyAsync(x.words + 2, words, 16, cudaMemcpyHostToDevice, stream), "coo words") &&
-               cuda_ok(cudaStreamSynchronize(stream), "coo words sync");
+        return cuda_ok(cudaMemcpyAsync(x.words + 2, words, 16, cudaMemcpyHostToDevice, stream), "coo words");
     }
     s->shift = bits_for(w[0] / B);
     s->single = bits_for(s->RB - 1u) + s->shift <= 31u;

@@ -199,7 +199,9 @@ constexpr uint32_t kTpTileCoo = 8192;
 constexpr uint32_t kTpChunk = 8192;  // entries per pass-2 chunk (staged whole in shared memory)
 constexpr uint32_t kTpGran = 256;    // entries per warp per step; rows are looked up per granule
 
-constexpr uint32_t kTpSlice = 64;    // tiles or chunks per slice of the offset scan
+// Tiles or chunks per slice of the offset scan: 64, or 16 where that leaves only
+// a few CTAs with a long chain each (365 tiles: 12 us by 64, 6 by 16).
+constexpr uint32_t tp_slice_len(uint32_t rows) { return rows <= 8192u ? 16u : 64u; }
 
 // Counts of a pass, one row per tile or chunk and one column per digit, and
 // what the scan over the rows of a segment makes of them: pass 1 has one
@@ -225,7 +227,7 @@ struct tp2_layout {
     uint32_t *gran_row;     // [nnz / kTpGran + 1] row holding entry j * kTpGran
     void *scan_tmp;
     std::size_t scan_bytes, bytes;
-    uint32_t K, tiles1, max_chunks, slices1, max_slices, low_bits;
+    uint32_t K, tiles1, max_chunks, slice1, slice2, slices1, max_slices, low_bits;
 };
 
 bool tp2_applicable(uint32_t cDim, uint32_t uDim) {
@@ -241,8 +243,10 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     const uint32_t tile = granules ? kTpTileCsr : kTpTileCoo;
     l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + tile - 1u) / tile);
     l->max_chunks = nnz / kTpChunk + l->K + 1u;
-    l->slices1 = (l->tiles1 + kTpSlice - 1u) / kTpSlice;
-    l->max_slices = l->max_chunks / kTpSlice + l->K + 1u;
+    l->slice1 = tp_slice_len(l->tiles1);
+    l->slice2 = tp_slice_len(l->max_chunks);
+    l->slices1 = (l->tiles1 + l->slice1 - 1u) / l->slice1;
+    l->max_slices = l->max_chunks / l->slice2 + l->K + 1u;
     scratch_carver c(base, cap);
     l->status = c.take<uint32_t>(4);
     auto counts = [&](tp_counts *t, std::size_t rows, std::size_t slices, std::size_t digits) {
@@ -335,23 +339,23 @@ __global__ void __launch_bounds__(kTpThreads) tp_hist1_kernel(const uint32_t *__
     if (bad) status_or(status, bad);
 }
 
-// The offset scan, over slices of kTpSlice rows so that a segment of many rows
+// The offset scan, over slices of 16 or 64 rows so that a segment of many rows
 // is not one serial chain: slice sums, a scan of each segment's slices, then
 // the rows of every slice.  Rows are D counters wide and a warp reads 32 of
 // them together (the counts used to lie digit by digit, one sector apart for a
 // CTA that wants its row of them; scanned as one array of 12 M words they took
 // 100 us and 256 scattered reads per chunk at 300,000 x 32,768).
-__device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, uint32_t rows) {
+__device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, uint32_t rows, uint32_t len) {
     if (range != nullptr) return range[blockIdx.x];
-    return make_uint2(blockIdx.x * kTpSlice, min(rows, (blockIdx.x + 1u) * kTpSlice));
+    return make_uint2(blockIdx.x * len, min(rows, (blockIdx.x + 1u) * len));
 }
 
 // flag (here and below): nothing runs where it is given and clear.
 __global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint32_t *__restrict__ flag,
-                                                            const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, const uint2 *__restrict__ range,
+                                                            const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
                                                             uint32_t *__restrict__ slices) {
     if (flag != nullptr && *flag == 0u) return;
-    const uint2 r = tp_slice_rows(range, rows);
+    const uint2 r = tp_slice_rows(range, rows, len);
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t sum = 0u;
 #pragma unroll 16
@@ -399,13 +403,13 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(const uint32_t *__r
 
 // start[segment * D + d]: global slot of the digit's first entry
 __global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint32_t *__restrict__ flag,
-                                                             const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, const uint2 *__restrict__ range,
+                                                             const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
                                                              const uint32_t *__restrict__ segment,
                                                              const uint32_t *__restrict__ slices,
                                                              const uint32_t *__restrict__ start, uint32_t limit,
                                                              uint32_t *__restrict__ base) {
     if (flag != nullptr && *flag == 0u) return;
-    const uint2 r = tp_slice_rows(range, rows);
+    const uint2 r = tp_slice_rows(range, rows, len);
     const std::size_t c0 = (segment != nullptr ? (std::size_t) segment[blockIdx.x] : 0u) * D;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t run = slices[(std::size_t) blockIdx.x * D + d] + (c0 + d < limit ? start[c0 + d] : 0u);
@@ -916,7 +920,7 @@ __global__ void __launch_bounds__(1024) tp_chunks_kernel(const tp2_layout l) {
     const uint32_t nc = n != 0u ? (b + n - 1u) / kTpChunk + 1u - b / kTpChunk : 0u;
     uint32_t chunks, slices;
     const uint32_t fc = block_exclusive_scan(nc, smem, chunks);
-    const uint32_t fs = block_exclusive_scan((nc + kTpSlice - 1u) / kTpSlice, smem, slices);
+    const uint32_t fs = block_exclusive_scan((nc + l.slice2 - 1u) / l.slice2, smem, slices);
     if (k < K) {
         first[k] = fc;
         slice[k] = l.slice_first[k] = fs;
@@ -943,8 +947,8 @@ __global__ void __launch_bounds__(1024) tp_chunks_kernel(const tp2_layout l) {
         uint2 r = make_uint2(0u, 0u);
         if (id < slices) {
             bk = tp_find(slice, K, id);
-            r.x = first[bk] + (id - slice[bk]) * kTpSlice;
-            r.y = min(first[bk + 1u], r.x + kTpSlice);
+            r.x = first[bk] + (id - slice[bk]) * l.slice2;
+            r.y = min(first[bk + 1u], r.x + l.slice2);
         }
         l.slice_bucket[id] = bk;
         l.slice_range[id] = r;
@@ -1337,7 +1341,7 @@ int tp_count_chunks(const uint32_t *flag, uint32_t uDim, const tp2_layout &l, ui
                               : resident_grid((const void *) tp_hist2_kernel<LB>, kTpThreads, 0, l.max_chunks);
     tp_hist2_kernel<LB><<<grid, kTpThreads, 0, stream>>>(flag, l.tmp_key, l.chunk_range, l.max_chunks, l.two.cnt);
     if (!launch_ok("tp_hist2_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, l.slice_range, l.two.slices);
+    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, 0u, l.slice_range, l.two.slices);
     if (!launch_ok("tp_slice_sums_kernel")) return 0;
     tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(flag, l.two.slices, D, l.slice_first, 0u, uDim,
                                                                   flag == nullptr ? out_ptr : nullptr);
@@ -1345,7 +1349,7 @@ int tp_count_chunks(const uint32_t *flag, uint32_t uDim, const tp2_layout &l, ui
     if (flag == nullptr &&
         !scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream))
         return 0;
-    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, l.slice_range, l.slice_bucket,
+    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, 0u, l.slice_range, l.slice_bucket,
                                                             l.two.slices, out_ptr, uDim, l.two.base);
     return launch_ok("tp_slice_apply_kernel");
 }
@@ -1385,14 +1389,14 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
     hist1<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K, l.one.cnt,
                                                                     l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, nullptr, l.one.slices);
+    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, l.one.slices);
     if (!launch_ok("tp_slice_sums_kernel")) return 0;
     tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(nullptr, l.one.slices, l.K, nullptr, l.slices1, l.K,
                                                                           l.total1);
     if (!launch_ok("tp_slice_scan_kernel")) return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
     if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, nullptr, nullptr, l.one.slices,
+    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr, l.one.slices,
                                                          l.start1, l.K, l.one.base);
     if (!launch_ok("tp_slice_apply_kernel")) return 0;
     if (csr) {

@@ -123,8 +123,10 @@ def blocked_ell_shape(csr: CSR, block_size: int, keep_bitmaps: bool = True, stre
     nbytes = C.c_size_t()
     _abi.check(lib.cs_b200_blocked_ell_scratch_bytes(csr.rows, csr.cols, block_size, C.byref(nbytes)), "scratch")
     scratch = _scratch(nbytes.value) if keep_bitmaps else None
-    shape = torch.zeros(2, dtype=torch.int64, device="cuda")
-    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    # one cleared block: width, total blocks, then the status and the word after it
+    # (where blocked_ell_from_csr counts the stored values)
+    words = torch.zeros(3, dtype=torch.int64, device="cuda")
+    shape, status = words[:2], words[2:].view(torch.int32)[:1]
     v = csr.view()
     _abi.check(lib.cs_b200_blocked_ell_shape(C.byref(v), block_size, ptr(shape), ptr(scratch),
                                              nbytes.value if keep_bitmaps else 0, ptr(status), stream_handle(stream)),
@@ -142,15 +144,14 @@ def blocked_ell_from_csr(csr: CSR, block_size: int, stream=None, check_status: b
     out = BlockedELL(csr.rows, csr.cols, block_size, ell_cols,
                      torch.empty(rb * width, dtype=torch.int32, device="cuda"),
                      torch.empty(csr.rows * ell_cols, dtype=torch.float16, device="cuda"), 0)
-    nnz = torch.zeros(1, dtype=torch.int32, device="cuda")
+    after = status.as_strided((2,), (1,), status.storage_offset())  # the status and the count behind it
     v, dv = csr.view(), out.view()
-    _abi.check(lib.cs_b200_blocked_ell_emit(C.byref(v), C.byref(dv), ptr(nnz), ptr(scratch), scratch.numel(),
+    _abi.check(lib.cs_b200_blocked_ell_emit(C.byref(v), C.byref(dv), ptr(after[1:]), ptr(scratch), scratch.numel(),
                                             ptr(status), stream_handle(stream)), "blocked_ell_emit")
-    out.nnz = int(nnz.cpu().view(torch.int32)[0]) & 0xFFFFFFFF
-    if check_status:
-        st = int(status.cpu()[0])
-        if st:
-            raise _abi.CellShardError(f"blocked_ell conversion flagged invalid input (status 0x{st:x})")
+    st, nnz = after.tolist()
+    out.nnz = nnz & 0xFFFFFFFF
+    if check_status and st:
+        raise _abi.CellShardError(f"blocked_ell conversion flagged invalid input (status 0x{st & 0xFFFFFFFF:x})")
     return out
 
 
@@ -400,7 +401,8 @@ def blocked_ell_from_coo(rows: int, cols_src: int, row_idx: torch.Tensor, col_id
     nbytes = C.c_size_t()
     _abi.check(lib.cs_b200_coo_blocked_ell_scratch_bytes(n, rows, cols, block_size, C.byref(nbytes)), "coo scratch")
     scratch = _scratch(nbytes.value)
-    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    words = torch.zeros(3, dtype=torch.int64, device="cuda")  # both nnz counts, then the status
+    nnz, status = words[:2], words[2:].view(torch.int32)[:1]
     width, total = C.c_uint32(), C.c_uint64()
     s = stream_handle(stream)
     fm = ptr(feature_to_global) if feature_to_global is not None else None
@@ -411,16 +413,15 @@ def blocked_ell_from_coo(rows: int, cols_src: int, row_idx: torch.Tensor, col_id
     out = BlockedELL(rows, cols, block_size, W * block_size,
                      torch.empty(max(RB * W, 1), dtype=torch.int32, device="cuda"),
                      torch.empty(max(rows * W * block_size, 1), dtype=torch.float16, device="cuda"), 0)
-    nnz = torch.zeros(2, dtype=torch.int64, device="cuda")
     dv = out.view()
     dv.blockColIdx, dv.val = out.bci.data_ptr(), out.val.data_ptr()
     _abi.check(lib.cs_b200_coo_blocked_ell_emit(C.byref(v), fm, cols, ptr(scratch), nbytes.value, C.byref(dv),
                                                 nnz.data_ptr(), s), "coo emit")
-    counts = [int(x) for x in nnz.cpu()]
+    *counts, st = words.tolist()
     out.nnz = counts[1]
     out.bci = out.bci[:RB * W]
     out.val = out.val[:rows * W * block_size]
-    return out, counts, int(status.item()), total.value
+    return out, counts, (st & 0xFFFFFFFF ^ 0x80000000) - 0x80000000, total.value  # the status as the int32 it is
 
 
 def cspack_store(path, m) -> None:

@@ -89,3 +89,21 @@ def test_csr_rows_in_any_column_order(cuda, orc, cols, block, repeat):
     ref = orc.blocked_ell_from_csr(rows, cols, ptr, idx, val, block)
     assert out.ell_cols == ref["ell_cols"] and out.nnz == ref["nnz"]
     assert np.array_equal(np_u32(out.bci), ref["bci"]) and np.array_equal(np_u16(out.val), ref["val"])
+
+
+@pytest.mark.parametrize("rows,cols,longest", [(1, 900, 900), (70, 6_100, 700), (5_000, 1_000, 40), (9_001, 300, 290)])
+@pytest.mark.parametrize("block", [8, 24])
+def test_short_rows_in_runs(cuda, orc, rows, cols, longest, block):
+    """A warp per row: runs of rows over row-block borders, rows past 256 entries."""
+    from cellshard_b200.device import blocked_ell_from_csr
+
+    rng = np.random.default_rng(rows + block)
+    n = rng.integers(0, longest + 1, rows)
+    n[rng.random(rows) < 0.1] = longest
+    ptr = np.concatenate([[0], np.cumsum(n)]).astype(np.uint32)
+    idx = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in n]).astype(np.uint32)
+    val = rng.integers(0, 60_000, len(idx)).astype(np.uint16)
+    out = blocked_ell_from_csr(to_device_csr(rows, cols, ptr, idx, val), block)
+    ref = orc.blocked_ell_from_csr(rows, cols, ptr, idx, val, block)
+    assert out.ell_cols == ref["ell_cols"] and out.nnz == ref["nnz"]
+    assert np.array_equal(np_u32(out.bci), ref["bci"]) and np.array_equal(np_u16(out.val), ref["val"])
