@@ -31,17 +31,6 @@ namespace {
 constexpr unsigned kEmitThreads = 256;
 constexpr unsigned kSegHalves = 32768; // 64 KB row segment in shared memory
 
-// How an emit treats rows out of column order.  Default: checked row by row, a
-// repeated column keeps its last value.  With a flag, all rows come in any
-// order, and either (first) a repeated column only sets the flag, or (second)
-// the emit runs only where the flag is set.
-struct emit_order {
-    uint32_t *flag;
-    bool first;
-    __device__ __forceinline__ bool skips() const { return flag != nullptr && !first && *flag == 0u; }
-    __device__ __forceinline__ bool flag_repeats() const { return flag != nullptr && first; }
-};
-
 __device__ __forceinline__ uint32_t div_b(uint32_t c, uint32_t B, int shift) {
     return shift >= 0 ? (c >> shift) : (c / B);
 }
@@ -161,12 +150,105 @@ __global__ void __launch_bounds__(WARPS * 32) bell_shape_kernel(
     }
 }
 
+// The shape of rows in any column order, a warp per row: beside the row block's
+// bitmap over column blocks every row has one over its columns, in which a
+// repeated column meets its own bit.  Bound by issue slots and the two shared
+// updates an entry; repeats found here spare the emit a mark per entry and, after
+// it, a second partition and emit behind a device flag (100,000 x 32,768, 131 M
+// entries: shape 196 us, emit 1,333; 12 before the emit marked: 228 and 1,390).
+constexpr unsigned kAnyWarps = 8;
+template <bool kPow2>
+__global__ void __launch_bounds__(kAnyWarps * 32) bell_shape_any_kernel(
+    const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, uint32_t rows, uint32_t cols, uint32_t nnz,
+    uint32_t B, int shift, uint32_t row_blocks, uint32_t words, uint32_t *__restrict__ bitmaps,
+    unsigned long long *__restrict__ shape, uint32_t *status, uint32_t *__restrict__ repeats) {
+    extern __shared__ __align__(16) uint32_t any_smem[];
+    const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5, warps = blockDim.x >> 5;
+    const uint32_t col_words = ((cols + 31u) / 32u + 3u) & ~3u;
+    uint32_t *mine = any_smem + (std::size_t) warp * col_words;             // [col_words] the warp's row
+    uint32_t *bits = any_smem + (std::size_t) warps * col_words;            // [words] the row block
+    __shared__ uint32_t warp_count[kAnyWarps];
+    constexpr uint32_t kNone = 0xffffffffu; // no column: every row's are below cols
+    uint32_t local_max = 0u, bad = 0u, twice = 0u;
+    unsigned long long local_total = 0ull;
+    for (uint32_t rb = blockIdx.x; rb < row_blocks; rb += gridDim.x) {
+        for (uint32_t w = t; w < words; w += blockDim.x) bits[w] = 0u;
+        __syncthreads();
+        const uint32_t r_end = min(rows, rb * B + B);
+        for (uint32_t r = rb * B + warp; r < r_end; r += warps) {
+            const uint32_t a = ptr[r], e = ptr[r + 1u];
+            if (e < a || e > nnz) {
+                bad |= CS_STATUS_BAD_POINTERS;
+                continue;
+            }
+            for (uint32_t w = lane * 4u; w < col_words; w += 128u)
+                *reinterpret_cast<uint4 *>(mine + w) = make_uint4(0u, 0u, 0u, 0u);
+            __syncwarp();
+            auto mark = [&](uint32_t c) {
+                const uint32_t bit = 1u << (c & 31u), bc = kPow2 ? c >> shift : c / B;
+                twice |= atomicOr(mine + (c >> 5), bit) & bit;
+                atomicOr(bits + (bc >> 5), 1u << (bc & 31u));
+            };
+            constexpr unsigned U = 8;
+            uint32_t i = a;
+            for (; i + 32u * U <= e; i += 32u * U) {
+                uint32_t c[U], top = 0u;
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u) {
+                    c[u] = __ldg(idx + i + 32u * u + lane);
+                    top = max(top, c[u]);
+                }
+                if (top >= cols) {
+                    bad |= CS_STATUS_INDEX_RANGE;
+                } else {
+#pragma unroll
+                    for (unsigned u = 0; u < U; ++u) mark(c[u]);
+                }
+            }
+            uint32_t c[U];
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u) c[u] = i + 32u * u + lane < e ? __ldg(idx + i + 32u * u + lane) : kNone;
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u) {
+                if (c[u] < cols) mark(c[u]);
+                else if (c[u] != kNone) bad |= CS_STATUS_INDEX_RANGE;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t cnt = 0u;
+        for (uint32_t w = t; w < words; w += blockDim.x) {
+            const uint32_t word = bits[w];
+            cnt += __popc(word);
+            bitmaps[(std::size_t) rb * words + w] = word;
+        }
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0u) warp_count[warp] = cnt;
+        __syncthreads(); // also before the next row block clears the bitmap
+        if (t == 0u) {
+            uint32_t all = 0u;
+            for (unsigned w = 0; w < warps; ++w) all += warp_count[w];
+            local_max = max(local_max, all);
+            local_total += all;
+        }
+    }
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    twice = __any_sync(0xffffffffu, twice != 0u);
+    if (lane == 0u) {
+        status_or(status, bad);
+        if (twice) atomicOr(repeats, 1u);
+    }
+    if (t == 0u) {
+        if (local_max != 0u) atomicMax(shape, (unsigned long long) local_max);
+        if (local_total != 0ull) atomicAdd(shape + 1, local_total);
+    }
+}
+
 __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci, uint16_t *__restrict__ out_val,
-    uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
-    if (order.skips()) return;
+    uint32_t *__restrict__ d_nnz, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char emit_smem[];
     uint16_t *buf = reinterpret_cast<uint16_t *>(emit_smem);                  // [kSegHalves]
     uint32_t *seen = reinterpret_cast<uint32_t *>(buf + kSegHalves);          // [kSegHalves / 32]
@@ -255,8 +337,7 @@ __global__ void __launch_bounds__(kEmitThreads) bell_emit_kernel(
                         if (pos < seg_len && (atomicOr(seen + (pos >> 5), bit) & bit)) repeated = 1;
                     }
                     if (__syncthreads_or(repeated) && threadIdx.x == 0) {
-                        if (order.flag_repeats()) atomicOr(order.flag, 1u);
-                        for (uint32_t i = a; i < e && !order.flag_repeats(); ++i) {
+                        for (uint32_t i = a; i < e; ++i) {
                             const uint32_t pos = cell(idx[i]);
                             if (pos < seg_len) buf[pos] = val[i];
                         }
@@ -332,15 +413,14 @@ __device__ __forceinline__ void write_block_columns(const uint2 *ix, uint32_t wo
 // A row whose columns are not strictly increasing marks one bit per cell in
 // `seen`; one that repeats a column is redone in CSR order by one thread (the
 // reference's overwrite order).
-// kAny (rows in any column order, as the COO partition leaves them): every row
-// marks its cells while it places them, with no order check.
+// kAny: rows in any column order that repeat no column (the COO partition's,
+// checked by its shape pass): placed without a check.
 template <int NBUF, bool kAny>
 __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci, uint16_t *__restrict__ out_val,
-    uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
-    if (kAny && order.skips()) return;
+    uint32_t *__restrict__ d_nnz, uint32_t *status) {
     extern __shared__ __align__(128) unsigned char tma_smem[];
     constexpr int PF = 8;                    // entries per thread prefetched for the next row
     constexpr bool kTakeBack = NBUF <= 2;    // small rows: a few vector stores clear them
@@ -438,10 +518,6 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                     for (uint32_t k = threadIdx.x * 8u; k < ell_cols; k += blockDim.x * 8u)
                         *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
                 }
-                if constexpr (!kAny) __syncthreads();
-            }
-            if constexpr (kAny) {
-                for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
                 __syncthreads();
             }
             int unordered = 0, repeated = 0;
@@ -462,7 +538,6 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             auto place = [&](uint32_t c, uint16_t v) {
                 const uint32_t p = cell(c);
                 if (p != kNone) {
-                    if constexpr (kAny) mark(p);
                     buf[p] = v;
                     row_nnz += half_nonzero(v);
                 }
@@ -496,7 +571,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
             bool all_held = n <= PF * kEmitThreads;
             fence_proxy_async_smem();
             if constexpr (kAny) {
-                repeated = __syncthreads_or(repeated);
+                __syncthreads();
             } else if (__syncthreads_or(unordered)) {
                 for (uint32_t k = threadIdx.x; k < seen_words; k += blockDim.x) seen[k] = 0u;
                 __syncthreads();
@@ -508,9 +583,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_tma_kernel(
                 for (uint32_t i = a + PF * kEmitThreads + threadIdx.x; i < e; i += blockDim.x) mark(cell(__ldg(idx + i)));
                 repeated = __syncthreads_or(repeated);
             }
-            if (kAny && order.first) {
-                if (repeated && threadIdx.x == 0) atomicOr(order.flag, 1u);
-            } else if (repeated) {
+            if (!kAny && repeated) {
                 if (threadIdx.x == 0) {
                     for (uint32_t i = a; i < e; ++i) {
                         const uint32_t p = cell(idx[i]);
@@ -562,8 +635,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
     const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, uint32_t rows,
     uint32_t cols, uint32_t nnz, uint32_t B, int shift, uint32_t words, uint32_t width, uint32_t ell_cols,
     uint32_t run_rows, const uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ out_bci,
-    uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status, const emit_order order) {
-    if (kAny && order.skips()) return;
+    uint16_t *__restrict__ out_val, uint32_t *__restrict__ d_nnz, uint32_t *status) {
     extern __shared__ __align__(128) unsigned char tma_smem[];
     constexpr int PF = 8;
     const uint32_t row_bytes = ell_cols * 2u;
@@ -648,8 +720,6 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             __syncwarp();
             for (uint32_t k = lane * 8u; k < ell_cols; k += 256u)
                 *reinterpret_cast<uint4 *>(buf + k) = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (kAny)
-                for (uint32_t k = lane; k < seen_words; k += 32u) seen[k] = 0u;
             __syncwarp();
             int unordered = 0, repeated = 0;
             uint32_t row_nnz = 0u;
@@ -663,10 +733,6 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
             auto place = [&](uint32_t c, uint16_t v) {
                 const uint32_t p = cell(c);
                 if (p == 0xffffffffu) return;
-                if constexpr (kAny) {
-                    const uint32_t bit = 1u << (p & 31u);
-                    if (atomicOr(seen + (p >> 5), bit) & bit) repeated = 1;
-                }
                 buf[p] = v;
                 row_nnz += half_nonzero(v);
             };
@@ -707,10 +773,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) bell_emit_warp_kernel(
                     if (p != 0xffffffffu && (atomicOr(seen + (p >> 5), bit) & bit)) repeated = 1;
                 }
             }
-            repeated = __any_sync(0xffffffffu, repeated);
-            if (kAny && order.first) {
-                if (repeated && lane == 0u) atomicOr(order.flag, 1u);
-            } else if (repeated) {
+            if (!kAny && __any_sync(0xffffffffu, repeated)) {
                 __syncwarp();
                 if (lane == 0u) {
                     for (uint32_t i = a; i < e; ++i) {
@@ -802,10 +865,39 @@ int blocked_ell_shape_launch(const cs_compressed_view *src, uint32_t B, uint64_t
     return launch(bell_shape_kernel<8>, 8u);
 }
 
+// a row block of fewer rows than warps would leave some idle
+static unsigned any_order_warps(uint32_t B) { return B < kAnyWarps ? B : kAnyWarps; }
+
+static std::size_t any_order_smem(uint32_t cols, uint32_t B) {
+    return ((std::size_t) any_order_warps(B) * (((cols + 31u) / 32u + 3u) & ~3u) + col_words(cols, B)) * sizeof(uint32_t);
+}
+
+bool blocked_ell_any_order_fits(uint32_t cols, uint32_t B) {
+    return B != 0u && any_order_smem(cols, B) <= 200u * 1024u;
+}
+
+int blocked_ell_shape_any_order(const cs_compressed_view *src, uint32_t B, uint64_t *d_shape, uint32_t *bitmaps,
+                                uint32_t *d_status, uint32_t *repeats, cudaStream_t stream) {
+    const uint32_t row_blocks = (uint32_t) (((uint64_t) src->rows + B - 1u) / B);
+    const uint32_t words = col_words(src->cols, B);
+    if (row_blocks == 0u || words == 0u) return 1;
+    const std::size_t smem = any_order_smem(src->cols, B);
+    auto kern = pow2_shift(B) >= 0 ? bell_shape_any_kernel<true> : bell_shape_any_kernel<false>;
+    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
+                 "bell_shape_any smem attribute"))
+        return 0;
+    const unsigned threads = any_order_warps(B) * 32u;
+    const unsigned grid = resident_grid((const void *) kern, threads, smem, row_blocks);
+    kern<<<grid, threads, smem, stream>>>(src->majorPtr, src->minorIdx, src->rows, src->cols, src->nnz, B,
+                                                  pow2_shift(B), row_blocks, words, bitmaps,
+                                                  reinterpret_cast<unsigned long long *>(d_shape), d_status, repeats);
+    return launch_ok("bell_shape_any_kernel");
+}
+
 namespace {
 template <bool kAny>
 int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
-                const uint32_t *bitmaps, uint32_t *d_status, const emit_order order, cudaStream_t stream) {
+                const uint32_t *bitmaps, uint32_t *d_status, cudaStream_t stream) {
     const uint32_t B = dst->block_size;
     const uint32_t words = col_words(src->cols, B);
     const uint32_t width = dst->ell_cols / B;
@@ -840,7 +932,7 @@ int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, u
                 kern<<<grid, kEmitThreads, wsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                             src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                             dst->ell_cols, run_rows, bitmaps, dst->blockColIdx,
-                                                            dst->val, d_nnz, d_status, order);
+                                                            dst->val, d_nnz, d_status);
                 return launch_ok("bell_emit_warp_kernel");
             };
             if (nbuf == 4) return launch(bell_emit_warp_kernel<4, kAny>);
@@ -862,7 +954,7 @@ int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, u
                 kern<<<tgrid, kEmitThreads, tsmem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                               src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                               dst->ell_cols, bitmaps, dst->blockColIdx, dst->val,
-                                                              d_nnz, d_status, order);
+                                                              d_nnz, d_status);
                 return launch_ok("bell_emit_tma_kernel");
             };
             if (nbuf == 8) return launch(bell_emit_tma_kernel<8, kAny>);
@@ -882,19 +974,19 @@ int emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, u
     bell_emit_kernel<<<grid, kEmitThreads, smem, stream>>>(src->majorPtr, src->minorIdx, src->val, src->rows,
                                                            src->cols, src->nnz, B, pow2_shift(B), words, width,
                                                            dst->ell_cols, bitmaps, dst->blockColIdx, dst->val, d_nnz,
-                                                           d_status, order);
+                                                           d_status);
     return launch_ok("bell_emit_kernel");
 }
 } // namespace
 
 int blocked_ell_emit_launch(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
                             const uint32_t *bitmaps, uint32_t *d_status, cudaStream_t stream) {
-    return emit_launch<false>(src, dst, d_nnz, bitmaps, d_status, emit_order{nullptr, false}, stream);
+    return emit_launch<false>(src, dst, d_nnz, bitmaps, d_status, stream);
 }
 
 int blocked_ell_emit_any_order(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
-                               const uint32_t *bitmaps, uint32_t *flag, bool flag_repeats, cudaStream_t stream) {
-    return emit_launch<true>(src, dst, d_nnz, bitmaps, nullptr, emit_order{flag, flag_repeats}, stream);
+                               const uint32_t *bitmaps, cudaStream_t stream) {
+    return emit_launch<true>(src, dst, d_nnz, bitmaps, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -204,24 +204,22 @@ std::size_t sort_pairs_u32_scratch_bytes(uint32_t n);
 int sort_pairs_u32(const uint32_t *keys, const uint32_t *vals, uint32_t n, uint32_t *out_keys, uint32_t *out_vals,
                    void *tmp, std::size_t tmp_bytes, cudaStream_t stream);
 
-// COO entries by rows, a row's entries in any order (transpose.cu), and again
-// in their own order where *flag is set.  scratch_bytes is 0 where it does not
-// apply (no entries, too many rows, columns too wide).
+// COO entries by rows, a row's entries in any order or, `stable`, in their own
+// (transpose.cu).  scratch_bytes is 0 where it does not apply (no entries, too
+// many rows, columns too wide).
 std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t cols);
 int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row, const uint32_t *col,
-                   const uint32_t *map, const uint16_t *val, uint32_t *out_ptr, uint32_t *out_col, uint16_t *out_val,
-                   void *scratch, std::size_t scratch_bytes, cudaStream_t stream);
+                   const uint32_t *map, const uint16_t *val, bool stable, uint32_t *out_ptr, uint32_t *out_col,
+                   uint16_t *out_val, void *scratch, std::size_t scratch_bytes, cudaStream_t stream);
 
-int partition_rows_stable(const uint32_t *flag, uint32_t *nnz_count, uint32_t n, uint32_t rows, uint32_t cols,
-                          const uint32_t *row, const uint32_t *col, const uint32_t *map, const uint16_t *val,
-                          const uint32_t *row_ptr, uint32_t *out_col, uint16_t *out_val, void *scratch,
-                          std::size_t scratch_bytes, cudaStream_t stream);
-
-// CSR -> Blocked-ELL emit of rows whose columns stand in any order
-// (blocked_ell.cu).  flag_repeats: a row that repeats a column only sets *flag;
-// otherwise nothing runs unless *flag is set, and repeats keep the last value.
+// CSR -> Blocked-ELL of rows whose columns stand in any order (blocked_ell.cu):
+// the shape pass sets *repeats where a row repeats a column; the emit is for
+// rows that do not.  Only where the rows' column bitmaps fit shared memory.
+bool blocked_ell_any_order_fits(uint32_t cols, uint32_t B);
+int blocked_ell_shape_any_order(const cs_compressed_view *src, uint32_t B, uint64_t *d_shape, uint32_t *bitmaps,
+                                uint32_t *d_status, uint32_t *repeats, cudaStream_t stream);
 int blocked_ell_emit_any_order(const cs_compressed_view *src, const cs_blocked_ell_view *dst, uint32_t *d_nnz,
-                               const uint32_t *bitmaps, uint32_t *flag, bool flag_repeats, cudaStream_t stream);
+                               const uint32_t *bitmaps, cudaStream_t stream);
 
 // Owned device memory and stream for the synchronous host entry points.
 struct dmem {

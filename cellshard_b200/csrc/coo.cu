@@ -14,8 +14,7 @@
 // the library's CSR -> Blocked-ELL shape and emit, which place a row's values
 // whatever the order of its columns and count nnz the same way.  Only a
 // repeated (row, column), whose last value stays, needs the entries' order: the
-// emit flags it, and the partition (stable this time) and the emit, launched
-// again behind the flag, then run.  The
+// shape pass finds them, and the partition then runs again, stable.  The
 // partition takes up to 2,097,152 rows whose row digit and column fit one
 // word; past that the entries are stably sorted by column and then by row and
 // gathered.  100,000 x 32,768, 131 M shuffled entries, plan + emit: 19.9 ms
@@ -45,11 +44,12 @@ namespace {
 
 constexpr uint32_t kInvalid = 0xffffffffu;
 
-// words (16): [8] the partition route found a repeated (row, column);
-// [0] largest mapped column, [1] dropped entries, [2] width, [3] route
-// (0 two sorts, 1 one sort, 2 CSR), [4] key shift, [5] kept entries, [6] rows
-// decrease somewhere, [7] the CSR route's nnz
-constexpr uint32_t kRouteTwoSorts = 0u, kRouteOneSort = 1u, kRouteCsr = 2u, kRouteCsrSorted = 3u;
+// words: [0] largest mapped column, [1] dropped entries, [2] width, [3] route
+// (0 two sorts, 1 one sort, 2 CSR, 3 CSR after a stable sort, 4 CSR in any
+// column order), [4] key shift, [5] kept entries, [6] rows decrease somewhere,
+// [7] the CSR route's nnz
+constexpr uint32_t kRouteTwoSorts = 0u, kRouteOneSort = 1u, kRouteCsr = 2u, kRouteCsrSorted = 3u,
+                   kRouteCsrAny = 4u;
 
 // The CSR route's column-block bitmaps (one bit per column block per row
 // block) must stay small next to the entries themselves.
@@ -61,7 +61,7 @@ bool csr_route_fits(uint32_t n, uint32_t rows, uint32_t cols, uint32_t B) {
 
 struct coo_scratch {
     uint32_t *words;
-    unsigned long long *shape;   // CSR route: width, pairs
+    unsigned long long *shape;   // CSR route: width, pairs, a repeated (row, column)
     uint32_t *csr_ptr, *mcol;    // CSR route: row pointers, mapped (and row-sorted) columns
     uint16_t *sval;              // CSR route after the row sort: values in row order
     void *csr_tmp;
@@ -75,8 +75,8 @@ void carve(void *base, uint32_t n, uint32_t rows, uint32_t cols, uint32_t B, coo
     const uint32_t RB = (uint32_t) (((uint64_t) rows + B - 1u) / B);
     scratch_carver c(base, ~std::size_t(0));
     const std::size_t n1 = (std::size_t) n + 1u;
-    x->words = c.take<uint32_t>(16);
-    x->shape = c.take<unsigned long long>(2);
+    x->words = c.take<uint32_t>(8);
+    x->shape = c.take<unsigned long long>(3);
     x->csr_ptr = c.take<uint32_t>((std::size_t) rows + 1u);
     x->mcol = c.take<uint32_t>(n1);
     x->sval = c.take<uint16_t>(n1);
@@ -428,11 +428,16 @@ int coo_plan(const cs_coo_view *src, const uint32_t *map, uint32_t cols, uint32_
         const bool sorted = w[6] != 0u;
         route = sorted ? kRouteCsrSorted : kRouteCsr;
         const uint32_t *rows_in_order = src->rowIdx;
+        auto by_rows = [&](bool stable) {
+            return partition_rows(n, src->rows, cols, src->rowIdx, src->colIdx, map, src->val, stable, x.csr_ptr,
+                                  x.mcol, x.sval, x.part_tmp, x.part_bytes, stream);
+        };
         if (sorted && x.part_bytes != 0u) {
-            if (!partition_rows(n, src->rows, cols, src->rowIdx, src->colIdx, map, src->val, x.csr_ptr, x.mcol, x.sval,
-                                x.part_tmp, x.part_bytes, stream))
-                return 0;
+            // past the columns whose bitmaps fit, repeats cannot be looked for: stable at once
+            const bool any = blocked_ell_any_order_fits(cols, B);
+            if (!by_rows(!any)) return 0;
             rows_in_order = nullptr;
+            if (any) route = kRouteCsrAny;
         } else if (sorted) {
             // stable by (mapped) column, then stable by row: rows in order, columns ascending
             // inside a row, repeated (row, column) entries next to each other in COO order
@@ -463,13 +468,20 @@ int coo_plan(const cs_coo_view *src, const uint32_t *map, uint32_t cols, uint32_
             if (!launch_ok("coo_row_ptr_kernel")) return 0;
         }
         const cs_compressed_view v = csr_of(src, map, cols, x, sorted);
-        unsigned long long shape[2] = {0, 0};
-        if (!cuda_ok(cudaMemsetAsync(x.shape, 0, 16, stream), "shape clear") ||
-            !cs_b200_blocked_ell_shape(&v, B, (uint64_t *) x.shape, x.csr_tmp, x.csr_bytes, status,
-                                       reinterpret_cast<cs_stream_t>(stream)) ||
-            !cuda_ok(cudaMemcpyAsync(shape, x.shape, 16, cudaMemcpyDeviceToHost, stream), "D2H shape") ||
+        unsigned long long shape[3] = {0, 0, 0};
+        if (!cuda_ok(cudaMemsetAsync(x.shape, 0, 24, stream), "shape clear") ||
+            !(route == kRouteCsrAny
+                  ? blocked_ell_shape_any_order(&v, B, (uint64_t *) x.shape, (uint32_t *) x.csr_tmp, status,
+                                                (uint32_t *) (x.shape + 2), stream)
+                  : cs_b200_blocked_ell_shape(&v, B, (uint64_t *) x.shape, x.csr_tmp, x.csr_bytes, status,
+                                              reinterpret_cast<cs_stream_t>(stream))) ||
+            !cuda_ok(cudaMemcpyAsync(shape, x.shape, 24, cudaMemcpyDeviceToHost, stream), "D2H shape") ||
             !cuda_ok(cudaStreamSynchronize(stream), "coo csr shape sync"))
             return 0;
+        if (shape[2] != 0u) { // a repeated (row, column): its last value is the one in the entries' order
+            if (!by_rows(true)) return 0;
+            route = kRouteCsrSorted;
+        }
         s->width = (uint32_t) shape[0];
         s->groups = shape[1];
         // copied from pageable memory: taken before the call returns, so nothing waits
@@ -550,20 +562,14 @@ int coo_emit(const cs_coo_view *src, const uint32_t *map, uint32_t cols, const v
         set_error("coo_blocked_ell_emit: null destination arrays");
         return 0;
     }
-    if (route == kRouteCsr || route == kRouteCsrSorted) {
-        const cs_compressed_view v = csr_of(src, map, cols, x, route == kRouteCsrSorted);
-        if (!cuda_ok(cudaMemsetAsync(x.words + 7, 0, 8, stream), "csr nnz clear")) return 0;
-        if (route == kRouteCsrSorted && x.part_bytes != 0u) {
-            const uint32_t *bits = (const uint32_t *) x.csr_tmp;
-            if (!blocked_ell_emit_any_order(&v, dst, x.words + 7, bits, x.words + 8, true, stream) ||
-                !partition_rows_stable(x.words + 8, x.words + 7, n, src->rows, cols, src->rowIdx, src->colIdx, map,
-                                       src->val, x.csr_ptr, x.mcol, x.sval, x.part_tmp, x.part_bytes, stream) ||
-                !blocked_ell_emit_any_order(&v, dst, x.words + 7, bits, x.words + 8, false, stream))
-                return 0;
-        } else if (!cs_b200_blocked_ell_emit(&v, dst, x.words + 7, x.csr_tmp, x.csr_bytes, nullptr,
-                                             reinterpret_cast<cs_stream_t>(stream))) {
+    if (route == kRouteCsr || route == kRouteCsrSorted || route == kRouteCsrAny) {
+        const cs_compressed_view v = csr_of(src, map, cols, x, route != kRouteCsr);
+        if (!cuda_ok(cudaMemsetAsync(x.words + 7, 0, 4, stream), "csr nnz clear") ||
+            !(route == kRouteCsrAny
+                  ? blocked_ell_emit_any_order(&v, dst, x.words + 7, (const uint32_t *) x.csr_tmp, stream)
+                  : cs_b200_blocked_ell_emit(&v, dst, x.words + 7, x.csr_tmp, x.csr_bytes, nullptr,
+                                             reinterpret_cast<cs_stream_t>(stream))))
             return 0;
-        }
         coo_nnz_from_csr_kernel<<<1, 32, 0, stream>>>(x.words + 7, (unsigned long long *) d_nnz);
         return launch_ok("coo_nnz_from_csr_kernel");
     }

@@ -20,6 +20,8 @@
 // caller's scratch; the two-pass path keeps repeated entries, in row order.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace csb {
 namespace {
 
@@ -350,11 +352,8 @@ __device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, 
     return make_uint2(blockIdx.x * len, min(rows, (blockIdx.x + 1u) * len));
 }
 
-// flag (here and below): nothing runs where it is given and clear.
-__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint32_t *__restrict__ flag,
-                                                            const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
+__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
                                                             uint32_t *__restrict__ slices) {
-    if (flag != nullptr && *flag == 0u) return;
     const uint2 r = tp_slice_rows(range, rows, len);
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
         uint32_t sum = 0u;
@@ -366,13 +365,11 @@ __global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint32_t *__re
 
 // One segment (blockIdx.x) and 32 digits (blockIdx.y) per CTA: 32 threads per
 // digit, each over a run of the segment's slices.  totals[segment * D + d] for
-// digits below `limit` in all (null: not wanted).
-__global__ void __launch_bounds__(1024) tp_slice_scan_kernel(const uint32_t *__restrict__ flag,
-                                                             uint32_t *__restrict__ slices, uint32_t D,
+// digits below `limit` in all.
+__global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restrict__ slices, uint32_t D,
                                                              const uint32_t *__restrict__ seg_first, uint32_t n_slices,
                                                              uint32_t limit, uint32_t *__restrict__ totals) {
     __shared__ uint32_t part[32][33];
-    if (flag != nullptr && *flag == 0u) return;
     const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, d = blockIdx.y * 32u + x;
     const uint32_t s0 = seg_first != nullptr ? seg_first[blockIdx.x] : 0u;
     const uint32_t s1 = seg_first != nullptr ? seg_first[blockIdx.x + 1u] : n_slices;
@@ -388,7 +385,7 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(const uint32_t *__r
         const uint32_t v = part[x][y], incl = warp_inclusive_scan(v);
         part[x][y] = incl - v;
         const std::size_t c = (std::size_t) blockIdx.x * D + blockIdx.y * 32u + y;
-        if (totals != nullptr && x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
+        if (x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
     }
     __syncthreads();
     if (d < D) {
@@ -402,13 +399,11 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(const uint32_t *__r
 }
 
 // start[segment * D + d]: global slot of the digit's first entry
-__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint32_t *__restrict__ flag,
-                                                             const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
+__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
                                                              const uint32_t *__restrict__ segment,
                                                              const uint32_t *__restrict__ slices,
                                                              const uint32_t *__restrict__ start, uint32_t limit,
                                                              uint32_t *__restrict__ base) {
-    if (flag != nullptr && *flag == 0u) return;
     const uint2 r = tp_slice_rows(range, rows, len);
     const std::size_t c0 = (segment != nullptr ? (std::size_t) segment[blockIdx.x] : 0u) * D;
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
@@ -722,8 +717,8 @@ std::size_t tp_scatter1_csr_smem(uint32_t K) { return sizeof(tp_tile_smem) + ((s
 // column.  Random rows leave nothing to rank by but the counters themselves: a
 // thread's entries take their places in a bucket by shared atomics, in any
 // order, which costs ~50 warp instructions per 32 entries against ~230 of the
-// ballots below.  Only a repeated (row, column) needs the order of the entries,
-// and the Blocked-ELL emit finds those: the ballot kernels then run again.
+// ballots below.  Only a repeated (row, column) needs the order of the entries;
+// the shape pass that follows finds those, and the ballot kernels then run.
 constexpr unsigned kTpThreadsCoo = 512;
 constexpr unsigned kTpPerCoo = kTpTileCoo / kTpThreadsCoo;
 
@@ -786,16 +781,12 @@ std::size_t tp_scatter1_coo_smem(uint32_t K) {
     return (std::size_t) kTpTileCoo * 8u + ((std::size_t) 2u * K + 1u) * 4u;
 }
 
-// The same in the order of the entries (stable), where `flag` is set: a
-// tile's entries are ranked in 32-entry batches by ballots, one per bucket bit.
-// Clears *nnz for the emit that follows.
+// The same in the order of the entries (stable): a tile's entries are ranked in
+// 32-entry batches by ballots, one per bucket bit.
 __global__ void __launch_bounds__(kTpThreads) tp_scatter1_coo_stable_kernel(
-    const uint32_t *__restrict__ flag, uint32_t *__restrict__ nnz_count, const uint32_t *__restrict__ idx,
-    const uint16_t *__restrict__ val, uint32_t uDim, uint32_t nnz, uint32_t low_bits, uint32_t K, uint32_t tiles1,
-    const tp_counts one, const uint32_t *__restrict__ pay, const uint32_t *__restrict__ pay_map,
-    uint32_t *__restrict__ tmp_key, uint16_t *__restrict__ tmp_val) {
-    if (*flag == 0u) return;
-    if (blockIdx.x == 0u && threadIdx.x == 0u) *nnz_count = 0u;
+    const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, const uint32_t *__restrict__ pay,
+    const uint32_t *__restrict__ pay_map, uint32_t uDim, uint32_t nnz, uint32_t low_bits, uint32_t K,
+    const tp_counts one, uint32_t *__restrict__ tmp_key, uint16_t *__restrict__ tmp_val) {
     extern __shared__ __align__(16) uint32_t tp_s[];
     __shared__ uint32_t scan33[33];
     // staged entry: key | value << 32 | bucket << 48
@@ -807,84 +798,81 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_coo_stable_kernel(
     sg.cnt = reinterpret_cast<uint16_t *>(sg.fill + K);                    // [kTpWarps][K]
     sg.bas = sg.cnt + kTpWarps * K;                                        // [kTpWarps][K]
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    for (uint32_t tile = blockIdx.x; tile < tiles1; tile += gridDim.x) {
-        __syncthreads();
-        const uint32_t a = tile * kTpTileCoo, e = min(nnz - a, kTpTileCoo) + a;
-        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
-            run[k] = one.base[(std::size_t) tile * K + k];
-            sg.lb[k] = one.cnt[(std::size_t) tile * K + k];
-            sg.fill[k] = 0u;
+    const uint32_t a = blockIdx.x * kTpTileCoo, e = min(nnz - a, kTpTileCoo) + a;
+    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
+        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        sg.lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
+        sg.fill[k] = 0u;
+    }
+    for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
+    __syncthreads();
+    block_scan_small<4>(sg.lb, K, scan33);
+    const unsigned lt = (1u << lane) - 1u;
+    uint16_t *my_cnt = sg.cnt + warp * K;
+    uint16_t *my_bas = sg.bas + warp * K;
+    uint32_t ncc[kTpBatches], npp[kTpBatches];
+    const uint32_t low_mask = (1u << low_bits) - 1u;
+    uint16_t nvv[kTpBatches];
+    auto fetch = [&](uint32_t sc) {
+        const uint32_t n = min(kTpSub, e - sc);
+        const uint32_t wa = sc + min(n, warp * kTpGran), we = sc + min(n, (warp + 1u) * kTpGran);
+#pragma unroll
+        for (unsigned q = 0; q < kTpBatches; ++q) {
+            const uint32_t i = wa + q * 32u + lane;
+            const bool in = i < we;
+            ncc[q] = in ? __ldg(idx + i) : uDim;
+            nvv[q] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
+            npp[q] = in ? __ldg(pay + i) : 0u;
         }
-        for (uint32_t k = threadIdx.x; k < kTpWarps * K; k += blockDim.x) sg.cnt[k] = 0u;
-        __syncthreads();
-        block_scan_small<4>(sg.lb, K, scan33);
-        const unsigned lt = (1u << lane) - 1u;
-        uint16_t *my_cnt = sg.cnt + warp * K;
-        uint16_t *my_bas = sg.bas + warp * K;
-        uint32_t ncc[kTpBatches], npp[kTpBatches];
-        const uint32_t low_mask = (1u << low_bits) - 1u;
-        uint16_t nvv[kTpBatches];
-        auto fetch = [&](uint32_t sc) {
-            const uint32_t n = min(kTpSub, e - sc);
-            const uint32_t wa = sc + min(n, warp * kTpGran), we = sc + min(n, (warp + 1u) * kTpGran);
+    };
+    fetch(a);
+    for (uint32_t sc0 = a; sc0 < e; sc0 += kTpSub) {
+        uint32_t cc[kTpBatches], pk[kTpBatches], rl[kTpBatches];
+        uint16_t vv[kTpBatches];
 #pragma unroll
-            for (unsigned q = 0; q < kTpBatches; ++q) {
-                const uint32_t i = wa + q * 32u + lane;
-                const bool in = i < we;
-                ncc[q] = in ? __ldg(idx + i) : uDim;
-                nvv[q] = in ? __ldg(reinterpret_cast<const unsigned short *>(val) + i) : (uint16_t) 0u;
-                npp[q] = in ? __ldg(pay + i) : 0u;
-            }
-        };
-        fetch(a);
-        for (uint32_t sc0 = a; sc0 < e; sc0 += kTpSub) {
-            uint32_t cc[kTpBatches], pk[kTpBatches], rl[kTpBatches];
-            uint16_t vv[kTpBatches];
+        for (unsigned q = 0; q < kTpBatches; ++q) {
+            cc[q] = ncc[q];
+            vv[q] = nvv[q];
+            rl[q] = pay_map != nullptr && cc[q] < uDim ? __ldg(pay_map + npp[q]) : npp[q];
+        }
+        if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
 #pragma unroll
-            for (unsigned q = 0; q < kTpBatches; ++q) {
-                cc[q] = ncc[q];
-                vv[q] = nvv[q];
-                rl[q] = pay_map != nullptr && cc[q] < uDim ? __ldg(pay_map + npp[q]) : npp[q];
-            }
-            if (sc0 + kTpSub < e) fetch(sc0 + kTpSub);
-#pragma unroll
-            for (unsigned q = 0; q < kTpBatches; ++q) {
-                const bool ok = cc[q] < uDim;
-                const uint32_t k = cc[q] >> low_bits;
-                pk[q] = warp_match_digit<10>(k, ok);
-                if (ok && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[k] += (uint16_t) __popc(pk[q]);
-                __syncwarp();
-            }
-            __syncthreads();
-            tp_stage_prefix<kTpWarps>(sg, K);
-            __syncthreads();
-#pragma unroll
-            for (unsigned q = 0; q < kTpBatches; ++q) {
-                const bool ok = cc[q] < uDim;
-                const uint32_t k = cc[q] >> low_bits;
-                uint32_t lp = 0u;
-                if (ok) lp = my_bas[k] + __popc(pk[q] & lt);
-                __syncwarp();
-                if (ok) {
-                    if (lp < kTpTileCoo)
-                        st[lp] = (unsigned long long) tp_pack(rl[q], cc[q] & low_mask, low_bits) |
-                                 ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
-                    if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
-                }
-                __syncwarp();
-            }
+        for (unsigned q = 0; q < kTpBatches; ++q) {
+            const bool ok = cc[q] < uDim;
+            const uint32_t k = cc[q] >> low_bits;
+            pk[q] = warp_match_digit<10>(k, ok);
+            if (ok && lane == (unsigned) (__ffs(pk[q]) - 1)) my_cnt[k] += (uint16_t) __popc(pk[q]);
+            __syncwarp();
         }
         __syncthreads();
-        const uint32_t placed = min(sg.lb[K], kTpTileCoo);
-        // run[k] - lb[k]: the global slot of staging slot 0 for bucket k
-        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) run[k] -= sg.lb[k];
+        tp_stage_prefix<kTpWarps>(sg, K);
         __syncthreads();
-        for (uint32_t j = threadIdx.x; j < placed; j += blockDim.x) {
-            const unsigned long long v = st[j];
-            const uint32_t g = run[(uint32_t) (v >> 48)] + j;
-            tmp_key[g] = (uint32_t) v;
-            tmp_val[g] = (uint16_t) (v >> 32);
+#pragma unroll
+        for (unsigned q = 0; q < kTpBatches; ++q) {
+            const bool ok = cc[q] < uDim;
+            const uint32_t k = cc[q] >> low_bits;
+            uint32_t lp = 0u;
+            if (ok) lp = my_bas[k] + __popc(pk[q] & lt);
+            __syncwarp();
+            if (ok) {
+                if (lp < kTpTileCoo)
+                    st[lp] = (unsigned long long) tp_pack(rl[q], cc[q] & low_mask, low_bits) |
+                             ((unsigned long long) vv[q] << 32) | ((unsigned long long) k << 48);
+                if (lane == (unsigned) (__ffs(pk[q]) - 1)) my_bas[k] += (uint16_t) __popc(pk[q]);
+            }
+            __syncwarp();
         }
+    }
+    __syncthreads();
+    const uint32_t placed = min(sg.lb[K], kTpTileCoo);
+    // run[k] - lb[k]: the global slot of staging slot 0 for bucket k
+    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) run[k] -= sg.lb[k];
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < placed; j += blockDim.x) {
+        const unsigned long long v = st[j];
+        const uint32_t g = run[(uint32_t) (v >> 48)] + j;
+        tmp_key[g] = (uint32_t) v;
+        tmp_val[g] = (uint16_t) (v >> 32);
     }
 }
 
@@ -957,39 +945,34 @@ __global__ void __launch_bounds__(1024) tp_chunks_kernel(const tp2_layout l) {
 
 // one histogram per warp while eight of them fit (LB = 8), one per CTA above
 template <int LB>
-__global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ flag,
-                                                             const uint32_t *__restrict__ tmp_key,
-                                                             const uint2 *__restrict__ chunk_range, uint32_t chunks,
+__global__ void __launch_bounds__(kTpThreads) tp_hist2_kernel(const uint32_t *__restrict__ tmp_key,
+                                                             const uint2 *__restrict__ chunk_range,
                                                              uint16_t *__restrict__ cnt) {
     constexpr uint32_t D = 1u << LB;
     constexpr unsigned kCopies = LB == 8 ? kTpWarps : 1u;
     __shared__ uint32_t h[kCopies][D];
-    if (flag != nullptr && *flag == 0u) return;
     const unsigned copy = (threadIdx.x >> 5) % kCopies;
-    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
-        for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
-        __syncthreads();
-        const uint32_t b = chunk_range[chunk].x, e = chunk_range[chunk].y;
-        constexpr unsigned U = 4;
-        for (uint32_t i0 = b; i0 < e; i0 += U * blockDim.x) {
-            uint32_t kk[U];
+    for (uint32_t d = threadIdx.x; d < kCopies * D; d += blockDim.x) (&h[0][0])[d] = 0u;
+    __syncthreads();
+    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
+    constexpr unsigned U = 4;
+    for (uint32_t i0 = b; i0 < e; i0 += U * blockDim.x) {
+        uint32_t kk[U];
 #pragma unroll
-            for (unsigned u = 0; u < U; ++u) {
-                const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
-                kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu; // no packed key: see partition_low_bits
-            }
-#pragma unroll
-            for (unsigned u = 0; u < U; ++u)
-                if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][tp_digit<LB>(kk[u])], 1u);
+        for (unsigned u = 0; u < U; ++u) {
+            const uint32_t i = i0 + u * blockDim.x + threadIdx.x;
+            kk[u] = i < e ? __ldg(tmp_key + i) : 0xffffffffu; // no packed key: see partition_low_bits
         }
-        __syncthreads();
-        for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
-            uint32_t t = 0u;
 #pragma unroll
-            for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
-            cnt[(std::size_t) chunk * D + d] = (uint16_t) t;
-        }
-        if (chunk + gridDim.x < chunks) __syncthreads();
+        for (unsigned u = 0; u < U; ++u)
+            if (kk[u] != 0xffffffffu) atomicAdd(&h[copy][tp_digit<LB>(kk[u])], 1u);
+    }
+    __syncthreads();
+    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+        uint32_t t = 0u;
+#pragma unroll
+        for (unsigned w = 0; w < kCopies; ++w) t += h[w][d];
+        cnt[(std::size_t) blockIdx.x * D + d] = (uint16_t) t;
     }
 }
 
@@ -1064,15 +1047,13 @@ __device__ void tp_rank_ballots(const uint32_t *__restrict__ tmp_key, const uint
 
 // Pass 2 by ballots: a chunk of one bucket reordered by the low digit in shared
 // memory (stable), then written out as one run per key.  Sparse transposes, and
-// COO entries where `flag` is set (null: always).
+// COO entries whose order counts.
 template <int LB>
-__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ flag,
-                                                                const uint32_t *__restrict__ tmp_key,
+__global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
                                                                 const uint16_t *__restrict__ tmp_val,
-                                                                const uint2 *__restrict__ chunk_range, uint32_t chunks,
+                                                                const uint2 *__restrict__ chunk_range,
                                                                 const tp_counts two, uint32_t *__restrict__ out_idx,
                                                                 uint16_t *__restrict__ out_val) {
-    if (flag != nullptr && *flag == 0u) return;
     extern __shared__ __align__(16) uint32_t tp_s2[];
     constexpr uint32_t D = 1u << LB;
     __shared__ uint32_t gbase[D];
@@ -1086,30 +1067,27 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
     sg.bas = sg.cnt + kTpWarps * D;                                        // [kTpWarps][D]
     sg.lb = lb;
     sg.fill = fill;
-    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
-        const uint32_t b = chunk_range[chunk].x, e = chunk_range[chunk].y;
-        if (b >= e) continue;
-        __syncthreads();
-        for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
-            lb[d] = two.cnt[(std::size_t) chunk * D + d];
-            gbase[d] = two.base[(std::size_t) chunk * D + d];
-            fill[d] = 0u;
+    const uint32_t b = chunk_range[blockIdx.x].x, e = chunk_range[blockIdx.x].y;
+    if (b >= e) return;
+    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
+        lb[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
+        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
+        fill[d] = 0u;
 #pragma unroll
-            for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
-        }
-        __syncthreads();
-        block_scan_small<(D / kTpThreads)>(lb, D, scan33);
-        tp_rank_ballots<LB, kTpWarps>(tmp_key, tmp_val, b, e, sg, st_key, st_val);
-        // global slot of staging slot 0 for digit d
-        for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
-        __syncthreads();
-        const uint32_t n = min(e - b, kTpChunk);
-        for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-            const uint32_t key = st_key[j];
-            const uint32_t g = gbase[tp_digit<LB>(key)] + j;
-            out_idx[g] = tp_payload<LB>(key);
-            out_val[g] = st_val[j];
-        }
+        for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
+    }
+    __syncthreads();
+    block_scan_small<(D / kTpThreads)>(lb, D, scan33);
+    tp_rank_ballots<LB, kTpWarps>(tmp_key, tmp_val, b, e, sg, st_key, st_val);
+    // global slot of staging slot 0 for digit d
+    for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) gbase[d] -= lb[d];
+    __syncthreads();
+    const uint32_t n = min(e - b, kTpChunk);
+    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+        const uint32_t key = st_key[j];
+        const uint32_t g = gbase[tp_digit<LB>(key)] + j;
+        out_idx[g] = tp_payload<LB>(key);
+        out_val[g] = st_val[j];
     }
 }
 
@@ -1330,37 +1308,23 @@ int tp_smem(K kernel, std::size_t smem, const char *what) {
     return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem), what);
 }
 
-// Counts of `l`'s pass-1 result (low digit of LB bits), the row pointers and
-// every chunk's offsets; with a flag, the chunks' offsets again where it is
-// set, in grids of one wave.
-template <int LB>
-int tp_count_chunks(const uint32_t *flag, uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, cudaStream_t stream) {
-    constexpr uint32_t D = 1u << LB;
-    const unsigned grid = flag == nullptr
-                              ? l.max_chunks
-                              : resident_grid((const void *) tp_hist2_kernel<LB>, kTpThreads, 0, l.max_chunks);
-    tp_hist2_kernel<LB><<<grid, kTpThreads, 0, stream>>>(flag, l.tmp_key, l.chunk_range, l.max_chunks, l.two.cnt);
-    if (!launch_ok("tp_hist2_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, 0u, l.slice_range, l.two.slices);
-    if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(flag, l.two.slices, D, l.slice_first, 0u, uDim,
-                                                                  flag == nullptr ? out_ptr : nullptr);
-    if (!launch_ok("tp_slice_scan_kernel")) return 0;
-    if (flag == nullptr &&
-        !scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream))
-        return 0;
-    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(flag, l.two.cnt, D, 0u, 0u, l.slice_range, l.slice_bucket,
-                                                            l.two.slices, out_ptr, uDim, l.two.base);
-    return launch_ok("tp_slice_apply_kernel");
-}
-
-// Pass 2.  rows: the payloads of a bucket never decrease (the transpose); any:
+// Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).  rows: the payloads of a bucket never decrease (the transpose); any:
 // entries of one key in any order (COO).
 template <int LB, tp_rank kRank>
 int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
                    cudaStream_t stream) {
     static_assert(kRank != tp_rank::rows || LB == (int) kTpBucketBits, "the row ranking has 256 digits");
-    if (!tp_count_chunks<LB>(nullptr, uDim, l, out_ptr, stream)) return 0;
+    tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_range, l.two.cnt);
+    if (!launch_ok("tp_hist2_kernel")) return 0;
+    constexpr uint32_t D = 1u << LB;
+    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, 0u, l.slice_range, l.two.slices);
+    if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(l.two.slices, D, l.slice_first, 0u, uDim, out_ptr);
+    if (!launch_ok("tp_slice_scan_kernel")) return 0;
+    if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
+    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, 0u, l.slice_range, l.slice_bucket,
+                                                            l.two.slices, out_ptr, uDim, l.two.base);
+    if (!launch_ok("tp_slice_apply_kernel")) return 0;
     if constexpr (kRank == tp_rank::rows) {
         if (!tp_smem(tp_scatter2_rows_kernel, sizeof(tp_rows_smem), "scatter2 smem attribute")) return 0;
         tp_scatter2_rows_kernel<<<l.max_chunks, kTpThreads2, sizeof(tp_rows_smem), stream>>>(
@@ -1373,15 +1337,16 @@ int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32
     } else {
         constexpr std::size_t smem = tp_scatter2_smem(LB);
         if (!tp_smem(tp_scatter2_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
-        tp_scatter2_kernel<LB><<<l.max_chunks, kTpThreads, smem, stream>>>(nullptr, l.tmp_key, l.tmp_val, l.chunk_range,
-                                                                           l.max_chunks, l.two, out_idx, out_val);
+        tp_scatter2_kernel<LB><<<l.max_chunks, kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range, l.two,
+                                                                           out_idx, out_val);
     }
     return launch_ok("tp_scatter2_kernel");
 }
 
-// Pass 1: `ptr` is null for COO (payloads `pay` through `pay_map`).
+// Pass 1: `ptr` is null for COO (payloads `pay` through `pay_map`; `stable`
+// keeps the entries' order).
 int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *ptr, const uint32_t *key,
-                  const uint16_t *val, const uint32_t *pay, const uint32_t *pay_map, const tp2_layout &l,
+                  const uint16_t *val, const uint32_t *pay, const uint32_t *pay_map, bool stable, const tp2_layout &l,
                   cudaStream_t stream) {
     const bool csr = ptr != nullptr, vec = (reinterpret_cast<uintptr_t>(key) & 15u) == 0u;
     auto hist1 = csr ? (vec ? tp_hist1_kernel<kTpTileCsr, true> : tp_hist1_kernel<kTpTileCsr, false>)
@@ -1389,14 +1354,14 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
     hist1<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K, l.one.cnt,
                                                                     l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, l.one.slices);
+    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, l.one.slices);
     if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(nullptr, l.one.slices, l.K, nullptr, l.slices1, l.K,
+    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(l.one.slices, l.K, nullptr, l.slices1, l.K,
                                                                           l.total1);
     if (!launch_ok("tp_slice_scan_kernel")) return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
     if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(nullptr, l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr, l.one.slices,
+    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr, l.one.slices,
                                                          l.start1, l.K, l.one.base);
     if (!launch_ok("tp_slice_apply_kernel")) return 0;
     if (csr) {
@@ -1404,6 +1369,12 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
         if (!tp_smem(tp_scatter1_csr_kernel, smem, "scatter1 smem attribute")) return 0;
         tp_scatter1_csr_kernel<<<l.tiles1, kTpThreads1, smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.K, l.one,
                                                                         l.gran_row, l.tmp_key, l.tmp_val);
+    } else if (stable) {
+        const std::size_t smem = tp_scatter1_smem(l.K);
+        if (!tp_smem(tp_scatter1_coo_stable_kernel, smem, "scatter1 smem attribute")) return 0;
+        tp_scatter1_coo_stable_kernel<<<l.tiles1, kTpThreads, smem, stream>>>(key, val, pay, pay_map, uDim, nnz,
+                                                                              l.low_bits, l.K, l.one, l.tmp_key,
+                                                                              l.tmp_val);
     } else {
         const std::size_t smem = tp_scatter1_coo_smem(l.K);
         if (!tp_smem(tp_scatter1_coo_kernel, smem, "scatter1 smem attribute")) return 0;
@@ -1418,7 +1389,7 @@ int transpose2_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t
                       const tp2_layout &l, cudaStream_t stream) {
     tp_gran_rows_kernel<<<(cDim + 255u) / 256u, 256, 0, stream>>>(ptr, cDim, l.gran_row);
     if (!launch_ok("tp_gran_rows_kernel")) return 0;
-    return tp_first_pass(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, l, stream) &&
+    return tp_first_pass(cDim, uDim, nnz, ptr, idx, val, nullptr, nullptr, false, l, stream) &&
            ((double) nnz >= kTpRowsKernelMin * (double) cDim * (double) l.K
                 ? tp_second_pass<(int) kTpBucketBits, tp_rank::rows>(uDim, l, out_ptr, out_idx, out_val, stream)
                 : tp_second_pass<(int) kTpBucketBits, tp_rank::ballots>(uDim, l, out_ptr, out_idx, out_val, stream));
@@ -1486,7 +1457,7 @@ int transpose_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t 
 }
 
 // COO entries by rows: row pointers, columns (through `map` when given) and
-// values, a row's entries in any order.  Every row is below `rows` and every
+// values, a row's entries in any order or, `stable`, in their own.  Every row is below `rows` and every
 // mapped column below `cols`.  Two passes move 22 bytes an entry in runs; the
 // two stable 32-bit sorts and the random gathers that this replaces moved over
 // 100, most of them one sector per entry.
@@ -1499,8 +1470,8 @@ std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t col
 }
 
 int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row, const uint32_t *col,
-                   const uint32_t *map, const uint16_t *val, uint32_t *out_ptr, uint32_t *out_col, uint16_t *out_val,
-                   void *scratch, std::size_t scratch_bytes, cudaStream_t stream) {
+                   const uint32_t *map, const uint16_t *val, bool stable, uint32_t *out_ptr, uint32_t *out_col,
+                   uint16_t *out_val, void *scratch, std::size_t scratch_bytes, cudaStream_t stream) {
     const uint32_t lb = partition_low_bits(rows, cols);
     if (n == 0u || rows == 0u || lb == 0u) {
         set_error("partition_rows: %u rows by %u columns outside its range", rows, cols);
@@ -1513,55 +1484,18 @@ int partition_rows(uint32_t n, uint32_t rows, uint32_t cols, const uint32_t *row
         return 0;
     }
     if (!cuda_ok(cudaMemsetAsync(l.status, 0, 16, stream), "partition status memset") ||
-        !tp_first_pass(0u, rows, n, nullptr, row, val, col, map, l, stream))
+        !tp_first_pass(0u, rows, n, nullptr, row, val, col, map, stable, l, stream))
         return 0;
+    auto second = [&](auto low) {
+        constexpr int LB = decltype(low)::value;
+        return stable ? tp_second_pass<LB, tp_rank::ballots>(rows, l, out_ptr, out_col, out_val, stream)
+                      : tp_second_pass<LB, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
+    };
     switch (lb) {
-        case 8u: return tp_second_pass<8, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
-        case 9u: return tp_second_pass<9, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
-        case 10u: return tp_second_pass<10, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
-        default: return tp_second_pass<11, tp_rank::any>(rows, l, out_ptr, out_col, out_val, stream);
-    }
-}
-
-// The same entries again in their own order (stable), where *flag is set, from
-// the pass-1 offsets and chunks that partition_rows left in `scratch` (a chunk
-// may end inside a tile's run, so its counts are taken anew); *nnz_count is
-// cleared with it.  Where the flag is clear, the launches are all it costs.
-template <int LB>
-static int partition_rows_stable_lb(uint32_t rows, const tp2_layout &l, const uint32_t *flag, const uint32_t *row_ptr,
-                                    uint32_t *out_col, uint16_t *out_val, cudaStream_t stream) {
-    constexpr std::size_t smem = tp_scatter2_smem(LB);
-    if (!tp_count_chunks<LB>(flag, rows, l, const_cast<uint32_t *>(row_ptr), stream)) return 0; // read only
-    if (!tp_smem(tp_scatter2_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
-    tp_scatter2_kernel<LB><<<resident_grid((const void *) tp_scatter2_kernel<LB>, kTpThreads, smem, l.max_chunks),
-                             kTpThreads, smem, stream>>>(flag, l.tmp_key, l.tmp_val, l.chunk_range, l.max_chunks, l.two,
-                                                         out_col, out_val);
-    return launch_ok("tp_scatter2_kernel");
-}
-
-int partition_rows_stable(const uint32_t *flag, uint32_t *nnz_count, uint32_t n, uint32_t rows, uint32_t cols,
-                          const uint32_t *row, const uint32_t *col, const uint32_t *map, const uint16_t *val,
-                          const uint32_t *row_ptr, uint32_t *out_col, uint16_t *out_val, void *scratch,
-                          std::size_t scratch_bytes, cudaStream_t stream) {
-    const uint32_t lb = partition_low_bits(rows, cols);
-    tp2_layout l;
-    tp2_make_layout(rows, n, lb == 0u ? kTpBucketBits : lb, false, scratch, scratch_bytes, &l);
-    if (n == 0u || rows == 0u || lb == 0u || scratch == nullptr || l.bytes > scratch_bytes) {
-        set_error("partition_rows_stable: outside its range");
-        return 0;
-    }
-    const std::size_t smem = tp_scatter1_smem(l.K);
-    if (!tp_smem(tp_scatter1_coo_stable_kernel, smem, "scatter1 smem attribute")) return 0;
-    tp_scatter1_coo_stable_kernel<<<resident_grid((const void *) tp_scatter1_coo_stable_kernel, kTpThreads, smem,
-                                                  l.tiles1),
-                                    kTpThreads, smem, stream>>>(flag, nnz_count, row, val, rows, n, l.low_bits, l.K,
-                                                                l.tiles1, l.one, col, map, l.tmp_key, l.tmp_val);
-    if (!launch_ok("tp_scatter1_kernel")) return 0;
-    switch (lb) {
-        case 8u: return partition_rows_stable_lb<8>(rows, l, flag, row_ptr, out_col, out_val, stream);
-        case 9u: return partition_rows_stable_lb<9>(rows, l, flag, row_ptr, out_col, out_val, stream);
-        case 10u: return partition_rows_stable_lb<10>(rows, l, flag, row_ptr, out_col, out_val, stream);
-        default: return partition_rows_stable_lb<11>(rows, l, flag, row_ptr, out_col, out_val, stream);
+        case 8u: return second(std::integral_constant<int, 8>{});
+        case 9u: return second(std::integral_constant<int, 9>{});
+        case 10u: return second(std::integral_constant<int, 10>{});
+        default: return second(std::integral_constant<int, 11>{});
     }
 }
 

@@ -107,3 +107,14 @@ def test_short_rows_in_runs(cuda, orc, rows, cols, longest, block):
     ref = orc.blocked_ell_from_csr(rows, cols, ptr, idx, val, block)
     assert out.ell_cols == ref["ell_cols"] and out.nnz == ref["nnz"]
     assert np.array_equal(np_u32(out.bci), ref["bci"]) and np.array_equal(np_u16(out.val), ref["val"])
+
+
+@pytest.mark.parametrize("rows,cols,n,block,repeat", [
+    (300, 1_000, 60_000, 1, 0), (300, 1_000, 60_000, 1, 3),  # one row per row block: one warp
+    (301, 1_003, 90_000, 3, 1),                              # no power of two
+    (90, 2_049, 80_000, 32, 0), (90, 2_049, 80_000, 32, 2),  # rows of several 256-column rounds
+    (40, 203_000, 30_000, 16, 2),                            # the widest rows of which bitmaps fit, and
+    (40, 210_000, 30_000, 16, 0), (40, 210_000, 30_000, 16, 2),  # wider: in the entries' order at once
+])
+def test_shuffled_coo_repeats_in_the_shape_pass(cuda, orc, rows, cols, n, block, repeat):
+    test_shuffled_coo(cuda, orc, rows, cols, n, block, 0, repeat, False)
