@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "moments_device.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace csb {
@@ -52,9 +53,10 @@ struct moments_layout {
     uint32_t *num_chunks;      // [1]
     chunk_desc *chunks;        // [max_chunks]
     uint32_t *sorted_rows;     // [rows]
-    float *partials;           // [max_chunks * 4 * cols]
+    float *partials;           // [max_chunks * 4 * pstride]
     std::size_t bytes;
-    uint32_t row_blocks, words, tiles, max_chunks, chunk_rows, col_blocks;
+    uint32_t row_blocks, words, tiles, max_chunks, chunk_rows, col_blocks, pstride;
+    bool short_chunks;         // see moments_accumulate_kernel
 };
 
 // Rows per chunk where the caller leaves it open.  A chunk's CTAs walk its rows
@@ -63,8 +65,8 @@ struct moments_layout {
 // partials a column, 16 / chunk_rows of the rows' own bytes.  Halved to 256
 // rows (6 %) while there are under 1,000 CTAs, and on to 64 only while there
 // are under two per SM.  us per call by 2,048 / 256 / 64 rows: 8,192 x 2,000
-// 95 / 49 / 33; 100,000 x 5,000 (16 groups) 349 / 179 / 258; 20,000 x 8,000 (64
-// groups) 80 / 80 / 103; 50,000 x 32,768 493 / 531 / 735 (1,024 taken: 494).
+// (8 groups) 99 / 52 / 36; 100,000 x 5,000 (16) 344 / 177 / 217; 20,000 x 8,000
+// (64) 78 / 76 / 83; 50,000 x 32,768 (64) 479 / 489 / 572 (1,024: 480).
 uint32_t default_chunk_rows(uint32_t rows, uint32_t col_blocks, uint32_t block_size, uint32_t groups) {
     const uint64_t segs = (uint64_t) col_blocks * ((block_size + 7u) / 8u);
     const uint64_t tiles = (segs + kAccThreads - 1u) / kAccThreads;
@@ -76,8 +78,9 @@ uint32_t default_chunk_rows(uint32_t rows, uint32_t col_blocks, uint32_t block_s
     return chunk;
 }
 
+// padded: the partials' columns in multiples of eight, for 16-byte stores.
 bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *p, void *base, std::size_t cap,
-                 moments_layout *lay) {
+                 moments_layout *lay, bool padded = true) {
     const uint32_t B = src->block_size;
     lay->row_blocks = (src->rows + B - 1u) / B;
     lay->col_blocks = (src->cols + B - 1u) / B;
@@ -86,6 +89,7 @@ bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *
     lay->chunk_rows = p->chunk_rows == 0u ? default_chunk_rows(src->rows, lay->col_blocks, B, p->group_count) : p->chunk_rows;
     const std::size_t G = p->group_count;
     lay->max_chunks = (uint32_t) ((src->rows + lay->chunk_rows - 1u) / lay->chunk_rows + G);
+    lay->short_chunks = std::min<std::size_t>(lay->chunk_rows, G != 0u ? src->rows / G : 0u) <= 512u;
     scratch_carver c(base, cap);
     lay->index = c.take<uint2>((std::size_t) lay->row_blocks * lay->words + 1);
     lay->tile_counts = c.take<uint32_t>((std::size_t) lay->tiles * G + 1);
@@ -95,7 +99,8 @@ bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *
     lay->num_chunks = c.take<uint32_t>(1);
     lay->chunks = c.take<chunk_desc>(lay->max_chunks);
     lay->sorted_rows = c.take<uint32_t>((std::size_t) src->rows + 1);
-    lay->partials = c.take<float>((std::size_t) lay->max_chunks * 4u * src->cols + 1);
+    lay->pstride = padded && src->cols <= 0xfffffff8u ? (src->cols + 7u) & ~7u : src->cols;
+    lay->partials = c.take<float>((std::size_t) lay->max_chunks * 4u * lay->pstride + 1);
     lay->bytes = c.used;
     return c.fits();
 }
@@ -172,9 +177,10 @@ __global__ void __launch_bounds__(kIndexWarps * 32) moments_index_kernel(const u
 __device__ __forceinline__ uint32_t row_group(uint32_t r, uint32_t rows, const uint8_t *keep, const uint32_t *labels,
                                               uint32_t G) {
     if (r >= rows) return G;
-    if (keep != nullptr && keep[r] == 0u) return G;
-    const uint32_t g = labels != nullptr ? labels[r] : 0u;
-    return g < G ? g : G;
+    // both loads at once: the label does not wait for the mask
+    const uint32_t g = labels != nullptr ? __ldg(labels + r) : 0u;
+    const bool kept = keep == nullptr || __ldg(keep + r) != 0u;
+    return kept && g < G ? g : G;
 }
 
 __global__ void __launch_bounds__(kSortThreads) moments_tile_hist_kernel(uint32_t rows, const uint8_t *__restrict__ keep,
@@ -184,10 +190,15 @@ __global__ void __launch_bounds__(kSortThreads) moments_tile_hist_kernel(uint32_
     for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) hist[g] = 0u;
     __syncthreads();
     const uint32_t base = blockIdx.x * kTileRows;
-    for (uint32_t i = threadIdx.x; i < kTileRows; i += blockDim.x) {
-        const uint32_t g = row_group(base + i, rows, keep, labels, G);
-        if (g < G) atomicAdd(hist + g, 1u);
-    }
+    // a small matrix is a few CTAs that wait for memory: all rows of a thread
+    // are loaded before any is counted (here and in the scatter)
+    uint32_t g[kTileRows / kSortThreads];
+#pragma unroll
+    for (uint32_t k = 0; k < kTileRows / kSortThreads; ++k)
+        g[k] = row_group(base + k * kSortThreads + threadIdx.x, rows, keep, labels, G);
+#pragma unroll
+    for (uint32_t k = 0; k < kTileRows / kSortThreads; ++k)
+        if (g[k] < G) atomicAdd(hist + g[k], 1u);
     __syncthreads();
     for (uint32_t g = threadIdx.x; g < G; g += blockDim.x)
         tile_counts[(std::size_t) blockIdx.x * G + g] = hist[g];
@@ -259,15 +270,18 @@ __global__ void __launch_bounds__(kSortThreads) moments_tile_scatter_kernel(uint
                                                                             uint32_t *__restrict__ sorted_rows) {
     extern __shared__ uint32_t warp_counts[]; // [kSortWarps][G]
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    constexpr uint32_t rows_per_warp = kTileRows / kSortWarps, batches = rows_per_warp / 32u;
+    const uint32_t wbase = blockIdx.x * kTileRows + warp * rows_per_warp;
+    uint32_t group[batches], peers_of[batches];
+#pragma unroll
+    for (uint32_t b = 0; b < batches; ++b) group[b] = row_group(wbase + b * 32u + lane, rows, keep, labels, G);
     for (uint32_t i = threadIdx.x; i < kSortWarps * G; i += blockDim.x) warp_counts[i] = 0u;
     __syncthreads();
-    constexpr uint32_t rows_per_warp = kTileRows / kSortWarps;
-    const uint32_t wbase = blockIdx.x * kTileRows + warp * rows_per_warp;
     uint32_t *my = warp_counts + (std::size_t) warp * G;
-    for (uint32_t b = 0; b < rows_per_warp; b += 32u) {
-        const uint32_t r = wbase + b + lane;
-        const uint32_t g = row_group(r, rows, keep, labels, G);
-        const uint32_t peers = __match_any_sync(0xffffffffu, g);
+#pragma unroll
+    for (uint32_t b = 0; b < batches; ++b) {
+        const uint32_t g = group[b];
+        const uint32_t peers = peers_of[b] = __match_any_sync(0xffffffffu, g);
         if (g < G && lane == (unsigned) (__ffs(peers) - 1)) my[g] += __popc(peers);
         __syncwarp();
     }
@@ -282,10 +296,9 @@ __global__ void __launch_bounds__(kSortThreads) moments_tile_scatter_kernel(uint
     }
     __syncthreads();
     const unsigned lt = (1u << lane) - 1u;
-    for (uint32_t b = 0; b < rows_per_warp; b += 32u) {
-        const uint32_t r = wbase + b + lane;
-        const uint32_t g = row_group(r, rows, keep, labels, G);
-        const uint32_t peers = __match_any_sync(0xffffffffu, g);
+#pragma unroll
+    for (uint32_t b = 0; b < batches; ++b) {
+        const uint32_t r = wbase + b * 32u + lane, g = group[b], peers = peers_of[b];
         uint32_t base = 0u;
         if (g < G) base = my[g];
         __syncwarp();
@@ -332,10 +345,16 @@ struct many_partition_rows {
     }
 };
 
-template <int L, bool COMP, typename Rows>
+// kVecStore: partials in 16-byte stores.  A thread's eight columns stand side by
+// side, so a scalar store of a warp is 32 sectors for 128 bytes: half of the time
+// of chunks of a dozen rows (3,000 x 20,000, 250 groups: 111 us, 52 with 16-byte
+// stores), nothing at 2,048 rows, where the registers in fours cost the row loop
+// 1.6 % (500,000 x 32,768, 64 groups: 3.99 and 4.06 ms).  Taken up to 512 rows;
+// both meet at about 1,200.
+template <int L, bool COMP, bool kVecStore, typename Rows>
 __global__ void __launch_bounds__(kAccThreads, 2) moments_accumulate_kernel(
-    Rows rows_of, uint32_t block_size, uint32_t col_blocks, uint32_t cols, const chunk_desc *__restrict__ chunks,
-    const uint32_t *__restrict__ num_chunks, float *__restrict__ partials, const uint32_t *__restrict__ chunk_first,
+    Rows rows_of, uint32_t block_size, uint32_t col_blocks, uint32_t cols, uint32_t pstride,
+    const chunk_desc *__restrict__ chunks, const uint32_t *__restrict__ num_chunks, float *__restrict__ partials, const uint32_t *__restrict__ chunk_first,
     uint32_t g_lo, uint32_t g_hi) {
     using entry = typename Rows::entry;
     extern __shared__ __align__(16) unsigned char acc_smem[];
@@ -420,18 +439,27 @@ __global__ void __launch_bounds__(kAccThreads, 2) moments_accumulate_kernel(
             }
         }
     }
-    // tail rows (fewer than a batch); their index entries are in e_next
+    // tail rows (fewer than a batch); their index entries are in e_next.  All
+    // values are loaded before any is added: a group of few rows is all tail
+    if (i < n) {
+        raw_vec<L> raw[kBatch];
+        uint32_t has = 0u;
 #pragma unroll
-    for (unsigned u = 0; u < kBatch; ++u) {
-        if (i + u < n) {
-            const uint2 e = e_next[u];
+        for (unsigned u = 0; u < kBatch; ++u) {
+            const uint2 e = e_next[u]; // zero past the last row
+            zero_raw<L>(raw[u]);
             if (e.x & bitmask) {
-                raw_vec<L> raw;
+                has |= 1u << u;
                 const uint32_t slot = e.y + __popc(e.x & below);
                 load_raw<L>(rows_of.row(chunk_rows_smem[i + u]) + (std::size_t) slot * block_size + lane_off,
-                            raw);
+                            raw[u]);
+            }
+        }
+#pragma unroll
+        for (unsigned u = 0; u < kBatch; ++u) {
+            if ((has >> u) & 1u) {
                 float x[L];
-                unpack<L>(raw, x);
+                unpack<L>(raw[u], x);
 #pragma unroll
                 for (int j = 0; j < L; ++j) {
                     if (COMP) {
@@ -446,94 +474,154 @@ __global__ void __launch_bounds__(kAccThreads, 2) moments_accumulate_kernel(
         }
     }
     const std::size_t f0 = (std::size_t) b * block_size + lane_off;
-    float *p = partials + (std::size_t) c * 4u * cols;
+    if (f0 >= cols) return;
+    float *p = partials + (std::size_t) c * 4u * pstride + f0;
+    // in padded columns a segment, which starts at a multiple of its L, ends inside them
+    const bool vec = kVecStore && (pstride & 7u) == 0u && (reinterpret_cast<uintptr_t>(partials) & 15u) == 0u;
+    auto store = [&](const float (&x)[L], uint32_t k) {
+        float *to = p + (std::size_t) k * pstride;
+        if constexpr (kVecStore && L % 4 == 0) {
+            if (vec) {
 #pragma unroll
-    for (int j = 0; j < L; ++j) {
-        const std::size_t f = f0 + j;
-        if (f < cols) {
-            p[f] = s_hi[j];
-            p[cols + f] = s_lo[j];
-            p[2u * (std::size_t) cols + f] = q_hi[j];
-            p[3u * (std::size_t) cols + f] = q_lo[j];
+                for (int j = 0; j < L; j += 4)
+                    *reinterpret_cast<float4 *>(to + j) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+                return;
+            }
         }
-    }
+#pragma unroll
+        for (int j = 0; j < L; ++j)
+            if (f0 + j < cols) to[j] = x[j];
+    };
+    store(s_hi, 0u);
+    store(s_lo, 1u);
+    store(q_hi, 2u);
+    store(q_lo, 3u);
 }
 
 // ---------------------------------------------------------------------------
 // 4. Combine.
 // ---------------------------------------------------------------------------
+// a / b from y, the rounded 1 / b: the product corrected twice by its exact
+// remainder, which is the correctly rounded quotient (P. Markstein, Computation
+// of elementary functions on the IBM RISC System/6000 processor, 1990) where b
+// is a whole number of 32 bits and nothing is near the ends of the double range;
+// infinities and NaN pass through the product.
+__device__ __forceinline__ double divide_by(double a, double b, double y) {
+    const double q0 = a * y;
+    const double q1 = fma(fma(-q0, b, a), y, q0);
+    const double q2 = fma(fma(-q1, b, a), y, q1);
+    return isinf(q0) ? q0 : q2;
+}
+
+// A thread adds C columns, 256 apart.  Bound by issue slots where a group has
+// one or two chunks: two divisions an output, by the group's row counts, were
+// half of the instructions; four columns share the reciprocals (250 groups of
+// 20,000 columns: 58 -> 32 us).
+template <int C>
 __global__ void __launch_bounds__(256) moments_combine_kernel(
-    uint32_t cols, uint32_t G, uint32_t scheme, uint32_t ddof, const uint32_t *__restrict__ chunk_first,
-    const uint32_t *__restrict__ group_rows, const float *__restrict__ partials, const uint8_t *__restrict__ feature_keep,
-    float *__restrict__ out_sum, float *__restrict__ out_sumsq, float *__restrict__ out_mean, float *__restrict__ out_var,
+    uint32_t cols, uint32_t pstride, uint32_t G, uint32_t scheme, uint32_t ddof,
+    const uint32_t *__restrict__ chunk_first, const uint32_t *__restrict__ group_rows,
+    const float *__restrict__ partials, const uint8_t *__restrict__ feature_keep, float *__restrict__ out_sum,
+    float *__restrict__ out_sumsq, float *__restrict__ out_mean, float *__restrict__ out_var,
     double *__restrict__ out_mean64, double *__restrict__ out_var64, uint32_t *__restrict__ out_group_rows,
     uint32_t g_base) {
     const uint32_t g = g_base + blockIdx.y;
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t f0 = blockIdx.x * (256u * C) + threadIdx.x;
     if (g >= G) return;
-    if (f == 0 && out_group_rows != nullptr) out_group_rows[g] = group_rows[g];
-    if (f >= cols) return;
+    if (f0 == 0 && out_group_rows != nullptr) out_group_rows[g] = group_rows[g];
     const uint32_t c0 = chunk_first[g], c1 = chunk_first[g + 1];
     const uint32_t n = group_rows[g];
-    const bool kept = feature_keep == nullptr || feature_keep[f] != 0u;
-    const std::size_t o = (std::size_t) g * cols + f;
-    float rs = 0.0f, rq = 0.0f, rm = 0.0f, rv = 0.0f;
-    double dm = 0.0, dv = 0.0;
-    if (kept) {
-        if (scheme == CS_MOMENTS_TWOSUM_F64_COMBINE) {
-            double s = 0.0, q = 0.0;
-#pragma unroll 8
-            for (uint32_t c = c0; c < c1; ++c) {
-                const float *p = partials + (std::size_t) c * 4u * cols;
-                s += (double) p[f] + (double) p[cols + f];
-                q += (double) p[2u * (std::size_t) cols + f] + (double) p[3u * (std::size_t) cols + f];
+    bool kept[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        const uint32_t f = f0 + 256u * k;
+        kept[k] = f < cols && (feature_keep == nullptr || feature_keep[f] != 0u);
+    }
+    float rs[C], rq[C], rm[C], rv[C];
+    double dm[C], dv[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        rs[k] = rq[k] = rm[k] = rv[k] = 0.0f;
+        dm[k] = dv[k] = 0.0;
+    }
+    if (scheme == CS_MOMENTS_TWOSUM_F64_COMBINE) {
+        double s[C], q[C];
+#pragma unroll
+        for (int k = 0; k < C; ++k) s[k] = q[k] = 0.0;
+#pragma unroll (8 / C)
+        for (uint32_t c = c0; c < c1; ++c) {
+            const float *p = partials + (std::size_t) c * 4u * pstride + f0;
+            float x[C][4];
+#pragma unroll
+            for (int k = 0; k < C; ++k)
+#pragma unroll
+                for (unsigned a = 0; a < 4u; ++a) x[k][a] = kept[k] ? p[a * (std::size_t) pstride + 256u * k] : 0.0f;
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                s[k] += (double) x[k][0] + (double) x[k][1];
+                q[k] += (double) x[k][2] + (double) x[k][3];
             }
-            rs = (float) s;
-            rq = (float) q;
-            if (n > 0u) {
-                dm = s / (double) n;
+        }
+        const double by_n = (double) n, by_dof = (double) (n > ddof ? n - ddof : 1u);
+        const double inv_n = 1.0 / by_n, inv_dof = 1.0 / by_dof;
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            rs[k] = (float) s[k];
+            rq[k] = (float) q[k];
+            if (kept[k] && n > 0u) {
+                dm[k] = C == 1 ? s[k] / by_n : divide_by(s[k], by_n, inv_n);
                 if (n > ddof) {
-                    double m2 = q - s * dm;
+                    double m2 = q[k] - s[k] * dm[k];
                     if (m2 < 0.0) m2 = 0.0;
-                    dv = m2 / (double) (n - ddof);
+                    dv[k] = C == 1 ? m2 / by_dof : divide_by(m2, by_dof, inv_dof);
                 }
             }
-            rm = (float) dm;
-            rv = (float) dv;
-        } else {
+            rm[k] = (float) dm[k];
+            rv[k] = (float) dv[k];
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            if (!kept[k]) continue;
             float s_hi = 0.0f, s_lo = 0.0f, q_hi = 0.0f, q_lo = 0.0f;
             for (uint32_t c = c0; c < c1; ++c) {
-                const float *p = partials + (std::size_t) c * 4u * cols;
+                const float *p = partials + (std::size_t) c * 4u * pstride + f0 + 256u * k;
                 if (scheme == CS_MOMENTS_TWOSUM_F32) {
-                    two_sum_acc(s_hi, s_lo, p[f]);
-                    s_lo = __fadd_rn(s_lo, p[cols + f]);
-                    two_sum_acc(q_hi, q_lo, p[2u * (std::size_t) cols + f]);
-                    q_lo = __fadd_rn(q_lo, p[3u * (std::size_t) cols + f]);
+                    two_sum_acc(s_hi, s_lo, p[0]);
+                    s_lo = __fadd_rn(s_lo, p[pstride]);
+                    two_sum_acc(q_hi, q_lo, p[2u * (std::size_t) pstride]);
+                    q_lo = __fadd_rn(q_lo, p[3u * (std::size_t) pstride]);
                 } else {
-                    s_hi = __fadd_rn(s_hi, p[f]);
-                    q_hi = __fadd_rn(q_hi, p[2u * (std::size_t) cols + f]);
+                    s_hi = __fadd_rn(s_hi, p[0]);
+                    q_hi = __fadd_rn(q_hi, p[2u * (std::size_t) pstride]);
                 }
             }
-            rs = __fadd_rn(s_hi, s_lo);
-            rq = __fadd_rn(q_hi, q_lo);
+            rs[k] = __fadd_rn(s_hi, s_lo);
+            rq[k] = __fadd_rn(q_hi, q_lo);
             if (n > 0u) {
-                rm = __fdiv_rn(rs, (float) n);
+                rm[k] = __fdiv_rn(rs[k], (float) n);
                 if (n > ddof) {
-                    float m2 = __fsub_rn(rq, __fmul_rn(rs, rm));
+                    float m2 = __fsub_rn(rq[k], __fmul_rn(rs[k], rm[k]));
                     if (m2 < 0.0f) m2 = 0.0f;
-                    rv = __fdiv_rn(m2, (float) (n - ddof));
+                    rv[k] = __fdiv_rn(m2, (float) (n - ddof));
                 }
             }
-            dm = rm;
-            dv = rv;
+            dm[k] = rm[k];
+            dv[k] = rv[k];
         }
     }
-    out_sum[o] = rs;
-    out_sumsq[o] = rq;
-    if (out_mean != nullptr) out_mean[o] = rm;
-    if (out_var != nullptr) out_var[o] = rv;
-    if (out_mean64 != nullptr) out_mean64[o] = dm;
-    if (out_var64 != nullptr) out_var64[o] = dv;
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        const uint32_t f = f0 + 256u * k;
+        if (f >= cols) continue;
+        const std::size_t o = (std::size_t) g * cols + f;
+        out_sum[o] = rs[k];
+        out_sumsq[o] = rq[k];
+        if (out_mean != nullptr) out_mean[o] = rm[k];
+        if (out_var != nullptr) out_var[o] = rv[k];
+        if (out_mean64 != nullptr) out_mean64[o] = dm[k];
+        if (out_var64 != nullptr) out_var64[o] = dv[k];
+    }
 }
 
 template <int L, bool COMP, typename Rows>
@@ -542,12 +630,13 @@ int launch_accumulate_rows(const Rows &rows_of, uint32_t block_size, uint32_t co
     const uint32_t segs = lay.col_blocks * (block_size / L);
     dim3 grid(lay.max_chunks, (segs + kAccThreads - 1u) / kAccThreads);
     const std::size_t smem = (std::size_t) lay.chunk_rows * sizeof(typename Rows::entry);
-    auto kern = moments_accumulate_kernel<L, COMP, Rows>;
+    auto kern = lay.short_chunks ? moments_accumulate_kernel<L, COMP, true, Rows>
+                                 : moments_accumulate_kernel<L, COMP, false, Rows>;
     if (smem > 48u * 1024u &&
         !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
                  "moments smem attribute"))
         return 0;
-    kern<<<grid, kAccThreads, smem, stream>>>(rows_of, block_size, lay.col_blocks, cols, lay.chunks, lay.num_chunks,
+    kern<<<grid, kAccThreads, smem, stream>>>(rows_of, block_size, lay.col_blocks, cols, lay.pstride, lay.chunks, lay.num_chunks,
                                               lay.partials, chunk_first, g_lo, g_hi);
     return launch_ok("moments_accumulate_kernel");
 }
@@ -665,11 +754,16 @@ int sort_rows_by_label(const moments_layout &lay, uint32_t rows, const uint8_t *
 int combine_groups(const moments_layout &lay, uint32_t cols, const cs_group_moments_params *params,
                    const uint8_t *d_feature_keep, const cs_group_moments_out *out, uint32_t g_lo, uint32_t g_hi,
                    cudaStream_t stream) {
-    dim3 grid((cols + 255u) / 256u == 0u ? 1u : (cols + 255u) / 256u, g_hi - g_lo);
-    moments_combine_kernel<<<grid, 256, 0, stream>>>(cols, params->group_count, params->scheme, params->ddof,
-                                                     lay.chunk_first, lay.group_rows, lay.partials, d_feature_keep,
-                                                     out->sum, out->sumsq, out->mean, out->var, out->mean64,
-                                                     out->var64, out->group_rows, g_lo);
+    // four columns a thread once that still fills the device (two CTAs of 256 per SM)
+    const uint32_t four = std::max(1u, (cols + 1023u) / 1024u), one = std::max(1u, (cols + 255u) / 256u);
+    auto launch = [&](auto kern, uint32_t tiles) {
+        kern<<<dim3(tiles, g_hi - g_lo), 256, 0, stream>>>(cols, lay.pstride, params->group_count, params->scheme,
+                                                           params->ddof, lay.chunk_first, lay.group_rows, lay.partials,
+                                                           d_feature_keep, out->sum, out->sumsq, out->mean, out->var,
+                                                           out->mean64, out->var64, out->group_rows, g_lo);
+    };
+    if ((uint64_t) four * (g_hi - g_lo) >= 296u) launch(moments_combine_kernel<4>, four);
+    else launch(moments_combine_kernel<1>, one);
     return launch_ok("moments_combine_kernel");
 }
 
@@ -700,7 +794,10 @@ static int moments_run(const cs_blocked_ell_view *src, const uint8_t *d_row_keep
         return 0;
     }
     moments_layout lay;
-    if (!make_layout(src, params, d_scratch, scratch_bytes, &lay) || d_scratch == nullptr) {
+    // scratch without room for the padding (the static array's limit counts none) is taken too
+    if ((!make_layout(src, params, d_scratch, scratch_bytes, &lay) &&
+         !make_layout(src, params, d_scratch, scratch_bytes, &lay, false)) ||
+        d_scratch == nullptr) {
         set_error("group_moments: scratch too small (%zu bytes, need %zu)", scratch_bytes, lay.bytes);
         return 0;
     }
@@ -804,12 +901,12 @@ std::size_t column_block_index_bytes(const cs_blocked_ell_view *src) {
     return (row_blocks * words + 1u) * sizeof(uint2);
 }
 
-// Scratch bytes the moments reduction needs for (src, params); 0 when the
+// Scratch bytes the moments reduction needs at least for (src, params); 0 when the
 // arguments are invalid (the error message is set).
 std::size_t group_moments_scratch_needed(const cs_blocked_ell_view *src, const cs_group_moments_params *params) {
     if (!validate(src, params)) return 0;
     moments_layout lay;
-    make_layout(src, params, nullptr, 0, &lay);
+    make_layout(src, params, nullptr, 0, &lay, false);
     return lay.bytes;
 }
 
