@@ -673,7 +673,7 @@ def coo_lines(lib, timed, emit, csr, no_cpu=False):
     ms_plan_u = timed(plan_fn)
     ms_emit_u = timed(emit_fn)
     ex = {"plan_ms": ms_plan_u, "emit_ms": ms_emit_u, "rows_per_s": R / ((ms_plan_u + ms_emit_u) * 1e-3),
-          "note": "entries shuffled: stable radix sort by row + gather, then the CSR route; time only"}
+          "note": "entries shuffled: two counting-sort passes by row, then the CSR route; time only"}
     if cpu_u is not None:
         ex["cpu_baseline"] = cpu_u
     emit("coo_blocked_ell_unordered", ms_plan_u + ms_emit_u, 0, ex)

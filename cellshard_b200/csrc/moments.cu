@@ -86,7 +86,8 @@ bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *
     lay->col_blocks = (src->cols + B - 1u) / B;
     lay->words = (lay->col_blocks + 31u) / 32u;
     lay->tiles = (src->rows + kTileRows - 1u) / kTileRows;
-    lay->chunk_rows = p->chunk_rows == 0u ? default_chunk_rows(src->rows, lay->col_blocks, B, p->group_count) : p->chunk_rows;
+    lay->chunk_rows =
+        p->chunk_rows == 0u ? default_chunk_rows(src->rows, lay->col_blocks, B, p->group_count) : p->chunk_rows;
     const std::size_t G = p->group_count;
     lay->max_chunks = (uint32_t) ((src->rows + lay->chunk_rows - 1u) / lay->chunk_rows + G);
     lay->short_chunks = std::min<std::size_t>(lay->chunk_rows, G != 0u ? src->rows / G : 0u) <= 512u;
@@ -350,12 +351,12 @@ struct many_partition_rows {
 // of chunks of a dozen rows (3,000 x 20,000, 250 groups: 111 us, 52 with 16-byte
 // stores), nothing at 2,048 rows, where the registers in fours cost the row loop
 // 1.6 % (500,000 x 32,768, 64 groups: 3.99 and 4.06 ms).  Taken up to 512 rows;
-// both meet at about 1,200.
+// by these two figures the forms meet at about 1,200.
 template <int L, bool COMP, bool kVecStore, typename Rows>
 __global__ void __launch_bounds__(kAccThreads, 2) moments_accumulate_kernel(
     Rows rows_of, uint32_t block_size, uint32_t col_blocks, uint32_t cols, uint32_t pstride,
-    const chunk_desc *__restrict__ chunks, const uint32_t *__restrict__ num_chunks, float *__restrict__ partials, const uint32_t *__restrict__ chunk_first,
-    uint32_t g_lo, uint32_t g_hi) {
+    const chunk_desc *__restrict__ chunks, const uint32_t *__restrict__ num_chunks, float *__restrict__ partials,
+    const uint32_t *__restrict__ chunk_first, uint32_t g_lo, uint32_t g_hi) {
     using entry = typename Rows::entry;
     extern __shared__ __align__(16) unsigned char acc_smem[];
     entry *chunk_rows_smem = reinterpret_cast<entry *>(acc_smem);
@@ -636,8 +637,8 @@ int launch_accumulate_rows(const Rows &rows_of, uint32_t block_size, uint32_t co
         !cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
                  "moments smem attribute"))
         return 0;
-    kern<<<grid, kAccThreads, smem, stream>>>(rows_of, block_size, lay.col_blocks, cols, lay.pstride, lay.chunks, lay.num_chunks,
-                                              lay.partials, chunk_first, g_lo, g_hi);
+    kern<<<grid, kAccThreads, smem, stream>>>(rows_of, block_size, lay.col_blocks, cols, lay.pstride, lay.chunks,
+                                              lay.num_chunks, lay.partials, chunk_first, g_lo, g_hi);
     return launch_ok("moments_accumulate_kernel");
 }
 

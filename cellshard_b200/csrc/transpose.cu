@@ -170,16 +170,17 @@ __global__ void __launch_bounds__(kThreads) tr_scatter_kernel(const uint32_t *__
 // at once; at 32,768 columns that leaves hundreds of MB of partially written
 // sectors open, far beyond L2.  Here the column key is sorted in two stable
 // counting-sort passes whose open write frontier is small:
-//   pass 1  by bucket = column >> 8 (<= 1,024 buckets), tiles of 8,192
-//           consecutive entries; entries become packed words (row >> 5,
+//   pass 1  by bucket = column >> 8 (<= 1,024 buckets), tiles of 4,096 (COO:
+//           8,192) consecutive entries; entries become packed words (row >> 5,
 //           column & 255, row & 31) + values: the upper bits are the place of
 //           the entry's bit in pass 2's bitmap.
 //   pass 2  inside each bucket by column & 255, in chunks of <= 8,192 that
 //           never cross a bucket, writing straight into the CSC.
 // Each tile or chunk is reordered whole in shared memory and leaves as one
 // run per digit, so global writes are long runs, not scattered entries.
-// Both passes rank entries in input order (warp match on the digit plus
-// per-warp running counts), so the result is the stable transpose.
+// Both passes rank entries in input order (runs of a row's entries in one
+// bucket; a bitmap of each column's rows, or ballots), so the result is the
+// stable transpose.
 // Needs cDim < 2^24 and uDim <= 262,144.
 //
 // The same two passes also put COO entries in row order (partition_rows_*
@@ -352,7 +353,9 @@ __device__ __forceinline__ uint2 tp_slice_rows(const uint2 *__restrict__ range, 
     return make_uint2(blockIdx.x * len, min(rows, (blockIdx.x + 1u) * len));
 }
 
-__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
+__global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
+                                                            uint32_t rows, uint32_t len,
+                                                            const uint2 *__restrict__ range,
                                                             uint32_t *__restrict__ slices) {
     const uint2 r = tp_slice_rows(range, rows, len);
     for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
@@ -399,7 +402,9 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restric
 }
 
 // start[segment * D + d]: global slot of the digit's first entry
-__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D, uint32_t rows, uint32_t len, const uint2 *__restrict__ range,
+__global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
+                                                             uint32_t rows, uint32_t len,
+                                                             const uint2 *__restrict__ range,
                                                              const uint32_t *__restrict__ segment,
                                                              const uint32_t *__restrict__ slices,
                                                              const uint32_t *__restrict__ start, uint32_t limit,
@@ -1308,8 +1313,9 @@ int tp_smem(K kernel, std::size_t smem, const char *what) {
     return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem), what);
 }
 
-// Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).  rows: the payloads of a bucket never decrease (the transpose); any:
-// entries of one key in any order (COO).
+// Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).  rows: the
+// payloads of a bucket never decrease (the transpose); any: entries of one key
+// in any order (COO); ballots: in their own order.
 template <int LB, tp_rank kRank>
 int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32_t *out_idx, uint16_t *out_val,
                    cudaStream_t stream) {
@@ -1361,7 +1367,8 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
     if (!launch_ok("tp_slice_scan_kernel")) return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
     if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr, l.one.slices,
+    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr,
+                                                         l.one.slices,
                                                          l.start1, l.K, l.one.base);
     if (!launch_ok("tp_slice_apply_kernel")) return 0;
     if (csr) {
@@ -1457,10 +1464,10 @@ int transpose_launch(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t 
 }
 
 // COO entries by rows: row pointers, columns (through `map` when given) and
-// values, a row's entries in any order or, `stable`, in their own.  Every row is below `rows` and every
-// mapped column below `cols`.  Two passes move 22 bytes an entry in runs; the
-// two stable 32-bit sorts and the random gathers that this replaces moved over
-// 100, most of them one sector per entry.
+// values, a row's entries in any order or, `stable`, in their own.  Every row
+// is below `rows` and every mapped column below `cols`.  Two passes move 22 bytes
+// an entry in runs; the two stable 32-bit sorts and the random gathers that this
+// replaces moved over 100, most of them one sector per entry.
 std::size_t partition_rows_scratch_bytes(uint32_t n, uint32_t rows, uint32_t cols) {
     const uint32_t lb = partition_low_bits(rows, cols);
     if (n == 0u || rows == 0u || lb == 0u) return 0u;
