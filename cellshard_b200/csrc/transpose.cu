@@ -211,8 +211,18 @@ constexpr uint32_t tp_slice_len(uint32_t rows) { return rows <= 8192u ? 16u : 64
 // segment (all tiles), pass 2 one per bucket (its chunks).
 struct tp_counts {
     uint16_t *cnt;      // [rows][D]
-    uint32_t *base;     // [rows][D] global slot of the row's first entry of the digit
+    uint32_t *base;     // [rows][D] global slot of the row's first entry of the digit, less its start
     uint32_t *slices;   // [slices][D] sums, then exclusive prefixes inside the segment
+    const uint32_t *start;   // [segments * D, `limit` of them] first slot of the digit; null where base has it
+    const uint32_t *segment; // [rows] (null: one segment)
+    uint32_t limit;
+    // global slot of the row's first entry of digit d (kAdd: start is given)
+    template <bool kAdd>
+    __device__ __forceinline__ uint32_t first(uint32_t row, uint32_t D, uint32_t d) const {
+        if constexpr (!kAdd) return base[(std::size_t) row * D + d];
+        const std::size_t c = (segment != nullptr ? (std::size_t) segment[row] * D : 0u) + d;
+        return base[(std::size_t) row * D + d] + (c < limit ? start[c] : 0u);
+    }
 };
 
 struct tp2_layout {
@@ -269,6 +279,11 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     l->slice_bucket = c.take<uint32_t>(l->max_slices);
     l->slice_range = c.take<uint2>(l->max_slices);
     l->slice_first = c.take<uint32_t>((std::size_t) l->K + 1u);
+    l->one.start = l->two.start = nullptr; // see tp_offsets
+    l->one.segment = nullptr;
+    l->one.limit = l->K;
+    l->two.segment = l->chunk_bucket;
+    l->two.limit = uDim;
     l->scan_bytes = scan_u32_scratch_bytes(uDim);
     l->scan_tmp = c.take<char>(l->scan_bytes);
     l->bytes = c.used;
@@ -421,6 +436,54 @@ __global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__r
     }
 }
 
+// The three at once for few rows: a segment and 32 digits per CTA as in
+// tp_slice_scan_kernel, over the rows themselves.  A digit's 32 threads walk
+// rows / 32 each, twice, and the scatter adds the digits' starts (two dependent
+// loads in every CTA): four launches fewer, for up to 1,024 tiles or chunks.  us
+// a call by three kernels / this: transposes of 43 tiles 126 / 110, of 240
+// 121 / 99, of 733 154 / 135, of 2,929 260 / 256, of 8,789 573 / 606, of 24,000
+// 1,329 / 1,467.  A scatter that asks at run time whether to add costs the large
+// COO partitions 2 %, so it is compiled both ways.
+constexpr uint32_t kTpDirectRows = 1024;
+__global__ void __launch_bounds__(1024) tp_rows_scan_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
+                                                            uint32_t rows, const uint32_t *__restrict__ seg_first,
+                                                            const uint2 *__restrict__ range, uint32_t limit,
+                                                            uint32_t *__restrict__ base,
+                                                            uint32_t *__restrict__ totals) {
+    __shared__ uint32_t part[32][33];
+    const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, d = blockIdx.y * 32u + x;
+    uint32_t r0 = 0u, r1 = rows;
+    if (seg_first != nullptr) {
+        const uint32_t s0 = seg_first[blockIdx.x], s1 = seg_first[blockIdx.x + 1u];
+        r0 = s0 < s1 ? range[s0].x : 0u;
+        r1 = s0 < s1 ? range[s1 - 1u].y : 0u;
+    }
+    const uint32_t per = (r1 - r0 + 31u) / 32u;
+    const uint32_t a = min(r1, r0 + y * per), e = min(r1, a + per);
+    uint32_t sum = 0u;
+    if (d < D) {
+#pragma unroll 8
+        for (uint32_t i = a; i < e; ++i) sum += __ldg(cnt + (std::size_t) i * D + d);
+    }
+    part[y][x] = sum;
+    __syncthreads();
+    {
+        const uint32_t v = part[x][y], incl = warp_inclusive_scan(v);
+        part[x][y] = incl - v;
+        const std::size_t c = (std::size_t) blockIdx.x * D + blockIdx.y * 32u + y;
+        if (x == 31u && blockIdx.y * 32u + y < D && c < limit) totals[c] = incl;
+    }
+    __syncthreads();
+    if (d < D) {
+        uint32_t run = part[y][x];
+#pragma unroll 8
+        for (uint32_t i = a; i < e; ++i) {
+            base[(std::size_t) i * D + d] = run;
+            run += __ldg(cnt + (std::size_t) i * D + d);
+        }
+    }
+}
+
 // Block-wide exclusive scan of n <= Q * blockDim.x values in place (each
 // thread scans up to Q consecutive entries); out[n] receives the total.
 template <int Q>
@@ -549,6 +612,7 @@ struct tp_tile_smem {
     uint32_t scan33[33], scan33b[33];
 };
 
+template <bool kAdd>
 __global__ void __launch_bounds__(kTpThreads1, 4)
     tp_scatter1_csr_kernel(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx,
                            const uint16_t *__restrict__ val, uint32_t cDim, uint32_t uDim, uint32_t nnz, uint32_t K,
@@ -583,7 +647,7 @@ __global__ void __launch_bounds__(kTpThreads1, 4)
         }
     }
     for (uint32_t k = t; k < K; k += kTpThreads1) {
-        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        run[k] = one.first<kAdd>(blockIdx.x, K, k);
         lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
     }
     for (uint32_t k = t; k < kTpWarps1 * K2; k += kTpThreads1) sm.cnt[k] = 0u;
@@ -727,6 +791,7 @@ std::size_t tp_scatter1_csr_smem(uint32_t K) { return sizeof(tp_tile_smem) + ((s
 constexpr unsigned kTpThreadsCoo = 512;
 constexpr unsigned kTpPerCoo = kTpTileCoo / kTpThreadsCoo;
 
+template <bool kAdd>
 __global__ void __launch_bounds__(kTpThreadsCoo, 2)
     tp_scatter1_coo_kernel(const uint32_t *__restrict__ key, const uint16_t *__restrict__ val,
                            const uint32_t *__restrict__ pay, const uint32_t *__restrict__ pay_map, uint32_t uDim,
@@ -750,7 +815,7 @@ __global__ void __launch_bounds__(kTpThreadsCoo, 2)
         vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
     }
     for (uint32_t k = t; k < K; k += kTpThreadsCoo) {
-        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        run[k] = one.first<kAdd>(blockIdx.x, K, k);
         at[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
     }
     if (pay_map != nullptr)
@@ -788,6 +853,7 @@ std::size_t tp_scatter1_coo_smem(uint32_t K) {
 
 // The same in the order of the entries (stable): a tile's entries are ranked in
 // 32-entry batches by ballots, one per bucket bit.
+template <bool kAdd>
 __global__ void __launch_bounds__(kTpThreads) tp_scatter1_coo_stable_kernel(
     const uint32_t *__restrict__ idx, const uint16_t *__restrict__ val, const uint32_t *__restrict__ pay,
     const uint32_t *__restrict__ pay_map, uint32_t uDim, uint32_t nnz, uint32_t low_bits, uint32_t K,
@@ -805,7 +871,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter1_coo_stable_kernel(
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t a = blockIdx.x * kTpTileCoo, e = min(nnz - a, kTpTileCoo) + a;
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
-        run[k] = one.base[(std::size_t) blockIdx.x * K + k];
+        run[k] = one.first<kAdd>(blockIdx.x, K, k);
         sg.lb[k] = one.cnt[(std::size_t) blockIdx.x * K + k];
         sg.fill[k] = 0u;
     }
@@ -1053,7 +1119,7 @@ __device__ void tp_rank_ballots(const uint32_t *__restrict__ tmp_key, const uint
 // Pass 2 by ballots: a chunk of one bucket reordered by the low digit in shared
 // memory (stable), then written out as one run per key.  Sparse transposes, and
 // COO entries whose order counts.
-template <int LB>
+template <int LB, bool kAdd>
 __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t *__restrict__ tmp_key,
                                                                 const uint16_t *__restrict__ tmp_val,
                                                                 const uint2 *__restrict__ chunk_range,
@@ -1076,7 +1142,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
     if (b >= e) return;
     for (uint32_t d = threadIdx.x; d < D; d += kTpThreads) {
         lb[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
-        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
+        gbase[d] = two.first<kAdd>(blockIdx.x, D, d);
         fill[d] = 0u;
 #pragma unroll
         for (unsigned w = 0; w < kTpWarps; ++w) sg.cnt[w * D + d] = 0u;
@@ -1098,7 +1164,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_scatter2_kernel(const uint32_t 
 
 // Pass 2 of COO entries, in any order inside a row: as tp_scatter1_coo_kernel,
 // by shared atomics on the row's next staging slot.
-template <int LB>
+template <int LB, bool kAdd>
 __global__ void __launch_bounds__(kTpThreadsCoo, 2)
     tp_scatter2_coo_kernel(const uint32_t *__restrict__ tmp_key, const uint16_t *__restrict__ tmp_val,
                            const uint2 *__restrict__ chunk_range, const tp_counts two, uint32_t *__restrict__ out_idx,
@@ -1125,7 +1191,7 @@ __global__ void __launch_bounds__(kTpThreadsCoo, 2)
     }
     for (uint32_t d = t; d < D; d += kTpThreadsCoo) {
         at[d] = two.cnt[(std::size_t) blockIdx.x * D + d];
-        gbase[d] = two.base[(std::size_t) blockIdx.x * D + d];
+        gbase[d] = two.first<kAdd>(blockIdx.x, D, d);
     }
     __syncthreads();
     block_scan_small<(D + kTpThreadsCoo - 1u) / kTpThreadsCoo>(at, D, scan33);
@@ -1186,6 +1252,7 @@ struct tp_rows_smem {
 static_assert(sizeof(uint32_t) * kTpSpanWords * 256u >= 2u * kTpWarps2 * 256u * sizeof(uint16_t),
               "the ballot counters fit the bitmap's place");
 
+template <bool kAdd>
 __global__ void __launch_bounds__(kTpThreads2, 2)
     tp_scatter2_rows_kernel(const uint32_t *__restrict__ tmp_key, const uint16_t *__restrict__ tmp_val,
                             const uint2 *__restrict__ chunk_range, const tp_counts two,
@@ -1220,7 +1287,7 @@ __global__ void __launch_bounds__(kTpThreads2, 2)
     }
     if (t < 256u) {
         sm.lb[t] = two.cnt[(std::size_t) blockIdx.x * 256u + t];
-        sm.gbase[t] = two.base[(std::size_t) blockIdx.x * 256u + t];
+        sm.gbase[t] = two.first<kAdd>(blockIdx.x, 256u, t);
     }
     if (t == 0u) sm.dup = 0u;
     const uint32_t w_first = __ldg(tmp_key + b) >> (LB + 5), w_last = __ldg(tmp_key + e - 1u) >> (LB + 5);
@@ -1313,6 +1380,33 @@ int tp_smem(K kernel, std::size_t smem, const char *what) {
     return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem), what);
 }
 
+// The totals of `t`'s digits, and its offsets: complete but for the digits'
+// starts, which the scatter then adds (t->start), where no segment has more than
+// kTpDirectRows rows; else tp_offsets_apply adds them once they are scanned.
+// rows [0, rows) in slices of len, or the segments' slices `range`.
+int tp_offsets(tp_counts *t, uint32_t D, uint32_t rows, uint32_t most_rows, uint32_t len, uint32_t slices,
+               uint32_t segments, const uint32_t *seg_first, const uint2 *range, uint32_t limit, uint32_t *totals,
+               const uint32_t *start, cudaStream_t stream) {
+    const dim3 grid(segments, (D + 31u) / 32u);
+    if (most_rows <= kTpDirectRows) {
+        t->start = start;
+        tp_rows_scan_kernel<<<grid, 1024, 0, stream>>>(t->cnt, D, rows, seg_first, range, limit, t->base, totals);
+        return launch_ok("tp_rows_scan_kernel");
+    }
+    tp_slice_sums_kernel<<<slices, 256, 0, stream>>>(t->cnt, D, rows, len, range, t->slices);
+    if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    tp_slice_scan_kernel<<<grid, 1024, 0, stream>>>(t->slices, D, seg_first, slices, limit, totals);
+    return launch_ok("tp_slice_scan_kernel");
+}
+
+int tp_offsets_apply(const tp_counts &t, uint32_t D, uint32_t rows, uint32_t len, uint32_t slices, const uint2 *range,
+                     const uint32_t *segment, uint32_t limit, const uint32_t *start, cudaStream_t stream) {
+    if (t.start != nullptr) return 1;
+    tp_slice_apply_kernel<<<slices, 256, 0, stream>>>(t.cnt, D, rows, len, range, segment, t.slices, start, limit,
+                                                      t.base);
+    return launch_ok("tp_slice_apply_kernel");
+}
+
 // Counts and pass 2 of `l`'s pass-1 result (low digit of LB bits).  rows: the
 // payloads of a bucket never decrease (the transpose); any: entries of one key
 // in any order (COO); ballots: in their own order.
@@ -1323,30 +1417,27 @@ int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32
     tp_hist2_kernel<LB><<<l.max_chunks, kTpThreads, 0, stream>>>(l.tmp_key, l.chunk_range, l.two.cnt);
     if (!launch_ok("tp_hist2_kernel")) return 0;
     constexpr uint32_t D = 1u << LB;
-    tp_slice_sums_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, 0u, l.slice_range, l.two.slices);
-    if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(l.K, D / 32u), 1024, 0, stream>>>(l.two.slices, D, l.slice_first, 0u, uDim, out_ptr);
-    if (!launch_ok("tp_slice_scan_kernel")) return 0;
-    if (!scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream)) return 0;
-    tp_slice_apply_kernel<<<l.max_slices, 256, 0, stream>>>(l.two.cnt, D, 0u, 0u, l.slice_range, l.slice_bucket,
-                                                            l.two.slices, out_ptr, uDim, l.two.base);
-    if (!launch_ok("tp_slice_apply_kernel")) return 0;
-    if constexpr (kRank == tp_rank::rows) {
-        if (!tp_smem(tp_scatter2_rows_kernel, sizeof(tp_rows_smem), "scatter2 smem attribute")) return 0;
-        tp_scatter2_rows_kernel<<<l.max_chunks, kTpThreads2, sizeof(tp_rows_smem), stream>>>(
-            l.tmp_key, l.tmp_val, l.chunk_range, l.two, out_idx, out_val);
-    } else if constexpr (kRank == tp_rank::any) {
-        constexpr std::size_t smem = tp_scatter2_coo_smem(LB);
-        if (!tp_smem(tp_scatter2_coo_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
-        tp_scatter2_coo_kernel<LB><<<l.max_chunks, kTpThreadsCoo, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range,
-                                                                                  l.two, out_idx, out_val);
-    } else {
-        constexpr std::size_t smem = tp_scatter2_smem(LB);
-        if (!tp_smem(tp_scatter2_kernel<LB>, smem, "scatter2 smem attribute")) return 0;
-        tp_scatter2_kernel<LB><<<l.max_chunks, kTpThreads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range, l.two,
-                                                                           out_idx, out_val);
-    }
-    return launch_ok("tp_scatter2_kernel");
+    tp_counts two = l.two;
+    if (!tp_offsets(&two, D, 0u, l.max_chunks, 0u, l.max_slices, l.K, l.slice_first, l.slice_range, uDim, out_ptr,
+                    out_ptr, stream) ||
+        !scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream) ||
+        !tp_offsets_apply(two, D, 0u, 0u, l.max_slices, l.slice_range, l.slice_bucket, uDim, out_ptr, stream))
+        return 0;
+    const bool add = two.start != nullptr;
+    auto launch = [&](auto kern, unsigned threads, std::size_t smem) {
+        if (!tp_smem(kern, smem, "scatter2 smem attribute")) return 0;
+        kern<<<l.max_chunks, threads, smem, stream>>>(l.tmp_key, l.tmp_val, l.chunk_range, two, out_idx, out_val);
+        return launch_ok("tp_scatter2_kernel");
+    };
+    if constexpr (kRank == tp_rank::rows)
+        return launch(add ? tp_scatter2_rows_kernel<true> : tp_scatter2_rows_kernel<false>, kTpThreads2,
+                      sizeof(tp_rows_smem));
+    else if constexpr (kRank == tp_rank::any)
+        return launch(add ? tp_scatter2_coo_kernel<LB, true> : tp_scatter2_coo_kernel<LB, false>, kTpThreadsCoo,
+                      tp_scatter2_coo_smem(LB));
+    else
+        return launch(add ? tp_scatter2_kernel<LB, true> : tp_scatter2_kernel<LB, false>, kTpThreads,
+                      tp_scatter2_smem(LB));
 }
 
 // Pass 1: `ptr` is null for COO (payloads `pay` through `pay_map`; `stable`
@@ -1360,33 +1451,30 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
     hist1<<<l.tiles1, kTpThreads, (std::size_t) l.K * 4u, stream>>>(key, nnz, uDim, l.low_bits, l.K, l.one.cnt,
                                                                     l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
-    tp_slice_sums_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, l.one.slices);
-    if (!launch_ok("tp_slice_sums_kernel")) return 0;
-    tp_slice_scan_kernel<<<dim3(1u, (l.K + 31u) / 32u), 1024, 0, stream>>>(l.one.slices, l.K, nullptr, l.slices1, l.K,
-                                                                          l.total1);
-    if (!launch_ok("tp_slice_scan_kernel")) return 0;
+    tp_counts one = l.one;
+    if (!tp_offsets(&one, l.K, l.tiles1, l.tiles1, l.slice1, l.slices1, 1u, nullptr, nullptr, l.K, l.total1, l.start1,
+                    stream))
+        return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
-    if (!launch_ok("tp_chunks_kernel")) return 0;
-    tp_slice_apply_kernel<<<l.slices1, 256, 0, stream>>>(l.one.cnt, l.K, l.tiles1, l.slice1, nullptr, nullptr,
-                                                         l.one.slices,
-                                                         l.start1, l.K, l.one.base);
-    if (!launch_ok("tp_slice_apply_kernel")) return 0;
+    if (!launch_ok("tp_chunks_kernel") ||
+        !tp_offsets_apply(one, l.K, l.tiles1, l.slice1, l.slices1, nullptr, nullptr, l.K, l.start1, stream))
+        return 0;
+    const bool add = one.start != nullptr;
     if (csr) {
+        auto kern = add ? tp_scatter1_csr_kernel<true> : tp_scatter1_csr_kernel<false>;
         const std::size_t smem = tp_scatter1_csr_smem(l.K);
-        if (!tp_smem(tp_scatter1_csr_kernel, smem, "scatter1 smem attribute")) return 0;
-        tp_scatter1_csr_kernel<<<l.tiles1, kTpThreads1, smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.K, l.one,
-                                                                        l.gran_row, l.tmp_key, l.tmp_val);
-    } else if (stable) {
-        const std::size_t smem = tp_scatter1_smem(l.K);
-        if (!tp_smem(tp_scatter1_coo_stable_kernel, smem, "scatter1 smem attribute")) return 0;
-        tp_scatter1_coo_stable_kernel<<<l.tiles1, kTpThreads, smem, stream>>>(key, val, pay, pay_map, uDim, nnz,
-                                                                              l.low_bits, l.K, l.one, l.tmp_key,
-                                                                              l.tmp_val);
+        if (!tp_smem(kern, smem, "scatter1 smem attribute")) return 0;
+        kern<<<l.tiles1, kTpThreads1, smem, stream>>>(ptr, key, val, cDim, uDim, nnz, l.K, one, l.gran_row, l.tmp_key,
+                                                      l.tmp_val);
     } else {
-        const std::size_t smem = tp_scatter1_coo_smem(l.K);
-        if (!tp_smem(tp_scatter1_coo_kernel, smem, "scatter1 smem attribute")) return 0;
-        tp_scatter1_coo_kernel<<<l.tiles1, kTpThreadsCoo, smem, stream>>>(key, val, pay, pay_map, uDim, nnz, l.low_bits,
-                                                                          l.K, l.one, l.tmp_key, l.tmp_val);
+        auto any = add ? tp_scatter1_coo_kernel<true> : tp_scatter1_coo_kernel<false>;
+        auto in_order = add ? tp_scatter1_coo_stable_kernel<true> : tp_scatter1_coo_stable_kernel<false>;
+        auto kern = stable ? in_order : any;
+        const std::size_t smem = stable ? tp_scatter1_smem(l.K) : tp_scatter1_coo_smem(l.K);
+        if (!tp_smem(kern, smem, "scatter1 smem attribute")) return 0;
+        kern<<<l.tiles1, stable ? kTpThreads : kTpThreadsCoo, smem, stream>>>(key, val, pay, pay_map, uDim, nnz,
+                                                                              l.low_bits, l.K, one, l.tmp_key,
+                                                                              l.tmp_val);
     }
     return launch_ok("tp_scatter1_kernel");
 }

@@ -118,3 +118,9 @@ def test_short_rows_in_runs(cuda, orc, rows, cols, longest, block):
 ])
 def test_shuffled_coo_repeats_in_the_shape_pass(cuda, orc, rows, cols, n, block, repeat):
     test_shuffled_coo(cuda, orc, rows, cols, n, block, 0, repeat, False)
+
+
+@pytest.mark.parametrize("n,repeat", [(8_390_000, 0), (8_800_000, 2)])
+def test_shuffled_coo_of_many_tiles(cuda, orc, n, repeat):
+    """Around 1,024 tiles of 8,192 entries: offsets by one kernel or in slices."""
+    test_shuffled_coo(cuda, orc, 700, 100_000, n, 16, 0, repeat, False)

@@ -70,3 +70,24 @@ def test_gap_of_empty_rows_inside_a_tile(cuda, orc, gap):
     rptr, ridx, rval = orc.csr_transpose(gap + 7, cols, ptr, idx, val)
     assert np.array_equal(np_u32(t.ptr), rptr) and np.array_equal(np_u32(t.idx), ridx)
     assert np.array_equal(np_u16(t.val), rval)
+
+
+@pytest.mark.parametrize("n", [1_024 * 4_096, 1_024 * 4_096 + 1, 1_027 * 4_096 + 77])
+def test_tiles_around_the_direct_offset_scan(cuda, n):
+    """The most tiles whose offsets come from one kernel, and more."""
+    from cellshard_b200.device import transpose
+
+    rng = np.random.default_rng(n)
+    rows, cols, per = 9_000, 1_500, n // 9_000
+    count = np.full(rows, per)
+    count[:n - per * rows] += 1
+    ptr = np.concatenate([[0], np.cumsum(count)]).astype(np.uint32)
+    first = rng.integers(0, cols, rows)
+    within = np.arange(n) - np.repeat(ptr[:-1].astype(np.int64), count)
+    idx = ((np.repeat(first, count) + within) % cols).astype(np.uint32)  # distinct in a row, in any order
+    val = (np.arange(n) * 7 % 60_000).astype(np.uint16)
+    t = transpose(to_device_csr(rows, cols, ptr, idx, val))
+    order = np.argsort(idx, kind="stable")
+    row = np.repeat(np.arange(rows, dtype=np.uint32), count)
+    assert np.array_equal(np_u32(t.ptr), np.concatenate([[0], np.cumsum(np.bincount(idx, minlength=cols))]))
+    assert np.array_equal(np_u32(t.idx), row[order]) and np.array_equal(np_u16(t.val), val[order])
