@@ -874,7 +874,7 @@ static std::size_t any_order_smem(uint32_t cols, uint32_t B) {
 }
 
 bool blocked_ell_any_order_fits(uint32_t cols, uint32_t B) {
-    return B != 0u && any_order_smem(cols, B) <= 200u * 1024u;
+    return B != 0u && any_order_smem(cols, B) <= 200u * 1024u && col_words(cols, B) <= kMaxShapeWords;
 }
 
 int blocked_ell_shape_any_order(const cs_compressed_view *src, uint32_t B, uint64_t *d_shape, uint32_t *bitmaps,

@@ -124,3 +124,18 @@ def test_shuffled_coo_repeats_in_the_shape_pass(cuda, orc, rows, cols, n, block,
 def test_shuffled_coo_of_many_tiles(cuda, orc, n, repeat):
     """Around 1,024 tiles of 8,192 entries: offsets by one kernel or in slices."""
     test_shuffled_coo(cuda, orc, 700, 100_000, n, 16, 0, repeat, False)
+
+
+def test_shuffled_coo_past_the_column_blocks_is_refused(cuda):
+    """131,072 column blocks at most, in any order of the entries."""
+    import torch
+
+    from cellshard_b200 import _abi
+    from cellshard_b200.device import blocked_ell_from_coo
+
+    row, col, val = _entries(40, 140_000, 30_000, 5)
+    for order in (np.arange(len(row)), np.argsort(row, kind="stable")):
+        dev = [torch.from_numpy(a[order].view(t).copy()).cuda()
+               for a, t in ((row, np.int32), (col, np.int32), (val, np.float16))]
+        with pytest.raises(_abi.CellShardError, match="column-block limit"):
+            blocked_ell_from_coo(40, 140_000, *dev, 1, 140_000)
