@@ -107,6 +107,21 @@ bool make_layout(const cs_blocked_ell_view *src, const cs_group_moments_params *
     return c.fits();
 }
 
+// A smaller matrix may ask for more scratch than a larger one (shorter chunks),
+// so scratch that was sized for the larger one, or for unpadded partials as the
+// static array's limit counts them, takes longer chunks, at last of 2,048 rows
+// without the padding.
+template <typename Make>
+bool fit_scratch(const cs_group_moments_params *params, Make make) {
+    cs_group_moments_params p = *params;
+    if (make(p, true)) return true;
+    if (params->chunk_rows == 0u)
+        for (p.chunk_rows = 128u; p.chunk_rows <= kDefaultChunkRows; p.chunk_rows *= 2u)
+            if (make(p, true)) return true;
+    p.chunk_rows = params->chunk_rows == 0u ? kDefaultChunkRows : params->chunk_rows;
+    return make(p, false);
+}
+
 // ---------------------------------------------------------------------------
 // 1. Column-block index per row block.
 // ---------------------------------------------------------------------------
@@ -816,9 +831,9 @@ static int moments_run(const cs_blocked_ell_view *src, const uint8_t *d_row_keep
         return 0;
     }
     moments_layout lay;
-    // scratch without room for the padding (the static array's limit counts none) is taken too
-    if ((!make_layout(src, params, d_scratch, scratch_bytes, &lay) &&
-         !make_layout(src, params, d_scratch, scratch_bytes, &lay, false)) ||
+    if (!fit_scratch(params, [&](const cs_group_moments_params &p, bool padded) {
+            return make_layout(src, &p, d_scratch, scratch_bytes, &lay, padded);
+        }) ||
         d_scratch == nullptr) {
         set_error("group_moments: scratch too small (%zu bytes, need %zu)", scratch_bytes, lay.bytes);
         return 0;
@@ -1032,8 +1047,9 @@ int validate_parts(const cs_blocked_ell_view *parts, uint32_t count, const cs_gr
 }
 
 bool make_parts_layout(const cs_blocked_ell_view *parts, uint32_t count, const cs_blocked_ell_view &whole,
-                       const cs_group_moments_params *params, void *base, std::size_t cap, parts_layout *pl) {
-    make_layout(&whole, params, base, cap, &pl->base);
+                       const cs_group_moments_params *params, void *base, std::size_t cap, parts_layout *pl,
+                       bool padded = true) {
+    make_layout(&whole, params, base, cap, &pl->base, padded);
     const uint32_t B = whole.block_size;
     std::size_t blocks = 0;
     for (uint32_t k = 0; k < count; ++k) blocks += (parts[k].rows + B - 1u) / B;
@@ -1075,7 +1091,10 @@ extern "C" int cs_b200_group_moments_blocked_ell_parts(const cs_blocked_ell_view
         return 0;
     }
     parts_layout pl;
-    if (!make_parts_layout(parts, count, whole, params, d_scratch, scratch_bytes, &pl) || d_scratch == nullptr) {
+    if (!fit_scratch(params, [&](const cs_group_moments_params &p, bool padded) {
+            return make_parts_layout(parts, count, whole, &p, d_scratch, scratch_bytes, &pl, padded);
+        }) ||
+        d_scratch == nullptr) {
         set_error("group_moments_parts: scratch too small (%zu bytes, need %zu)", scratch_bytes, pl.bytes);
         return 0;
     }

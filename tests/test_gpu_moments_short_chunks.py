@@ -61,3 +61,48 @@ def test_short_chunks(cuda, rows, cols, block, groups):
         tol = 2.0 ** -52 * np.abs(s * mean) / np.maximum(n - 1.0, 1.0) + 2.0 ** -51 * var
         assert np.all(np.abs(got["var64"] - var) <= tol)
         assert np.array_equal(got["mean"], mean.astype(np.float32))
+
+
+@pytest.mark.parametrize("rows,cols", [(8_000, 900), (8_000, 901), (3_000, 2_003)])
+def test_scratch_sized_for_longer_chunks(cuda, rows, cols):
+    """Scratch for chunks of 512 or 2,048 rows, padded or not, does where the
+    default is 64: the sums are those of the full scratch."""
+    import torch
+
+    from cellshard_b200 import _abi
+    from cellshard_b200.device import blocked_ell_from_csr, ptr as dptr, stream_handle
+
+    lib = _abi.load()
+    p, idx, val = random_csr(rows, cols, 0.03, rows + cols, 0.1)
+    bell = blocked_ell_from_csr(to_device_csr(rows, cols, p, idx, val), 16)
+    labels = torch.arange(rows, dtype=torch.int32, device="cuda") % 3
+    v = bell.view()
+    parts = (_abi.BlockedEllView * 1)(v)
+
+    def need(chunk, many):
+        prm, n = _abi.GroupMomentsParams(3, 2, 1, chunk), C.c_size_t()
+        call = (lambda: lib.cs_b200_group_moments_parts_scratch_bytes(parts, 1, C.byref(prm), C.byref(n))) if many \
+            else (lambda: lib.cs_b200_group_moments_scratch_bytes(C.byref(v), C.byref(prm), C.byref(n)))
+        _abi.check(call(), "scratch")
+        return n.value
+
+    results = []
+    for many in (False, True):
+        assert need(0, many) > need(512, many) > need(2048, many)
+        short = need(2048, many) - (4 if cols % 8 and not many else 0)
+        for room in (need(0, many), need(512, many), need(2048, many), short):
+            scratch = torch.full((room,), 0xff, dtype=torch.uint8, device="cuda")
+            out = [torch.full((3, cols), -1.0, device="cuda") for _ in range(2)]
+            status = torch.zeros(1, dtype=torch.int32, device="cuda")
+            o, prm = _abi.GroupMomentsOut(*[dptr(t) for t in out]), _abi.GroupMomentsParams(3, 2, 1, 0)
+            o.status = dptr(status)
+            if many:
+                ok = lib.cs_b200_group_moments_blocked_ell_parts(parts, 1, None, None, None, dptr(labels), C.byref(prm),
+                                                                 C.byref(o), dptr(scratch), room, stream_handle())
+            else:
+                ok = lib.cs_b200_group_moments_blocked_ell(C.byref(v), None, None, dptr(labels), C.byref(prm),
+                                                           C.byref(o), dptr(scratch), room, stream_handle())
+            _abi.check(ok, "moments")
+            results.append(torch.stack(out).cpu().numpy())
+    for r in results[1:]:
+        assert np.array_equal(r, results[0])  # whole counts: exact
