@@ -20,6 +20,7 @@
 // caller's scratch; the two-pass path keeps repeated entries, in row order.
 #include "common.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace csb {
@@ -204,7 +205,8 @@ constexpr uint32_t kTpGran = 256;    // entries per warp per step; rows are look
 
 // Tiles or chunks per slice of the offset scan: 64, or 16 where that leaves only
 // a few CTAs with a long chain each (365 tiles: 12 us by 64, 6 by 16).
-constexpr uint32_t tp_slice_len(uint32_t rows) { return rows <= 8192u ? 16u : 64u; }
+constexpr uint32_t kTpShortSlices = 8192;
+constexpr uint32_t tp_slice_len(uint32_t rows) { return rows <= kTpShortSlices ? 16u : 64u; }
 
 // Counts of a pass, one row per tile or chunk and one column per digit, and
 // what the scan over the rows of a segment makes of them: pass 1 has one
@@ -267,8 +269,10 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
         t->base = c.take<uint32_t>(rows * digits);
         t->slices = c.take<uint32_t>(slices * digits);
     };
-    counts(&l->one, l->tiles1, l->slices1, l->K);
-    counts(&l->two, l->max_chunks, l->max_slices, D);
+    // room for the short slices of fewer rows too: scratch for many entries does for fewer
+    counts(&l->one, l->tiles1, std::max(l->slices1, std::min(l->tiles1, kTpShortSlices) / 16u), l->K);
+    counts(&l->two, l->max_chunks, std::max(l->max_slices, std::min(l->max_chunks, kTpShortSlices) / 16u + l->K + 1u),
+           D);
     l->total1 = c.take<uint32_t>(l->K);
     l->start1 = c.take<uint32_t>((std::size_t) l->K + 1u);
     l->tmp_key = c.take<uint32_t>((std::size_t) nnz + 1u);
@@ -276,8 +280,8 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     l->gran_row = granules ? c.take<uint32_t>((std::size_t) nnz / kTpGran + 1u) : nullptr;
     l->chunk_bucket = c.take<uint32_t>(l->max_chunks);
     l->chunk_range = c.take<uint2>(l->max_chunks);
-    l->slice_bucket = c.take<uint32_t>(l->max_slices);
-    l->slice_range = c.take<uint2>(l->max_slices);
+    l->slice_bucket = c.take<uint32_t>(std::max(l->max_slices, kTpShortSlices / 16u + l->K + 1u));
+    l->slice_range = c.take<uint2>(std::max(l->max_slices, kTpShortSlices / 16u + l->K + 1u));
     l->slice_first = c.take<uint32_t>((std::size_t) l->K + 1u);
     l->one.start = l->two.start = nullptr; // see tp_offsets
     l->one.segment = nullptr;
