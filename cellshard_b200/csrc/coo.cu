@@ -382,6 +382,17 @@ coo_decode decoder(const cs_coo_view *src, const uint32_t *map, const coo_scratc
     return d;
 }
 
+// What the emit reads of the CSR route, written on the device before the plan's
+// last wait: width, route (a repeated cell takes the stable order), kept entries.
+__global__ void coo_csr_words_kernel(const unsigned long long *__restrict__ shape, uint32_t route, uint32_t n_valid,
+                                     uint32_t *__restrict__ words) {
+    if (threadIdx.x != 0u) return;
+    words[2] = (uint32_t) shape[0];
+    words[3] = shape[2] != 0u ? kRouteCsrSorted : route;
+    words[4] = 0u;
+    words[5] = n_valid;
+}
+
 // The CSR view of the CSR route (row pointers and mapped or row-sorted columns
 // in the scratch).
 cs_compressed_view csr_of(const cs_coo_view *src, const uint32_t *map, uint32_t cols, const coo_scratch &x,
@@ -474,19 +485,19 @@ int coo_plan(const cs_coo_view *src, const uint32_t *map, uint32_t cols, uint32_
                   ? blocked_ell_shape_any_order(&v, B, (uint64_t *) x.shape, (uint32_t *) x.csr_tmp, status,
                                                 (uint32_t *) (x.shape + 2), stream)
                   : cs_b200_blocked_ell_shape(&v, B, (uint64_t *) x.shape, x.csr_tmp, x.csr_bytes, status,
-                                              reinterpret_cast<cs_stream_t>(stream))) ||
+                                              reinterpret_cast<cs_stream_t>(stream))))
+            return 0;
+        coo_csr_words_kernel<<<1, 32, 0, stream>>>(x.shape, route, s->n_valid, x.words);
+        if (!launch_ok("coo_csr_words_kernel") ||
             !cuda_ok(cudaMemcpyAsync(shape, x.shape, 24, cudaMemcpyDeviceToHost, stream), "D2H shape") ||
             !cuda_ok(cudaStreamSynchronize(stream), "coo csr shape sync"))
             return 0;
-        if (shape[2] != 0u) { // a repeated (row, column): its last value is the one in the entries' order
-            if (!by_rows(true)) return 0;
-            route = kRouteCsrSorted;
-        }
         s->width = (uint32_t) shape[0];
         s->groups = shape[1];
-        // copied from pageable memory: taken before the call returns, so nothing waits
-        const uint32_t words[4] = {s->width, route, 0u, s->n_valid};
-        return cuda_ok(cudaMemcpyAsync(x.words + 2, words, 16, cudaMemcpyHostToDevice, stream), "coo words");
+        if (shape[2] == 0u) return 1;
+        // a repeated (row, column): its last value is the one in the entries' order.  The plan has
+        // finished when it returns, so that the emit may run on another stream
+        return by_rows(true) && cuda_ok(cudaStreamSynchronize(stream), "coo stable partition sync");
     }
     s->shift = bits_for(w[0] / B);
     s->single = bits_for(s->RB - 1u) + s->shift <= 31u;

@@ -243,10 +243,15 @@ typedef struct CS_ALIGN16 cs_coo_view {
 
 /* Shape of one block size: width and the count of (row block, block column)
  * pairs; the plan stays in the scratch for the emit of the same block size.
- * Entries whose rows never decrease, with every mapped column below cols,
- * take the CSR route (row pointers from the row runs, then the CSR ->
- * Blocked-ELL shape and emit); others are sorted by (row block, block
- * column).  Synchronises (two small reads of sizes). */
+ * Where every row is below src->rows and every mapped column below cols (and
+ * the column-block bitmaps stay small next to the entries), the CSR route:
+ * row pointers from the row runs of entries whose rows never decrease, others
+ * put by rows in two counting-sort passes (by two stable sorts past 2,097,152
+ * rows), then the CSR -> Blocked-ELL shape and emit.  Otherwise the entries are
+ * sorted by (row block, block column).  Synchronises (two small reads of
+ * sizes, and a wait where a repeated (row, column) makes it order the entries
+ * again): the plan is complete when the call returns, so the emit may run on
+ * another stream. */
 CS_API int cs_b200_coo_blocked_ell_scratch_bytes(uint32_t nnz, uint32_t rows, uint32_t cols, uint32_t block_size,
                                                  size_t *out_bytes);
 CS_API int cs_b200_coo_blocked_ell_plan(const cs_coo_view *src,
