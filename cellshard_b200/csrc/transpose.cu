@@ -1253,6 +1253,7 @@ struct tp_rows_smem {
     uint16_t val[kTpChunk];                // staged values
     uint32_t gbase[256], lb[257], fill[256], scan33[33], dup;
 };
+static_assert(0xffffffffu - kTpRounds * kTpSpanKeys >= kTpSpanKeys, "no entry is past every span of a chunk");
 static_assert(sizeof(uint32_t) * kTpSpanWords * 256u >= 2u * kTpWarps2 * 256u * sizeof(uint16_t),
               "the ballot counters fit the bitmap's place");
 
@@ -1281,10 +1282,14 @@ __global__ void __launch_bounds__(kTpThreads2, 2)
         for (unsigned q = 0; q < kTpPerThread; q += 2u)
             vv[q / 2u] = (uint32_t) __ldcs(vp + q * kTpThreads2) | (uint32_t) __ldcs(vp + (q + 1u) * kTpThreads2) << 16;
     } else {
+        // no entry: the word before the first span.  A round's k0 lies at most kTpRounds spans
+        // behind it, so the difference wraps to near 2^32, past every span (the word of all
+        // ones would be inside a span that starts in the last 36 * 32 rows below 2^24)
+        const uint32_t none = (__ldg(tmp_key + b) >> (LB + 5) << (LB + 5)) - 1u;
 #pragma unroll
         for (unsigned q = 0; q < kTpPerThread; ++q) {
             const bool in = q * kTpThreads2 + t < n;
-            kk[q] = in ? __ldcs(kp + q * kTpThreads2) : 0xffffffffu;
+            kk[q] = in ? __ldcs(kp + q * kTpThreads2) : none;
             const uint32_t v = in ? (uint32_t) __ldcs(vp + q * kTpThreads2) : 0u;
             vv[q / 2u] = (q & 1u) ? vv[q / 2u] | v << 16 : v;
         }
@@ -1305,13 +1310,14 @@ __global__ void __launch_bounds__(kTpThreads2, 2)
     if (!ballots) {
         for (uint32_t w0 = w_first; w0 <= w_last; w0 += kTpSpanWords) {
             const uint32_t words = min(kTpSpanWords, w_last - w0 + 1u), k0 = w0 << (LB + 5);
+            const uint32_t span = words << (LB + 5); // the words past it are not cleared
             for (uint32_t w = t; w < words * 64u; w += kTpThreads2)
                 reinterpret_cast<uint4 *>(sm.bits)[w] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
 #pragma unroll
             for (unsigned q = 0; q < kTpPerThread; ++q) {
-                const uint32_t x = kk[q] - k0; // no entry: past every span
-                if (x < kTpSpanKeys) atomicOr(sm.bits + (x >> 5), 1u << (x & 31u));
+                const uint32_t x = kk[q] - k0;
+                if (x < span) atomicOr(sm.bits + (x >> 5), 1u << (x & 31u));
             }
             __syncthreads();
             // two threads per column, each with half of the words: the prefix
@@ -1339,7 +1345,7 @@ __global__ void __launch_bounds__(kTpThreads2, 2)
 #pragma unroll
             for (unsigned q = 0; q < kTpPerThread; ++q) {
                 const uint32_t x = kk[q] - k0;
-                if (x < kTpSpanKeys) {
+                if (x < span) {
                     const uint32_t lp = sm.pre[x >> 5] + __popc(sm.bits[x >> 5] & ((1u << (x & 31u)) - 1u));
                     sm.key[lp] = kk[q]; // lp < n: the column's slots start at lb and hold its entries
                     sm.val[lp] = (uint16_t) ((q & 1u) ? vv[q / 2u] >> 16 : vv[q / 2u]);

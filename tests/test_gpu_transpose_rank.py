@@ -91,3 +91,38 @@ def test_tiles_around_the_direct_offset_scan(cuda, n):
     row = np.repeat(np.arange(rows, dtype=np.uint32), count)
     assert np.array_equal(np_u32(t.ptr), np.concatenate([[0], np.cumsum(np.bincount(idx, minlength=cols))]))
     assert np.array_equal(np_u32(t.idx), row[order]) and np.array_equal(np_u16(t.val), val[order])
+
+
+@pytest.mark.parametrize("last,short", [
+    ((1 << 24) - 2, 2),      # the last word of the range
+    ((1 << 24) - 102, 2),    # the word before it
+    ((1 << 24) - 620, 30),   # the first chunk start at which the word of all ones lies in the span
+])
+def test_most_rows(cuda, last, short):
+    """2^24 - 1 rows; the last chunk, `short` entries below a whole one, ends in row `last`."""
+    import torch
+
+    from cellshard_b200.device import CSR, transpose
+
+    rows, cols, chunk = (1 << 24) - 1, 256, 8_192
+    # 3 entries in most rows, 16 in the last 600 that hold any; enough for the row ranking (3 a row)
+    count = np.full(rows, 3, np.int64)
+    count[last + 1:] = 0
+    count[last - 599:last + 1] = 16
+    need = max(0, 3 * rows - int(count.sum()))
+    count[1:need + 2 * chunk:2] += 2
+    over = (int(count.sum()) + short) % chunk  # one entry fewer in `over` early rows
+    count[1:2 * over:2] -= 1
+    n = int(count.sum())
+    assert n % chunk == chunk - short and n >= 3 * rows
+    ptr = np.concatenate([[0], np.cumsum(count)])
+    row = torch.repeat_interleave(torch.arange(rows, device="cuda", dtype=torch.int32),
+                                  torch.from_numpy(count).cuda())
+    at = torch.arange(n, device="cuda") - torch.from_numpy(ptr[:-1]).cuda()[row.long()]
+    col = ((row * 7 + at * 16 + 15) % cols).to(torch.int32)  # distinct in a row, in any order
+    val = (torch.arange(n, device="cuda") % 30_011).to(torch.int16)
+    t = transpose(CSR(rows, cols, torch.from_numpy(ptr.astype(np.uint32).view(np.int32)).cuda(), col,
+                      val.view(torch.float16)))
+    _, order = torch.sort(col.to(torch.uint8), stable=True)
+    assert np.array_equal(np_u32(t.ptr), np.concatenate([[0], np.cumsum(np.bincount(col.cpu(), minlength=cols))]))
+    assert torch.equal(t.idx, row[order]) and torch.equal(t.val.view(torch.int16), val[order])
