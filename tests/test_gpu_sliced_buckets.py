@@ -65,3 +65,34 @@ def test_split_by_widths(cuda, orc, kind, rows, h, gaps):
         assert [int(np_u32(s.slice_widths)[0]) for s in bp.segments] == [s.col_idx.numel() // s.rows if s.rows else 0
                                                                          for s in bp.segments]
         assert np_u16(bp.val).size >= bp.plan["value_entries"]
+
+
+@pytest.mark.parametrize("requested", [3, 4, 512])
+def test_more_buckets_than_widths_of_many_rows(cuda, requested):
+    """A million rows of three widths: one segment per width, however many are asked
+    for, without a programme over the rows (512 levels of it take seconds)."""
+    import time
+
+    import torch
+
+    from cellshard_b200.device import SlicedELL, bucketed_sliced_ell
+
+    rows, w = 1_000_000, 4
+    live = torch.randint(0, 3, (rows,), generator=torch.Generator().manual_seed(1)) + 1  # 1..3 of the slice's 4 slots
+    col = torch.where(torch.arange(w)[None, :] < live[:, None], torch.arange(w, dtype=torch.int32)[None, :],
+                      torch.full((), -1, dtype=torch.int32)).reshape(-1).cuda()
+    val = torch.ones(rows * w, dtype=torch.float16, device="cuda")
+    one = [torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, rows], [w], [0])]
+    sell = SlicedELL(rows, 9, int(live.sum()), rows, *one, col, val)
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    bp = bucketed_sliced_ell(sell, requested)
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 0.5
+    n = torch.bincount(live, minlength=4)[1:].tolist()
+    assert bp.segment_row_offsets == [0, n[0], n[0] + n[1], rows]
+    assert [s.col_idx.numel() for s in bp.segments] == [n[0], 2 * n[1], 3 * n[2]]
+    order = torch.argsort(live, stable=True)
+    assert np.array_equal(np_u32(bp.exec_to_canonical_rows), order.numpy())
+    for k, s in enumerate(bp.segments):
+        assert torch.equal(s.col_idx.view(-1, k + 1), torch.arange(k + 1, dtype=torch.int32, device="cuda").expand(n[k], -1))
