@@ -242,7 +242,7 @@ struct tp2_layout {
     uint32_t *gran_row;     // [nnz / kTpGran + 1] row holding entry j * kTpGran
     void *scan_tmp;
     std::size_t scan_bytes, bytes;
-    uint32_t K, tiles1, max_chunks, slice1, slice2, slices1, max_slices, low_bits;
+    uint32_t K, tiles1, max_chunks, most_chunks, slice1, slice2, slices1, max_slices, low_bits;
 };
 
 bool tp2_applicable(uint32_t cDim, uint32_t uDim) {
@@ -258,6 +258,7 @@ void tp2_make_layout(uint32_t uDim, uint32_t nnz, uint32_t low_bits, bool granul
     const uint32_t tile = granules ? kTpTileCsr : kTpTileCoo;
     l->tiles1 = nnz == 0u ? 1u : (uint32_t) (((std::size_t) nnz + tile - 1u) / tile);
     l->max_chunks = nnz / kTpChunk + l->K + 1u;
+    l->most_chunks = std::min(l->max_chunks, nnz / kTpChunk + 2u); // of one bucket
     l->slice1 = tp_slice_len(l->tiles1);
     l->slice2 = tp_slice_len(l->max_chunks);
     l->slices1 = (l->tiles1 + l->slice1 - 1u) / l->slice1;
@@ -377,7 +378,8 @@ __global__ void __launch_bounds__(256) tp_slice_sums_kernel(const uint16_t *__re
                                                             const uint2 *__restrict__ range,
                                                             uint32_t *__restrict__ slices) {
     const uint2 r = tp_slice_rows(range, rows, len);
-    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+    const uint32_t d = blockIdx.y * blockDim.x + threadIdx.x;
+    if (d < D) {
         uint32_t sum = 0u;
 #pragma unroll 16
         for (uint32_t i = r.x; i < r.y; ++i) sum += __ldg(cnt + (std::size_t) i * D + d);
@@ -420,6 +422,38 @@ __global__ void __launch_bounds__(1024) tp_slice_scan_kernel(uint32_t *__restric
     }
 }
 
+// The same, or (T = uint16_t) the scan of the rows themselves, by a thread per
+// digit: many segments of few slices or rows each, which the CTAs of 1,024
+// threads above mostly leave idle.  range: null where seg_first counts in's rows.
+template <typename T>
+__global__ void __launch_bounds__(256) tp_segment_scan_kernel(const T *in, uint32_t D,
+                                                              const uint32_t *__restrict__ seg_first,
+                                                              const uint2 *__restrict__ range, uint32_t limit,
+                                                              uint32_t *out, uint32_t *__restrict__ totals) {
+    const uint32_t d = blockIdx.y * blockDim.x + threadIdx.x;
+    if (d >= D) return;
+    uint32_t r0 = seg_first[blockIdx.x], r1 = seg_first[blockIdx.x + 1u];
+    if (range != nullptr) {
+        const uint32_t s0 = r0, s1 = r1;
+        r0 = s0 < s1 ? range[s0].x : 0u;
+        r1 = s0 < s1 ? range[s1 - 1u].y : 0u;
+    }
+    constexpr uint32_t U = 8; // loads in flight; `out` may be `in`
+    uint32_t run = 0u;
+    for (uint32_t i0 = r0; i0 < r1; i0 += U) {
+        uint32_t v[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) v[u] = i0 + u < r1 ? (uint32_t) in[(std::size_t) (i0 + u) * D + d] : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            if (i0 + u < r1) out[(std::size_t) (i0 + u) * D + d] = run;
+            run += v[u];
+        }
+    }
+    const std::size_t c = (std::size_t) blockIdx.x * D + d;
+    if (c < limit) totals[c] = run;
+}
+
 // start[segment * D + d]: global slot of the digit's first entry
 __global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__restrict__ cnt, uint32_t D,
                                                              uint32_t rows, uint32_t len,
@@ -430,7 +464,8 @@ __global__ void __launch_bounds__(256) tp_slice_apply_kernel(const uint16_t *__r
                                                              uint32_t *__restrict__ base) {
     const uint2 r = tp_slice_rows(range, rows, len);
     const std::size_t c0 = (segment != nullptr ? (std::size_t) segment[blockIdx.x] : 0u) * D;
-    for (uint32_t d = threadIdx.x; d < D; d += blockDim.x) {
+    const uint32_t d = blockIdx.y * blockDim.x + threadIdx.x;
+    if (d < D) {
         uint32_t run = slices[(std::size_t) blockIdx.x * D + d] + (c0 + d < limit ? start[c0 + d] : 0u);
 #pragma unroll 16
         for (uint32_t i = r.x; i < r.y; ++i) {
@@ -1391,20 +1426,38 @@ int tp_smem(K kernel, std::size_t smem, const char *what) {
 }
 
 // The totals of `t`'s digits, and its offsets: complete but for the digits'
-// starts, which the scatter then adds (t->start), where no segment has more than
-// kTpDirectRows rows; else tp_offsets_apply adds them once they are scanned.
-// rows [0, rows) in slices of len, or the segments' slices `range`.
-int tp_offsets(tp_counts *t, uint32_t D, uint32_t rows, uint32_t most_rows, uint32_t len, uint32_t slices,
-               uint32_t segments, const uint32_t *seg_first, const uint2 *range, uint32_t limit, uint32_t *totals,
-               const uint32_t *start, cudaStream_t stream) {
-    const dim3 grid(segments, (D + 31u) / 32u);
-    if (most_rows <= kTpDirectRows) {
+// starts, which the scatter then adds (t->start), where the rows are few (in each
+// segment, or kTpDirectRows in all); else tp_offsets_apply adds them once they are
+// scanned.  rows [0, rows) in slices of len, or the segments' slices `range`; a
+// segment has at most most_rows of the total_rows.
+// us of a transpose into 262,144 columns (1,024 buckets; 1 M / 2 M / 6 M entries):
+// 101 / 121 / 233, with 32 threads a digit in every segment 144 / 163 / 279 (44 of
+// them in 8,192 CTAs of the second pass's scan).
+int tp_offsets(tp_counts *t, uint32_t D, uint32_t rows, uint32_t total_rows, uint32_t most_rows, uint32_t len,
+               uint32_t slices, uint32_t segments, const uint32_t *seg_first, const uint2 *range, uint32_t limit,
+               uint32_t *totals, const uint32_t *start, cudaStream_t stream) {
+    const dim3 grid(segments, (D + 31u) / 32u), by_digit(segments, (D + 255u) / 256u);
+    // a serial step per 8 rows of the longest segment there can be against 8 CTAs of 1,024
+    // threads a segment, two to an SM: they cost the same at about four segments a row
+    auto few = [&](uint32_t n) { return segments > 1u && n <= segments / 4u; };
+    if (few(most_rows)) {
+        t->start = start;
+        tp_segment_scan_kernel<<<by_digit, 256, 0, stream>>>(t->cnt, D, seg_first, range, limit, t->base, totals);
+        return launch_ok("tp_segment_scan_kernel");
+    }
+    if (total_rows <= kTpDirectRows) {
         t->start = start;
         tp_rows_scan_kernel<<<grid, 1024, 0, stream>>>(t->cnt, D, rows, seg_first, range, limit, t->base, totals);
         return launch_ok("tp_rows_scan_kernel");
     }
-    tp_slice_sums_kernel<<<slices, 256, 0, stream>>>(t->cnt, D, rows, len, range, t->slices);
+    const dim3 by_slice(slices, (D + 255u) / 256u);
+    tp_slice_sums_kernel<<<by_slice, 256, 0, stream>>>(t->cnt, D, rows, len, range, t->slices);
     if (!launch_ok("tp_slice_sums_kernel")) return 0;
+    if (few(most_rows / len + 2u)) {
+        tp_segment_scan_kernel<<<by_digit, 256, 0, stream>>>((const uint32_t *) t->slices, D, seg_first, nullptr, limit,
+                                                             t->slices, totals);
+        return launch_ok("tp_segment_scan_kernel");
+    }
     tp_slice_scan_kernel<<<grid, 1024, 0, stream>>>(t->slices, D, seg_first, slices, limit, totals);
     return launch_ok("tp_slice_scan_kernel");
 }
@@ -1412,8 +1465,8 @@ int tp_offsets(tp_counts *t, uint32_t D, uint32_t rows, uint32_t most_rows, uint
 int tp_offsets_apply(const tp_counts &t, uint32_t D, uint32_t rows, uint32_t len, uint32_t slices, const uint2 *range,
                      const uint32_t *segment, uint32_t limit, const uint32_t *start, cudaStream_t stream) {
     if (t.start != nullptr) return 1;
-    tp_slice_apply_kernel<<<slices, 256, 0, stream>>>(t.cnt, D, rows, len, range, segment, t.slices, start, limit,
-                                                      t.base);
+    tp_slice_apply_kernel<<<dim3(slices, (D + 255u) / 256u), 256, 0, stream>>>(t.cnt, D, rows, len, range, segment,
+                                                                                  t.slices, start, limit, t.base);
     return launch_ok("tp_slice_apply_kernel");
 }
 
@@ -1428,8 +1481,8 @@ int tp_second_pass(uint32_t uDim, const tp2_layout &l, uint32_t *out_ptr, uint32
     if (!launch_ok("tp_hist2_kernel")) return 0;
     constexpr uint32_t D = 1u << LB;
     tp_counts two = l.two;
-    if (!tp_offsets(&two, D, 0u, l.max_chunks, 0u, l.max_slices, l.K, l.slice_first, l.slice_range, uDim, out_ptr,
-                    out_ptr, stream) ||
+    if (!tp_offsets(&two, D, 0u, l.max_chunks, l.most_chunks, l.slice2, l.max_slices, l.K, l.slice_first,
+                    l.slice_range, uDim, out_ptr, out_ptr, stream) ||
         !scan_exclusive_u32(out_ptr, out_ptr, uDim, true, l.scan_tmp, l.scan_bytes, stream) ||
         !tp_offsets_apply(two, D, 0u, 0u, l.max_slices, l.slice_range, l.slice_bucket, uDim, out_ptr, stream))
         return 0;
@@ -1462,8 +1515,8 @@ int tp_first_pass(uint32_t cDim, uint32_t uDim, uint32_t nnz, const uint32_t *pt
                                                                     l.status);
     if (!launch_ok("tp_hist1_kernel")) return 0;
     tp_counts one = l.one;
-    if (!tp_offsets(&one, l.K, l.tiles1, l.tiles1, l.slice1, l.slices1, 1u, nullptr, nullptr, l.K, l.total1, l.start1,
-                    stream))
+    if (!tp_offsets(&one, l.K, l.tiles1, l.tiles1, l.tiles1, l.slice1, l.slices1, 1u, nullptr, nullptr, l.K, l.total1,
+                    l.start1, stream))
         return 0;
     tp_chunks_kernel<<<1, 1024, 0, stream>>>(l);
     if (!launch_ok("tp_chunks_kernel") ||

@@ -126,3 +126,33 @@ def test_most_rows(cuda, last, short):
     _, order = torch.sort(col.to(torch.uint8), stable=True)
     assert np.array_equal(np_u32(t.ptr), np.concatenate([[0], np.cumsum(np.bincount(col.cpu(), minlength=cols))]))
     assert torch.equal(t.idx, row[order]) and torch.equal(t.val.view(torch.int16), val[order])
+
+
+@pytest.mark.parametrize("cols,n,skew", [
+    (262_144, 300_000, 0.0),      # 1,024 buckets of a chunk each
+    (262_144, 2_080_700, 0.9),    # the longest bucket that a thread per digit walks, nearly all entries in it
+    (262_144, 2_089_000, 0.9),    # one more: in slices
+    (262_144, 9_000_000, 0.5),
+    (120_000, 900_000, 0.3),      # fewer chunks than one scan takes, either way
+    (120_000, 980_000, 0.3),
+    (16_000, 5_000_000, 0.0),     # few buckets
+])
+def test_offsets_of_many_buckets(cuda, cols, n, skew):
+    """Second-pass offsets over many buckets, one of them holding up to nearly all entries."""
+    import torch
+
+    from cellshard_b200.device import CSR, transpose
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rows = 4_000
+    row = torch.sort(torch.randint(0, rows, (n,), generator=g, device="cuda")).values
+    col = torch.randint(0, cols, (n,), generator=g, device="cuda")
+    hot = torch.rand(n, generator=g, device="cuda") < skew
+    col = torch.where(hot, col % 256 + 256 * 3, col)  # rows repeat columns; input order decides
+    val = (torch.arange(n, device="cuda") % 30_011).to(torch.int16)
+    ptr = torch.zeros(rows + 1, dtype=torch.int64, device="cuda")
+    torch.cumsum(torch.bincount(row, minlength=rows), 0, out=ptr[1:])
+    t = transpose(CSR(rows, cols, ptr.to(torch.int32), col.to(torch.int32), val.view(torch.float16)))
+    order = torch.sort(col, stable=True).indices
+    assert torch.equal(t.ptr[1:].long(), torch.cumsum(torch.bincount(col, minlength=cols), 0))
+    assert torch.equal(t.idx.long(), row[order]) and torch.equal(t.val.view(torch.int16), val[order])
