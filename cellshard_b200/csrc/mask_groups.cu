@@ -708,11 +708,26 @@ __global__ void __launch_bounds__(kCodesWarps * 32, 1)
     const uint32_t gmask = group_count >= 32u ? 0xffffffffu : (1u << group_count) - 1u;
     for (uint32_t c = threadIdx.x; c < kept_words; c += blockDim.x) kept[c] = 0u;
     if constexpr (kBitmap) __syncthreads();
-    for (uint32_t c = threadIdx.x; c < src.cols; c += blockDim.x) {
-        const bool keep = feature_kept(masks.feature_keep, c);
-        const uint32_t m = keep ? __ldg(group_masks + c) & gmask : 0u;
-        code[c] = kBitmap ? m : m | (keep ? 0x80000000u : 0u);
-        if (kBitmap && keep) atomicOr(kept + (c >> 5), 1u << (c & 31u));
+    // eight columns a thread in flight: a small matrix waits for the table (500 x 33,000:
+    // 25 us a call, 37 one by one)
+    constexpr unsigned U = 8;
+    for (uint32_t c0 = threadIdx.x; c0 < src.cols; c0 += blockDim.x * U) {
+        uint32_t m[U];
+        bool keep[U];
+#pragma unroll
+        for (unsigned u = 0; u < U; ++u) {
+            const uint32_t c = c0 + blockDim.x * u;
+            m[u] = c < src.cols ? __ldg(group_masks + c) & gmask : 0u;
+            keep[u] = c < src.cols && feature_kept(masks.feature_keep, c);
+        }
+#pragma unroll
+        for (unsigned u = 0; u < U; ++u) {
+            const uint32_t c = c0 + blockDim.x * u;
+            if (c >= src.cols) break;
+            if (!keep[u]) m[u] = 0u;
+            code[c] = kBitmap ? m[u] : m[u] | (keep[u] ? 0x80000000u : 0u);
+            if (kBitmap && keep[u]) atomicOr(kept + (c >> 5), 1u << (c & 31u));
+        }
     }
     __syncthreads();
     const wide_table tbl{code, kept};
@@ -781,11 +796,28 @@ int launch_codes(reduce_codes_kernel_t<View> k, const View &src, const uint32_t 
     return launch_ok(name);
 }
 
-// Shared bytes of the wide kernel, 0 where it does not apply: 16 to 32 groups
-// and a table that fits beside the stages.
-std::size_t wide_smem_bytes(const uint32_t *masks, uint32_t group_count, uint32_t cols) {
+// Whether rows and entries pay for the wide kernel's table, which every CTA
+// builds, and its 148 CTAs' start.  It saves 84 entries' worth a row (the general
+// kernel's group sums meet in shared memory) and something an entry, more with
+// 32 accumulators a lane (17 groups up) than with 16; with 32 groups the bitmap
+// costs some of it back.  Fitted over 1,940 matrices of 2,500 to 33,000 columns,
+// 8 to 1,500 entries a row, 75 to 165,000 rows: 4 of them are slower than by the
+// general kernel, by 9 % at most.  us general / wide, 24 groups: 500 x 33,000 of 100
+// entries 13 / 25, 20,000 x 33,000 of 100 41 / 42, 60,000 x 33,000 of 60 86 / 65, 8,000 x
+// 33,000 of 1,600 152 / 88.  nnz 0: not counted (a segment's view), 100 a row taken.
+bool wide_pays(uint32_t rows, uint32_t nnz, uint32_t cols, uint32_t group_count) {
+    const double entries = nnz != 0u ? (double) nnz : 100.0 * rows;
+    const double scale = group_count == 16u ? 2.5 : group_count == 32u ? 1.3 : 1.0;
+    return 84.0 * rows + entries >= scale * (0.9e6 + 60.0 * cols);
+}
+
+// Shared bytes of the wide kernel, 0 where it does not apply: 16 to 32 groups,
+// a matrix that pays for the table, and a table that fits beside the stages.
+template <typename View>
+std::size_t wide_smem_bytes(const View &src, const uint32_t *masks, uint32_t group_count) {
     if (masks == nullptr || group_count < 16u || group_count > 32u) return 0u;
-    const std::size_t words = (std::size_t) cols + (group_count == 32u ? (cols + 31u) / 32u : 0u) + 1u;
+    if (!wide_pays(src.rows, src.nnz, src.cols, group_count)) return 0u;
+    const std::size_t words = (std::size_t) src.cols + (group_count == 32u ? (src.cols + 31u) / 32u : 0u) + 1u;
     const std::size_t bytes = (words & ~(std::size_t) 1u) * 4u + kCodesWarps * kWideStage * sizeof(uint2);
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -2052,7 +2084,7 @@ extern "C" int cs_b200_group_reduce_sliced_ell(const cs_sliced_ell_view *src, co
                                                 *src, d_feature_group_masks, group_count, m, *filter, *out, csmem,
                                                 as_stream(s), "group_reduce_sell_codes_kernel");
     }
-    if (const std::size_t wsmem = vec ? wide_smem_bytes(d_feature_group_masks, group_count, src->cols) : 0u)
+    if (const std::size_t wsmem = vec ? wide_smem_bytes(*src, d_feature_group_masks, group_count) : 0u)
         return launch_codes<cs_sliced_ell_view>(group_count == 32u
                                                     ? group_reduce_wide_kernel<cs_sliced_ell_view, true>
                                                     : group_reduce_wide_kernel<cs_sliced_ell_view, false>,
@@ -2093,7 +2125,7 @@ extern "C" int cs_b200_group_reduce_compressed(const cs_compressed_view *src, co
                                                 *src, d_feature_group_masks, group_count, m, *filter, *out, csmem,
                                                 as_stream(s), "group_reduce_csr_codes_kernel");
     }
-    if (const std::size_t wsmem = vec ? wide_smem_bytes(d_feature_group_masks, group_count, src->cols) : 0u)
+    if (const std::size_t wsmem = vec ? wide_smem_bytes(*src, d_feature_group_masks, group_count) : 0u)
         return launch_codes<cs_compressed_view>(group_count == 32u
                                                     ? group_reduce_wide_kernel<cs_compressed_view, true>
                                                     : group_reduce_wide_kernel<cs_compressed_view, false>,
