@@ -139,3 +139,38 @@ def test_shuffled_coo_past_the_column_blocks_is_refused(cuda):
                for a, t in ((row, np.int32), (col, np.int32), (val, np.float16))]
         with pytest.raises(_abi.CellShardError, match="column-block limit"):
             blocked_ell_from_coo(40, 140_000, *dev, 1, 140_000)
+
+
+@pytest.mark.parametrize("cols,block", [
+    (1_100, 24), (9_000, 16),               # rows by a warp, by a CTA
+    (333, 3), (1_201, 1), (40_000, 16),     # no bulk stores: odd row sizes, two segments
+])
+@pytest.mark.parametrize("equal", [False, True])
+def test_rows_that_repeat_a_column(cuda, orc, cols, block, equal):
+    """Repeated columns with other values, the same one, NaN and zeros among them, in any order: the
+    last value stays, and a cell counts once."""
+    from cellshard_b200.device import blocked_ell_from_csr
+
+    rng = np.random.default_rng(cols + block)
+    rows = 61
+    parts, vals = [], []
+    for r in range(rows):
+        c = rng.permutation(cols)[:int(rng.integers(1, min(cols, 3_000)))]
+        v = rng.integers(0, 3, len(c)).astype(np.float16)
+        v[rng.random(len(c)) < 0.05] = np.nan
+        if r % 3:
+            k = rng.integers(0, len(c), 4)
+            more = v[k] if equal else rng.integers(0, 5, 4).astype(np.float16)
+            p = rng.permutation(len(c) + 4)
+            c, v = np.append(c, c[k])[p], np.append(v, more)[p]
+        if r % 5 == 0:  # next to each other
+            o = np.argsort(c, kind="stable")
+            c, v = c[o], v[o]
+        parts.append(c)
+        vals.append(v)
+    ptr = np.concatenate([[0], np.cumsum([len(c) for c in parts])]).astype(np.uint32)
+    idx, val = np.concatenate(parts).astype(np.uint32), np.concatenate(vals).view(np.uint16)
+    out = blocked_ell_from_csr(to_device_csr(rows, cols, ptr, idx, val), block)
+    ref = orc.blocked_ell_from_csr(rows, cols, ptr, idx, val, block)
+    assert out.ell_cols == ref["ell_cols"] and out.nnz == ref["nnz"]
+    assert np.array_equal(np_u32(out.bci), ref["bci"]) and np.array_equal(np_u16(out.val), ref["val"])
