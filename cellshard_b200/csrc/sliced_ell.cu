@@ -131,7 +131,10 @@ __global__ void __launch_bounds__(kWarps * 32) sell_emit_vec_kernel(const uint32
         const uint32_t w = widths[s];
         const std::size_t base = (std::size_t) slot_offsets[s] + (std::size_t) (r - s * h) * w;
         const uint32_t a = ptr[r];
-        sell_emit_row_vec<GL>(idx, val, a, ptr[r + 1u] - a, w, base, col_idx, out_val, gl);
+        if constexpr (GL == 32u)
+            sell_emit_row_vec<GL>(idx, val, a, ptr[r + 1u] - a, w, base, col_idx, out_val, gl);
+        else
+            sell_emit_short_row_vec<GL>(idx, val, a, ptr[r + 1u] - a, w, base, col_idx, out_val, gl);
     }
 }
 

@@ -119,3 +119,26 @@ def test_sliced_matches_reference_gpu_route(cuda, orc):
     out = sliced_ell_from_csr(to_device_csr(rows, cols, ptr, idx, val), 32)
     assert np.array_equal(np_u32(out.col_idx), ref_col)
     assert np.array_equal(np_u16(out.val), ref_val)
+
+
+@pytest.mark.parametrize("mean", [1, 3, 25, 95, 97, 300])  # eight lanes a row below 96 entries, a warp above
+@pytest.mark.parametrize("h", [1, 5, 32])
+def test_sliced_ell_row_sizes(cuda, orc, mean, h):
+    """Every row size from none to past a step of the group, rows at every offset from a vector boundary."""
+    from cellshard_b200.device import sliced_ell_from_csr
+
+    rng = np.random.default_rng(mean + h)
+    rows, cols = 1_201, 2_000
+    n = np.minimum(rng.poisson(mean, rows), cols)
+    n[:80] = np.arange(80) % (2 * mean + 2)
+    if mean > 80:  # the short first rows made up for in the last ones
+        n[-200:] += (mean * rows - int(n.sum())) // 200
+    ptr = np.concatenate([[0], np.cumsum(n)]).astype(np.uint32)
+    idx = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in n]).astype(np.uint32)
+    val = rng.integers(0, 65_536, len(idx)).astype(np.uint16)
+    assert (len(idx) / rows >= 96) == (mean > 96)
+    out = sliced_ell_from_csr(to_device_csr(rows, cols, ptr, idx, val), h)
+    ref = orc.sliced_ell_from_csr(rows, ptr, idx, val, h)
+    offs, widths, col, v = _host(out)
+    assert np.array_equal(offs, ref["offsets"]) and np.array_equal(widths, ref["widths"])
+    assert np.array_equal(col, ref["col_idx"]) and np.array_equal(v, ref["val"])
