@@ -617,12 +617,17 @@ cs_batch_tiles default_tiles(const std::vector<cs_batch_part> &parts) {
         rows += p.src.rows;
         nnz += p.src.nnz;
     }
-    // about eight emit items per CTA, so that the last ones leave few CTAs idle
-    // (400,000 rows: 1.34 ms at 64 rows an item, 1.42 at 512)
-    t.emit_rows = 512u;
-    while (t.emit_rows > 32u && rows / t.emit_rows < 8u * 3u * (uint64_t) sm_count()) t.emit_rows /= 2u;
     const double mean = rows ? (double) nnz / (double) rows : 0.0;
     t.emit_lanes = mean >= 96.0 ? 32u : (mean >= 24.0 ? 16u : 8u);
+    // Long rows: about eight emit items per CTA, so that the last ones leave few CTAs
+    // idle (400,000 rows of 819: 1.34 ms at 64 rows an item, 1.42 at 512).  Short rows:
+    // an item of few of them is less work than taking it, so only as small as gives
+    // the SMs one each (us a run at 512 / 128 / 32 rows an item: 100,000 rows of 12
+    // 97 / 98 / 102, 200,000 of 12 149 / 165 / 153, 50,000 of 5 64 / 68 / 70; 10,000 of 80
+    // 76 / 45 / 43).
+    t.emit_rows = 512u;
+    const uint64_t items = t.emit_lanes == 32u ? 8u * 3u * (uint64_t) sm_count() : 128u;
+    while (t.emit_rows > 32u && rows / t.emit_rows < items) t.emit_rows /= 2u;
     t.ctas_per_sm = 0u; // 0 = as many as fit
     return t;
 }

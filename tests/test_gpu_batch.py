@@ -189,3 +189,36 @@ def test_batch_autotune_and_generated_partitions(cuda, orc):
     assert deferred == 0 and err == 0
     for h, r in zip(hp, results):
         _check_part(orc, h, r, bucket_count=8)
+
+
+@pytest.mark.parametrize("rows,per,emit_rows", [
+    (100_000, 12, 512),   # short rows are not cut into items that cost more than their work
+    (10_000, 12, 64),     # but for the SMs to get one each
+    (90, 12, 32),
+    (20_000, 120, 32),    # long rows: eight items per CTA, down to 32 rows
+])
+def test_default_emit_items(cuda, rows, per, emit_rows):
+    import torch
+
+    from cellshard_b200.batch import BatchSlicedConverter
+    from cellshard_b200.device import CSR, sliced_ell_from_csr
+
+    parts = []
+    for k in range(3):
+        r = rows // 3 + k - 1
+        n = torch.full((r,), per, dtype=torch.int64)
+        n[::7] += k
+        ptr = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(n, 0)]).to(torch.int32).cuda()
+        nnz = int(n.sum())
+        parts.append(CSR(r, 1_000, ptr, (torch.arange(nnz, device="cuda") * 7 % 1_000).to(torch.int32),
+                         (torch.arange(nnz, device="cuda") % 2_000).to(torch.float16)))
+    conv = BatchSlicedConverter(parts)
+    assert conv.tiles()["emit_rows"] == emit_rows
+    conv.run()
+    results, deferred, err = conv.results()
+    assert deferred == 0 and err == 0
+    for p, r in zip(parts, results):
+        want = sliced_ell_from_csr(p, r.slice_rows)
+        assert torch.equal(r.sliced.slice_widths, want.slice_widths)
+        assert torch.equal(r.sliced.col_idx, want.col_idx)
+        assert torch.equal(r.sliced.val.view(torch.int16), want.val.view(torch.int16))
