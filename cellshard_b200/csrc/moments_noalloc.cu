@@ -72,15 +72,15 @@ extern "C" int cs_b200_group_moments_blocked_ell_noalloc(const cs_blocked_ell_vi
                                                           const uint8_t *d_feature_keep, const uint32_t *d_row_labels,
                                                           const cs_group_moments_params *params,
                                                           const cs_group_moments_out *out, cs_stream_t stream) {
-    // chunks of 2,048 rows by default: shorter ones, which the entry point with
-    // caller scratch takes for small matrices, would need more of the static array
-    cs_group_moments_params whole;
-    if (params != nullptr && params->chunk_rows == 0u) {
-        whole = *params;
-        whole.chunk_rows = 2048u;
-        params = &whole;
+    // What the array must hold at least: chunks of 2,048 rows.  Where the default's
+    // shorter ones fit too, the reduction takes them (see fit_scratch), and its results
+    // are those of the entry point with caller scratch bit for bit.
+    cs_group_moments_params least;
+    if (params != nullptr) {
+        least = *params;
+        if (least.chunk_rows == 0u) least.chunk_rows = 2048u;
     }
-    const std::size_t need = group_moments_scratch_needed(src, params);
+    const std::size_t need = group_moments_scratch_needed(src, params != nullptr ? &least : nullptr);
     if (need == 0) return 0;
     if (need > (std::size_t) CS_NOALLOC_SCRATCH_BYTES) {
         set_error("group_moments_noalloc: this partition needs %zu bytes of scratch but the static scratch holds "

@@ -887,7 +887,7 @@ typedef struct CS_ALIGN16 cs_group_moments_params {
     uint32_t group_count; /* G, 1..CS_MAX_MOMENT_GROUPS */
     uint32_t scheme;      /* CS_MOMENTS_* */
     uint32_t ddof;        /* variance divisor is n - ddof (0 or 1) */
-    uint32_t chunk_rows;  /* rows per work chunk, 0 = default */
+    uint32_t chunk_rows;  /* rows per work chunk, 0 = default: 64 to 2,048 by the size of the matrix */
     /* Optional (NULL = built by every call): device address of the partition's
      * column-block index, built once by cs_b200_group_moments_build_index for
      * this partition (it depends only on blockColIdx, so it stays valid while
@@ -949,7 +949,10 @@ CS_API int cs_b200_group_moments_build_index(const cs_blocked_ell_view *src, voi
  * padding at the end (the layout cs_b200_blocked_ell_emit and
  * convert::blocked_ell_from_compressed produce); other layouts set
  * CS_STATUS_BLOCK_COL_ORDER.  Deterministic: the same inputs give the same
- * bits regardless of stream contention. */
+ * bits regardless of stream contention, with any scratch of at least the size
+ * that cs_b200_group_moments_scratch_bytes asks for.  With chunk_rows 0 less is
+ * taken down to what chunks of 2,048 rows need: the rows are then added in
+ * longer chunks, which may round the last bit of a sum otherwise. */
 CS_API int cs_b200_group_moments_blocked_ell(const cs_blocked_ell_view *src,
                                       const uint8_t *d_row_keep,
                                       const uint8_t *d_feature_keep,
@@ -971,9 +974,10 @@ CS_API int cs_b200_group_moments_blocked_ell(const cs_blocked_ell_view *src,
  * footprint behind the owner's back).  It allocates nothing: its scratch is
  * a fixed CS_NOALLOC_SCRATCH_BYTES device array inside the library, located
  * once per device with cudaGetSymbolAddress on the first call on that device
- * (make that first call before any stream capture).  Calls whose scratch need
- * (cs_b200_group_moments_scratch_bytes) exceeds CS_NOALLOC_SCRATCH_BYTES
- * return 0 with a message.  All calls share the array and it keeps the last
+ * (make that first call before any stream capture).  Calls that do not fit
+ * CS_NOALLOC_SCRATCH_BYTES (chunk_rows 0: with chunks of 2,048 rows) return 0
+ * with a message; where cs_b200_group_moments_scratch_bytes fits, the results
+ * are those of the call with caller scratch bit for bit.  All calls share the array and it keeps the last
  * call's contents (nothing needs clearing: every byte read is written earlier
  * in the same call); calls that overlap on the GPU race on it, so the caller
  * serialises them.  The located address is kept for the life of the process:

@@ -56,3 +56,37 @@ def test_default_chunks(cuda, rows, cols, density, block, groups):
     if done:
         for w, k in zip(want, ("sum", "sumsq")):
             assert np.array_equal(out[k].cpu().numpy().astype(np.float64), w), k
+
+
+@pytest.mark.parametrize("rows,cols,groups,chunk", [(8_192, 2_000, 8, 0), (3_000, 700, 9, 0), (3_000, 700, 9, 96),
+                                                    (3_000, 4_000, 250, 0)])
+def test_noalloc_gives_the_same_bits(cuda, rows, cols, groups, chunk):
+    """Values that are no whole numbers: the order of the sums shows in the 64-bit results."""
+    import torch
+
+    from cellshard_b200 import _abi
+    from cellshard_b200.device import blocked_ell_from_csr, ptr as dptr, stream_handle
+
+    p, idx, val = random_csr(rows, cols, 0.06, rows, 0.1, integer=False)
+    bell = blocked_ell_from_csr(to_device_csr(rows, cols, p, idx, val), 16)
+    lab = torch.from_numpy(np.random.default_rng(rows).integers(0, groups, rows).astype(np.int32)).cuda()
+    lib = _abi.load()
+    v, prm, n = bell.view(), _abi.GroupMomentsParams(groups, 2, 1, chunk), C.c_size_t()
+    _abi.check(lib.cs_b200_group_moments_scratch_bytes(C.byref(v), C.byref(prm), C.byref(n)), "scratch")
+    assert n.value <= 64 << 20
+    scratch = torch.empty(n.value, dtype=torch.uint8, device="cuda")
+    got = []
+    for noalloc in (False, True):
+        out = [torch.zeros(groups, cols, dtype=t, device="cuda") for t in 4 * [torch.float32] + 2 * [torch.float64]]
+        o = _abi.GroupMomentsOut(*(dptr(t) for t in out))
+        if noalloc:
+            ok = lib.cs_b200_group_moments_blocked_ell_noalloc(C.byref(v), None, None, dptr(lab), C.byref(prm),
+                                                               C.byref(o), stream_handle())
+        else:
+            ok = lib.cs_b200_group_moments_blocked_ell(C.byref(v), None, None, dptr(lab), C.byref(prm), C.byref(o),
+                                                       dptr(scratch), n.value, stream_handle())
+        _abi.check(ok, "group_moments")
+        got.append(out)
+    assert float(got[0][0].abs().sum()) > 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
