@@ -241,6 +241,15 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+def moments_chunk_rows(bell):
+    """Rows per chunk that the library takes by default for this matrix: those whose scratch it asks for."""
+    from cellshard_b200 import runtime
+
+    need = runtime.group_moments_scratch_bytes(bell, GROUPS)
+    return next(c for c in (2048, 1024, 512, 256, 128, 64)
+                if runtime.group_moments_scratch_bytes(bell, GROUPS, chunk_rows=c) == need)
+
+
 def workload_config(spec):
     return {"workload": "masked grouped moments (sum, sumsq, mean, var) over a Blocked-ELL-16 partition",
             "rows": spec.rows, "cols": spec.cols, "density": 0.04, "block_size": BLOCK, "groups": GROUPS,
@@ -380,7 +389,7 @@ def run_product(args):
 
     W = bell.ell_width
     rb_kept = int(np.unique(np.flatnonzero(rk) // BLOCK).size)
-    cr = args.chunk_rows or 2048
+    cr = args.chunk_rows or moments_chunk_rows(bell)
     chunks_per_group = [(n + cr - 1) // cr for n in np.bincount(lab[rk == 1], minlength=GROUPS)]
     n_chunks = int(sum(chunks_per_group))
     acc_bytes = kept_rows * bell.ell_cols * 2 + n_chunks * spec.cols * 16

@@ -62,3 +62,22 @@ def test_single_process_keeps_its_values():
 
     assert bench.max_over_ranks(None, [1, 2.5], "cpu") == [1.0, 2.5]
     assert bench.whole_job_rate(1, 10, 2.0) == pytest.approx(5000.0)
+
+
+@pytest.mark.parametrize("rows,cols,chunk", [(500_000, 32_768, 2_048), (60_000, 32_768, 1_024), (120_000, 8_000, 512),
+                                             (30_000, 2_000, 64)])
+def test_roofline_counts_the_chunks_that_the_library_takes(rows, cols, chunk):
+    sys.path.insert(0, str(ROOT))
+    import bench
+    from cellshard_b200 import _abi, build
+
+    build.build()
+
+    class Bell:
+        @staticmethod
+        def view():
+            v = _abi.BlockedEllView()
+            v.rows, v.cols, v.block_size, v.ell_cols = rows, cols, bench.BLOCK, cols
+            return v
+
+    assert bench.moments_chunk_rows(Bell) == chunk
