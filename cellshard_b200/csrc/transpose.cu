@@ -648,7 +648,7 @@ struct tp_tile_smem {
     uint32_t heads[kTpTileWords], starts[kTpTileWords]; // bits: run heads, row starts
     uint16_t heads_pre[kTpTileWords], starts_pre[kTpTileWords];
     uint16_t row_of[kTpTileRows];        // row - the tile's first row
-    uint32_t scan33[33], scan33b[33];
+    uint32_t scan33[33];
 };
 
 template <bool kAdd>

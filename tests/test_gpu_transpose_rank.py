@@ -156,3 +156,41 @@ def test_offsets_of_many_buckets(cuda, cols, n, skew):
     order = torch.sort(col, stable=True).indices
     assert torch.equal(t.ptr[1:].long(), torch.cumsum(torch.bincount(col, minlength=cols), 0))
     assert torch.equal(t.idx.long(), row[order]) and torch.equal(t.val.view(torch.int16), val[order])
+
+
+@pytest.mark.parametrize("cols,sections", [
+    (256, [(9_000, 9)]),                                       # a round a chunk, or two
+    (256, [(20_000, 12), (20_000, 3.4), (9_000, 2.4)]),        # two and three rounds
+    (256, [(30_000, 12), (25_000, 2.0), (2_000, 20)]),         # four, the most
+    (256, [(30_000, 12), (25_000, 1.9), (25_000, 1.75)]),      # around the edge to five, ranked by ballots
+    (256, [(30_000, 12), (4_600, 0), (9_000, 2.2), (70_000, 0.01), (40_000, 12)]),  # gaps of empty rows
+    (300, [(30_000, 14), (15_000, 4.0)]),                      # a second bucket of 44 columns
+    (1_000, [(12_000, 60), (12_000, 9)]),
+    (262_144, [(40, 4_400)]),                                  # the most buckets
+])
+@pytest.mark.parametrize("repeat,unsorted", [(0, False), (0, True), (5, True), (2_000, False)])
+def test_row_ranking_rounds(cuda, orc, cols, sections, repeat, unsorted):
+    """Matrices that take the row ranking (three entries per row and 256 columns), with chunks of one
+    to five rounds of 1,152 rows."""
+    from cellshard_b200.device import transpose
+
+    rows = sum(r for r, _ in sections)
+    rng = np.random.default_rng(rows + cols + repeat)
+    n = np.concatenate([rng.poisson(per, r) for r, per in sections])
+    row = np.repeat(np.arange(rows), n)
+    key = np.unique(row.astype(np.int64) * cols + rng.integers(0, cols, len(row)))
+    row, col = key // cols, key % cols
+    if repeat:
+        at = rng.choice(len(row), repeat, replace=False)
+        row, col = np.insert(row, at, row[at]), np.insert(col, at, col[at])
+    if unsorted:
+        p = np.lexsort((rng.random(len(row)), row))
+        row, col = row[p], col[p]
+    assert len(row) >= 3 * rows * -(-cols // 256)
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=rows))]).astype(np.uint32)
+    idx, val = col.astype(np.uint32), rng.integers(1, 60_000, len(col)).astype(np.uint16)
+    t = transpose(to_device_csr(rows, cols, ptr, idx, val))
+    rptr, ridx, rval = orc.csr_transpose(rows, cols, ptr, idx, val)
+    assert np.array_equal(np_u32(t.ptr), rptr)
+    assert np.array_equal(np_u32(t.idx), ridx)
+    assert np.array_equal(np_u16(t.val), rval)
