@@ -65,7 +65,8 @@ struct moments_layout {
 // few SMs (8,192 x 2,000, 8 groups: 12 CTAs); every chunk costs 32 bytes of
 // partials a column, 16 / chunk_rows of the rows' own bytes.  Halved to 256
 // rows (6 %) while there are under 1,000 CTAs, and on to 64 only while there
-// are under two per SM.  us per call by 2,048 / 256 / 64 rows: 8,192 x 2,000
+// are under two per SM of this chip (written out, so that the order of the sums
+// does not depend on the device).  us per call by 2,048 / 256 / 64 rows: 8,192 x 2,000
 // (8 groups) 99 / 52 / 36; 100,000 x 5,000 (16) 344 / 177 / 217; 20,000 x 8,000
 // (64) 78 / 76 / 83; 50,000 x 32,768 (64) 479 / 489 / 572 (1,024: 480).
 uint32_t default_chunk_rows(uint32_t rows, uint32_t col_blocks, uint32_t block_size, uint32_t groups) {
@@ -799,7 +800,7 @@ int combine_groups(const moments_layout &lay, uint32_t cols, const cs_group_mome
                                                            d_feature_keep, out->sum, out->sumsq, out->mean, out->var,
                                                            out->mean64, out->var64, out->group_rows, g_lo);
     };
-    if ((uint64_t) four * (g_hi - g_lo) >= 296u) launch(moments_combine_kernel<4>, four);
+    if ((uint64_t) four * (g_hi - g_lo) >= 2u * (uint64_t) sm_count()) launch(moments_combine_kernel<4>, four);
     else launch(moments_combine_kernel<1>, one);
     return launch_ok("moments_combine_kernel");
 }
