@@ -66,17 +66,21 @@ struct moments_layout {
 // partials a column, 16 / chunk_rows of the rows' own bytes.  Halved to 256
 // rows (6 %) while there are under 1,000 CTAs, and on to 64 only while there
 // are under two per SM of this chip (written out, so that the order of the sums
-// does not depend on the device).  us per call by 2,048 / 256 / 64 rows: 8,192 x 2,000
-// (8 groups) 99 / 52 / 36; 100,000 x 5,000 (16) 344 / 177 / 217; 20,000 x 8,000
-// (64) 78 / 76 / 83; 50,000 x 32,768 (64) 479 / 489 / 572 (1,024: 480).
+// does not depend on the device).  Not past 250 chunks a group: the combine walks a
+// group's chunks one after the other, 0.125 us each where columns and groups are few
+// (600,000 x 2,000, one group: 484 us with 2,048 rows, 581 with 512).  us per call by
+// 2,048 / 256 / 64 rows: 8,192 x 2,000 (8 groups) 99 / 52 / 36; 100,000 x 5,000 (16)
+// 344 / 177 / 217; 20,000 x 8,000 (64) 78 / 76 / 83; 50,000 x 32,768 (64) 479 / 489 / 572
+// (1,024: 480).
 uint32_t default_chunk_rows(uint32_t rows, uint32_t col_blocks, uint32_t block_size, uint32_t groups) {
     const uint64_t segs = (uint64_t) col_blocks * ((block_size + 7u) / 8u);
     const uint64_t tiles = (segs + kAccThreads - 1u) / kAccThreads;
     // about half of the groups end in a chunk of their own
     auto ctas = [&](uint32_t chunk) { return (rows / chunk + groups / 2u) * tiles; };
+    auto may_halve = [&](uint32_t chunk) { return rows / groups <= 250u * (chunk / 2u); };
     uint32_t chunk = kDefaultChunkRows;
-    while (chunk > 256u && ctas(chunk) < 1000u) chunk /= 2u;
-    while (chunk > 64u && ctas(chunk) < 296u) chunk /= 2u;
+    while (chunk > 256u && ctas(chunk) < 1000u && may_halve(chunk)) chunk /= 2u;
+    while (chunk > 64u && ctas(chunk) < 296u && may_halve(chunk)) chunk /= 2u;
     return chunk;
 }
 
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(1024) moments_group_scan_kernel(uint32_t G, ui
                                                                   uint32_t *__restrict__ num_chunks,
                                                                   chunk_desc *__restrict__ chunks) {
     __shared__ uint32_t smem[33];
+    __shared__ uint32_t first[1024], begin[1024], len[1024];
     if constexpr (kTiles) {
         for (uint32_t g = threadIdx.x >> 5; g < G; g += blockDim.x >> 5)
             group_tiles(g, tiles, G, tile_counts, group_rows);
@@ -270,16 +275,33 @@ __global__ void __launch_bounds__(1024) moments_group_scan_kernel(uint32_t G, ui
         uint32_t tot_n, tot_c;
         const uint32_t ex_n = block_exclusive_scan(n, smem, tot_n);
         const uint32_t ex_c = block_exclusive_scan(nc, smem, tot_c);
+        const uint32_t off = carry_rows + ex_n, cf = carry_chunks + ex_c;
         if (g < G) {
-            const uint32_t off = carry_rows + ex_n;
-            const uint32_t cf = carry_chunks + ex_c;
             group_offsets[g] = off;
             chunk_first[g] = cf;
-            for (uint32_t c = 0; c < nc; ++c) {
-                const uint32_t b = off + c * chunk_rows;
-                const uint32_t e = (c + 1u == nc) ? off + n : b + chunk_rows;
-                if (cf + c < max_chunks) chunks[cf + c] = chunk_desc{g, b, e, 0u};
+        }
+        auto cut = [&](uint32_t id, uint32_t group, uint32_t from, uint32_t upto) {
+            if (id < max_chunks) chunks[id] = chunk_desc{group, from, min(from + chunk_rows, upto), 0u};
+        };
+        if (__syncthreads_or(nc > 8u)) { // a thread per chunk: its group is the last that starts at or before it
+            first[threadIdx.x] = ex_c;
+            begin[threadIdx.x] = off;
+            len[threadIdx.x] = n;
+            __syncthreads();
+            for (uint32_t c = threadIdx.x; c < tot_c; c += blockDim.x) {
+                uint32_t lo = 0u, hi = blockDim.x - 1u;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1u) >> 1;
+                    if (first[mid] <= c)
+                        lo = mid;
+                    else
+                        hi = mid - 1u;
+                }
+                cut(carry_chunks + c, g0 + lo, begin[lo] + (c - first[lo]) * chunk_rows, begin[lo] + len[lo]);
             }
+            __syncthreads();
+        } else {
+            for (uint32_t c = 0; c < nc; ++c) cut(cf + c, g, off + c * chunk_rows, off + n);
         }
         carry_rows += tot_n;
         carry_chunks += tot_c;
@@ -547,7 +569,8 @@ __device__ __forceinline__ double divide_by(double a, double b, double y) {
 // one or two chunks: two divisions an output, by the group's row counts, were
 // half of the instructions; four columns share the reciprocals (250 groups of
 // 20,000 columns: 58 -> 32 us).
-template <int C>
+// kLong: groups of many chunks (one column a thread).
+template <int C, bool kLong>
 __global__ void __launch_bounds__(256) moments_combine_kernel(
     uint32_t cols, uint32_t pstride, uint32_t G, uint32_t scheme, uint32_t ddof,
     const uint32_t *__restrict__ chunk_first, const uint32_t *__restrict__ group_rows,
@@ -567,6 +590,20 @@ __global__ void __launch_bounds__(256) moments_combine_kernel(
         const uint32_t f = f0 + 256u * k;
         kept[k] = f < cols && (feature_keep == nullptr || feature_keep[f] != 0u);
     }
+    // kBatch consecutive chunks' partials of the thread's column (column 0's, unused,
+    // where it has none).  A group of hundreds of chunks is a chain of their latencies:
+    // loaded without a condition in the way, a batch is one (200,000 x 2,000 in one
+    // group, 782 chunks: 98 us, 331 one by one).  Groups of few chunks go without: the
+    // registers cost them more (6,000 x 8,000, 20 groups: 58 us a call, 62 with batches;
+    // 20,000 x 33,000, 600 groups 482 and 534).
+    constexpr uint32_t kBatchChunks = 16u;
+    auto load_batch = [&](uint32_t c, float (&x)[kBatchChunks][4]) {
+        const float *p = partials + (std::size_t) c * 4u * pstride + (kept[0] ? f0 : 0u);
+#pragma unroll
+        for (uint32_t u = 0; u < kBatchChunks; ++u)
+#pragma unroll
+            for (unsigned a = 0; a < 4u; ++a) x[u][a] = __ldg(p + (u * 4u + a) * (std::size_t) pstride);
+    };
     float rs[C], rq[C], rm[C], rv[C];
     double dm[C], dv[C];
 #pragma unroll
@@ -578,8 +615,20 @@ __global__ void __launch_bounds__(256) moments_combine_kernel(
         double s[C], q[C];
 #pragma unroll
         for (int k = 0; k < C; ++k) s[k] = q[k] = 0.0;
+        uint32_t c = c0;
+        if constexpr (kLong) {
+            for (; c + kBatchChunks <= c1; c += kBatchChunks) {
+                float x[kBatchChunks][4];
+                load_batch(c, x);
+#pragma unroll
+                for (uint32_t u = 0; u < kBatchChunks; ++u) {
+                    s[0] += (double) x[u][0] + (double) x[u][1];
+                    q[0] += (double) x[u][2] + (double) x[u][3];
+                }
+            }
+        }
 #pragma unroll (8 / C)
-        for (uint32_t c = c0; c < c1; ++c) {
+        for (; c < c1; ++c) {
             const float *p = partials + (std::size_t) c * 4u * pstride + f0;
             float x[C][4];
 #pragma unroll
@@ -614,17 +663,30 @@ __global__ void __launch_bounds__(256) moments_combine_kernel(
         for (int k = 0; k < C; ++k) {
             if (!kept[k]) continue;
             float s_hi = 0.0f, s_lo = 0.0f, q_hi = 0.0f, q_lo = 0.0f;
-            for (uint32_t c = c0; c < c1; ++c) {
-                const float *p = partials + (std::size_t) c * 4u * pstride + f0 + 256u * k;
+            auto add = [&](const float (&x)[4]) {
                 if (scheme == CS_MOMENTS_TWOSUM_F32) {
-                    two_sum_acc(s_hi, s_lo, p[0]);
-                    s_lo = __fadd_rn(s_lo, p[pstride]);
-                    two_sum_acc(q_hi, q_lo, p[2u * (std::size_t) pstride]);
-                    q_lo = __fadd_rn(q_lo, p[3u * (std::size_t) pstride]);
+                    two_sum_acc(s_hi, s_lo, x[0]);
+                    s_lo = __fadd_rn(s_lo, x[1]);
+                    two_sum_acc(q_hi, q_lo, x[2]);
+                    q_lo = __fadd_rn(q_lo, x[3]);
                 } else {
-                    s_hi = __fadd_rn(s_hi, p[0]);
-                    q_hi = __fadd_rn(q_hi, p[2u * (std::size_t) pstride]);
+                    s_hi = __fadd_rn(s_hi, x[0]);
+                    q_hi = __fadd_rn(q_hi, x[2]);
                 }
+            };
+            uint32_t c = c0;
+            if constexpr (kLong) {
+                for (; c + kBatchChunks <= c1; c += kBatchChunks) {
+                    float x[kBatchChunks][4];
+                    load_batch(c, x);
+#pragma unroll
+                    for (uint32_t u = 0; u < kBatchChunks; ++u) add(x[u]);
+                }
+            }
+            for (; c < c1; ++c) {
+                const float *p = partials + (std::size_t) c * 4u * pstride + f0 + 256u * k;
+                const float x[4] = {p[0], p[pstride], p[2u * (std::size_t) pstride], p[3u * (std::size_t) pstride]};
+                add(x);
             }
             rs[k] = __fadd_rn(s_hi, s_lo);
             rq[k] = __fadd_rn(q_hi, q_lo);
@@ -800,8 +862,10 @@ int combine_groups(const moments_layout &lay, uint32_t cols, const cs_group_mome
                                                            d_feature_keep, out->sum, out->sumsq, out->mean, out->var,
                                                            out->mean64, out->var64, out->group_rows, g_lo);
     };
-    if ((uint64_t) four * (g_hi - g_lo) >= 2u * (uint64_t) sm_count()) launch(moments_combine_kernel<4>, four);
-    else launch(moments_combine_kernel<1>, one);
+    const bool many_chunks = lay.max_chunks / params->group_count > 32u;
+    if ((uint64_t) four * (g_hi - g_lo) >= 2u * (uint64_t) sm_count()) launch(moments_combine_kernel<4, false>, four);
+    else if (many_chunks) launch(moments_combine_kernel<1, true>, one);
+    else launch(moments_combine_kernel<1, false>, one);
     return launch_ok("moments_combine_kernel");
 }
 

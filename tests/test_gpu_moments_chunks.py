@@ -90,3 +90,33 @@ def test_noalloc_gives_the_same_bits(cuda, rows, cols, groups, chunk):
     assert float(got[0][0].abs().sum()) > 0
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("groups", [1, 3, 1_024, 1_025, 2_000])
+@pytest.mark.parametrize("chunk", [0, 64])
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+def test_groups_of_many_chunks(cuda, groups, chunk, scheme):
+    """Most rows in the first and the last group, groups of none between them: chunks cut by a thread
+    each, over the 1,024 groups of a pass too, and combined in batches.  Whole counts: exact sums."""
+    import torch
+
+    from cellshard_b200 import runtime
+    from cellshard_b200.device import blocked_ell_from_csr
+
+    rows, cols = 9_001, 300
+    p, idx, val = random_csr(rows, cols, 0.03, groups, 0.1)
+    bell = blocked_ell_from_csr(to_device_csr(rows, cols, p, idx, val), 8)
+    rng = np.random.default_rng(groups)
+    lab = rng.integers(0, groups, rows) // 2 * 2
+    lab[rng.random(rows) < 0.4] = 0
+    lab[rng.random(rows) < 0.4] = groups - 1
+    row = np.repeat(np.arange(rows), np.diff(p.astype(np.int64)))
+    x = val.view(np.float16).astype(np.float64)
+    got = runtime.compute_sparse_group_moments(bell, groups, None, None,
+                                               torch.from_numpy(lab.astype(np.int32)).cuda(), scheme=scheme,
+                                               chunk_rows=chunk)
+    for k, v in (("sum", x), ("sumsq", x * x)):
+        want = np.zeros((groups, cols))
+        np.add.at(want, (lab[row], idx.astype(np.int64)), v)
+        assert np.array_equal(got[k].cpu().numpy().astype(np.float64), want), k
+    assert np.array_equal(got["group_rows"].cpu().numpy(), np.bincount(lab, minlength=groups))
