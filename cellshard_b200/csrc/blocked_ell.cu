@@ -9,12 +9,14 @@
 //           blocks from the row block's contiguous CSR index range; popc gives
 //           the distinct count, atomicMax the global ell_width.  The bitmaps
 //           are kept in scratch for the emit pass.
-//   emit    one CTA per output row assembles the row's padded ELL segment in
-//           shared memory (zero, scatter, then 16-byte streaming stores), the
-//           slot of column block b being prefix(word) + popc(word & below(b)),
-//           which is exactly the rank of b in the ascending qsort order.  The
-//           first row of each row block also writes the row block's
-//           blockColIdx (set bits in ascending order, CS_INVALID_COL padding).
+//   emit    a warp per output row of up to 12 KB, a CTA per longer one, assembles
+//           the padded row in shared memory and sends it with one bulk store;
+//           rows over 64 KB or off a 16-byte boundary leave in segments by
+//           streaming stores.  The slot of column block b is
+//           prefix(word) + popc(word & below(b)), which is exactly the rank
+//           of b in the ascending qsort order.  The first row of each row
+//           block also writes the row block's blockColIdx (set bits in
+//           ascending order, CS_INVALID_COL padding).
 //
 // Values of duplicate columns inside one row resolve to the last occurrence
 // (the reference's overwrite order).  A row whose columns ascend has none (a

@@ -1,6 +1,7 @@
-// Sliced-ELL row emission of the single-partition and batched converters: row r owns the w slots [base, base + w) of its slice; its n
-// real (column, value) pairs go into the first n slots in CSR order, the rest
-// is padding (CS_INVALID_COL, 0) -- sliced_ell_from_compressed.cuh:49-80.
+// Sliced-ELL row emission of the single-partition and batched converters: row r
+// owns the w slots [base, base + w) of its slice; its n real (column, value)
+// pairs go into the first n slots in CSR order, the rest is padding
+// (CS_INVALID_COL, 0) -- sliced_ell_from_compressed.cuh:49-80.
 //
 // A group of GL lanes (GL in {32, 16, 8, 4}) writes one row.  Real slots are
 // copied lane by lane, so loads and stores are whole lines whatever the two

@@ -775,9 +775,10 @@ CS_API int cs_b200_bucketed_blocked_ell_fill(const cs_blocked_ell_view *part,
                                              cs_stream_t stream);
 
 CS_API int cs_b200_bucketed_sliced_ell_scratch_bytes(uint32_t rows, uint32_t max_segments, size_t *out_bytes);
-/* Live-slot counts and the stable sort on the device; the split (a
- * sequential dynamic programme over the sorted widths, as the reference's)
- * runs on the host over the widths copied back.  requested 0 chooses as
+/* Live-slot counts, their histogram and the stable sort on the device; the
+ * split (the reference's sequential dynamic programme) runs on the host over
+ * the distinct widths and their row counts, which give the cuts of the
+ * programme over all rows.  requested 0 chooses as
  * choose_bucket_count_for_sliced_part. */
 CS_API int cs_b200_bucketed_sliced_ell_plan(const cs_sliced_ell_view *part,
                                             uint32_t requested,
