@@ -212,3 +212,28 @@ def test_staged_group_bytes(cs_lib):
     assert cs_lib.cs_b200_device_partition_bytes_blocked_ell(C.byref(parts[0]), C.byref(one)) == 1
     assert n.value == one.value
     assert np.int64(n.value) > 0
+
+
+def test_sort_scratch_never_falls_with_the_entries(cs_lib):
+    """Scratch sized for more entries does for fewer: the two-pass sort's counts, offsets and slices,
+    across the lengths at which its slices change."""
+    import random
+
+    rng = random.Random(7)
+    n = C.c_size_t()
+
+    def transpose(rows, cols, nnz):
+        assert cs_lib.cs_b200_compressed_transpose_scratch_bytes(rows, cols, nnz, C.byref(n)) == 1
+        return n.value
+
+    def coo(rows, cols, nnz):
+        assert cs_lib.cs_b200_coo_blocked_ell_scratch_bytes(nnz, rows, cols, 16, C.byref(n)) == 1
+        return n.value
+
+    edges = [8_192 * 4_096, 8_192 * 8_192, 1_024 * 4_096, 1_024 * 8_192]
+    for size in (transpose, coo):
+        for _ in range(400):
+            rows, cols = rng.randint(1, 2_000_000), rng.randint(1, 262_144)
+            a = rng.choice(edges) + rng.randint(-20_000, 20_000) if rng.random() < 0.5 else rng.randint(0, 1 << 31)
+            b = a + rng.choice([1, 4_096, 8_192, 1 << 20, 1 << 26])
+            assert size(rows, cols, a) <= size(rows, cols, b), (size.__name__, rows, cols, a, b)
